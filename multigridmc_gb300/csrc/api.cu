@@ -8,6 +8,7 @@
 // when the noise comes from the in-kernel Philox generator.
 #include <algorithm>
 #include <array>
+#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -104,6 +105,10 @@ struct Level {
     unsigned *counter = nullptr;  // CTA counter of k_bt_solve
     int sweep_tx = 0;             // CTA width of the colour passes chosen by the autotuner (0: sweep_block())
     int sweep_threads = 0;        // and its thread count, 128 or 256 (0: RBP_THREADS)
+    // constant stencil with equal weights at +-dx, +-dy, +-dz (to rounding):
+    // wc[|dz| * 4 + |dy| * 2 + |dx|] (k_sweep_row_sym)
+    bool sym = false;
+    double wc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     void *adj[4] = {nullptr, nullptr, nullptr, nullptr};  // adjoint: x-bar, f-bar, two work vectors (T, padded)
     CUtensorMap xmap{}, fmap{};  // 3D tile maps of x and f for the residual-restriction
     bool tma = false;            // maps valid (3D, rows of a multiple of 16 bytes)
@@ -444,10 +449,96 @@ static void launch_sweep_t(Sampler &S, const Level &lv, bool forward, T *x, cons
     }
 }
 
-// 2^dim colours, one launch per colour
+// Launch of a pair of colours on whole rows: `tx` threads along x, CTAs of
+// `nt` threads (more where a row needs them).
+struct RowLaunch {
+    dim3 grid, block;
+    bool trigger;  // let the next launch start early
+};
+static RowLaunch row_launch(const Grid3 &g, int work, int nt, int pb, int pc) {
+    int tx = 8;
+    while (tx < work) tx *= 2;
+    RowLaunch r;
+    r.block = dim3(tx, std::max(1, nt / tx), 1);
+    const int nb = (g.N1 - pb + 1) / 2, nc = (g.N2 - pc + 1) / 2;
+    r.grid = dim3(1, (nb + r.block.y - 1) / r.block.y, nc);
+    r.trigger = false;
+    return r;
+}
+static i64 row_warps(const RowLaunch &r) {
+    return (i64)r.grid.y * r.grid.z * ((r.block.x * r.block.y + 31) / 32);
+}
+
+// CTAs of the pair kernels: 128 threads in FP32, 64 in FP64, where few warps
+// per CTA spread a small level over the SMs.  The next launch starts early
+// wherever it helps: always in FP32 (63^3: 7.4 -> 6.3 us per sweep, 127^3:
+// 16.7 -> 14.9), in FP64 up to four warps per SM (31^3: 9.6 -> 8.4 us, 2D
+// 31^2 3.7 -> 3.0; but 63^3 18.7 -> 23.9 and 39 x 47 x 55 15.0 -> 18.5: the
+// early CTAs take whichever SMs are free first and leave the FP64 units
+// unevenly loaded).
+static constexpr int ROW_NT32 = 128, ROW_NT64 = 64;
+
+// 2^dim colours: two per launch where a CTA can own a row, else one
 template <typename T, bool EXACT, int NOISE>
 static void launch_colour_passes(Sampler &S, const Level &lv, bool forward, T *x, const T *f, const StencilArg<T> &s,
                                  const NoiseArgs &nz) {
+    const bool pdl = S.pdl && lv.g.pdl;
+    const VarField<T> vf = var_field<T>(lv);
+    if (lv.g.N0 <= ROW_PAIR_MAX_N0) {
+        const int npair = lv.ncol / 2;
+        for (int q = 0; q < npair; ++q) {
+            const int pr = forward ? q : npair - 1 - q, pb = pr & 1, pc = pr >> 1;
+            if (lv.g.N1 <= pb || lv.g.N2 <= pc) continue;
+            if constexpr (std::is_same<T, double>::value && !EXACT) {
+                // FP64 chains (FP32 chains' set-up sweeps keep the ordered
+                // sums): symmetric stencils by classes of rows, in 3D and,
+                // for rows of up to 128 points, in 2D (383 x 239: 6.9 us per
+                // sweep against 6.2 for the pairs, 63 x 63: 3.1 against 3.9)
+                if (!S.fp32 && lv.sym && lv.var == 0 && lv.g.N0 <= (S.dim == 2 ? 128 : ROW_SYM_THREADS)) {
+                    RowLaunch r = row_launch(lv.g, lv.g.N0, ROW_NT64, pb, pc);
+                    r.trigger = row_warps(r) <= 4 * S.nsm;
+                    SymWeights w;
+                    std::copy(lv.wc, lv.wc + 8, w.wc);
+                    w.sd = s.sd;
+                    w.od = s.omega_diag;
+                    w.om1 = 1.0 - s.omega;
+                    const size_t sm = sizeof(double) * (r.block.x + 2) * r.block.y * (S.dim == 2 ? 2 : 4);
+                    if (S.dim == 2)
+                        plaunch(pdl, k_sweep_row_sym<9, NOISE>, r.grid, r.block, sm, S.stream, x, f, lv.g, w, pb, pc,
+                                forward ? 0 : 1, nz, (int)r.trigger);
+                    else
+                        plaunch(pdl, k_sweep_row_sym<27, NOISE>, r.grid, r.block, sm, S.stream, x, f, lv.g, w, pb, pc,
+                                forward ? 0 : 1, nz, (int)r.trigger);
+                    S.launches++;
+                    continue;
+                }
+            }
+            RowLaunch r = row_launch(lv.g, (lv.g.N0 + 1) / 2, sizeof(T) == 4 ? ROW_NT32 : ROW_NT64, pb, pc);
+            r.trigger = sizeof(T) == 4 || row_warps(r) <= 4 * S.nsm;
+            const size_t sm = sizeof(T) * (r.block.x + 1) * r.block.y;
+            auto go = [&](auto kernel) {
+                plaunch(pdl, kernel, r.grid, r.block, sm, S.stream, x, f, lv.g, s, pb, pc, forward ? 0 : 1, nz, vf,
+                        (int)r.trigger);
+            };
+            if (S.dim == 2) {
+                if (lv.var == 2)
+                    go(k_sweep_row_pair<T, 9, EXACT, NOISE, 2>);
+                else if (lv.var == 1)
+                    go(k_sweep_row_pair<T, 9, EXACT, NOISE, 1>);
+                else
+                    go(k_sweep_row_pair<T, 9, EXACT, NOISE, 0>);
+            } else {
+                if (lv.var == 2)
+                    go(k_sweep_row_pair<T, 27, EXACT, NOISE, 2>);
+                else if (lv.var == 1)
+                    go(k_sweep_row_pair<T, 27, EXACT, NOISE, 1>);
+                else
+                    go(k_sweep_row_pair<T, 27, EXACT, NOISE, 0>);
+            }
+            S.launches++;
+        }
+        return;
+    }
     for (int cc = 0; cc < lv.ncol; ++cc) {
         const int colour = forward ? cc : lv.ncol - 1 - cc;
         const int pa = colour & 1, pb = (colour >> 1) & 1, pc = (colour >> 2) & 1;
@@ -455,13 +546,12 @@ static void launch_colour_passes(Sampler &S, const Level &lv, bool forward, T *x
         if (na <= 0 || nb <= 0 || nc <= 0) continue;
         const dim3 blk = level_block(lv, na);
         dim3 grid((na + blk.x - 1) / blk.x, (nb + blk.y - 1) / blk.y, nc);
-        const VarField<T> vf = var_field<T>(lv);
         if (lv.var == 2)
-            plaunch(S.pdl && lv.g.pdl, k_sweep_c27_pass<T, EXACT, NOISE, 2>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, nz, vf);
+            plaunch(pdl, k_sweep_c27_pass<T, EXACT, NOISE, 2>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, nz, vf);
         else if (lv.var == 1)
-            plaunch(S.pdl && lv.g.pdl, k_sweep_c27_pass<T, EXACT, NOISE, 1>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, nz, vf);
+            plaunch(pdl, k_sweep_c27_pass<T, EXACT, NOISE, 1>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, nz, vf);
         else
-            plaunch(S.pdl && lv.g.pdl, k_sweep_c27_pass<T, EXACT, NOISE, 0>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, nz, vf);
+            plaunch(pdl, k_sweep_c27_pass<T, EXACT, NOISE, 0>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, nz, vf);
         S.launches++;
     }
 }
@@ -839,6 +929,25 @@ static int stencil_npt(int ncol, const double st[27]) {
         if ((dx != 0) + (dy != 0) + (dz != 0) > 1 && st[k] != 0.0) return 27;
     }
     return 7;
+}
+
+// Weights by class (|dz|, |dy|, |dx|): true if the weights of every class are
+// equal to rounding (the Galerkin products of a symmetric stencil differ by a
+// few ulp of the largest weight); wc holds their means.
+static bool symmetric_classes(const double st[27], double wc[8]) {
+    int cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    double big = 0.0;
+    std::fill(wc, wc + 8, 0.0);
+    auto cls = [](int k) { return (k / 9 != 1) * 4 + ((k / 3) % 3 != 1) * 2 + (k % 3 != 1); };
+    for (int k = 0; k < 27; ++k) {
+        wc[cls(k)] += st[k];
+        cnt[cls(k)]++;
+        big = std::max(big, std::fabs(st[k]));
+    }
+    for (int q = 0; q < 8; ++q) wc[q] /= cnt[q];
+    for (int k = 0; k < 27; ++k)
+        if (!(std::fabs(st[k] - wc[cls(k)]) <= 32 * DBL_EPSILON * big)) return false;
+    return true;
 }
 
 __global__ void k_scatter(const unsigned *__restrict__ idx, const double *__restrict__ val, i64 cnt, double *__restrict__ dst) {
@@ -1223,6 +1332,7 @@ void Sampler::build(const mgmc_operator_desc &op) {
         lv.sd = std::sqrt(lv.diag * (2. - P.omega) / P.omega);
         lv.ncol = colour_count(dim, st);
         lv.npt = stencil_npt(lv.ncol, st);
+        lv.sym = symmetric_classes(st, lv.wc);
         // programmatic dependent launch pays off for the short kernels of
         // the coarser levels; the many-CTA kernels of large levels run
         // without its per-CTA wait
@@ -1341,6 +1451,7 @@ void Sampler::autotune_sweeps() {
     for (int lev = 0; lev < nlev; ++lev) {
         if (lev == nlev - 1 && chol) break;
         Level &lv = L[lev];
+        if (lv.npt != 7 && lv.g.N0 <= ROW_PAIR_MAX_N0) continue;  // whole rows: no width to choose
         ensure_scratch(lev);
         const bool vec = fp32 && !exact && lv.npt == 7 && (lv.g.sy % 4) == 0 && (lv.g.sz % 4) == 0 && lv.var != 2;
         const int count = vec ? (lv.g.N0 + 8) / 8 : (lv.g.N0 + 1) / 2;
@@ -2749,6 +2860,17 @@ void BatchGroup::sor(int lev, bool forward, cudaStream_t st) {
             else
                 k_sweep_rb_vec_batch<NOISE_PHILOX, false, false><<<grid, blk, 0, st>>>(la[lev], ca, g, colour, pass,
                                                                                       inv, (unsigned)lev);
+            batch_launch_check(0);
+        }
+    } else if (g.N0 <= ROW_PAIR_MAX_N0) {
+        const int npair = lv.ncol / 2;
+        for (int q = 0; q < npair; ++q) {
+            const int pr = forward ? q : npair - 1 - q, pb = pr & 1, pc = pr >> 1;
+            if (g.N1 <= pb || g.N2 <= pc) continue;
+            const RowLaunch r = row_launch(g, (g.N0 + 1) / 2, ROW_NT32, pb, pc);
+            const dim3 grid(r.grid.x, r.grid.y, r.grid.z * G);
+            k_sweep_row_pair_batch<NOISE_PHILOX><<<grid, r.block, sizeof(float) * (r.block.x + 1) * r.block.y, st>>>(
+                la[lev], ca, g, pb, pc, forward ? 0 : 1, (int)r.grid.z, inv, (unsigned)lev);
             batch_launch_check(0);
         }
     } else {

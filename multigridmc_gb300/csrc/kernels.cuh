@@ -204,8 +204,9 @@ __device__ __forceinline__ T stencil_row_acc(const XA &xa, const StencilArg<T> &
 #pragma unroll
         for (int q = 0; q < 7; ++q) res = A::add(res, A::mul(vweight<T, VAR>(s, vf, P, ks[q]), xa(dzs[q], dys[q], dxs[q])));
     } else {
+        constexpr int ZLO = NPT == 9 ? 0 : -1, ZHI = NPT == 9 ? 0 : 1;  // a 2D level has no neighbours in z
 #pragma unroll
-        for (int dz = -1; dz <= 1; ++dz)
+        for (int dz = ZLO; dz <= ZHI; ++dz)
 #pragma unroll
             for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
@@ -545,6 +546,214 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_c27_pass(T *__restrict__ 
                                                                 VarField<T> vf) {
     if (g.pdl) pdl_begin();
     sweep_c27_body<T, EXACT, NOISE, VAR>(x, f, g, s, colour, nz, vf, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// ------------------------------------------- two colours of a row per launch
+// The colours of a 27-point (9-point in 2D) level come in pairs that share
+// the parities of b and c and differ in the parity of a.  A point of the
+// second colour of a pair has neighbours of the first one in its own row
+// only, so a CTA that owns whole rows runs both colours of the pair: the
+// rows around are read once for both, and a sweep takes half the launches.
+// The update of every point, the order of its sum included, is that of the
+// one-colour pass.
+//
+// What bounds it: on levels of up to 63^3 points the round trip of one
+// dependent launch (parameters, one L2 load, the sum, one store), above that
+// the L2 traffic.  The normals do not depend on the launch before, so they
+// are drawn before the wait for it (`wait`), and with `trigger` the next
+// launch's CTAs start, and draw theirs, while this one's loads are in flight.
+// (GB300, a whole sweep with Philox noise in a graph of dependent launches,
+// one-colour passes -> row pairs: FP32 127^3 31.5 -> 17.7 us, 63^3 15.4 ->
+// 6.8, 31^3 14.1 -> 5.9; FP64 31^3 22.3 -> 13.0, 15^3 20.8 -> 12.7.)
+//
+// Thread t of a row owns the points 2t and 2t + 1: the four positions 2t ..
+// 2t + 3 of the nine (three) rows around, two aligned pair loads each where
+// the pitches are even.  One Philox block holds the normals of four points
+// of one parity of a group of eight, so of the four threads of a group the
+// even ones draw the even points' block, the odd ones the odd points', and
+// neighbours swap.
+constexpr int ROW_PAIR_THREADS = 256;                 // most threads of a CTA
+constexpr int ROW_PAIR_MAX_N0 = 2 * ROW_PAIR_THREADS; // longest row a CTA can own
+
+template <typename T>
+struct Pair;
+template <>
+struct Pair<float> {
+    typedef float2 type;
+};
+template <>
+struct Pair<double> {
+    typedef double2 type;
+};
+
+template <typename T, int NPT, bool EXACT, int NOISE, int VAR>
+__device__ __forceinline__ void sweep_row_pair_body(T *__restrict__ x, const T *__restrict__ f, const Grid3 &g,
+                                                    const StencilArg<T> &s, int pb, int pc, int odd_first,
+                                                    const NoiseArgs &nz, const VarField<T> &vf, int by, int bz,
+                                                    T *sh, bool wait, bool trigger) {
+    constexpr int NR = NPT == 9 ? 3 : 9;  // rows of the stencil
+    const int t = threadIdx.x, a0 = 2 * t;
+    const int b = 2 * (by * blockDim.y + threadIdx.y) + pb, c = 2 * bz + pc;
+    const bool row_in = b < g.N1 && c < g.N2;
+    const bool in0 = row_in && a0 < g.N0, in1 = row_in && a0 + 1 < g.N0;
+    T xi0 = T(0), xi1 = T(0);
+    if (NOISE == NOISE_PHILOX) {  // point_normals of the two points
+        const unsigned G0 = (unsigned)((g.N0 + 7) >> 3);
+        const unsigned grp = (unsigned)(((u64)c * g.N1 + b) * G0 + (t >> 2));
+        const float4 r = normals4(philox4x32_10(noise_ctr(nz, grp, PURPOSE_POINT, t & 1), noise_key(nz)));
+        const float own = pick(r, t & 3), other = __shfl_xor_sync(0xffffffffu, pick(r, (t & 3) ^ 1), 1);
+        xi0 = (T)((t & 1) ? other : own);
+        xi1 = (T)((t & 1) ? own : other);
+    }
+    if (wait) pdl_begin();
+    if (trigger) pdl_trigger();
+    const i64 P = g.pad(a0, b, c);
+    if (NOISE == NOISE_INJECTED) {
+        if (in0) xi0 = (T)nz.buf[g.compact(a0, b, c)];
+        if (in1) xi1 = (T)nz.buf[g.compact(a0 + 1, b, c)];
+    }
+    T v[NR][4], f0 = T(0), f1 = T(0);
+    if (in0) {
+        f0 = f[P];
+        if (in1) f1 = f[P + 1];
+        const bool even = (g.sy & 1) == 0 && (g.sz & 1) == 0;  // then P - 1 is even too
+        typedef typename Pair<T>::type T2;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const T *q = x + P - 1 + (NR == 9 ? (r / 3 - 1) * g.sz : 0) + (r % 3 - 1) * g.sy;
+            if (even) {
+                const T2 u = *reinterpret_cast<const T2 *>(q), w = *reinterpret_cast<const T2 *>(q + 2);
+                v[r][0] = u.x;
+                v[r][1] = u.y;
+                v[r][2] = w.x;
+                v[r][3] = w.y;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[r][j] = j < 3 || in1 ? q[j] : T(0);
+            }
+        }
+    }
+    constexpr int OWN = NR / 2;
+    auto updated = [&](int o, T fv, T xi) {  // point 2t + o
+        return sor_value<T, NPT, EXACT, VAR>(
+            [&](int dz, int dy, int dx) { return v[(NR == 9 ? (dz + 1) * 3 : 0) + dy + 1][1 + o + dx]; }, v[OWN][1 + o],
+            fv, s, P + o, NOISE != NOISE_NONE, xi, vf);
+    };
+    // the first colour's new values reach the neighbouring threads through
+    // shared memory (one slot per thread and row, one more at the row's end)
+    T *row = sh + threadIdx.y * (blockDim.x + 1);
+    if (!odd_first) {
+        T n = T(0);
+        if (in0) x[P] = n = v[OWN][1] = updated(0, f0, xi0);
+        row[t] = n;
+        if (t == 0) row[blockDim.x] = T(0);
+        __syncthreads();
+        v[OWN][3] = row[t + 1];
+        if (in1) x[P + 1] = updated(1, f1, xi1);
+    } else {
+        T n = T(0);
+        if (in1) x[P + 1] = n = v[OWN][2] = updated(1, f1, xi1);
+        row[t + 1] = n;
+        if (t == 0) row[0] = T(0);
+        __syncthreads();
+        v[OWN][0] = row[t];
+        if (in0) x[P] = updated(0, f0, xi0);
+    }
+}
+
+template <typename T, int NPT, bool EXACT, int NOISE, int VAR>
+__global__ void __launch_bounds__(ROW_PAIR_THREADS)
+    k_sweep_row_pair(T *__restrict__ x, const T *__restrict__ f, Grid3 g, StencilArg<T> s, int pb, int pc, int odd_first,
+                     NoiseArgs nz, VarField<T> vf, int trigger) {
+    extern __shared__ __align__(16) unsigned char row_sm[];
+    sweep_row_pair_body<T, NPT, EXACT, NOISE, VAR>(x, f, g, s, pb, pc, odd_first, nz, vf, blockIdx.y, blockIdx.z,
+                                                   reinterpret_cast<T *>(row_sm), g.pdl != 0, trigger != 0);
+}
+
+// The same pair of colours for FP64 chains whose constant stencil has equal
+// weights at +-dx, +-dy, +-dz (Level::sym).  GB300 issues about two FP64
+// operations per clock per SM -- one instruction of a warp holds the FP64
+// unit of its SM partition for 64 clocks -- so the count of FP64
+// instructions is what a launch takes.  The rows around are first added by
+// class (|dy|, |dz|), each sum is shared with the two neighbours in x, and
+// the diagonal term drops out of x + (omega / d)(c - sum):
+//   x'' = (1 - omega) x + (omega / d)(sd xi + f - sum over the neighbours),
+// 21 FP64 instructions per point instead of 30 (8 instead of 30 in 2D, where
+// the one-colour pass also multiplied the zero weights of the planes above
+// and below).  One thread per point: a warp per 32 points spreads a small
+// level over more FP64 units than two points per thread do.
+// wc[|dz| * 4 + |dy| * 2 + |dx|]: the weight of a class.
+struct SymWeights {
+    double wc[8];
+    double sd, od, om1;  // noise scale, omega / d, 1 - omega
+};
+
+// a float that is zero or normal as a double, by its bits (the conversion
+// instruction would take the FP64 unit)
+__device__ __forceinline__ double widen(float v) {
+    const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu;
+    const unsigned hi = (u & 0x80000000u) | (m < 0x00800000u ? 0u : (m >> 3) + 0x38000000u);
+    return __hiloint2double((int)hi, m < 0x00800000u ? 0 : (int)(u << 29));
+}
+
+constexpr int ROW_SYM_THREADS = 512;  // most threads of a CTA, and the longest row
+
+template <int NPT, int NOISE>
+__global__ void __launch_bounds__(ROW_SYM_THREADS)
+    k_sweep_row_sym(double *__restrict__ x, const double *__restrict__ f, Grid3 g, SymWeights w, int pb, int pc,
+                    int odd_first, NoiseArgs nz, int trigger) {
+    constexpr int NC = NPT == 9 ? 1 : 3;  // classes beside the own row
+    extern __shared__ __align__(16) unsigned char row_sm[];
+    const int a = threadIdx.x;
+    const int b = 2 * (blockIdx.y * blockDim.y + threadIdx.y) + pb, c = 2 * blockIdx.z + pc;
+    const bool in = a < g.N0 && b < g.N1 && c < g.N2;
+    double xi = 0.0;
+    if (NOISE == NOISE_PHILOX) xi = widen(pick(point_normals(nz, g, a, b, c), (a & 7) >> 1));
+    if (g.pdl) pdl_begin();
+    if (trigger) pdl_trigger();
+    const i64 P = g.pad(a, b, c);
+    if (NOISE == NOISE_INJECTED && in) xi = nz.buf[g.compact(a, b, c)];
+    // position a + 1 of the class rows; positions 0 and N0 + 1 are ghosts
+    const int pitch = blockDim.x + 2;
+    double *row = reinterpret_cast<double *>(row_sm) + threadIdx.y * (NC + 1) * pitch + 1 + a;
+    double s[NC + 1], cv = 0.0;
+#pragma unroll
+    for (int k = 0; k <= NC; ++k) s[k] = 0.0;
+    if (in) {
+        const double *q = x + P;
+        s[0] = q[0];
+        s[1] = q[-g.sy] + q[g.sy];
+        if (NPT == 27) {
+            s[2] = q[-g.sz] + q[g.sz];
+            s[3] = (q[-g.sz - g.sy] + q[-g.sz + g.sy]) + (q[g.sz - g.sy] + q[g.sz + g.sy]);
+        }
+        cv = f[P];
+    }
+#pragma unroll
+    for (int k = 0; k <= NC; ++k) {
+        row[k * pitch] = s[k];
+        if (a == 0) row[k * pitch - 1] = 0.0;
+        if (a == blockDim.x - 1) row[k * pitch + 1] = 0.0;
+    }
+    __syncthreads();
+    if (NOISE != NOISE_NONE) cv = fma(w.sd, xi, cv);
+#pragma unroll
+    for (int k = 1; k <= NC; ++k) {
+        cv = fma(-w.wc[2 * k], s[k], cv);
+        cv = fma(-w.wc[2 * k + 1], row[k * pitch - 1] + row[k * pitch + 1], cv);
+    }
+    const double keep = w.om1 == 0.0 ? 0.0 : w.om1 * s[0];
+    // own row: the first colour, then the second one from its new values
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if ((a & 1) == (h ^ odd_first)) {
+            const double v = fma(w.od, fma(-w.wc[1], row[-1] + row[1], cv), keep);
+            if (h == 0) row[0] = v;
+            if (in) x[P] = v;
+            if (h == 0 && !in) row[0] = 0.0;
+        }
+        if (h == 0) __syncthreads();
+    }
 }
 
 // ------------------------------------------------ lexicographic wavefront
@@ -2394,7 +2603,23 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_vec_batch(const BatchL
                                             bz);
 }
 
-// one colour of an 8-colour level, grid.z = chains x colour planes
+// a pair of colours of an 8-colour level, grid.z = chains x planes of the pair
+template <int NOISE>
+__global__ void __launch_bounds__(ROW_PAIR_THREADS)
+    k_sweep_row_pair_batch(const BatchLevelArg *__restrict__ la, const BatchChainArg *__restrict__ ca, Grid3 g, int pb,
+                           int pc, int odd_first, int ncz, unsigned invocation, unsigned level) {
+    __shared__ StencilArg<float> ss;
+    extern __shared__ __align__(16) unsigned char row_sm[];
+    const int chain = blockIdx.z / ncz, bz = blockIdx.z - chain * ncz;
+    const BatchLevelArg &a = la[chain];
+    load_stencil_shared(ss, a.s);
+    const NoiseArgs nz = batch_noise(ca[chain], invocation, level);
+    sweep_row_pair_body<float, 27, false, NOISE, 0>(a.x, a.f, g, ss, pb, pc, odd_first, nz, VarField<float>{nullptr, 0},
+                                                    blockIdx.y, bz, reinterpret_cast<float *>(row_sm), false, false);
+}
+
+// one colour of an 8-colour level with rows too long for a CTA, grid.z =
+// chains x colour planes
 template <int NOISE>
 __global__ void __launch_bounds__(RBP_THREADS) k_sweep_c27_batch(const BatchLevelArg *__restrict__ la,
                                                                  const BatchChainArg *__restrict__ ca, Grid3 g,
