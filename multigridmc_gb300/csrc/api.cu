@@ -449,6 +449,15 @@ static void launch_sweep_t(Sampler &S, const Level &lv, bool forward, T *x, cons
     }
 }
 
+static SymWeights sym_weights(const Level &lv, const StencilArg<double> &s) {
+    SymWeights w;
+    std::copy(lv.wc, lv.wc + 8, w.wc);
+    w.sd = s.sd;
+    w.od = s.omega_diag;
+    w.om1 = 1.0 - s.omega;
+    return w;
+}
+
 // Launch of a pair of colours on whole rows: `tx` threads along x, CTAs of
 // `nt` threads (more where a row needs them).
 struct RowLaunch {
@@ -497,11 +506,7 @@ static void launch_colour_passes(Sampler &S, const Level &lv, bool forward, T *x
                 if (!S.fp32 && lv.sym && lv.var == 0 && lv.g.N0 <= (S.dim == 2 ? 128 : ROW_SYM_THREADS)) {
                     RowLaunch r = row_launch(lv.g, lv.g.N0, ROW_NT64, pb, pc);
                     r.trigger = row_warps(r) <= 4 * S.nsm;
-                    SymWeights w;
-                    std::copy(lv.wc, lv.wc + 8, w.wc);
-                    w.sd = s.sd;
-                    w.od = s.omega_diag;
-                    w.om1 = 1.0 - s.omega;
+                    const SymWeights w = sym_weights(lv, s);
                     const size_t sm = sizeof(double) * (r.block.x + 2) * r.block.y * (S.dim == 2 ? 2 : 4);
                     if (S.dim == 2)
                         plaunch(pdl, k_sweep_row_sym<9, NOISE>, r.grid, r.block, sm, S.stream, x, f, lv.g, w, pb, pc,
@@ -684,6 +689,27 @@ void Sampler::sor(int lev, bool forward, bool noisy, void *x, void *f, int nspar
     if (noisy) inv++;
 }
 
+// k_resid_restrict_sym, CTAs of 64 threads at least
+static void launch_resid_restrict_sym(Sampler &S, const Level &lv, const Level &lc, const double *x, const double *f,
+                                      double *fc, double *xc, const StencilArg<double> &s) {
+    const SymWeights w = sym_weights(lv, s);
+    const int whole = lv.g.N0 <= 256;
+    int tx = 16;
+    while (tx < lv.g.N0 && tx < 256) tx *= 2;
+    const dim3 blk(tx, std::max(1, 64 / tx), 1);
+    const int txc = whole ? lc.g.N0 : (tx - 3) / 2;
+    const dim3 grid((lc.g.N0 + txc - 1) / txc, (lc.g.N1 + blk.y - 1) / blk.y, S.dim == 3 ? lc.g.N2 : 1);
+    const size_t sm = sizeof(double) * blk.y * 2 * (tx + 4);
+    auto go = [&](auto kernel) {
+        plaunch(S.pdl && lv.g.pdl, kernel, grid, blk, sm, S.stream, x, f, fc, xc, lv.g, lc.g, w, whole);
+    };
+    if (S.dim == 3)
+        lv.npt == 7 ? go(k_resid_restrict_sym<7>) : go(k_resid_restrict_sym<27>);
+    else
+        lv.npt == 7 ? go(k_resid_restrict_sym<5>) : go(k_resid_restrict_sym<9>);
+    S.launches++;
+}
+
 template <typename T>
 static void launch_resid_restrict(Sampler &S, int lev, const void *x, const void *f, void *fc, void *xc, bool zero_stencil) {
     Level &lv = S.L[lev], &lc = S.L[lev + 1];
@@ -705,6 +731,12 @@ static void launch_resid_restrict(Sampler &S, int lev, const void *x, const void
                     lv.g, lc.g, s, S.dim, vf);
         S.launches++;
         return;
+    }
+    if constexpr (std::is_same<T, double>::value) {
+        if (lv.sym && S.dim > 1 && !zero_stencil) {
+            launch_resid_restrict_sym(S, lv, lc, (const double *)x, (const double *)f, (double *)fc, (double *)xc, s);
+            return;
+        }
     }
     if (S.dim == 3 && !zero_stencil && lv.tma && x == lv.x && f == lv.f) {
         dim3 grid((lc.g.N0 + RR_TX - 1) / RR_TX, (lc.g.N1 + RR_TY - 1) / RR_TY, (lc.g.N2 + RR_TZ - 1) / RR_TZ);

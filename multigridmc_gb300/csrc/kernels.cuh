@@ -1656,6 +1656,101 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict_tma(const __grid_
     resid_restrict_tile<T, NPT>(xs, fs, rz, fc, xc, gf, gc, s, ca0, cb0, cc0);
 }
 
+// FP64 residual-restriction of a level whose constant stencil has equal
+// weights at +-dx, +-dy, +-dz (Level::sym; NPT 27 or 7 in 3D, 9 or 5 in 2D).
+// The FP64 unit takes two operations per clock per SM (k_sweep_row_sym), so
+// the sums are arranged for few of them: with E the sum of the two
+// neighbours along a direction, A_0 is a sum of w_ijk E_x^i E_y^j E_z^k
+// (i, j, k in {0, 1}) and the restriction a product of one-dimensional ones,
+// so R A_0 is the sum of w_ijk (R E^i)_x (R E^j)_y (R E^k)_z with the
+// one-dimensional rows R = (1/2, 1, 1/2) and R E = (1/2, 1, 1, 1, 1/2)
+// about the coarse point.  Each direction is applied at the resolution that
+// the ones before it left: 5 operations for both rows per column and coarse
+// plane, 10 per coarse row, 7 per coarse point, against 27 per fine point
+// and halo point for the residuals themselves.
+//
+// Thread t of a row owns the fine column a = x0 + t of one coarse row and
+// plane (25 values of x and 9 of f in 3D, all loads in flight together); only
+// the last direction, x, goes through shared memory.  Rows that fit a CTA are
+// taken whole (x0 = 0), longer ones in windows of blockDim.x columns that
+// overlap by three.  Two coarse rows per thread, or two to eight coarse planes
+// sliding through registers, load less and were slower on every level but one
+// (31^3 fine points, 27-point: 3.9 us, 6.0 with two rows, 6.5 with two planes;
+// 127^3, 7-point: 46.8, 50.5 with both; 63^3: 11.2, 10.2 with two rows): they
+// leave fewer warps for the FP64 units.  Measured in graphs of dependent
+// launches; residuals formed point by point in shared-memory tiles
+// (k_resid_restrict_tma) took 27 us on 31^3 and 63^3, 64 us on 127^3 under
+// ncu, where this kernel takes 5.5, 13 and 50.
+template <int NPT>
+__global__ void __launch_bounds__(256)
+    k_resid_restrict_sym(const double *__restrict__ x, const double *__restrict__ f, double *__restrict__ fc,
+                         double *__restrict__ xc, Grid3 gf, Grid3 gc, SymWeights w, int whole) {
+    if (gf.pdl) pdl_begin();
+    constexpr bool D3 = NPT == 27 || NPT == 7, FULL = NPT == 27 || NPT == 9;
+    constexpr int NPX = D3 ? 5 : 1, NPF = D3 ? 3 : 1;  // planes of x and f
+    extern __shared__ __align__(16) unsigned char rr_sym_sm[];
+    const int txc = whole ? gc.N0 : ((int)blockDim.x - 3) / 2;
+    const int ca0 = blockIdx.x * txc, x0 = whole ? 0 : 2 * ca0 - 1;
+    const int a = x0 + (int)threadIdx.x;
+    const int cb = blockIdx.y * blockDim.y + threadIdx.y, cc = D3 ? blockIdx.z : 0;
+    const bool col_in = a >= 0 && a < gf.N0;
+    // G and Q: blockDim.x + 4 values each, two zeros at either end
+    const int pitch = blockDim.x + 4;
+    double *sm = reinterpret_cast<double *>(rr_sym_sm) + threadIdx.y * 2 * pitch;
+    if (threadIdx.x < 2) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            sm[q * pitch + threadIdx.x] = 0.0;
+            sm[q * pitch + blockDim.x + 2 + threadIdx.x] = 0.0;
+        }
+    }
+    auto at = [&](const double *v, int b, int c) {  // zero outside the lattice
+        return col_in && b >= 0 && b < gf.N1 && c >= 0 && c < gf.N2 ? v[gf.pad(a, b, c)] : 0.0;
+    };
+    auto r1 = [](const double *q) { return fma(0.5, q[0] + q[2], q[1]); };                  // R
+    auto re = [](const double *q) { return fma(0.5, q[0] + q[4], (q[1] + q[3]) + q[2]); };  // R E
+    double xv[5][NPX], fv[3][NPF];
+#pragma unroll
+    for (int r = 0; r < 5; ++r)
+#pragma unroll
+        for (int p = 0; p < NPX; ++p) xv[r][p] = at(x, 2 * cb - 1 + r, D3 ? 2 * cc - 1 + p : 0);
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int p = 0; p < NPF; ++p) fv[r][p] = at(f, 2 * cb + r, D3 ? 2 * cc + p : 0);
+    double z0[5], z1[5], zf[3];  // (R)_z x, (R E)_z x, (R)_z f
+#pragma unroll
+    for (int r = 0; r < 5; ++r) {
+        z0[r] = D3 ? r1(xv[r] + NPX / 2 - D3) : xv[r][0];
+        z1[r] = D3 ? re(xv[r]) : 0.0;
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) zf[r] = D3 ? r1(fv[r]) : fv[r][0];
+    const double y0z0 = r1(z0 + 1), y1z0 = re(z0);
+    double P = fma(w.wc[2], y1z0, w.wc[0] * y0z0), Q = w.wc[1] * y0z0;
+    if (FULL) Q = fma(w.wc[3], y1z0, Q);
+    if (D3) {
+        const double y0z1 = r1(z1 + 1);
+        P = fma(w.wc[4], y0z1, P);
+        if (FULL) {
+            const double y1z1 = re(z1);
+            P = fma(w.wc[6], y1z1, P);
+            Q = fma(w.wc[5], y0z1, Q);
+            Q = fma(w.wc[7], y1z1, Q);
+        }
+    }
+    sm[2 + threadIdx.x] = r1(zf) - P;
+    sm[pitch + 2 + threadIdx.x] = Q;
+    __syncthreads();
+    const int ca = ca0 + (int)threadIdx.x;
+    if ((int)threadIdx.x < txc && ca < gc.N0 && cb < gc.N1) {
+        const double *g = sm + 2 + (2 * ca + 1 - x0), *q = g + pitch;
+        const i64 Pc = gc.pad(ca, cb, cc);
+        fc[Pc] = r1(g - 1) - re(q - 2);
+        if (xc) xc[Pc] = 0.0;  // the coarse sample starts from zero
+    }
+}
+
 // dst[row] += sign * sum_e B_e y_{col_e} / Sigma_{col_e} over the rows of B
 // (row-compressed): the B Sigma^{-1} B^T x part of A x.
 template <typename T>
