@@ -97,9 +97,13 @@ struct Level {
     double *Bval = nullptr;
     RowCsr Br;          // B by rows (double values)
     CorrRows C[2];      // C = M^{-1} B, forward / backward (T values)
+    CorrJob *Cjobs[2] = {nullptr, nullptr};  // the CTAs of k_lr_correct and their columns
+    int *Ccols[2] = {nullptr, nullptr};
+    int n_Cjobs[2] = {0, 0}, Cmode[2] = {0, 0}, Cquads[2] = {1, 1};
     double *SinvT[2] = {nullptr, nullptr};  // S^{-1} transposed, per sweep direction
     float2 *SinvT_ff[2] = {nullptr, nullptr};  // the same as float-float pairs (FP32 chain)
     double *y = nullptr, *z = nullptr, *part = nullptr;
+    void *w = nullptr;  // m values: the low-rank noise of the sweep in flight
     float *zf = nullptr, *Bvalf = nullptr;
     int bt_split = 1;  // blocks per column of the B^T x reduction
     unsigned *counter = nullptr;  // CTA counter of k_bt_solve
@@ -333,16 +337,6 @@ NoiseArgs Sampler::noise_args(int lev, i64 count) {
 // memory before its predecessor has completed and flushed.  This hides the launch latency between the short
 // dependent kernels of a multigrid step.
 constexpr i64 PDL_MAX_POINTS = i64(1) << 22;
-// supports of C up to this many rows take the fused solve + correction
-#ifndef MGMC_LR_FUSE_MAX_ROWS
-#define MGMC_LR_FUSE_MAX_ROWS 200000ll
-#endif
-constexpr i64 LR_FUSE_MAX_ROWS = MGMC_LR_FUSE_MAX_ROWS;
-// CTAs per SM of the fused solve + correction (each CTA repeats the solve)
-#ifndef MGMC_LR_APPLY_CTAS_PER_SM
-#define MGMC_LR_APPLY_CTAS_PER_SM 2
-#endif
-
 template <typename... KArgs, typename... Args>
 static void plaunch(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                     Args &&...args) {
@@ -596,6 +590,11 @@ static unsigned solve_block(int) { return 256u; }
 // its dynamic shared memory: u (m) and the partial products (256)
 static size_t solve_smem(int m) { return sizeof(double) * ((size_t)m + 256); }
 
+// dynamic shared memory of k_lr_correct: u and z (m values), products and sums
+static size_t lr_correct_smem(int m) {
+    return sizeof(double) * (2 * (size_t)m + 64 * 8 + LRC_MAX_M);
+}
+
 template <typename T>
 static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, const NoiseArgs &nz) {
     LowRankArg lr;
@@ -615,48 +614,29 @@ static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, cons
     lr.counter = lv.counter;
     const CorrRows &C = lv.C[dir];
     const i64 nrows = C.n1 + C.nm;
-    const dim3 bgrid(S.m, lv.bt_split);
-    if (nrows > LR_FUSE_MAX_ROWS) {
-        // large support: partial sums with the solve in their last CTA, then
-        // the correction on the whole GPU
-        const size_t smem = solve_smem(S.m);
-        if (noise == NOISE_NONE)
-            plaunch(S.pdl, k_bt_solve<T, NOISE_NONE, true>, bgrid, 256, smem, S.stream, (const T *)x, lr, nz);
-        else if (noise == NOISE_PHILOX)
-            plaunch(S.pdl, k_bt_solve<T, NOISE_PHILOX, true>, bgrid, 256, smem, S.stream, (const T *)x, lr, nz);
-        else
-            plaunch(S.pdl, k_bt_solve<T, NOISE_INJECTED, true>, bgrid, 256, smem, S.stream, (const T *)x, lr, nz);
-        const unsigned blocks = (unsigned)std::min<i64>(nblk(nrows, 4 * 256), 8 * S.nsm);
-        if (sizeof(T) == 4)
-            plaunch(S.pdl, k_lr_scatter<T, float>, blocks, 256, 0, S.stream, x, C, (const float *)lv.zf);
-        else
-            plaunch(S.pdl, k_lr_scatter<T, double>, blocks, 256, 0, S.stream, x, C, (const double *)lv.z);
-        S.launches++;
-    } else if (nrows > 0) {
-        plaunch(S.pdl, k_bt_partial<T>, bgrid, 256, 0, S.stream, (const T *)x, lr);
-        S.launches++;
-        // solve and correction in one launch; every CTA repeats the m x m
-        // solve, so the grid stays at a few CTAs per SM
-        const unsigned blocks = (unsigned)std::min<i64>(nblk(nrows, 256), MGMC_LR_APPLY_CTAS_PER_SM * S.nsm);
-        const size_t sm = sizeof(double) * (2 * (size_t)S.m + 256);
-        if (noise == NOISE_NONE)
-            plaunch(S.pdl, k_lr_apply<T, NOISE_NONE>, blocks, 256, sm, S.stream, x, lr, lv.bt_split, nz, C);
-        else if (noise == NOISE_PHILOX)
-            plaunch(S.pdl, k_lr_apply<T, NOISE_PHILOX>, blocks, 256, sm, S.stream, x, lr, lv.bt_split, nz, C);
-        else
-            plaunch(S.pdl, k_lr_apply<T, NOISE_INJECTED>, blocks, 256, sm, S.stream, x, lr, lv.bt_split, nz, C);
-    } else {
-        plaunch(S.pdl, k_bt_partial<T>, bgrid, 256, 0, S.stream, (const T *)x, lr);
-        S.launches++;
-        const size_t smem = solve_smem(S.m);
-        if (noise == NOISE_NONE)
-            plaunch(S.pdl, k_lr_solve<T, NOISE_NONE, true>, 1, solve_block(S.m), smem, S.stream, lr, lv.bt_split, nz);
-        else if (noise == NOISE_PHILOX)
-            plaunch(S.pdl, k_lr_solve<T, NOISE_PHILOX, true>, 1, solve_block(S.m), smem, S.stream, lr, lv.bt_split, nz);
-        else
-            plaunch(S.pdl, k_lr_solve<T, NOISE_INJECTED, true>, 1, solve_block(S.m), smem, S.stream, lr, lv.bt_split, nz);
-    }
-    S.launches += 1;
+    if (nrows == 0) return;  // empty columns: nothing to correct
+    lr.w = lv.w;
+    auto gather = [&](auto kernel) {
+        plaunch(S.pdl, kernel, dim3(S.m, lv.bt_split), 256, 0, S.stream, (const T *)x, lr, nz);
+    };
+    if (noise == NOISE_NONE)
+        gather(k_bt_partial<T, NOISE_NONE>);
+    else if (noise == NOISE_PHILOX)
+        gather(k_bt_partial<T, NOISE_PHILOX>);
+    else
+        gather(k_bt_partial<T, NOISE_INJECTED>);
+    auto correct = [&](auto kernel) {
+        plaunch(S.pdl, kernel, lv.n_Cjobs[dir], 256, lr_correct_smem(S.m), S.stream, x, lr, lv.bt_split, C,
+                (const CorrJob *)lv.Cjobs[dir], (const int *)lv.Ccols[dir]);
+    };
+    const int nq = lv.Cquads[dir];
+    if (lv.Cmode[dir] == 0)
+        nq == 1 ? correct(k_lr_correct<T, 0, 1>) : nq == 2 ? correct(k_lr_correct<T, 0, 2>) : correct(k_lr_correct<T, 0, 3>);
+    else if (lv.Cmode[dir] == 1)
+        nq == 1 ? correct(k_lr_correct<T, 1, 1>) : nq == 2 ? correct(k_lr_correct<T, 1, 2>) : correct(k_lr_correct<T, 1, 3>);
+    else
+        nq == 1 ? correct(k_lr_correct<T, 2, 1>) : nq == 2 ? correct(k_lr_correct<T, 2, 2>) : correct(k_lr_correct<T, 2, 3>);
+    S.launches += 2;
 }
 
 // SORSampler::apply (sor_sampler.cc:37-59) / SORSmoother::apply
@@ -795,6 +775,25 @@ static void launch_add_Bq(Sampler &S, Level &lv, void *dst, const double *y, dou
     S.launches++;
 }
 
+// dst -= B_c Sigma^{-1} B^T x: x on level lv, dst and B_c on the next one
+template <typename T>
+static void launch_resid_lowrank(Sampler &S, Level &lv, Level &lc, const void *x, void *dst) {
+    const RowCsr &B = lc.Br;
+    if (B.nrows == 0) return;
+    LowRankArg lr{};
+    lr.m = S.m;
+    lr.Bptr = lv.Bptr;
+    lr.Bidx = lv.Bidx;
+    lr.Bval = lv.Bval;
+    lr.Bvalf = lv.Bvalf;
+    lr.part = lv.part;
+    plaunch(S.pdl, k_bt_partial<T, NOISE_NONE>, dim3(S.m, lv.bt_split), 256, 0, S.stream, (const T *)x, lr, NoiseArgs{});
+    plaunch(S.pdl, k_resid_Bq<T>, nblk(B.nrows, 256), 256, sizeof(double) * S.m, S.stream, (T *)dst, B.nrows,
+            (const i64 *)B.rows, (const i64 *)B.ptr, (const int *)B.col, (const double *)B.val, (const double *)lv.part,
+            S.m, lv.bt_split, (const double *)S.d_sigma_inv);
+    S.launches += 2;
+}
+
 // residual f - A x of multigridmc_sampler.cc:124-125 restricted to the
 // next level (:126): R (f - A_0 x) - B_c Sigma^{-1} B^T x.
 void Sampler::resid_restrict(int lev) {
@@ -802,16 +801,10 @@ void Sampler::resid_restrict(int lev) {
     if (taping) tape.push_back(TapeEvent{EV_RESID, lev, true, tape_state(lev), nullptr, nullptr, NoiseArgs{}, NoiseArgs{}});
     if (fp32) {
         launch_resid_restrict<float>(*this, lev, lv.x, lv.f, lc.f, lc.x, false);
-        if (m > 0) {
-            launch_bt_plain<float>(*this, lv, lv.x);
-            launch_add_Bq<float>(*this, lc, lc.f, lv.y, -1.0);
-        }
+        if (m > 0) launch_resid_lowrank<float>(*this, lv, lc, lv.x, lc.f);
     } else {
         launch_resid_restrict<double>(*this, lev, lv.x, lv.f, lc.f, lc.x, false);
-        if (m > 0) {
-            launch_bt_plain<double>(*this, lv, lv.x);
-            launch_add_Bq<double>(*this, lc, lc.f, lv.y, -1.0);
-        }
+        if (m > 0) launch_resid_lowrank<double>(*this, lv, lc, lv.x, lc.f);
     }
     if (taping) {
         tape_last[lev + 1] = nullptr;  // the coarse state starts from zero
@@ -1046,6 +1039,7 @@ void Sampler::build_lowrank(int lev) {
     lv.y = alloc<double>(m);
     lv.z = alloc<double>(m);
     lv.zf = alloc<float>(m);
+    lv.w = alloc<double>(m);
     {
         i64 maxcol = 1;
         for (int j = 0; j < m; ++j) maxcol = std::max<i64>(maxcol, lv.Bh.ptr[j + 1] - lv.Bh.ptr[j]);
@@ -1092,7 +1086,7 @@ void Sampler::build_lowrank(int lev) {
             lr.Bvalf = lv.Bvalf;
             lr.y = lv.y;
             lr.part = lv.part;
-            k_bt_partial<double><<<dim3(m, lv.bt_split), 256, 0, stream>>>(xs, lr);
+            k_bt_partial<double, NOISE_NONE><<<dim3(m, lv.bt_split), 256, 0, stream>>>(xs, lr, nz);
             k_lr_solve<double, NOISE_NONE, false><<<1, solve_block(m), 0, stream>>>(lr, lv.bt_split, nz);
             CK(cudaMemcpyAsync(yh.data(), lv.y, m * sizeof(double), cudaMemcpyDeviceToHost, stream));
             CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), stream));
@@ -1133,6 +1127,85 @@ void Sampler::build_lowrank(int lev) {
                 pm.push_back((int)cm.size());
             }
             e = e1;
+        }
+        // both kinds of rows by column, then row, and the runs of them that
+        // the CTAs of k_lr_correct take: up to 256 multi-entry rows, or 512 to
+        // 3072 single-entry rows, the fewest that leave at most two CTAs per
+        // SM (gather and correction of 768,000 rows, FP32: 18.0, 12.0, 10.5,
+        // 7.8 us with 512, 1024, 2048, 3072 rows per CTA; of 70,000 rows
+        // 4.6, 4.4, 4.5, 4.6).  Where most rows have one entry (and none has
+        // too many), a run has at most LRC_MAX_COLS columns and its CTA forms
+        // those z only (mode 0: 256,000 rows 4.8 us, all of z in every CTA
+        // 6.0)
+        {
+            std::vector<size_t> ord(r1.size());
+            for (size_t k = 0; k < ord.size(); ++k) ord[k] = k;
+            std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return c1[a] < c1[b]; });
+            auto permute = [&](auto &v) {
+                auto w = v;
+                for (size_t k = 0; k < ord.size(); ++k) w[k] = v[ord[k]];
+                v.swap(w);
+            };
+            permute(r1);
+            permute(c1);
+            permute(v1);
+            const size_t nm = rm.size();
+            ord.resize(nm);
+            for (size_t k = 0; k < nm; ++k) ord[k] = k;
+            std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) {
+                return std::lexicographical_compare(cm.begin() + pm[a], cm.begin() + pm[a + 1], cm.begin() + pm[b],
+                                                    cm.begin() + pm[b + 1]);
+            });
+            std::vector<unsigned> rs;
+            std::vector<int> ps{0}, cs;
+            std::vector<double> vs;
+            for (size_t k : ord) {
+                rs.push_back(rm[k]);
+                cs.insert(cs.end(), cm.begin() + pm[k], cm.begin() + pm[k + 1]);
+                vs.insert(vs.end(), vm.begin() + pm[k], vm.begin() + pm[k + 1]);
+                ps.push_back((int)cs.size());
+            }
+            rm.swap(rs);
+            pm.swap(ps);
+            cm.swap(cs);
+            vm.swap(vs);
+            if (r1.size() > (size_t)INT32_MAX || cm.size() > (size_t)INT32_MAX)
+                fail(MGMC_ERR_UNSUPPORTED, "more than 2^31 support rows of C on a level");
+            std::vector<CorrJob> jobs;
+            std::vector<int> jcols;
+            int widest = 1;
+            for (size_t k = 0; k < nm; ++k) widest = std::max(widest, pm[k + 1] - pm[k]);
+            const int mode = m > LRC_MAX_M ? 2 : r1.size() >= 2 * nm && widest <= LRC_MAX_COLS ? 0 : 1;
+            const int max_cols = mode == 0 ? LRC_MAX_COLS : m;
+            lv.Cmode[dir] = mode;
+            int rows1 = 512;
+            while (rows1 < 3072 && (i64)rows1 * 2 * nsm < (i64)r1.size()) rows1 = rows1 < 1024 ? 1024 : rows1 + 1024;
+            lv.Cquads[dir] = (rows1 + 1023) / 1024;
+            std::vector<int> mark(m, -1);
+            auto add_jobs = [&](int multi, int n, int most, auto first, auto last) {  // entries first(r) .. last(r) of row r
+                for (int r = 0; r < n;) {
+                    CorrJob jb{r, r, multi, (int)jcols.size(), 0};
+                    while (r < n && r - jb.r0 < most) {
+                        int fresh = 0;
+                        for (const int *c = first(r); c != last(r); ++c) fresh += mark[*c] != (int)jobs.size();
+                        if (jb.nc + fresh > max_cols) break;
+                        for (const int *c = first(r); c != last(r); ++c)
+                            if (mark[*c] != (int)jobs.size()) {
+                                mark[*c] = (int)jobs.size();
+                                jcols.push_back(*c);
+                                jb.nc++;
+                            }
+                        ++r;
+                    }
+                    jb.r1 = r;
+                    jobs.push_back(jb);
+                }
+            };
+            add_jobs(0, (int)r1.size(), rows1, [&](int r) { return c1.data() + r; }, [&](int r) { return c1.data() + r + 1; });
+            add_jobs(1, (int)nm, 256, [&](int r) { return cm.data() + pm[r]; }, [&](int r) { return cm.data() + pm[r + 1]; });
+            lv.Cjobs[dir] = upload(jobs);
+            lv.Ccols[dir] = upload(jcols);
+            lv.n_Cjobs[dir] = (int)jobs.size();
         }
         CorrRows &C = lv.C[dir];
         C.n1 = (i64)r1.size();
@@ -1408,14 +1481,13 @@ void Sampler::build(const mgmc_operator_desc &op) {
         d_sigma_inv = upload(si);
         d_sigma_sqrt = upload(ss);
         d_sigma_sqrt_ff = upload(float_float(ss));
-        const size_t lr_smem = sizeof(double) * (2 * (size_t)m + 256);
-        if (lr_smem > 48 * 1024) {
-            raise_smem_limit(k_lr_apply<float, NOISE_NONE>, lr_smem);
-            raise_smem_limit(k_lr_apply<float, NOISE_PHILOX>, lr_smem);
-            raise_smem_limit(k_lr_apply<float, NOISE_INJECTED>, lr_smem);
-            raise_smem_limit(k_lr_apply<double, NOISE_NONE>, lr_smem);
-            raise_smem_limit(k_lr_apply<double, NOISE_PHILOX>, lr_smem);
-            raise_smem_limit(k_lr_apply<double, NOISE_INJECTED>, lr_smem);
+        if (lr_correct_smem(m) > 48 * 1024) {
+            raise_smem_limit(k_lr_correct<float, 2, 1>, lr_correct_smem(m));
+            raise_smem_limit(k_lr_correct<float, 2, 2>, lr_correct_smem(m));
+            raise_smem_limit(k_lr_correct<float, 2, 3>, lr_correct_smem(m));
+            raise_smem_limit(k_lr_correct<double, 2, 1>, lr_correct_smem(m));
+            raise_smem_limit(k_lr_correct<double, 2, 2>, lr_correct_smem(m));
+            raise_smem_limit(k_lr_correct<double, 2, 3>, lr_correct_smem(m));
         }
         for (size_t lev = 0; lev < L.size(); ++lev) build_lowrank((int)lev);
     }

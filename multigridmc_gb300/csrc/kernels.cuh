@@ -9,17 +9,19 @@
 //   k_sweep_rb_vec      one colour of the red-black SOR sweep of the 7-point
 //                       level, FP32, 8-point spans with float4 loads/stores
 //   k_sweep_rb_pass     the same, one point per thread (FP64, parity)
-//   k_sweep_c27_pass    one colour of the 8-colour SOR sweep of a 27-point level
+//   k_sweep_row_pair    two colours of the 8-colour (2D: 4-colour) SOR sweep of
+//                       a 27-point (9-point) level; k_sweep_row_sym: the same
+//                       for FP64 chains' symmetric stencils
+//   k_sweep_c27_pass    one colour of it, for rows too long for a CTA
 //   k_sweep_wavefront   lexicographic SOR sweep as a hyperplane wavefront
 //                       (one CTA; parity mode)
-//   k_bt_partial        partial sums of y = B^T x
-//   k_bt_solve          the partial sums and, in the last CTA, the solve
-//   k_lr_solve          y and the m x m low-rank solve
-//   k_lr_apply          the solve and x += C z over the rows of C = M^{-1} B
-//   k_lr_scatter        x += C z (large supports, after k_bt_solve)
+//   k_bt_partial        partial sums of y = B^T x, the low-rank noise
+//   k_lr_correct        the m x m solve and x += C z over the rows of C = M^{-1} B
+//   k_bt_solve          y = B^T x in one launch (k_lr_solve: from partial sums)
 //   k_resid_restrict_tma    f_c = R (f - A_0 x), TMA tiles (fused residual
 //                           + restriction; _tiled / plain variants otherwise)
-//   k_add_Bq            f_c -= B_c Sigma^{-1} y
+//   k_resid_restrict_sym    the same for FP64 chains' symmetric stencils
+//   k_resid_Bq          f_c -= B_c Sigma^{-1} y (k_add_Bq: elsewhere)
 //   k_prolong_add       x += alpha P x_c
 //   k_chol_gemv_*       coarse-level Cholesky sample (k_chol_subst: parity)
 //   k_step_end          observables z = b^T x, step counter
@@ -161,6 +163,14 @@ __device__ __forceinline__ float4 point_normals(const NoiseArgs &nz, const Grid3
     unsigned G0 = (unsigned)((g.N0 + 7) >> 3);
     unsigned grp = (unsigned)(((u64)c * g.N1 + b) * G0 + (a >> 3));
     return normals4(philox4x32_10(noise_ctr(nz, grp, PURPOSE_POINT, a & 1), noise_key(nz)));
+}
+
+// a float that is zero or normal as a double, by its bits (the conversion
+// instruction would take the FP64 unit)
+__device__ __forceinline__ double widen(float v) {
+    const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu;
+    const unsigned hi = (u & 0x80000000u) | (m < 0x00800000u ? 0u : (m >> 3) + 0x38000000u);
+    return __hiloint2double((int)hi, m < 0x00800000u ? 0 : (int)(u << 29));
 }
 
 // ------------------------------------------------------- exact arithmetic
@@ -566,6 +576,10 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_c27_pass(T *__restrict__ 
 // one-colour passes -> row pairs: FP32 127^3 31.5 -> 17.7 us, 63^3 15.4 ->
 // 6.8, 31^3 14.1 -> 5.9; FP64 31^3 22.3 -> 13.0, 15^3 20.8 -> 12.7.)
 //
+// x and f carry no __restrict__ here and in the kernels below that wait for
+// the launch before: loads of memory promised to be read-only may move above
+// the wait.
+//
 // Thread t of a row owns the points 2t and 2t + 1: the four positions 2t ..
 // 2t + 3 of the nine (three) rows around, two aligned pair loads each where
 // the pitches are even.  One Philox block holds the normals of four points
@@ -587,7 +601,7 @@ struct Pair<double> {
 };
 
 template <typename T, int NPT, bool EXACT, int NOISE, int VAR>
-__device__ __forceinline__ void sweep_row_pair_body(T *__restrict__ x, const T *__restrict__ f, const Grid3 &g,
+__device__ __forceinline__ void sweep_row_pair_body(T *x, const T *f, const Grid3 &g,
                                                     const StencilArg<T> &s, int pb, int pc, int odd_first,
                                                     const NoiseArgs &nz, const VarField<T> &vf, int by, int bz,
                                                     T *sh, bool wait, bool trigger) {
@@ -663,7 +677,7 @@ __device__ __forceinline__ void sweep_row_pair_body(T *__restrict__ x, const T *
 
 template <typename T, int NPT, bool EXACT, int NOISE, int VAR>
 __global__ void __launch_bounds__(ROW_PAIR_THREADS)
-    k_sweep_row_pair(T *__restrict__ x, const T *__restrict__ f, Grid3 g, StencilArg<T> s, int pb, int pc, int odd_first,
+    k_sweep_row_pair(T *x, const T *f, Grid3 g, StencilArg<T> s, int pb, int pc, int odd_first,
                      NoiseArgs nz, VarField<T> vf, int trigger) {
     extern __shared__ __align__(16) unsigned char row_sm[];
     sweep_row_pair_body<T, NPT, EXACT, NOISE, VAR>(x, f, g, s, pb, pc, odd_first, nz, vf, blockIdx.y, blockIdx.z,
@@ -688,19 +702,11 @@ struct SymWeights {
     double sd, od, om1;  // noise scale, omega / d, 1 - omega
 };
 
-// a float that is zero or normal as a double, by its bits (the conversion
-// instruction would take the FP64 unit)
-__device__ __forceinline__ double widen(float v) {
-    const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu;
-    const unsigned hi = (u & 0x80000000u) | (m < 0x00800000u ? 0u : (m >> 3) + 0x38000000u);
-    return __hiloint2double((int)hi, m < 0x00800000u ? 0 : (int)(u << 29));
-}
-
 constexpr int ROW_SYM_THREADS = 512;  // most threads of a CTA, and the longest row
 
 template <int NPT, int NOISE>
 __global__ void __launch_bounds__(ROW_SYM_THREADS)
-    k_sweep_row_sym(double *__restrict__ x, const double *__restrict__ f, Grid3 g, SymWeights w, int pb, int pc,
+    k_sweep_row_sym(double *x, const double *f, Grid3 g, SymWeights w, int pb, int pc,
                     int odd_first, NoiseArgs nz, int trigger) {
     constexpr int NC = NPT == 9 ? 1 : 3;  // classes beside the own row
     extern __shared__ __align__(16) unsigned char row_sm[];
@@ -791,12 +797,12 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     if (l == 0) sh[w] = v;
     __syncthreads();
     v = (threadIdx.x < NT / 32) ? sh[threadIdx.x] : 0.0;
-    if (w == 0) {
+    if (w == 0) {  // the sum of NT / 32 values, in lane 0
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        for (int o = NT / 64; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     }
     __syncthreads();
-    return v;  // valid in warp 0
+    return v;  // valid in thread 0
 }
 
 // ------------------------------------------------ float-float arithmetic
@@ -844,7 +850,7 @@ __device__ __forceinline__ ff32 ff_of(float2 v) { return {v.x, v.y}; }
 __device__ __forceinline__ double ff_to_double(ff32 a) { return (double)a.hi + (double)a.lo; }
 __device__ __forceinline__ float ff_to_float(ff32 a) { return __fadd_rn(a.hi, a.lo); }
 
-// block_sum's shuffle tree in float-float; the result is valid in warp 0
+// block_sum's shuffle tree in float-float; the result is valid in thread 0
 template <int NT>
 __device__ __forceinline__ ff32 block_sum_ff(ff32 v, float2 *sh) {
 #pragma unroll
@@ -856,7 +862,7 @@ __device__ __forceinline__ ff32 block_sum_ff(ff32 v, float2 *sh) {
     v = (threadIdx.x < NT / 32) ? ff_of(sh[threadIdx.x]) : ff32{0.f, 0.f};
     if (w == 0) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = NT / 64; o > 0; o >>= 1)
             v = ff_add(v, ff32{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
     }
     __syncthreads();
@@ -878,6 +884,7 @@ struct LowRankArg {
     double *part;       // m x P scratch: partial sums of B^T x (the FP32 chain
                         // stores float-float pairs, float2, in the same slots)
     unsigned *counter;  // CTA counter of k_bt_solve (reset by its last CTA)
+    void *w;                     // m scratch: Sigma^{1/2} xi' (double, or float2 for the FP32 chain)
     const float2 *SinvT_ff;      // SinvT as float-float pairs (FP32 chain)
     const float2 *sigma_sqrt_ff; // Sigma^{1/2} as float-float pairs (FP32 chain)
 };
@@ -891,10 +898,10 @@ struct LowRankArg {
 // thread's first index/value loads are issued before the wait for the
 // kernel that wrote x (`wait`: the caller has not waited yet).
 template <typename T>
-__device__ __forceinline__ void bt_partial_cta(const T *__restrict__ x, const LowRankArg &lr, double *sh, int j, int p,
-                                               int P, bool wait = false) {
+__device__ __forceinline__ void bt_partial_cta(const T *x, const LowRankArg &lr, double *sh, int j, int p, int P,
+                                               bool wait = false) {
     const i64 e0 = lr.Bptr[j], e1 = lr.Bptr[j + 1];
-    const i64 len = (e1 - e0 + P - 1) / P;
+    const i64 len = P == 1 ? e1 - e0 : (e1 - e0 + P - 1) / P;
     const i64 lo = e0 + p * len, hi = min(e1, lo + len);
     T tacc = T(0);
     i64 idx[8];
@@ -909,7 +916,10 @@ __device__ __forceinline__ void bt_partial_cta(const T *__restrict__ x, const Lo
     };
     i64 e = lo + threadIdx.x;
     load(e);
-    if (wait) pdl_begin();
+    if (wait) {
+        pdl_begin();
+        pdl_trigger();  // the correction's rows, S^{-1} and normals load meanwhile
+    }
     // eight index/value loads, then the eight gathers, in flight at once;
     // the products are added in entry order
     for (; e < hi; e += 8 * 256) {
@@ -930,10 +940,25 @@ __device__ __forceinline__ void bt_partial_cta(const T *__restrict__ x, const Lo
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_bt_partial(const T *__restrict__ x, LowRankArg lr) {
+// Also the low-rank noise Sigma^{1/2} xi' of the column (lr.w, unless null),
+// drawn before the wait by a thread that has little else to do.
+template <typename T, int NOISE>
+__global__ void __launch_bounds__(256) k_bt_partial(const T *x, LowRankArg lr, NoiseArgs nz) {
     __shared__ double sh[32];
-    bt_partial_cta<T>(x, lr, sh, blockIdx.x, blockIdx.y, gridDim.y, true);
+    const int j = blockIdx.x;
+    const bool draws = lr.w && blockIdx.y == 0 && threadIdx.x == 255;
+    float xif = 0.f;
+    if (draws && NOISE == NOISE_PHILOX)
+        xif = pick(normals4(philox4x32_10(noise_ctr(nz, (unsigned)(j >> 2), PURPOSE_LOWRANK, 0), noise_key(nz))), j & 3);
+    bt_partial_cta<T>(x, lr, sh, j, blockIdx.y, gridDim.y, true);
+    if (draws) {
+        if constexpr (sizeof(T) == 4) {
+            const ff32 w = ff_mul(ff_of(lr.sigma_sqrt_ff[j]), ff32{NOISE == NOISE_INJECTED ? (float)nz.buf[j] : xif, 0.f});
+            static_cast<float2 *>(lr.w)[j] = make_float2(w.hi, w.lo);
+        } else {
+            static_cast<double *>(lr.w)[j] = lr.sigma_sqrt[j] * (NOISE == NOISE_INJECTED ? nz.buf[j] : widen(xif));
+        }
+    }
 }
 
 // One CTA: y_k = sum_p part[k * P + p] (fixed order, so the result does not
@@ -1244,39 +1269,41 @@ __device__ __forceinline__ void corr_multi_row(T *__restrict__ x, const CorrRows
     x[row] = x[row] + acc;
 }
 
-// Four single-entry rows of a thread, r0 + j stride (j < 4): row index,
+// Four single-entry rows of a thread, r0 + j stride (j < 4) below r1: row index,
 // column, value and state loaded together; the update is the multi-entry
 // arithmetic with one product.  The state of rows loaded before the wait
-// for the previous kernel is read through L2 (see k_lr_scatter).
+// for the previous kernel is read through L2 (see k_lr_correct).
 template <typename T>
 struct CorrQuad {
     unsigned row[4];
     int col[4];
     T val[4], xv[4];
-    __device__ __forceinline__ void load(const T *__restrict__ x, const CorrRows &C, i64 r0, i64 stride,
-                                         bool before_wait) {
+    __device__ __forceinline__ void load(const T *x, const CorrRows &C, int r0, int stride, int r1, bool before_wait) {
         const T *v1 = static_cast<const T *>(C.v1);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const i64 r = r0 + j * stride;
-            const bool ok = r < C.n1;
+            const int r = r0 + j * stride;
+            const bool ok = r < r1;
             row[j] = ok ? C.r1[r] : 0u;
             col[j] = ok ? C.c1[r] : 0;
             val[j] = ok ? v1[r] : T(0);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            xv[j] = r0 + j * stride < C.n1 ? (before_wait ? __ldcg(x + row[j]) : x[row[j]]) : T(0);
+            xv[j] = r0 + j * stride < r1 ? (before_wait ? __ldcg(x + row[j]) : x[row[j]]) : T(0);
     }
     template <typename ZT>
-    __device__ __forceinline__ void apply(T *__restrict__ x, const CorrRows &C, i64 r0, i64 stride,
-                                          const ZT *z) const {
+    __device__ __forceinline__ void apply(T *x, int r0, int stride, int r1, const ZT *z) const {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (r0 + j * stride >= C.n1) continue;
-            T acc = T(0);
-            acc += val[j] * (T)z[col[j]];
-            x[row[j]] = xv[j] + acc;
+            if (r0 + j * stride >= r1) continue;
+            if (sizeof(T) == 4) {
+                T acc = T(0);
+                acc += val[j] * (T)z[col[j]];
+                x[row[j]] = xv[j] + acc;
+            } else {  // one FP64 instruction instead of two
+                x[row[j]] = fma(val[j], (T)z[col[j]], xv[j]);
+            }
         }
     }
 };
@@ -1290,7 +1317,7 @@ struct CorrMulti {
     unsigned row;
     int e0, e1, col0, col1;
     T val0, val1, xv;
-    __device__ __forceinline__ void load(const T *__restrict__ x, const CorrRows &C, i64 r, bool before_wait) {
+    __device__ __forceinline__ void load(const T *x, const CorrRows &C, i64 r, bool before_wait) {
         const T *vm = static_cast<const T *>(C.vm);
         row = C.rm[r];
         e0 = C.pm[r];
@@ -1302,7 +1329,7 @@ struct CorrMulti {
         xv = before_wait ? __ldcg(x + row) : x[row];
     }
     template <typename ZT>
-    __device__ __forceinline__ void apply(T *__restrict__ x, const CorrRows &C, const ZT *z) const {
+    __device__ __forceinline__ void apply(T *x, const CorrRows &C, const ZT *z) const {
         const T *vm = static_cast<const T *>(C.vm);
         T acc = T(0);
         acc += val0 * (T)z[col0];
@@ -1312,63 +1339,257 @@ struct CorrMulti {
     }
 };
 
-// Low-rank solve and correction in one launch: every CTA forms z itself
-// (the same arithmetic in the same order in every CTA, so all agree) and
-// adds C z on its share of the support rows of C = M^{-1} B, four rows per
-// thread and iteration with their loads issued together.  A thread's first
-// four rows do not depend on the partial sums the kernel before writes, so
-// they are loaded before the wait.
-template <typename T, int NOISE>
-__global__ void __launch_bounds__(256) k_lr_apply(T *__restrict__ x, LowRankArg lr, int P, NoiseArgs nz, CorrRows C) {
-    const i64 stride = (i64)gridDim.x * blockDim.x;
-    const i64 t0 = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    CorrQuad<T> q;
-    CorrMulti<T> mr;
-    if (t0 < C.n1) q.load(x, C, t0, stride, true);
-    if (t0 < C.nm) mr.load(x, C, t0, true);
-    pdl_begin();
+// Low-rank solve and correction in one launch, x += C z with
+// z = S^{-1}(Sigma^{1/2} xi' - y).  A CTA takes a run of rows of C (single- or
+// multi-entry ones, both sorted by column).  MODE 0, up to LRC_MAX_M columns
+// and mostly single-entry rows: it forms the z of the columns of its own rows
+// only, their products one per thread.  MODE 1, the same where columns overlap
+// throughout (coarse levels): all of z, S^{-1} loaded before the wait.  MODE 2:
+// all of z of more columns.  The FP32 chain forms every z_k in the same order wherever it
+// is formed (lr_solve_cta_ff's: 256 / m groups of terms per column, two
+// alternating sums in a group), so all CTAs and the batched kernels agree bit
+// for bit.
+//
+// What bounds it is the chain of dependent loads and sums behind the launch
+// that gathered x, so everything that does not depend on it -- the rows of C
+// with the state they correct, S^{-1} -- is loaded before the wait, while
+// k_bt_partial gathers (it lets this kernel start once the sweep has
+// completed, so the state is final; it is read through L2, the level at which
+// the sweep's writes are visible), and few registers keep all CTAs of a large
+// support resident.  (Gather and correction behind a short launch, the
+// kernels before -> these: FP64 m = 32, 8,000 rows 7.5 -> 4.5 us, 54,000 rows
+// 9.4 -> 6.0; FP32 m = 64, 19,000 rows 7.1 -> 4.4, 256,000 rows 9.6 -> 6.5.)
+constexpr int LRC_MAX_M = 64, LRC_MAX_COLS = 16;  // columns of S^{-1}, and of a CTA's rows, in mode 0
+
+struct CorrJob {
+    int r0, r1;      // rows
+    int multi;       // of the multi-entry rows
+    int c0, nc;      // their columns: cols[c0 .. c0 + nc)
+};
+
+template <typename T, int MODE, int NQ>
+__global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
+    k_lr_correct(T *x, LowRankArg lr, int P, CorrRows C, const CorrJob *__restrict__ jobs, const int *__restrict__ jobcols) {
+    typedef typename std::conditional<sizeof(T) == 4, float2, double>::type V;  // FP32 chain: float-float
     extern __shared__ double dyn[];
-    const int m = lr.m;
-    lr_solve_chain<T, NOISE, true>(lr, P, nz, dyn + m, dyn + 2 * m, dyn, blockIdx.x == 0);
-    // z (m values of type T at the start of dyn) is complete after the last
-    // __syncthreads of the solve
-    const T *zs = reinterpret_cast<const T *>(dyn);
-    for (i64 r0 = t0; r0 < C.n1; r0 += 4 * stride) {
-        q.apply(x, C, r0, stride, zs);
-        if (r0 + 4 * stride < C.n1) q.load(x, C, r0 + 4 * stride, stride, false);
+    const int m = lr.m, tid = threadIdx.x;
+    const CorrJob jb = jobs[blockIdx.x];
+    V *u = reinterpret_cast<V *>(dyn), *pr = u + m;
+    T *zs = reinterpret_cast<T *>(pr + (MODE ? 256 : 64 * 8));
+    const V *Sinv;
+    if constexpr (sizeof(T) == 4)
+        Sinv = lr.SinvT_ff;
+    else
+        Sinv = lr.SinvT;
+    const int row = jb.r0 + tid;
+    CorrQuad<T> q[NQ];
+    CorrMulti<T> mr;
+    if (jb.multi) {
+        if (row < jb.r1) mr.load(x, C, row, true);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NQ; ++i)
+            if (row + 1024 * i < jb.r1) q[i].load(x, C, row + 1024 * i, 256, jb.r1, true);
     }
-    for (i64 r = t0; r < C.nm; r += stride) {
-        if (r != t0) mr.load(x, C, r, false);
-        mr.apply(x, C, zs);
+    // terms of a column in groups g = 0 .. tpr - 1: columns g, g + tpr, ... of S^{-1}
+    const int cols = m < 256 ? m : 256, tpr = 256 / cols, groups = min(tpr, m);
+    const int g = MODE ? tid / cols : 0, kk = tid - g * cols, cnt = g < groups ? (m - g + tpr - 1) / tpr : 0;
+    const int warp = tid >> 5, lane = tid & 31;
+    V pv[MODE == 1 ? 16 : 4];
+    int kcol[2] = {0, 0};
+    if (MODE == 0) {  // warp w takes the columns w and w + 8, lanes l and l + 32 their terms
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (warp + 8 * i >= jb.nc) break;
+            kcol[i] = jobcols[jb.c0 + warp + 8 * i];
+            if (lane < m) pv[2 * i] = __ldg(Sinv + lane * m + kcol[i]);
+            if (lane + 32 < m) pv[2 * i + 1] = __ldg(Sinv + (lane + 32) * m + kcol[i]);
+        }
+    }
+    if (MODE == 1) {
+#pragma unroll
+        for (int i = 0; i < (MODE == 1 ? 16 : 0); ++i)
+            if (i < cnt) pv[i] = __ldg(Sinv + (g + i * tpr) * m + kk);
+    }
+    pdl_begin();
+    pdl_trigger();
+    // u = Sigma^{1/2} xi' - y, the partial sums of y in order
+    for (int k = tid; k < m; k += 256) {
+        const V *part = reinterpret_cast<const V *>(lr.part) + (i64)k * P;
+        const V w = __ldcg(static_cast<const V *>(lr.w) + k);
+        if constexpr (sizeof(T) == 4) {
+            ff32 t{0.f, 0.f};
+            for (int p0 = 0; p0 < P; p0 += 4) {
+                float2 pp[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) pp[r] = p0 + r < P ? __ldcg(part + p0 + r) : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    if (p0 + r < P) t = ff_add(t, ff_of(pp[r]));
+            }
+            const ff32 uk = ff_add(ff_of(w), ff_neg(t));
+            u[k] = make_float2(uk.hi, uk.lo);
+        } else {
+            double t = 0.0;
+            for (int p0 = 0; p0 < P; p0 += 4) {
+                double pp[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) pp[r] = p0 + r < P ? __ldcg(part + p0 + r) : 0.0;
+                t += (pp[0] + pp[1]) + (pp[2] + pp[3]);
+            }
+            u[k] = w - t;
+        }
+    }
+    __syncthreads();
+    if constexpr (MODE == 0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (warp + 8 * i >= jb.nc) break;
+            if constexpr (sizeof(T) == 4) {
+                // products, the two sums of each group (lane 2 g + h: h of
+                // group g; 2 groups <= 32), then z_k over the groups
+                V *p = pr + 64 * warp;
+                const ff32 v0 = lane < m ? ff_mul(ff_of(pv[2 * i]), ff_of(u[lane])) : ff32{0.f, 0.f};
+                const ff32 v1 = lane + 32 < m ? ff_mul(ff_of(pv[2 * i + 1]), ff_of(u[lane + 32])) : ff32{0.f, 0.f};
+                p[lane] = make_float2(v0.hi, v0.lo);
+                p[lane + 32] = make_float2(v1.hi, v1.lo);
+                __syncwarp();
+                ff32 a{0.f, 0.f};
+                if (lane < 2 * groups)
+                    for (int c = (lane >> 1) + (lane & 1) * tpr; c < m; c += 2 * tpr) a = ff_add(a, ff_of(p[c]));
+                a = ff_add(a, ff32{__shfl_xor_sync(0xffffffffu, a.hi, 1), __shfl_xor_sync(0xffffffffu, a.lo, 1)});
+                ff32 zk{0.f, 0.f};
+                for (int h = 0; h < groups; ++h)
+                    zk = ff_add(zk, ff32{__shfl_sync(0xffffffffu, a.hi, 2 * h), __shfl_sync(0xffffffffu, a.lo, 2 * h)});
+                if (lane == 0) zs[kcol[i]] = ff_to_float(zk);
+                __syncwarp();
+            } else {
+                double a = lane < m ? pv[2 * i] * u[lane] : 0.0;
+                if (lane + 32 < m) a = fma(pv[2 * i + 1], u[lane + 32], a);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                if (lane == 0) zs[kcol[i]] = a;
+            }
+        }
+        __syncthreads();
+    } else {  // every CTA forms all of z
+        for (int k0 = 0; k0 < m; k0 += cols) {
+            const int k = k0 + kk;
+            if (g < groups && k < m) {
+                const V *col = Sinv + k;
+                int c = g;
+                if constexpr (sizeof(T) == 4) {
+                    ff32 t0{0.f, 0.f}, t1{0.f, 0.f};
+                    if constexpr (MODE == 1) {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 2) {
+                            if (i < cnt) t0 = ff_add(t0, ff_mul(ff_of(pv[i]), ff_of(u[g + i * tpr])));
+                            if (i + 1 < cnt) t1 = ff_add(t1, ff_mul(ff_of(pv[i + 1]), ff_of(u[g + (i + 1) * tpr])));
+                        }
+                    } else {  // blocks of eight terms, the rest to the first sum
+                        for (; c + 7 * tpr < m; c += 8 * tpr) {
+                            float2 sv[8];
+#pragma unroll
+                            for (int r = 0; r < 8; ++r) sv[r] = __ldg(col + (i64)(c + r * tpr) * m);
+#pragma unroll
+                            for (int r = 0; r < 8; r += 2) {
+                                t0 = ff_add(t0, ff_mul(ff_of(sv[r]), ff_of(u[c + r * tpr])));
+                                t1 = ff_add(t1, ff_mul(ff_of(sv[r + 1]), ff_of(u[c + (r + 1) * tpr])));
+                            }
+                        }
+                        for (; c < m; c += tpr) t0 = ff_add(t0, ff_mul(ff_of(__ldg(col + (i64)c * m)), ff_of(u[c])));
+                    }
+                    const ff32 v = ff_add(t0, t1);
+                    pr[g * cols + kk] = make_float2(v.hi, v.lo);
+                } else {
+                    double t0 = 0.0, t1 = 0.0;
+                    if constexpr (MODE == 1) {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 2) {
+                            if (i < cnt) t0 = fma(pv[i], u[g + i * tpr], t0);
+                            if (i + 1 < cnt) t1 = fma(pv[i + 1], u[g + (i + 1) * tpr], t1);
+                        }
+                    } else {
+                        for (; c + 7 * tpr < m; c += 8 * tpr) {
+                            double sv[8];
+#pragma unroll
+                            for (int r = 0; r < 8; ++r) sv[r] = __ldg(col + (i64)(c + r * tpr) * m);
+#pragma unroll
+                            for (int r = 0; r < 8; r += 2) {
+                                t0 = fma(sv[r], u[c + r * tpr], t0);
+                                t1 = fma(sv[r + 1], u[c + (r + 1) * tpr], t1);
+                            }
+                        }
+                        for (; c < m; c += tpr) t0 = fma(__ldg(col + (i64)c * m), u[c], t0);
+                    }
+                    pr[g * cols + kk] = t0 + t1;
+                }
+            }
+            __syncthreads();
+            if (tid < cols && k0 + tid < m) {
+                if constexpr (sizeof(T) == 4) {
+                    ff32 zk{0.f, 0.f};
+                    for (int h = 0; h < groups; ++h) zk = ff_add(zk, ff_of(pr[h * cols + tid]));
+                    zs[k0 + tid] = ff_to_float(zk);
+                } else {
+                    double zk = 0.0;
+                    for (int h = 0; h < groups; ++h) zk += pr[h * cols + tid];
+                    zs[k0 + tid] = zk;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    if (jb.multi) {
+        if (row < jb.r1) mr.apply(x, C, zs);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NQ; ++i)
+            if (row + 1024 * i < jb.r1) q[i].apply(x, row + 1024 * i, 256, jb.r1, zs);
     }
 }
 
-// x[row] += sum_e C_e z_{col_e} over the support rows of C = M^{-1} B, with
-// the coefficients z of k_lr_solve (ZT = float: the FP32 chain's rounded
-// copy), four rows per thread and iteration with their loads issued together.
-// Only z comes from the kernel just before (k_bt_solve); the row indices,
-// columns, values and the state of a thread's first four rows do not, so
-// they are loaded before the wait for that kernel.  The state was written by
-// a kernel before k_bt_solve, which had completed when every CTA of
-// k_bt_solve passed its own wait, i.e. before this grid started; it is read
-// through L2 (ld.global.cg), the level at which those writes are visible.
-template <typename T, typename ZT>
-__global__ void __launch_bounds__(256) k_lr_scatter(T *__restrict__ x, CorrRows C, const ZT *__restrict__ z) {
-    const i64 stride = (i64)gridDim.x * blockDim.x;
-    const i64 t0 = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    CorrQuad<T> q;
-    CorrMulti<T> mr;
-    if (t0 < C.n1) q.load(x, C, t0, stride, true);
-    if (t0 < C.nm) mr.load(x, C, t0, true);
+// dst -= B_c Sigma^{-1} y over the rows of the coarse level's B, y from the
+// partial sums of k_bt_partial: the low-rank term of a residual-restriction
+// (k_add_Bq's arithmetic).  The rows are known before the wait; dst was
+// written by the kernel before k_bt_partial.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_resid_Bq(T *dst, i64 nrows, const i64 *__restrict__ rows, const i64 *__restrict__ ptr, const int *__restrict__ col,
+               const double *__restrict__ val, const double *lrpart, int m, int P, const double *__restrict__ sigma_inv) {
+    extern __shared__ double qs[];
+    const i64 r = (i64)blockIdx.x * 256 + threadIdx.x;
+    i64 row = 0, e0 = 0, e1 = 0;
+    double v0 = 0.0;
+    int c0 = 0;
+    if (r < nrows) {
+        row = rows[r];
+        e0 = ptr[r];
+        e1 = ptr[r + 1];
+        v0 = val[e0];
+        c0 = col[e0];
+    }
+    const double si = threadIdx.x < m ? sigma_inv[threadIdx.x] : 0.0;
     pdl_begin();
-    for (i64 r0 = t0; r0 < C.n1; r0 += 4 * stride) {
-        q.apply(x, C, r0, stride, z);
-        if (r0 + 4 * stride < C.n1) q.load(x, C, r0 + 4 * stride, stride, false);
+    pdl_trigger();
+    const T d = r < nrows ? dst[row] : T(0);
+    for (int k = threadIdx.x; k < m; k += 256) {
+        double y = 0.0;
+        if constexpr (sizeof(T) == 4) {
+            const float2 *part = reinterpret_cast<const float2 *>(lrpart) + (i64)k * P;
+            ff32 t{0.f, 0.f};
+            for (int p = 0; p < P; ++p) t = ff_add(t, ff_of(__ldcg(part + p)));
+            y = ff_to_double(t);
+        } else {
+            for (int p = 0; p < P; ++p) y += __ldcg(lrpart + (i64)k * P + p);
+        }
+        qs[k] = y * (k == (int)threadIdx.x ? si : sigma_inv[k]);
     }
-    for (i64 r = t0; r < C.nm; r += stride) {
-        if (r != t0) mr.load(x, C, r, false);
-        mr.apply(x, C, z);
-    }
+    __syncthreads();
+    if (r >= nrows) return;
+    double acc = v0 * qs[c0];
+    for (i64 e = e0 + 1; e < e1; ++e) acc += val[e] * qs[col[e]];
+    dst[row] = d + (T)(-1.0 * acc);
 }
 
 // ------------------------------------------------- residual + restriction
@@ -1683,8 +1904,8 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict_tma(const __grid_
 // ncu, where this kernel takes 5.5, 13 and 50.
 template <int NPT>
 __global__ void __launch_bounds__(256)
-    k_resid_restrict_sym(const double *__restrict__ x, const double *__restrict__ f, double *__restrict__ fc,
-                         double *__restrict__ xc, Grid3 gf, Grid3 gc, SymWeights w, int whole) {
+    k_resid_restrict_sym(const double *x, const double *f, double *fc, double *xc, Grid3 gf, Grid3 gc, SymWeights w,
+                         int whole) {
     if (gf.pdl) pdl_begin();
     constexpr bool D3 = NPT == 27 || NPT == 7, FULL = NPT == 27 || NPT == 9;
     constexpr int NPX = D3 ? 5 : 1, NPF = D3 ? 3 : 1;  // planes of x and f
