@@ -375,6 +375,15 @@ static dim3 level_block(const Level &lv, int count) {
     return sweep_block(count);
 }
 
+static SymWeights sym_weights(const Level &lv, const StencilArg<double> &s) {
+    SymWeights w;
+    std::copy(lv.wc, lv.wc + 8, w.wc);
+    w.sd = s.sd;
+    w.od = s.omega_diag;
+    w.om1 = 1.0 - s.omega;
+    return w;
+}
+
 template <typename T, bool EXACT, int NOISE>
 static void launch_colour_passes(Sampler &S, const Level &lv, bool forward, T *x, const T *f, const StencilArg<T> &s,
                                  const NoiseArgs &nz);
@@ -405,18 +414,25 @@ static void launch_sweep_t(Sampler &S, const Level &lv, bool forward, T *x, cons
                     // the colour-split f exists for level 0's own f only
                     const bool fs = v8 && S.fsplit && f == S.L[0].f && &lv == &S.L[0];
                     const float *fsc = fs ? S.fsplit + colour * S.fhalf : nullptr;
-                    if (lv.var == 1 && fs)
-                        plaunch(pd, k_sweep_rb_vec<NOISE, true, true, true>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vd, fsc);
-                    else if (lv.var == 1 && v8)
-                        plaunch(pd, k_sweep_rb_vec<NOISE, true, true, false>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vd, fsc);
-                    else if (lv.var == 1)
-                        plaunch(pd, k_sweep_rb_vec<NOISE, true, false, false>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vd, fsc);
-                    else if (fs)
-                        plaunch(pd, k_sweep_rb_vec<NOISE, false, true, true>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vd, fsc);
-                    else if (v8)
-                        plaunch(pd, k_sweep_rb_vec<NOISE, false, true, false>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vd, fsc);
-                    else
-                        plaunch(pd, k_sweep_rb_vec<NOISE, false, false, false>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vd, fsc);
+                    auto go = [&](auto kernel) {
+                        plaunch(pd, kernel, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vd, fsc);
+                    };
+                    auto pick = [&](auto early) {
+                        constexpr bool E = decltype(early)::value;
+                        if (lv.var == 1 && fs)
+                            go(k_sweep_rb_vec<NOISE, true, true, true, E>);
+                        else if (lv.var == 1 && v8)
+                            go(k_sweep_rb_vec<NOISE, true, true, false, E>);
+                        else if (lv.var == 1)
+                            go(k_sweep_rb_vec<NOISE, true, false, false, E>);
+                        else if (fs)
+                            go(k_sweep_rb_vec<NOISE, false, true, true, E>);
+                        else if (v8)
+                            go(k_sweep_rb_vec<NOISE, false, true, false, E>);
+                        else
+                            go(k_sweep_rb_vec<NOISE, false, false, false, E>);
+                    };
+                    pd ? pick(std::true_type{}) : pick(std::false_type{});
                     S.launches++;
                     continue;
                 }
@@ -426,30 +442,37 @@ static void launch_sweep_t(Sampler &S, const Level &lv, bool forward, T *x, cons
                 const dim3 blk = level_block(lv, na);
                 dim3 grid((na + blk.x - 1) / blk.x, (lv.g.N1 + blk.y - 1) / blk.y, lv.g.N2);
                 const VarField<T> vf = var_field<T>(lv);
+                const bool pd = S.pdl && lv.g.pdl;
+                // FP64: the next launch starts early up to four warps per SM (see ROW_NT64)
+                const i64 warps = (i64)grid.x * grid.y * grid.z * (blk.x * blk.y / 32);
+                const int trigger = sizeof(T) == 4 || warps <= 4 * S.nsm;
+                if constexpr (std::is_same<T, double>::value && !EXACT) {
+                    // FP64 chains (FP32 chains' set-up sweeps keep the ordered sums)
+                    if (!S.fp32 && lv.sym && lv.var == 0 && S.dim > 1) {
+                        const SymWeights w = sym_weights(lv, s);
+                        auto go = [&](auto kernel) {
+                            plaunch(pd, kernel, grid, blk, 0, S.stream, x, f, lv.g, w, colour, pass, nz, trigger);
+                        };
+                        if (S.dim == 3)
+                            w.om1 == 0.0 ? go(k_sweep_rb_sym<true, NOISE, true>) : go(k_sweep_rb_sym<true, NOISE, false>);
+                        else
+                            w.om1 == 0.0 ? go(k_sweep_rb_sym<false, NOISE, true>) : go(k_sweep_rb_sym<false, NOISE, false>);
+                        S.launches++;
+                        continue;
+                    }
+                }
                 if (lv.var == 1)
-                    plaunch(S.pdl && lv.g.pdl, k_sweep_rb_pass<T, EXACT, NOISE, 1>, grid, blk, 0, S.stream, x, f, lv.g, s, colour,
-                            pass, nz, vf);
+                    plaunch(pd, k_sweep_rb_pass<T, EXACT, NOISE, 1>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vf, trigger);
                 else if (lv.var == 2)
-                    plaunch(S.pdl && lv.g.pdl, k_sweep_rb_pass<T, EXACT, NOISE, 2>, grid, blk, 0, S.stream, x, f, lv.g, s, colour,
-                            pass, nz, vf);
+                    plaunch(pd, k_sweep_rb_pass<T, EXACT, NOISE, 2>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vf, trigger);
                 else
-                    plaunch(S.pdl && lv.g.pdl, k_sweep_rb_pass<T, EXACT, NOISE, 0>, grid, blk, 0, S.stream, x, f, lv.g, s, colour,
-                            pass, nz, vf);
+                    plaunch(pd, k_sweep_rb_pass<T, EXACT, NOISE, 0>, grid, blk, 0, S.stream, x, f, lv.g, s, colour, pass, nz, vf, trigger);
             }
             S.launches++;
         }
     } else {
         launch_colour_passes<T, EXACT, NOISE>(S, lv, forward, x, f, s, nz);
     }
-}
-
-static SymWeights sym_weights(const Level &lv, const StencilArg<double> &s) {
-    SymWeights w;
-    std::copy(lv.wc, lv.wc + 8, w.wc);
-    w.sd = s.sd;
-    w.od = s.omega_diag;
-    w.om1 = 1.0 - s.omega;
-    return w;
 }
 
 // Launch of a pair of colours on whole rows: `tx` threads along x, CTAs of
@@ -502,12 +525,14 @@ static void launch_colour_passes(Sampler &S, const Level &lv, bool forward, T *x
                     r.trigger = row_warps(r) <= 4 * S.nsm;
                     const SymWeights w = sym_weights(lv, s);
                     const size_t sm = sizeof(double) * (r.block.x + 2) * r.block.y * (S.dim == 2 ? 2 : 4);
+                    auto go = [&](auto kernel) {
+                        plaunch(pdl, kernel, r.grid, r.block, sm, S.stream, x, f, lv.g, w, pb, pc, forward ? 0 : 1, nz,
+                                (int)r.trigger);
+                    };
                     if (S.dim == 2)
-                        plaunch(pdl, k_sweep_row_sym<9, NOISE>, r.grid, r.block, sm, S.stream, x, f, lv.g, w, pb, pc,
-                                forward ? 0 : 1, nz, (int)r.trigger);
+                        w.om1 == 0.0 ? go(k_sweep_row_sym<9, NOISE, true>) : go(k_sweep_row_sym<9, NOISE, false>);
                     else
-                        plaunch(pdl, k_sweep_row_sym<27, NOISE>, r.grid, r.block, sm, S.stream, x, f, lv.g, w, pb, pc,
-                                forward ? 0 : 1, nz, (int)r.trigger);
+                        w.om1 == 0.0 ? go(k_sweep_row_sym<27, NOISE, true>) : go(k_sweep_row_sym<27, NOISE, false>);
                     S.launches++;
                     continue;
                 }
@@ -1556,9 +1581,17 @@ void Sampler::autotune_sweeps() {
         if (lev == nlev - 1 && chol) break;
         Level &lv = L[lev];
         if (lv.npt != 7 && lv.g.N0 <= ROW_PAIR_MAX_N0) continue;  // whole rows: no width to choose
-        ensure_scratch(lev);
         const bool vec = fp32 && !exact && lv.npt == 7 && (lv.g.sy % 4) == 0 && (lv.g.sz % 4) == 0 && lv.var != 2;
         const int count = vec ? (lv.g.N0 + 8) / 8 : (lv.g.N0 + 1) / 2;
+        // a level of at most eight warps per SM: small CTAs spread it best, and
+        // a launch's own time hides the shapes' differences from the tuner
+        if ((i64)count * lv.g.N1 * lv.g.N2 <= 256 * (i64)nsm) {
+            lv.sweep_threads = 64;
+            lv.sweep_tx = 8;
+            while (lv.sweep_tx < count && lv.sweep_tx < 64) lv.sweep_tx *= 2;
+            continue;
+        }
+        ensure_scratch(lev);
         int cap = 8;
         while (cap < count && cap < RBP_THREADS) cap *= 2;
         NoiseArgs nz{};

@@ -266,6 +266,13 @@ __device__ __forceinline__ void sor_point(T *__restrict__ x, const T *__restrict
                                          x[P], f[P], s, P, noisy, xi, vf);
 }
 
+// Constant stencil with equal weights at +-dx, +-dy, +-dz: wc[|dz| * 4 +
+// |dy| * 2 + |dx|] is the weight of a class.
+struct SymWeights {
+    double wc[8];
+    double sd, od, om1;  // noise scale, omega / d, 1 - omega (kernels' UNIT: omega = 1, om1 = 0)
+};
+
 // ------------------------------------------------- red-black SOR sweep
 // Noise of a 7-point level: the normals of the 4 points of one x-parity in
 // the 8-aligned group of padded positions P = a + 1 in [8q, 8q + 8) of row
@@ -292,21 +299,51 @@ __host__ __forceinline__ dim3 sweep_block(int count) {
     return dim3(tx, RBP_THREADS / tx, 1);
 }
 
+// The normals are drawn before the wait for the launch before, and with
+// `trigger` the next launch starts early (see k_sweep_row_pair).
 template <typename T, bool EXACT, int NOISE, int VAR = 0>
-__global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_pass(T *__restrict__ x, const T *__restrict__ f, Grid3 g,
-                                                               StencilArg<T> s, int colour, int reverse, NoiseArgs nz,
-                                                               VarField<T> vf) {
-    if (g.pdl) pdl_begin();
+__global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_pass(T *x, const T *f, Grid3 g, StencilArg<T> s, int colour,
+                                                               int reverse, NoiseArgs nz, VarField<T> vf, int trigger) {
     const int b = blockIdx.y * blockDim.y + threadIdx.y;
     const int c = reverse ? g.N2 - 1 - (int)blockIdx.z : (int)blockIdx.z;
-    if (b >= g.N1) return;
     const int p = (colour + b + c) & 1;
     const int a = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + p;
     T xi = T(0);
     if (NOISE == NOISE_PHILOX) xi = (T)pick(fine_normals(nz, g, a + 1, b, c), ((a + 1) & 7) >> 1);
-    if (a >= g.N0) return;
+    if (g.pdl) pdl_begin();
+    if (trigger) pdl_trigger();
+    if (a >= g.N0 || b >= g.N1) return;
     if (NOISE == NOISE_INJECTED) xi = (T)nz.buf[g.compact(a, b, c)];
     sor_point<T, 7, EXACT, VAR>(x, f, g, s, g.pad(a, b, c), NOISE != NOISE_NONE, xi, vf);
+}
+
+// The same colour pass for FP64 chains whose constant axis stencil has equal
+// weights at +-1 (Level::sym): 8 FP64 instructions per point (6 in 2D) instead
+// of 11, since the FP64 unit is what it waits for (see k_sweep_row_sym): the
+// neighbours are added in pairs, the diagonal drops out of
+// x'' = (1 - omega) x + (omega / d)(sd xi + f - sum over the neighbours), and
+// the normal is widened by its bits.
+template <bool D3, int NOISE, bool UNIT>
+__global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_sym(double *x, const double *f, Grid3 g, SymWeights w,
+                                                              int colour, int reverse, NoiseArgs nz, int trigger) {
+    const int b = blockIdx.y * blockDim.y + threadIdx.y;
+    const int c = reverse ? g.N2 - 1 - (int)blockIdx.z : (int)blockIdx.z;
+    const int p = (colour + b + c) & 1;
+    const int a = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + p;
+    double xi = 0.0;
+    if (NOISE == NOISE_PHILOX) xi = widen(pick(fine_normals(nz, g, a + 1, b, c), ((a + 1) & 7) >> 1));
+    if (g.pdl) pdl_begin();
+    if (trigger) pdl_trigger();
+    if (a >= g.N0 || b >= g.N1) return;
+    if (NOISE == NOISE_INJECTED) xi = nz.buf[g.compact(a, b, c)];
+    double *q = x + g.pad(a, b, c);
+    double cv = f[g.pad(a, b, c)];
+    const double sx = q[-1] + q[1], sy = q[-g.sy] + q[g.sy], sz = D3 ? q[-g.sz] + q[g.sz] : 0.0;
+    if (NOISE != NOISE_NONE) cv = fma(w.sd, xi, cv);
+    if (D3) cv = fma(-w.wc[4], sz, cv);
+    cv = fma(-w.wc[2], sy, cv);
+    cv = fma(-w.wc[1], sx, cv);
+    *q = UNIT ? w.od * cv : fma(w.od, cv, w.om1 * *q);
 }
 
 // 256-bit vector access (sm_100 and later): 8 floats at a 32-byte aligned
@@ -359,7 +396,9 @@ __device__ __forceinline__ void st8(float *p, const float *v) {
 // The body, with the CTA coordinates (bx, by, bz) passed in: the solo
 // kernel below and the batched kernel (k_sweep_rb_vec_batch) run the same
 // arithmetic.
-template <int NOISE, bool VD, bool V8, bool FS>
+// EARLY (levels in programmatic dependent launch): the normals are drawn before
+// the wait for the launch before, and the next launch starts early.
+template <int NOISE, bool VD, bool V8, bool FS, bool EARLY>
 __device__ __forceinline__ void sweep_rb_vec_body(float *__restrict__ x, const float *__restrict__ f, const Grid3 &g,
                                                   const StencilArg<float> &s, int colour, int reverse,
                                                   const NoiseArgs &nz, const float *__restrict__ vd,
@@ -368,8 +407,17 @@ __device__ __forceinline__ void sweep_rb_vec_body(float *__restrict__ x, const f
     const int c = reverse ? g.N2 - 1 - bz : bz;
     const int q = bx * blockDim.x + threadIdx.x;
     const int ngrp = (g.N0 + 8) >> 3;
-    if (q >= ngrp || b >= g.N1) return;
     const int P0 = 8 * q;
+    // points of the colour: padded P with (P - 1 + b + c) & 1 == colour; the
+    // two parities get separate code so that every register index is static
+    const int j0 = (colour + b + c + 1) & 1;  // first local index j (P = P0 + j) of the colour
+    float4 nrm = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (EARLY) {
+        if (NOISE == NOISE_PHILOX) nrm = fine_normals(nz, g, P0 + j0, b, c);
+        pdl_begin();
+        pdl_trigger();
+    }
+    if (q >= ngrp || b >= g.N1) return;
     const i64 rb = (i64)(c + 1) * g.sz + (i64)(b + 1) * g.sy;
     const float4 *xr = reinterpret_cast<const float4 *>(x + rb + P0);
     const float4 *xn = reinterpret_cast<const float4 *>(x + rb - g.sy + P0);
@@ -388,9 +436,6 @@ __device__ __forceinline__ void sweep_rb_vec_body(float *__restrict__ x, const f
             dv[0] = d0.x; dv[1] = d0.y; dv[2] = d0.z; dv[3] = d0.w; dv[4] = d1.x; dv[5] = d1.y; dv[6] = d1.z; dv[7] = d1.w;
         }
     }
-    // points of the colour: padded P with (P - 1 + b + c) & 1 == colour; the
-    // two parities get separate code so that every register index is static
-    const int j0 = (colour + b + c + 1) & 1;  // first local index j (P = P0 + j) of the colour
     if (V8) {
         v[0] = P0 > 0 ? x[rb + P0 - 1] : 0.f;
         ld8(x + rb + P0, v + 1);
@@ -423,8 +468,7 @@ __device__ __forceinline__ void sweep_rb_vec_body(float *__restrict__ x, const f
         zp[0] = u0.x; zp[1] = u0.y; zp[2] = u0.z; zp[3] = u0.w; zp[4] = u1.x; zp[5] = u1.y; zp[6] = u1.z; zp[7] = u1.w;
         fv[0] = f0.x; fv[1] = f0.y; fv[2] = f0.z; fv[3] = f0.w; fv[4] = f1.x; fv[5] = f1.y; fv[6] = f1.z; fv[7] = f1.w;
     }
-    float4 nrm = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (NOISE == NOISE_PHILOX) nrm = fine_normals(nz, g, P0 + j0, b, c);
+    if (!EARLY && NOISE == NOISE_PHILOX) nrm = fine_normals(nz, g, P0 + j0, b, c);
     auto upd = [&](int j, int k) {
         const int a = P0 + j - 1;
         if (a < 0 || a >= g.N0) return;
@@ -478,13 +522,12 @@ __device__ __forceinline__ void sweep_rb_vec_body(float *__restrict__ x, const f
     }
 }
 
-template <int NOISE, bool VD = false, bool V8 = false, bool FS = false>
+template <int NOISE, bool VD, bool V8, bool FS, bool EARLY>
 __global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_vec(float *__restrict__ x, const float *__restrict__ f,
                                                               Grid3 g, StencilArg<float> s, int colour, int reverse,
                                                               NoiseArgs nz, const float *__restrict__ vd,
                                                               const float *__restrict__ fsc) {
-    if (g.pdl) pdl_begin();
-    sweep_rb_vec_body<NOISE, VD, V8, FS>(x, f, g, s, colour, reverse, nz, vd, fsc, blockIdx.x, blockIdx.y, blockIdx.z);
+    sweep_rb_vec_body<NOISE, VD, V8, FS, EARLY>(x, f, g, s, colour, reverse, nz, vd, fsc, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // Level 0's f split by colour for the FP32 fine sweep: the value of point
@@ -696,15 +739,9 @@ __global__ void __launch_bounds__(ROW_PAIR_THREADS)
 // the one-colour pass also multiplied the zero weights of the planes above
 // and below).  One thread per point: a warp per 32 points spreads a small
 // level over more FP64 units than two points per thread do.
-// wc[|dz| * 4 + |dy| * 2 + |dx|]: the weight of a class.
-struct SymWeights {
-    double wc[8];
-    double sd, od, om1;  // noise scale, omega / d, 1 - omega
-};
-
 constexpr int ROW_SYM_THREADS = 512;  // most threads of a CTA, and the longest row
 
-template <int NPT, int NOISE>
+template <int NPT, int NOISE, bool UNIT>
 __global__ void __launch_bounds__(ROW_SYM_THREADS)
     k_sweep_row_sym(double *x, const double *f, Grid3 g, SymWeights w, int pb, int pc,
                     int odd_first, NoiseArgs nz, int trigger) {
@@ -748,12 +785,12 @@ __global__ void __launch_bounds__(ROW_SYM_THREADS)
         cv = fma(-w.wc[2 * k], s[k], cv);
         cv = fma(-w.wc[2 * k + 1], row[k * pitch - 1] + row[k * pitch + 1], cv);
     }
-    const double keep = w.om1 == 0.0 ? 0.0 : w.om1 * s[0];
+    const double keep = UNIT ? 0.0 : w.om1 * s[0];
     // own row: the first colour, then the second one from its new values
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         if ((a & 1) == (h ^ odd_first)) {
-            const double v = fma(w.od, fma(-w.wc[1], row[-1] + row[1], cv), keep);
+            const double c1 = fma(-w.wc[1], row[-1] + row[1], cv), v = UNIT ? w.od * c1 : fma(w.od, c1, keep);
             if (h == 0) row[0] = v;
             if (in) x[P] = v;
             if (h == 0 && !in) row[0] = 0.0;
@@ -2915,7 +2952,7 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_vec_batch(const BatchL
     load_stencil_shared(ss, a.s);
     const NoiseArgs nz = batch_noise(ca[chain], invocation, level);
     const float *fsc = FS ? a.fsplit + colour * a.fhalf : nullptr;
-    sweep_rb_vec_body<NOISE, false, V8, FS>(a.x, a.f, g, ss, colour, reverse, nz, nullptr, fsc, blockIdx.x, blockIdx.y,
+    sweep_rb_vec_body<NOISE, false, V8, FS, false>(a.x, a.f, g, ss, colour, reverse, nz, nullptr, fsc, blockIdx.x, blockIdx.y,
                                             bz);
 }
 

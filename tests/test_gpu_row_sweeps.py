@@ -1,7 +1,8 @@
-"""Colour passes of 9- and 27-point levels (two colours of a row per launch)
-against a plain numpy sweep in 64 bits, at the edges of their row widths:
-rows of one point, of odd and even length, one CTA's longest row and one
-point more (which runs one colour per launch)."""
+"""Colour passes against a plain numpy sweep in 64 bits: 9- and 27-point levels
+(two colours of a row per launch) at the edges of their row widths -- rows of
+one point, of odd and even length, one CTA's longest row and one point more
+(which runs one colour per launch) -- and red-black levels with pitches that
+take the vector pass and ones that do not."""
 import numpy as np
 import pytest
 
@@ -24,10 +25,13 @@ def _stencil(dim, symmetric):
     return st
 
 
-def _normals(a, b, c, N, level, sc, seed):
-    """Philox4x32-10 and Box-Muller in 64 bits: the normal of point (a, b, c)."""
+def _normals(a, b, c, N, level, sc, seed, axis=False):
+    """Philox4x32-10 and Box-Muller in 64 bits: the normal of point (a, b, c)
+    of a 3^dim-point level, or of a red-black one (axis)."""
     m = np.uint64(0xFFFFFFFF)
-    grp = ((c * N[1] + b) * ((N[0] + 7) >> 3) + (a >> 3)).astype(np.uint64)
+    groups = ((N[0] + 1) >> 3) + 1 if axis else (N[0] + 7) >> 3
+    a = a + 1 if axis else a
+    grp = ((c * N[1] + b) * groups + (a >> 3)).astype(np.uint64)
     ctr = [grp, (np.uint64(level << 8) | (a & 1).astype(np.uint64)), np.full_like(grp, sc & 0xFFFFFFFF),
            np.full_like(grp, sc >> 32)]
     k0, k1 = seed & 0xFFFFFFFF, seed >> 32
@@ -44,8 +48,10 @@ def _normals(a, b, c, N, level, sc, seed):
 def _sweep(st, dim, x, f, omega, forward):
     """One multicolour SOR sweep (colour = parities of a, b, c) of x[c, b, a]."""
     c, b, a = np.indices(x.shape)
-    colour = (a & 1) | (b & 1) << 1 | (c & 1) << 2
-    order = range(2 ** dim) if forward else reversed(range(2 ** dim))
+    axis = np.count_nonzero(st) <= 2 * dim + 1
+    colour = (a + b + c) & 1 if axis else (a & 1) | (b & 1) << 1 | (c & 1) << 2
+    ncol = 2 if axis else 2 ** dim
+    order = range(ncol) if forward else reversed(range(ncol))
     for k in order:
         xp = np.pad(x, 1)
         y = sum(st[(dz + 1) * 9 + (dy + 1) * 3 + dx + 1] *
@@ -62,9 +68,25 @@ SHAPES = [(2, 4, 4), (9, 3, 2), (16, 6, 5), (66, 5, 4), (33, 8), (130, 6), (131,
 @pytest.mark.parametrize("symmetric", [True, False])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_row_sweeps(shape, symmetric, precision):
-    dim, omega, seed = len(shape), 1.2, 5
+    _check(shape, _stencil(len(shape), symmetric), 1.2, precision)
+
+
+@pytest.mark.parametrize("precision", [M.FP64, M.FP32_MIXED])
+@pytest.mark.parametrize("omega", [1.0, 1.2])
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("shape", [(2, 3, 4), (8, 5, 4), (12, 8, 3), (33, 4, 5), (9,), (8, 6), (7, 5), (200, 16, 16)])
+def test_red_black_sweeps(shape, symmetric, omega, precision):
+    st = _stencil(len(shape), symmetric)
+    for k in range(27):
+        if sum(d != 1 for d in (k % 3, (k // 3) % 3, k // 9)) > 1:
+            st[k] = 0.0
+    _check(shape, st, omega, precision)
+
+
+def _check(shape, st, omega, precision):
+    dim, seed = len(shape), 5
     N = [s - 1 for s in shape] + [1] * (3 - dim)
-    st = _stencil(dim, symmetric)
+    axis = np.count_nonzero(st) <= 2 * dim + 1
     op = M.LinearOperator(shape, st)
     s = M.SSORSampler(op, omega=omega, precision=precision, seed=seed)
     rng = np.random.default_rng(2)
@@ -80,7 +102,7 @@ def test_row_sweeps(shape, symmetric, precision):
             cval = f.reshape(N[::-1])
             if noisy:
                 sd = np.sqrt(st[13] * (2 - omega) / omega)
-                cval = cval + sd * _normals(a, b, c, N, 0, 4095, seed)
+                cval = cval + sd * _normals(a, b, c, N, 0, 4095, seed, axis)
             want = _sweep(st, dim, x.reshape(N[::-1]), cval, omega, forward).reshape(-1)
             s.sor(0, M.FORWARD if forward else M.BACKWARD, f, x, with_noise=noisy)
             assert np.max(np.abs(x - want)) < (5e-4 if noisy else 27 * 8 * 4 * eps)
