@@ -3252,21 +3252,22 @@ mgmc_status mgmc_batch_destroy(mgmc_batch *b) {
 
 // --------------------------------------------- low-rank Cholesky sampler
 // LowRankCholeskySampler (cholesky_sampler.cc:41-129) on the GPU.  The
-// factors come from lowrank_cholesky_factors (setup.cc): D_k = L_kk^{-1}
-// and O_k = L_{k,k-1} of the block factor of A_0, and Q, QW, QWT.  A sample
-// is xi ~ N(0, 1) (n normals: Philox or injected), g = L^{-1} f block by
-// block (g_k = D_k (f_k - O_k g_{k-1})), g += QW (Q^T g), xi += g,
-// xi += QWT (Q^T xi), and x = L^{-T} xi block by block from the last
-// (x_k = D_k^T (xi_k - O_{k+1}^T x_{k+1})) -- dense FP64 matrix-vector
-// products (k_dgemv_rows, k_dgemv_cols_partial / _finish) captured into
-// one CUDA graph.
+// factors come from lowrank_cholesky_factors (setup.cc): D_k = L_kk^{-1},
+// O_k = L_{k,k-1} of the block factor of A_0, and Q, W of the low-rank term;
+// the set-up forms E_k = D_k O_k and G_k = D_k^T O_{k+1}^T on the device.  A
+// sample is xi ~ N(0, 1) (n normals: Philox or injected), g = L^{-1} f,
+// the low-rank part, and x = L^{-T} xi, each solve a product of all
+// triangular blocks and a chain of dense ones (k_chol_tri, k_chol_step),
+// captured into one CUDA graph.
 struct LrChol {
-    int device = 0, nb = 0, m = 0, noise = NOISE_PHILOX;
-    i64 n = 0, p = 0;
+    int device = 0, nb = 0, m = 0, noise = NOISE_PHILOX, nsm = 152;
+    i64 n = 0;
+    int p = 0, ld = 0;
     u64 seed = 0;
     cudaStream_t stream = nullptr;
-    double *D = nullptr, *O = nullptr, *Q = nullptr, *QW = nullptr, *QWT = nullptr;
-    double *f = nullptr, *x = nullptr, *xi = nullptr, *g = nullptr, *t = nullptr, *mt = nullptr, *part = nullptr;
+    double *D = nullptr, *DT = nullptr, *E = nullptr, *G = nullptr, *Q = nullptr, *W = nullptr;
+    double *f = nullptr, *x = nullptr, *xi = nullptr, *g = nullptr, *v = nullptr, *part = nullptr;  // blocks of ld
+    double *cvec = nullptr;  // n values: a caller's vector
     double *noise_buf = nullptr;
     i64 noise_cap = 0, noise_len = 0, noise_pos = 0;
     u64 *d_step = nullptr;
@@ -3274,7 +3275,6 @@ struct LrChol {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     std::vector<void *> owned;
-    static constexpr int RCH = 64;  // rows per partial sum of a transposed product
     ~LrChol() {
         if (gexec) cudaGraphExecDestroy(gexec);
         if (graph) cudaGraphDestroy(graph);
@@ -3287,74 +3287,55 @@ struct LrChol {
         owned.push_back(q);
         return q;
     }
-    template <typename P_>
-    P_ *upload(const std::vector<P_> &v) {
-        P_ *q = dupload(v, stream);
-        owned.push_back(q);
+    double *zeros(size_t count) {
+        double *q = alloc<double>(count);
+        CK(cudaMemsetAsync(q, 0, count * sizeof(double), stream));
         return q;
     }
-    // y = yadd + alpha A v, A rows x cols row-major
-    void rows(const double *A, i64 r, i64 c, i64 lda, const double *v, const double *yadd, double alpha, double *y,
-              bool lower) {
-        const unsigned blocks = (unsigned)((r * 32 + 255) / 256);
-        if (lower)
-            k_dgemv_rows<true><<<blocks, 256, 0, stream>>>(A, r, c, lda, v, yadd, alpha, y);
-        else
-            k_dgemv_rows<false><<<blocks, 256, 0, stream>>>(A, r, c, lda, v, yadd, alpha, y);
-    }
-    // y = yadd + alpha A^T v
-    void cols(const double *A, i64 r, i64 c, i64 lda, const double *v, const double *yadd, double alpha, double *y,
-              bool lower) {
-        const int nch = (int)((r + RCH - 1) / RCH);
-        const int bs = c >= 256 ? 256 : (int)((c + 31) / 32 * 32);
-        const dim3 grid((unsigned)((c + bs - 1) / bs), (unsigned)nch);
-        if (lower)
-            k_dgemv_cols_partial<true><<<grid, bs, 0, stream>>>(A, r, c, lda, v, RCH, part);
-        else
-            k_dgemv_cols_partial<false><<<grid, bs, 0, stream>>>(A, r, c, lda, v, RCH, part);
-        k_dgemv_cols_finish<<<(unsigned)((c + 255) / 256), 256, 0, stream>>>(part, nch, c, yadd, alpha, y);
+    i64 padded() const { return (i64)nb * ld; }
+    void set_factors(const LowRankCholeskyFactors &F);
+    // y -= A v, one block
+    void link(const double *A, const double *vec, double *y) {
+        // as many warps per CTA as make one CTA per SM
+        const int wpc = std::min(8, std::max(1, (p + nsm - 1) / nsm));
+        plaunch(true, k_chol_step, (p + wpc - 1) / wpc, 32 * wpc, 0, stream, A, p, ld, vec, y);
     }
     void sample() {
         NoiseArgs nz{};
         nz.seed = seed;
         nz.d_step = d_step;
-        nz.invocation = 0;
-        nz.level = 0;
+        const i64 np = padded(), mat = (i64)p * ld;
         if (noise == NOISE_INJECTED) {
             nz.buf = noise_buf + noise_pos;
-            k_cholesky_normals<NOISE_INJECTED><<<nblk(n, 256), 256, 0, stream>>>(nz, n, xi);
+            k_cholesky_normals<NOISE_INJECTED><<<nblk(np, 256), 256, 0, stream>>>(nz, nb, p, ld, xi);
         } else {
-            k_cholesky_normals<NOISE_PHILOX><<<nblk(n, 256), 256, 0, stream>>>(nz, n, xi);
+            k_cholesky_normals<NOISE_PHILOX><<<nblk(np, 256), 256, 0, stream>>>(nz, nb, p, ld, xi);
         }
-        // g = L^{-1} f
-        for (int k = 0; k < nb; ++k) {
-            const double *Dk = D + (size_t)k * p * p;
-            const double *v = f + k * p;
-            if (k > 0) {
-                rows(O + (size_t)k * p * p, p, p, p, g + (k - 1) * p, f + k * p, -1.0, t, false);
-                v = t;
-            }
-            rows(Dk, p, p, p, v, nullptr, 1.0, g + k * p, true);
+        auto triangular = [&](auto kernel, const double *A, const double *from, double *to) {
+            for (i64 k0 = 0; k0 < nb; k0 += 65535)  // grid.y carries the blocks
+                plaunch(true, kernel, dim3(((p + 1) / 2 + 7) / 8, (unsigned)std::min<i64>(nb - k0, 65535)), 256, 0, stream,
+                        A + k0 * mat, p, ld, from + k0 * ld, to + k0 * ld);
+        };
+        triangular(k_chol_tri<false>, D, f, g);
+        for (int k = 1; k < nb; ++k) link(E + k * mat, g + (i64)(k - 1) * ld, g + (i64)k * ld);
+        const unsigned rows = nblk(np, 128);
+        const size_t sm = m * sizeof(double);
+        if (m > 0) {
+            const int parts = (int)((np + CHOL_QT_ROWS - 1) / CHOL_QT_ROWS);
+            const double *cQ = Q, *cW = W, *cg = g, *cxi = xi, *cv = v, *cp = part;
+            plaunch(true, k_chol_qt, parts, 256, 0, stream, cQ, np, m, cg, part);
+            plaunch(true, k_chol_v<true>, 1, 1024, sm, stream, cp, parts, m, cW, v);
+            plaunch(true, k_chol_add<true>, rows, 128, sm, stream, xi, cg, cQ, np, m, cv);
+            plaunch(true, k_chol_qt, parts, 256, 0, stream, cQ, np, m, cxi, part);
+            plaunch(true, k_chol_v<false>, 1, 1024, sm, stream, cp, parts, m, cW, v);
+            plaunch(true, k_chol_add<false>, rows, 128, sm, stream, xi, cg, cQ, np, m, cv);
+        } else {
+            plaunch(true, k_chol_add<true>, rows, 128, 0, stream, xi, (const double *)g, (const double *)nullptr, np, 0,
+                    (const double *)nullptr);
         }
-        if (m > 0) {  // g += QW (Q^T g)
-            cols(Q, n, m, m, g, nullptr, 1.0, mt, false);
-            rows(QW, n, m, m, mt, g, 1.0, g, false);
-        }
-        k_axpy<double><<<nblk(n, 256), 256, 0, stream>>>(xi, g, 1.0, n);
-        if (m > 0) {  // xi += QWT (Q^T xi)
-            cols(Q, n, m, m, xi, nullptr, 1.0, mt, false);
-            rows(QWT, n, m, m, mt, xi, 1.0, xi, false);
-        }
-        // x = L^{-T} xi
-        for (int k = nb - 1; k >= 0; --k) {
-            const double *v = xi + k * p;
-            if (k + 1 < nb) {
-                cols(O + (size_t)(k + 1) * p * p, p, p, p, x + (k + 1) * p, xi + k * p, -1.0, t, false);
-                v = t;
-            }
-            cols(D + (size_t)k * p * p, p, p, p, v, nullptr, 1.0, x + k * p, true);
-        }
-        k_counter_advance<<<1, 1, 0, stream>>>(d_step);
+        triangular(k_chol_tri<true>, DT, xi, x);
+        for (int k = nb - 2; k >= 0; --k) link(G + k * mat, x + (i64)(k + 1) * ld, x + (i64)k * ld);
+        plaunch(true, k_counter_advance, 1, 1, 0, stream, d_step);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) fail(MGMC_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     }
@@ -3384,6 +3365,52 @@ struct LrChol {
     }
 };
 
+// The factors on the device: D and D^T with rows of ld, E_k = D_k O_k and
+// G_k = D_k^T O_{k+1}^T, Q by the blocks' rows (zero rows behind each block).
+void LrChol::set_factors(const LowRankCholeskyFactors &F) {
+    ld = (p + 3) / 4 * 4;
+    const i64 mat = (i64)p * ld, pp = (i64)p * p;
+    D = zeros((size_t)nb * mat);
+    DT = zeros((size_t)nb * mat);
+    E = zeros((size_t)nb * mat);
+    G = zeros((size_t)nb * mat);
+    struct Temp {
+        std::vector<double *> ptrs;
+        ~Temp() {
+            for (double *q : ptrs) cudaFree(q);
+        }
+    } temp;
+    auto up = [&](const std::vector<double> &h) {
+        temp.ptrs.push_back(dupload(h, stream));
+        return temp.ptrs.back();
+    };
+    const double *Dc = up(F.D), *Oc = up(F.O);
+    // grid.z carries the blocks: at most 65535 at a time
+    for (int k0 = 0; k0 < nb; k0 += 65535) {
+        const int nk = std::min(nb - k0, 65535), ne = std::min(nb - 1 - k0, 65535);
+        const dim3 t32((p + 31) / 32, (p + 31) / 32, nk);
+        k_chol_copy<false><<<t32, 256, 0, stream>>>(Dc + k0 * pp, D + k0 * mat, p, ld);
+        k_chol_copy<true><<<t32, 256, 0, stream>>>(Dc + k0 * pp, DT + k0 * mat, p, ld);
+        if (ne <= 0) continue;
+        const dim3 t64((p + 63) / 64, (p + 63) / 64, ne);
+        k_chol_gemm<<<t64, 256, 0, stream>>>(Dc + (k0 + 1) * pp, pp, p, 1, Oc + (k0 + 1) * pp, pp, p, 1,
+                                             E + (k0 + 1) * mat, mat, ld, p);
+        k_chol_gemm<<<t64, 256, 0, stream>>>(Dc + k0 * pp, pp, 1, p, Oc + (k0 + 1) * pp, pp, 1, p, G + k0 * mat, mat, ld, p);
+    }
+    CK(cudaGetLastError());
+    std::vector<double> Qp;
+    if (m > 0) {
+        Qp.assign((size_t)padded() * m, 0.0);
+        for (int k = 0; k < nb; ++k)
+            std::copy(F.Q.begin() + (size_t)k * p * m, F.Q.begin() + (size_t)(k + 1) * p * m, Qp.begin() + (size_t)k * ld * m);
+        Q = alloc<double>(Qp.size());
+        W = alloc<double>(F.W.size());
+        CK(cudaMemcpyAsync(Q, Qp.data(), Qp.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
+        CK(cudaMemcpyAsync(W, F.W.data(), F.W.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
+    }
+    CK(cudaStreamSynchronize(stream));
+}
+
 struct mgmc_lrchol {
     std::unique_ptr<LrChol> impl;
 };
@@ -3394,10 +3421,14 @@ static LrChol &lrimpl(mgmc_lrchol *s) {
     return *s->impl;
 }
 
-// n doubles host or device -> device buffer dst of the sampler
-static void lr_put(LrChol &S, const double *src, int on_device, double *dst) {
-    CK(cudaMemcpyAsync(dst, src, (size_t)S.n * sizeof(double), on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                       S.stream));
+// n doubles host or device -> f, in the blocks' layout
+static void lr_put_f(LrChol &S, const double *src, int on_device) {
+    if (!on_device) {
+        CK(cudaMemcpyAsync(S.cvec, src, (size_t)S.n * sizeof(double), cudaMemcpyHostToDevice, S.stream));
+        src = S.cvec;
+    }
+    k_chol_pad<<<nblk(S.padded(), 256), 256, 0, S.stream>>>(src, S.f, S.nb, S.p, S.ld);
+    CK(cudaGetLastError());
 }
 
 extern "C" {
@@ -3429,6 +3460,7 @@ mgmc_status mgmc_lrchol_create(const mgmc_operator_desc *op, int noise, uint64_t
         Sigma.assign(op->Sigma, op->Sigma + op->m);
     }
     LowRankCholeskyFactors F;
+    if (geo.n / geo.N[geo.dim - 1] > INT32_MAX / 8) fail(MGMC_ERR_UNSUPPORTED, "blocks too large");
     if (!lowrank_cholesky_factors(geo, op->stencil, B, Sigma, F))
         fail(MGMC_ERR_NOT_SPD, "the prior or the low-rank system is not positive definite");
     h = new mgmc_lrchol();
@@ -3439,28 +3471,26 @@ mgmc_status mgmc_lrchol_create(const mgmc_operator_desc *op, int noise, uint64_t
     CK(cudaStreamCreateWithFlags(&S.stream, cudaStreamNonBlocking));
     S.n = geo.n;
     S.nb = F.nb;
-    S.p = F.p;
+    S.p = (int)F.p;
     S.m = F.m;
+    CK(cudaDeviceGetAttribute(&S.nsm, cudaDevAttrMultiProcessorCount, device));
     S.noise = noise == MGMC_NOISE_INJECTED ? NOISE_INJECTED : NOISE_PHILOX;
     S.seed = seed;
-    S.D = S.upload(F.D);
-    S.O = S.upload(F.O);
+    S.set_factors(F);
     if (S.m > 0) {
-        S.Q = S.upload(F.Q);
-        S.QW = S.upload(F.QW);
-        S.QWT = S.upload(F.QWT);
+        S.v = S.alloc<double>(S.m);
+        S.part = S.alloc<double>((size_t)((S.padded() + CHOL_QT_ROWS - 1) / CHOL_QT_ROWS) * S.m);
+        if (S.m * sizeof(double) > 48 * 1024) {
+            raise_smem_limit(k_chol_v<true>, S.m * sizeof(double));
+            raise_smem_limit(k_chol_v<false>, S.m * sizeof(double));
+            raise_smem_limit(k_chol_add<true>, S.m * sizeof(double));
+            raise_smem_limit(k_chol_add<false>, S.m * sizeof(double));
+        }
     }
-    S.f = S.alloc<double>(S.n);
-    S.x = S.alloc<double>(S.n);
-    S.xi = S.alloc<double>(S.n);
-    S.g = S.alloc<double>(S.n);
-    S.t = S.alloc<double>(S.p);
-    S.mt = S.alloc<double>(std::max(S.m, 1));
-    const i64 maxr = std::max<i64>(S.n, S.p), maxc = std::max<i64>(S.p, S.m);
-    S.part = S.alloc<double>((size_t)((maxr + LrChol::RCH - 1) / LrChol::RCH) * maxc);
+    S.cvec = S.alloc<double>(S.n);
+    for (double **q : {&S.f, &S.x, &S.xi, &S.g}) *q = S.zeros((size_t)S.padded());
     S.d_step = S.alloc<u64>(1);
     CK(cudaMemsetAsync(S.d_step, 0, sizeof(u64), S.stream));
-    for (double *q : {S.f, S.x, S.xi, S.g}) CK(cudaMemsetAsync(q, 0, (size_t)S.n * sizeof(double), S.stream));
     CK(cudaStreamSynchronize(S.stream));
     *out = h;
     h = nullptr;
@@ -3493,7 +3523,7 @@ mgmc_status mgmc_lrchol_fix_rhs(mgmc_lrchol *s, const double *f, int on_device) 
     API_BEGIN
     LrChol &S = lrimpl(s);
     if (!f) fail(MGMC_ERR_INVALID_ARGUMENT, "null f");
-    lr_put(S, f, on_device, S.f);
+    lr_put_f(S, f, on_device);
     CK(cudaStreamSynchronize(S.stream));
     S.rhs_set = true;
     API_END
@@ -3504,14 +3534,15 @@ mgmc_status mgmc_lrchol_apply(mgmc_lrchol *s, const double *f, double *x, int on
     LrChol &S = lrimpl(s);
     if (!x) fail(MGMC_ERR_INVALID_ARGUMENT, "null x");
     if (f) {
-        lr_put(S, f, on_device, S.f);
+        lr_put_f(S, f, on_device);
         S.rhs_set = true;
     } else if (!S.rhs_set) {
         fail(MGMC_ERR_INVALID_ARGUMENT, "f is NULL but no right hand side has been set");
     }
     S.run();
-    CK(cudaMemcpyAsync(x, S.x, (size_t)S.n * sizeof(double), on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                       S.stream));
+    k_chol_unpad<<<nblk(S.padded(), 256), 256, 0, S.stream>>>(S.x, on_device ? x : S.cvec, S.nb, S.p, S.ld);
+    CK(cudaGetLastError());
+    if (!on_device) CK(cudaMemcpyAsync(x, S.cvec, (size_t)S.n * sizeof(double), cudaMemcpyDeviceToHost, S.stream));
     CK(cudaStreamSynchronize(S.stream));
     API_END
 }

@@ -2789,79 +2789,297 @@ __global__ void __launch_bounds__(256) k_step_end(const T *__restrict__ x, int n
 }
 
 // ------------------------------------------- low-rank Cholesky sampler
-// The sampler's solves with the block factor of A_0 and its low-rank
-// products are dense FP64 matrix-vector products of three kinds.
+// The block solves with L (blocks D_k = L_kk^{-1}, O_k = L_{k,k-1} of p x p)
+//   g_k = D_k (f_k - O_k g_{k-1}) = D_k f_k - E_k g_{k-1},      E_k = D_k O_k
+//   x_k = D_k^T (xi_k - O_{k+1}^T x_{k+1}) = D_k^T xi_k - G_k x_{k+1},
+//                                                   G_k = D_k^T O_{k+1}^T
+// are a product of all triangular blocks at once (k_chol_tri) and a chain of
+// one dense product per block (k_chol_step): half the dependent launches of
+// the form with two products per block, and every product reads rows.
+// Vectors are stored by blocks of ld doubles (p, padded with zeros to a
+// multiple of 4), matrices with rows of ld.
 
-// y_i = yadd_i + alpha sum_j A_ij v_j over a row-major rows x cols block
-// (leading dimension lda): one warp per row, lanes over the columns, a
-// warp-shuffle sum.  LOWER: the block is lower triangular (columns j <= i).
-// y may alias yadd (each row reads its own entry before writing it).
-template <bool LOWER>
-__global__ void __launch_bounds__(256) k_dgemv_rows(const double *__restrict__ A, i64 rows, i64 cols, i64 lda,
-                                                    const double *__restrict__ v, const double *yadd, double alpha,
-                                                    double *y) {
-    const i64 i = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (i >= rows) return;
-    const i64 jmax = LOWER ? min(i + 1, cols) : cols;
-    const double *Ai = A + i * lda;
-    double a0 = 0.0, a1 = 0.0;
-    i64 j = lane;
-    for (; j + 32 < jmax; j += 64) {
-        a0 = fma(Ai[j], v[j], a0);
-        a1 = fma(Ai[j + 32], v[j + 32], a1);
-    }
-    if (j < jmax) a0 = fma(Ai[j], v[j], a0);
-    double acc = a0 + a1;
+// y_k = A_k v_k for all blocks k = blockIdx.y, A_k triangular (UPPER: columns
+// j >= i).  A warp takes the rows i and p - 1 - i, together one full row, and
+// reduces both sums in five steps instead of ten: FP64 instructions, two per
+// clock per SM, bound it.
+template <bool UPPER>
+__global__ void __launch_bounds__(256) k_chol_tri(const double *__restrict__ A, int p, int ld, const double *v, double *y) {
+    const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5), k = blockIdx.y;
+    pdl_begin();
+    if (i >= (p + 1) / 2) return;
+    const int i2 = p - 1 - i;
+    const double2 *vk = reinterpret_cast<const double2 *>(v + (i64)k * ld);
+    auto row_sum = [&](int r) {
+        const double2 *a = reinterpret_cast<const double2 *>(A + ((i64)k * p + r) * ld);
+        const int q0 = UPPER ? r / 2 : 0, q1 = UPPER ? ld / 2 : r / 2 + 1;
+        double s0 = 0.0, s1 = 0.0;
+        int q = q0 + lane;
+        for (; q + 96 < q1; q += 128) {
+            double2 av[4], vv[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) y[i] = (yadd ? yadd[i] : 0.0) + alpha * acc;
+            for (int t = 0; t < 4; ++t) av[t] = __ldcs(a + q + 32 * t);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) vv[t] = vk[q + 32 * t];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                s0 = fma(av[t].x, vv[t].x, s0);
+                s1 = fma(av[t].y, vv[t].y, s1);
+            }
+        }
+        for (; q < q1; q += 32) {
+            const double2 av = __ldcs(a + q), vv = vk[q];
+            s0 = fma(av.x, vv.x, s0);
+            s1 = fma(av.y, vv.y, s1);
+        }
+        return s0 + s1;
+    };
+    const double a0 = row_sum(i), a1 = i2 == i ? 0.0 : row_sum(i2);
+    const double give = lane < 16 ? a1 : a0;  // lanes 0-15 reduce row i, 16-31 row i2
+    double s = (lane < 16 ? a0 : a1) + __shfl_xor_sync(0xffffffffu, give, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) y[(i64)k * ld + i] = s;
+    if (lane == 16 && i2 != i) y[(i64)k * ld + i2] = s;
 }
 
-// Partial sums of (A^T v)_j over row chunk blockIdx.y (rows [c rch,
-// (c + 1) rch)): part[c cols + j], one thread per column (coalesced row
-// reads).  LOWER: A is lower triangular, rows i >= j only.
-template <bool LOWER>
-__global__ void __launch_bounds__(256) k_dgemv_cols_partial(const double *__restrict__ A, i64 rows, i64 cols, i64 lda,
-                                                            const double *__restrict__ v, int rch,
-                                                            double *__restrict__ part) {
-    const i64 j = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
-    if (j >= cols) return;
-    i64 i0 = (i64)c * rch;
-    const i64 i1 = min(rows, i0 + rch);
-    if (LOWER && i0 < j) i0 = j;
-    double acc = 0.0;
-    for (i64 i = i0; i < i1; ++i) acc = fma(A[i * lda + j], v[i], acc);
-    part[(i64)c * cols + j] = acc;
+// One link of the chain: y -= A v, A p x p dense, one warp per row.  The row
+// does not depend on the launch before, so its first 1024 values are in
+// registers before the wait, and the next link starts at once to load its own:
+// what is left between two links is the read of v, 30 FP64 multiplications and
+// five additions.  (32^3 cells, p = 961: about 3.1 us per link.)
+__global__ void __launch_bounds__(256, 2) k_chol_step(const double *__restrict__ A, int p, int ld, const double *v, double *y) {
+    const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), n2 = ld / 2;
+    const double2 *a = reinterpret_cast<const double2 *>(A + (i64)min(row, p - 1) * ld);
+    const double2 *vv = reinterpret_cast<const double2 *>(v);
+    double2 av[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) av[t] = lane + 32 * t < n2 ? __ldcs(a + lane + 32 * t) : make_double2(0.0, 0.0);
+    pdl_begin();
+    pdl_trigger();
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (256 * h >= n2) break;
+        double2 w[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) w[t] = lane + 32 * (8 * h + t) < n2 ? vv[lane + 32 * (8 * h + t)] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            if (32 * (8 * h + t) >= n2) break;
+            s0 = fma(av[8 * h + t].x, w[t].x, s0);
+            s1 = fma(av[8 * h + t].y, w[t].y, s1);
+        }
+    }
+    for (int q = lane + 512; q < n2; q += 128) {
+        double2 b[4], w[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const bool in = q + 32 * t < n2;
+            b[t] = in ? __ldcs(a + q + 32 * t) : make_double2(0.0, 0.0);
+            w[t] = in ? vv[q + 32 * t] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            s0 = fma(b[t].x, w[t].x, s0);
+            s1 = fma(b[t].y, w[t].y, s1);
+        }
+    }
+    double s = s0 + s1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0 && row < p) y[row] -= s;
 }
 
-// y_j = yadd_j + alpha sum_c part[c cols + j], chunks in order (the result
-// does not depend on block timing).  y may alias yadd.
-__global__ void __launch_bounds__(256) k_dgemv_cols_finish(const double *__restrict__ part, int nch, i64 cols,
-                                                           const double *yadd, double alpha, double *y) {
-    const i64 j = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= cols) return;
-    double acc = 0.0;
-    for (int c = 0; c < nch; ++c) acc += part[(i64)c * cols + j];
-    y[j] = (yadd ? yadd[j] : 0.0) + alpha * acc;
+// Low-rank part, xi += g + Q (W^T - Id) Q^T g, then xi += Q (W - Id) Q^T xi:
+// each a product with Q^T (k_chol_qt), an m x m one (k_chol_v) and one with Q
+// (k_chol_add).  Q^T xi is formed from the updated xi although W^T Q^T g +
+// Q^T xi would save a pass over Q: W is small where the measurements are
+// accurate, and only the product with the rounded xi damps its rounding too
+// (16^3 posterior against the oracle: 1.1e-12 instead of below 1e-12).
+//
+// Partial sums of Q^T v over CHOL_QT_ROWS rows per CTA: part[cta * m + j].
+constexpr int CHOL_QT_ROWS = 128;
+__global__ void __launch_bounds__(256) k_chol_qt(const double *__restrict__ Q, i64 rows, int m, const double *v,
+                                                 double *part) {
+    __shared__ double sh[8][32];
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    pdl_begin();
+    pdl_trigger();
+    const i64 r0 = (i64)blockIdx.x * CHOL_QT_ROWS, r1 = min(rows, r0 + CHOL_QT_ROWS);
+    for (int j0 = 0; j0 < m; j0 += 32) {
+        const int j = j0 + l;
+        double t = 0.0;
+        if (j < m) {
+#pragma unroll 4
+            for (i64 r = r0 + w; r < r1; r += 8) t = fma(Q[r * m + j], v[r], t);
+        }
+        sh[w][l] = t;
+        __syncthreads();
+        if (w == 0 && j < m) {
+            double a = 0.0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a += sh[i][l];
+            part[(i64)blockIdx.x * m + j] = a;
+        }
+        __syncthreads();
+    }
+}
+
+// t = the sum of the parts and v = (W - Id) t (TRANSPOSE: (W^T - Id) t) in one
+// CTA of 1024 threads, eight lanes per sum
+template <bool TRANSPOSE>
+__global__ void __launch_bounds__(1024) k_chol_v(const double *part, int nparts, int m, const double *__restrict__ W,
+                                                 double *v) {
+    extern __shared__ double ts[];
+    pdl_begin();
+    pdl_trigger();
+    const int l = threadIdx.x & 7, q = threadIdx.x >> 3;
+    auto over8 = [](double a) {
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        return a;
+    };
+    for (int c0 = 0; c0 < m; c0 += 128) {
+        const int c = c0 + q;
+        double a = 0.0;
+        if (c < m) {
+#pragma unroll 4
+            for (int i = l; i < nparts; i += 8) a += part[(i64)i * m + c];
+        }
+        a = over8(a);
+        if (l == 0 && c < m) ts[c] = a;
+    }
+    __syncthreads();
+    for (int c0 = 0; c0 < m; c0 += 128) {
+        const int c = c0 + q;
+        double a = 0.0;
+        if (c < m)
+            for (int k = l; k < m; k += 8)
+                a = fma((TRANSPOSE ? W[(i64)k * m + c] : W[(i64)c * m + k]) - (k == c ? 1.0 : 0.0), ts[k], a);
+        a = over8(a);
+        if (l == 0 && c < m) v[c] = a;
+    }
+}
+
+// xi += Q v (ADD_G: + g), one thread per row
+template <bool ADD_G>
+__global__ void __launch_bounds__(128) k_chol_add(double *xi, const double *g, const double *__restrict__ Q, i64 rows, int m,
+                                                  const double *v) {
+    extern __shared__ double vs[];
+    pdl_begin();
+    pdl_trigger();
+    for (int j = threadIdx.x; j < m; j += blockDim.x) vs[j] = v[j];
+    __syncthreads();
+    const i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= rows) return;
+    double a0 = 0.0, a1 = 0.0;
+    const double *q = Q + r * m;
+    int j = 0;
+    for (; j + 3 < m; j += 4) {
+        const double q0 = q[j], q1 = q[j + 1], q2 = q[j + 2], q3 = q[j + 3];
+        a0 = fma(q0, vs[j], a0);
+        a1 = fma(q1, vs[j + 1], a1);
+        a0 = fma(q2, vs[j + 2], a0);
+        a1 = fma(q3, vs[j + 3], a1);
+    }
+    for (; j < m; ++j) a0 = fma(q[j], vs[j], a0);
+    a0 += a1;
+    if (ADD_G) a0 += g[r];
+    xi[r] += a0;
 }
 
 // xi_i ~ N(0, 1): Philox (counter: vertex group i / 4, purpose
-// PURPOSE_CHOLESKY, the sampler's step counter) or the injected normals
+// PURPOSE_CHOLESKY, the sampler's step counter) or the injected normals, into
+// blocks of ld (zeros behind the p values of a block)
 template <int NOISE>
-__global__ void __launch_bounds__(256) k_cholesky_normals(NoiseArgs nz, i64 n, double *__restrict__ xi) {
-    const i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (NOISE == NOISE_INJECTED) {
-        xi[i] = nz.buf[i];
-    } else {
-        const float4 r = normals4(philox4x32_10(noise_ctr(nz, (unsigned)(i >> 2), PURPOSE_CHOLESKY, 0), noise_key(nz)));
-        xi[i] = (double)pick(r, (int)(i & 3));
+__global__ void __launch_bounds__(256) k_cholesky_normals(NoiseArgs nz, int nb, int p, int ld, double *xi) {
+    const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (int)(t / ld), j = (int)(t - (i64)k * ld);
+    if (k >= nb) return;
+    const i64 i = (i64)k * p + j;
+    double v = 0.0;
+    if (j < p) {
+        if (NOISE == NOISE_INJECTED)
+            v = nz.buf[i];
+        else
+            v = (double)pick(normals4(philox4x32_10(noise_ctr(nz, (unsigned)(i >> 2), PURPOSE_CHOLESKY, 0), noise_key(nz))),
+                             (int)(i & 3));
+    }
+    xi[t] = v;
+}
+
+// compact vectors of nb p values to and from blocks of ld
+__global__ void __launch_bounds__(256) k_chol_pad(const double *__restrict__ src, double *__restrict__ dst, int nb, int p, int ld) {
+    const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (int)(t / ld), j = (int)(t - (i64)k * ld);
+    if (k < nb) dst[t] = j < p ? src[(i64)k * p + j] : 0.0;
+}
+__global__ void __launch_bounds__(256) k_chol_unpad(const double *__restrict__ src, double *__restrict__ dst, int nb, int p, int ld) {
+    const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (int)(t / ld), j = (int)(t - (i64)k * ld);
+    if (k < nb && j < p) dst[(i64)k * p + j] = src[t];
+}
+
+// Set-up: C_k(i, j) = sum_l A_k(i, l) B_k(l, j), p x p each, through strides
+// (A_k(i, l) at k as + i ai + l al, and so on); tiles of 64 x 64, 4 x 4 per
+// thread.
+__global__ void __launch_bounds__(256) k_chol_gemm(const double *__restrict__ A, i64 as, i64 ai, i64 al,
+                                                   const double *__restrict__ B, i64 bs, i64 bl, i64 bj,
+                                                   double *__restrict__ C, i64 cs, i64 ci, int p) {
+    __shared__ double At[16][64 + 1], Bt[16][64 + 1];
+    A += blockIdx.z * as;
+    B += blockIdx.z * bs;
+    C += blockIdx.z * cs;
+    const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double acc[4][4] = {};
+    for (int l0 = 0; l0 < p; l0 += 16) {
+        for (int t = threadIdx.x; t < 16 * 64; t += 256) {
+            // the index with the unit stride runs over the threads
+            const int la = al == 1 ? t & 15 : t >> 6, ia = al == 1 ? t >> 4 : t & 63;
+            At[la][ia] = i0 + ia < p && l0 + la < p ? A[(i0 + ia) * ai + (l0 + la) * al] : 0.0;
+            const int lb = bl == 1 ? t & 15 : t >> 6, jb = bl == 1 ? t >> 4 : t & 63;
+            Bt[lb][jb] = j0 + jb < p && l0 + lb < p ? B[(l0 + lb) * bl + (j0 + jb) * bj] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int l = 0; l < 16; ++l)
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[a][b] = fma(At[l][ty + 16 * a], Bt[l][tx + 16 * b], acc[a][b]);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if (i0 + ty + 16 * a < p && j0 + tx + 16 * b < p) C[(i0 + ty + 16 * a) * ci + j0 + tx + 16 * b] = acc[a][b];
+}
+
+// blocks of p x p values to blocks of p rows of ld, transposed or not
+template <bool TRANSPOSE>
+__global__ void __launch_bounds__(256) k_chol_copy(const double *__restrict__ src, double *__restrict__ dst, int p, int ld) {
+    __shared__ double tile[32][33];
+    src += (i64)blockIdx.z * p * p;
+    dst += (i64)blockIdx.z * p * ld;
+    const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int r = ty; r < 32; r += 8)
+        if (i0 + r < p && j0 + tx < p) tile[r][tx] = src[(i64)(i0 + r) * p + j0 + tx];
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+        if (TRANSPOSE) {
+            if (j0 + r < p && i0 + tx < p) dst[(i64)(j0 + r) * ld + i0 + tx] = tile[tx][r];
+        } else {
+            if (i0 + r < p && j0 + tx < p) dst[(i64)(i0 + r) * ld + j0 + tx] = tile[r][tx];
+        }
     }
 }
 
-__global__ void k_counter_advance(u64 *__restrict__ step) { *step += 1ull; }
+__global__ void k_counter_advance(u64 *step) {
+    pdl_begin();
+    *step += 1ull;
+}
 
 // ------------------------------------------------------- batched chains
 // Chains of one lattice geometry stepped together (FP32-mixed chains with

@@ -789,19 +789,7 @@ bool lowrank_cholesky_factors(const Geometry &g, const double st[27], const Spar
             W[(size_t)a * m + c] = (a == c ? 1.0 : 0.0) - d;
         }
     if (!dense_cholesky(W, m)) return false;
-    F.QW.assign((size_t)(n * m), 0.0);
-    F.QWT.assign((size_t)(n * m), 0.0);
-#pragma omp parallel for schedule(static) if (n > 4096)
-    for (int64_t i = 0; i < n; ++i)
-        for (int c = 0; c < m; ++c) {
-            double u = 0.0, l = 0.0;
-            for (int k = 0; k < m; ++k) {
-                u += F.Q[i * m + k] * (W[(size_t)c * m + k] - (k == c ? 1.0 : 0.0));  // (W^T - Id)[k][c]
-                l += F.Q[i * m + k] * (W[(size_t)k * m + c] - (k == c ? 1.0 : 0.0));  // (W - Id)[k][c]
-            }
-            F.QW[i * m + c] = u;
-            F.QWT[i * m + c] = l;
-        }
+    F.W = std::move(W);
     return true;
 }
 

@@ -107,12 +107,11 @@ std::vector<double> small_inverse(const std::vector<double> &S, int m);
 // D holds the blocks L_kk^{-1} and O the blocks L_{k,k-1} (block 0 zero),
 // row-major p x p each.  With measurements, V = L^{-1} B has the thin QR
 // V = Q R (R with a positive diagonal), W is the lower Cholesky factor of
-// Id - R (Sigma + V^T V)^{-1} R^T, and QW = Q (W^T - Id), QWT = Q (W - Id),
-// n x m row-major.
+// Id - R (Sigma + V^T V)^{-1} R^T (Q: n x m, W: m x m, row-major).
 struct LowRankCholeskyFactors {
     int nb = 0, m = 0;
     int64_t p = 0;
-    std::vector<double> D, O, Q, QW, QWT;
+    std::vector<double> D, O, Q, W;
 };
 // false if A_0 or Id - Lambda is not positive definite
 bool lowrank_cholesky_factors(const Geometry &g, const double st[27], const SparseCols &B,
