@@ -718,32 +718,33 @@ static void launch_resid_restrict_sym(Sampler &S, const Level &lv, const Level &
 template <typename T>
 static void launch_resid_restrict(Sampler &S, int lev, const void *x, const void *f, void *fc, void *xc, bool zero_stencil) {
     Level &lv = S.L[lev], &lc = S.L[lev + 1];
-    StencilArg<T> s = stencil_arg<T>(lv, S.P.omega);
-    if (zero_stencil)
-        for (int k = 0; k < 27; ++k) s.w[k] = T(0);
-    const i64 nc = lc.geo.n;
-    if (lv.var && !zero_stencil) {  // variable coefficients: the plain fused kernel
-        const VarField<T> vf = var_field<T>(lv);
-        const bool pdl = S.pdl && lv.g.pdl;
-        if (lv.npt == 7 && lv.var == 1)
-            plaunch(pdl, k_resid_restrict<T, 7, 1>, nblk(nc, 256), 256, 0, S.stream, (const T *)x, (const T *)f, (T *)fc, (T *)xc,
-                    lv.g, lc.g, s, S.dim, vf);
-        else if (lv.var == 1)
-            plaunch(pdl, k_resid_restrict<T, 27, 1>, nblk(nc, 256), 256, 0, S.stream, (const T *)x, (const T *)f, (T *)fc, (T *)xc,
-                    lv.g, lc.g, s, S.dim, vf);
-        else
-            plaunch(pdl, k_resid_restrict<T, 27, 2>, nblk(nc, 256), 256, 0, S.stream, (const T *)x, (const T *)f, (T *)fc, (T *)xc,
-                    lv.g, lc.g, s, S.dim, vf);
+    const StencilArg<T> s = stencil_arg<T>(lv, S.P.omega);
+    auto plain = [&](auto kernel) {  // k_resid_restrict
+        const dim3 grid((lc.g.N0 + RRS_TX - 1) / RRS_TX, S.dim > 1 ? lc.g.N1 : 1, S.dim > 2 ? lc.g.N2 : 1);
+        plaunch(S.pdl && lv.g.pdl, kernel, grid, RRS_THREADS, 0, S.stream, (const T *)x, (const T *)f, (T *)fc, (T *)xc, lv.g,
+                lc.g, s, S.dim, var_field<T>(lv));
         S.launches++;
+    };
+    if (zero_stencil) {
+        plain(k_resid_restrict<T, 7, 0, true>);
+        return;
+    }
+    if (lv.var) {  // variable coefficients
+        if (lv.npt == 7 && lv.var == 1)
+            plain(k_resid_restrict<T, 7, 1, false>);
+        else if (lv.var == 1)
+            S.dim == 2 ? plain(k_resid_restrict<T, 9, 1, false>) : plain(k_resid_restrict<T, 27, 1, false>);
+        else
+            S.dim == 2 ? plain(k_resid_restrict<T, 9, 2, false>) : plain(k_resid_restrict<T, 27, 2, false>);
         return;
     }
     if constexpr (std::is_same<T, double>::value) {
-        if (lv.sym && S.dim > 1 && !zero_stencil) {
+        if (lv.sym && S.dim > 1) {
             launch_resid_restrict_sym(S, lv, lc, (const double *)x, (const double *)f, (double *)fc, (double *)xc, s);
             return;
         }
     }
-    if (S.dim == 3 && !zero_stencil && lv.tma && x == lv.x && f == lv.f) {
+    if (S.dim == 3 && lv.tma && x == lv.x && f == lv.f) {
         dim3 grid((lc.g.N0 + RR_TX - 1) / RR_TX, (lc.g.N1 + RR_TY - 1) / RR_TY, (lc.g.N2 + RR_TZ - 1) / RR_TZ);
         const size_t sm = rr_tma_smem_bytes<T>();
         if (lv.npt == 7)
@@ -755,7 +756,7 @@ static void launch_resid_restrict(Sampler &S, int lev, const void *x, const void
         S.launches++;
         return;
     }
-    if (S.dim == 3 && !zero_stencil) {
+    if (S.dim == 3) {
         dim3 grid((lc.g.N0 + RR_TX - 1) / RR_TX, (lc.g.N1 + RR_TY - 1) / RR_TY, (lc.g.N2 + RR_TZ - 1) / RR_TZ);
         const size_t sm = rr_smem_bytes<T>();
         if (lv.npt == 7)
@@ -765,12 +766,10 @@ static void launch_resid_restrict(Sampler &S, int lev, const void *x, const void
         S.launches++;
         return;
     }
-    const VarField<T> vf0{nullptr, 0};
-    if (lv.npt == 7 && !zero_stencil)
-        plaunch(S.pdl && lv.g.pdl, k_resid_restrict<T, 7, 0>, nblk(nc, 256), 256, 0, S.stream, (const T *)x, (const T *)f, (T *)fc, (T *)xc, lv.g, lc.g, s, S.dim, vf0);
+    if (lv.npt == 7)
+        plain(k_resid_restrict<T, 7, 0, false>);
     else
-        plaunch(S.pdl && lv.g.pdl, k_resid_restrict<T, 27, 0>, nblk(nc, 256), 256, 0, S.stream, (const T *)x, (const T *)f, (T *)fc, (T *)xc, lv.g, lc.g, s, S.dim, vf0);
-    S.launches++;
+        S.dim == 2 ? plain(k_resid_restrict<T, 9, 0, false>) : plain(k_resid_restrict<T, 27, 0, false>);
 }
 
 // y = B^T x on the level (into the level's y unless `y` is given)

@@ -228,7 +228,7 @@ __device__ __forceinline__ T stencil_row_acc(const XA &xa, const StencilArg<T> &
 }
 
 template <typename T, int NPT, bool EXACT, int VAR = 0>
-__device__ __forceinline__ T stencil_row(const T *__restrict__ x, const Grid3 &g, const StencilArg<T> &s, i64 P,
+__device__ __forceinline__ T stencil_row(const T *x, const Grid3 &g, const StencilArg<T> &s, i64 P,
                                          const VarField<T> &vf = VarField<T>{nullptr, 0}) {
     return stencil_row_acc<T, NPT, EXACT, VAR>(
         [&](int dz, int dy, int dx) { return x[P + dz * g.sz + dy * g.sy + dx]; }, s, P, vf);
@@ -1634,43 +1634,47 @@ __global__ void __launch_bounds__(256)
 // r(a) = prod {1/2, 1, 1/2}: IntergridOperator::restrict
 // (intergrid_operator.hh:74-88) of the residual f - A_0 x
 // (multigridmc_sampler.cc:124-126), with the stencil part of A.
-template <typename T, int NPT, int VAR = 0>
-__global__ void __launch_bounds__(256) k_resid_restrict(const T *__restrict__ x, const T *__restrict__ f,
-                                                         T *__restrict__ fc, T *__restrict__ xc, Grid3 gf, Grid3 gc, StencilArg<T> s,
-                                                         int dim, VarField<T> vf) {
+//
+// One coarse row segment of RRS_TX points per CTA: a thread forms one residual
+// of its 33 x 3 x 3 fine footprint (33 x 3 in 2D), then one thread per coarse
+// point adds its taps in ascending order.  Rows of residuals are shared by
+// neighbouring CTAs' footprints, that is formed 9/4 times, but a level has
+// enough CTAs: one thread per coarse point, which formed its 27 residuals one
+// after the other, left all but a few SMs idle on the coarse levels (27-point
+// fields, FP32: 77 us for 15^3 coarse points, 73 for 7^3 under ncu).  ZERO:
+// the restriction of f alone.
+constexpr int RRS_TX = 16, RRS_FW = 2 * RRS_TX + 1, RRS_THREADS = 320;  // >= 33 * 9
+
+template <typename T, int NPT, int VAR, bool ZERO>
+__global__ void __launch_bounds__(RRS_THREADS) k_resid_restrict(const T *x, const T *f, T *fc, T *xc, Grid3 gf, Grid3 gc,
+                                                                StencilArg<T> s, int dim, VarField<T> vf) {
     if (gf.pdl) pdl_begin();
-    i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    i64 nc = (i64)gc.N0 * gc.N1 * gc.N2;
-    if (t >= nc) return;
-    int a = (int)(t % gc.N0), b = (int)((t / gc.N0) % gc.N1), c = (int)(t / ((i64)gc.N0 * gc.N1));
-    // fine 0-based coordinates of the centre 2 (a+1) - 1
-    int fa = 2 * a + 1, fb = dim > 1 ? 2 * b + 1 : 0, fc_ = dim > 2 ? 2 * c + 1 : 0;
-    const int zlo = dim > 2 ? -1 : 0, ylo = dim > 1 ? -1 : 0;
+    __shared__ T res[9 * RRS_FW];
+    const int ca0 = blockIdx.x * RRS_TX, cb = blockIdx.y, cc = blockIdx.z;
+    const int nr = dim > 2 ? 9 : dim > 1 ? 3 : 1;  // rows of the footprint
+    const int row = threadIdx.x / RRS_FW, la = threadIdx.x - row * RRS_FW;
+    if (row < nr) {
+        const int a = 2 * ca0 + la, b = dim > 1 ? 2 * cb + row % 3 : 0, c = dim > 2 ? 2 * cc + row / 3 : 0;
+        T v = T(0);
+        if (a < gf.N0) {
+            const i64 P = gf.pad(a, b, c);
+            v = ZERO ? f[P] : f[P] - stencil_row<T, NPT, false, VAR>(x, gf, s, P, vf);
+        }
+        res[threadIdx.x] = v;
+    }
+    __syncthreads();
+    const int ca = ca0 + (int)threadIdx.x;
+    if (threadIdx.x >= RRS_TX || ca >= gc.N0) return;
     T acc = T(0);
-    for (int az = zlo; az <= -zlo; ++az)
-        for (int ay = ylo; ay <= -ylo; ++ay)
-            for (int ax = -1; ax <= 1; ++ax) {
-                T wr = T((ax ? 0.5 : 1.0) * (ay ? 0.5 : 1.0) * (az ? 0.5 : 1.0));
-                i64 P = gf.pad(fa + ax, fb + ay, fc_ + az);
-                T res = T(0);
-                if (VAR) {
-                    res = stencil_row<T, NPT, false, VAR>(x, gf, s, P, vf);
-                } else if (NPT == 7) {
-                    res = s.w[4] * x[P - gf.sz] + s.w[10] * x[P - gf.sy] + s.w[12] * x[P - 1] + s.w[13] * x[P] +
-                          s.w[14] * x[P + 1] + s.w[16] * x[P + gf.sy] + s.w[22] * x[P + gf.sz];
-                } else {
+    for (int r = 0; r < nr; ++r)
 #pragma unroll
-                    for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-                        for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-                            for (int dx = -1; dx <= 1; ++dx)
-                                res += s.w[(dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)] * x[P + dz * gf.sz + dy * gf.sy + dx];
-                }
-                acc += wr * (f[P] - res);
-            }
-    fc[gc.pad(a, b, c)] = acc;
-    if (xc) xc[gc.pad(a, b, c)] = T(0);  // the coarse sample starts from zero
+        for (int ax = 0; ax < 3; ++ax) {
+            const T wr = T((ax == 1 ? 1.0 : 0.5) * (dim > 1 && r % 3 != 1 ? 0.5 : 1.0) * (dim > 2 && r / 3 != 1 ? 0.5 : 1.0));
+            acc += wr * res[r * RRS_FW + 2 * threadIdx.x + ax];
+        }
+    const i64 Pc = gc.pad(ca, dim > 1 ? cb : 0, dim > 2 ? cc : 0);
+    fc[Pc] = acc;
+    if (xc) xc[Pc] = T(0);  // the coarse sample starts from zero
 }
 
 // 3D-tiled variant: a CTA owns RR_TX x RR_TY x RR_TZ coarse points.  It
