@@ -114,6 +114,7 @@ struct Level {
     bool sym = false;
     double wc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     void *adj[4] = {nullptr, nullptr, nullptr, nullptr};  // adjoint: x-bar, f-bar, two work vectors (T, padded)
+    bool adj_clear = false;  // adj[2] is zero at this point of the adjoint being issued
     CUtensorMap xmap{}, fmap{};  // 3D tile maps of x and f for the residual-restriction
     bool tma = false;            // maps valid (3D, rows of a multiple of 16 bytes)
     // variable coefficients: 0 the constant stencil st; 1 a per-point centre
@@ -230,7 +231,6 @@ struct Sampler {
     void build(const mgmc_operator_desc &op);
     void build_lowrank(int lev);
     void make_tile_maps(Level &lv);
-    double *adj_m = nullptr;  // m-vector for the adjoint's transposed low-rank solve
     void ensure_adjoint();
     // parameter adjoint: a replay of one step records the input and output
     // state of every sweep, the state entering each residual and every
@@ -253,7 +253,7 @@ struct Sampler {
     double *pa_gs = nullptr, *pa_gsig = nullptr;  // gradient accumulators
     double *pa_part = nullptr;
     int pa_part_cap = 0;
-    double *pa_Bu = nullptr, *pa_Bv = nullptr, *pa_xi = nullptr, *pa_xic = nullptr, *pa_U = nullptr;
+    double *pa_xic = nullptr, *pa_U = nullptr;
     void *pa_phi = nullptr, *pa_cv = nullptr, *pa_mu = nullptr;
     // with Philox noise every launch of the replay and the reverse pass has
     // the same arguments at every call (the tape's buffers are reused, the
@@ -621,8 +621,9 @@ static size_t lr_correct_smem(int m) {
 }
 
 template <typename T>
-static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, const NoiseArgs &nz) {
-    LowRankArg lr;
+static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, const NoiseArgs &nz, double *zpub = nullptr) {
+    LowRankArg lr{};
+    lr.zpub = zpub;
     lr.m = S.m;
     lr.Bptr = lv.Bptr;
     lr.Bidx = lv.Bidx;
@@ -1062,6 +1063,7 @@ void Sampler::build_lowrank(int lev) {
     }
     lv.y = alloc<double>(m);
     lv.z = alloc<double>(m);
+    CK(cudaMemsetAsync(lv.z, 0, m * sizeof(double), stream));
     lv.zf = alloc<float>(m);
     lv.w = alloc<double>(m);
     {
@@ -1215,8 +1217,8 @@ void Sampler::build_lowrank(int lev) {
                         if (jb.nc + fresh > max_cols) break;
                         for (const int *c = first(r); c != last(r); ++c)
                             if (mark[*c] != (int)jobs.size()) {
+                                jcols.push_back(*c | (mark[*c] < 0 ? CORR_OWNER : 0));
                                 mark[*c] = (int)jobs.size();
-                                jcols.push_back(*c);
                                 jb.nc++;
                             }
                         ++r;
@@ -1888,16 +1890,15 @@ struct BorrowLevel0 {
 // x <- x + M_d^{-1}(c - A_0 x), M_d = D / omega + (A_0's part before the
 // point in the sweep order), and for symmetric A_0, M_d^T is the splitting
 // of the opposite direction, so M_d^{-T} v is a noise-free sweep of the
-// opposite direction from x = 0 with right hand side v.  The low-rank
-// correction x <- (I - C S^{-1} B^T) x (C = M_d^{-1} B) has transpose
-// I - B S^{-T} B^T M_d^{-T}; R = P^T; the coarse Cholesky sample
+// opposite direction from x = 0 with right hand side v; with the low-rank
+// term, M_f^{-T} v (M_f = M_d + B Sigma^{-1} B^T) is that sweep with its own
+// correction (adjoint_sor).  R = P^T; the coarse Cholesky sample
 // L^{-T}(xi + L^{-1} f) has the symmetric linear part Q_c^{-1}.  No
 // counterpart in the reference.
 void Sampler::ensure_adjoint() {
     for (auto &lv : L)
         for (int k = 0; k < 4; ++k)
             if (!lv.adj[k]) lv.adj[k] = talloc(lv.geo.nalloc);
-    if (!adj_m) adj_m = alloc<double>((size_t)std::max(m, 1));
 }
 
 template <typename T>
@@ -1925,38 +1926,50 @@ static void launch_apply_stencil(Sampler &S, const Level &lv, const void *x, voi
         plaunch(false, k_apply_stencil<T, 0>, nb, 256, 0, S.stream, (const T *)x, (T *)y, lv.g, s, vf);
 }
 
-// out = M^{-T} v for the sweep of direction `forward` on level lev
+// a -= A_0 u, b += u, zero = 0 on a level
 template <typename T>
-static void adj_msolve(Sampler &S, int lev, bool forward, const void *v, void *out) {
-    Level &lv = S.L[lev];
-    adj_zero<T>(S, lv, out);
-    NoiseArgs nz{};
-    nz.d_step = S.d_step;
-    launch_sweep(S, lv, !forward, NOISE_NONE, out, v, nz, S.fp32, false);
+static void launch_adj_update(Sampler &S, const Level &lv, const void *u, void *a, void *b, void *zero) {
+    int tx = 8;
+    while (tx < lv.g.N0 && tx < 128) tx *= 2;
+    const dim3 blk(tx, 256 / tx), grid((lv.g.N0 + tx - 1) / tx, (lv.g.N1 + blk.y - 1) / blk.y, lv.g.N2);
+    const StencilArg<T> s = stencil_arg<T>(lv, S.P.omega);
+    const VarField<T> vf = var_field<T>(lv);
+    auto go = [&](auto kernel) {
+        plaunch(S.pdl && lv.g.pdl, kernel, grid, blk, 0, S.stream, (const T *)u, (T *)a, (T *)b, (T *)zero, lv.g, s, vf);
+    };
+    if (lv.var == 2)
+        S.dim == 2 ? go(k_adj_update<T, 9, 2>) : go(k_adj_update<T, 27, 2>);
+    else if (lv.npt == 7)
+        lv.var ? go(k_adj_update<T, 7, 1>) : go(k_adj_update<T, 7, 0>);
+    else if (S.dim == 2)
+        lv.var ? go(k_adj_update<T, 9, 1>) : go(k_adj_update<T, 9, 0>);
+    else
+        lv.var ? go(k_adj_update<T, 27, 1>) : go(k_adj_update<T, 27, 0>);
 }
 
-template <typename T>
-static void adj_apply_a0(Sampler &S, Level &lv, const void *x, void *y) {
-    launch_apply_stencil<T>(S, lv, x, y);
-}
-
-// adjoint of one SOR sweep of direction `forward` with its low-rank
-// correction: a = x-bar (in/out), b = f-bar (accumulated)
+// The adjoint of one SOR sweep of direction `forward` with its low-rank
+// correction, x'' = x + M_f^{-1}(c - A x), M_f = M + B Sigma^{-1} B^T:
+// u = M_f^{-T} x-bar is the noise-free sweep of the opposite direction with
+// its correction from x = 0 with right hand side x-bar (for symmetric A_0,
+// M^T is the splitting of the opposite direction), f-bar += u and
+// x-bar -= A u = A_0 u - B z, z the correction's coefficients
+// (Sigma^{-1} B^T u = -z).  a = x-bar (in/out), b = f-bar (accumulated).
 template <typename T>
 static void adjoint_sor(Sampler &S, int lev, bool forward) {
     Level &lv = S.L[lev];
-    void *a = lv.adj[0], *b = lv.adj[1], *w = lv.adj[2], *u = lv.adj[3];
-    if (S.m > 0) {
-        adj_msolve<T>(S, lev, forward, a, w);  // w = M^{-T} a
-        launch_bt_plain<T>(S, lv, w);          // y = B^T w
-        k_sinvt_q<<<(S.m + 255) / 256, 256, 0, S.stream>>>(lv.SinvT[forward ? 0 : 1], lv.y, S.d_sigma_sqrt, S.adj_m, S.m);
-        launch_add_Bq<T>(S, lv, a, S.adj_m, -1.0);  // a -= B S^{-T} y
-    }
-    adj_msolve<T>(S, lev, forward, a, u);  // u = M^{-T} a
+    T *a = (T *)lv.adj[0], *b = (T *)lv.adj[1], *u = (T *)lv.adj[2], *next = (T *)lv.adj[3];
+    if (!lv.adj_clear) adj_zero<T>(S, lv, u);
+    NoiseArgs nz{};
+    nz.d_step = S.d_step;
+    launch_sweep(S, lv, !forward, NOISE_NONE, u, a, nz, S.fp32, false);
+    if (S.m > 0) launch_lowrank<T>(S, lv, forward ? 1 : 0, NOISE_NONE, u, nz, lv.z);
     if (S.param_adj) S.pgrad_sweep<T>(S.tape_pop(Sampler::EV_SWEEP, lev, forward), u);
-    adj_axpy<T>(S, lv, b, u, 1.0);        // f-bar += u
-    adj_apply_a0<T>(S, lv, u, w);
-    adj_axpy<T>(S, lv, a, w, -1.0);       // a -= A_0 u
+    launch_adj_update<T>(S, lv, u, a, b, next);
+    if (S.m > 0 && lv.Br.nrows > 0)
+        plaunch(S.pdl, k_add_Bz<T>, nblk(lv.Br.nrows, 256), 256, 0, S.stream, a, lv.Br.nrows, (const i64 *)lv.Br.rows,
+                (const i64 *)lv.Br.ptr, (const int *)lv.Br.col, (const double *)lv.Br.val, (const double *)lv.z);
+    std::swap(lv.adj[2], lv.adj[3]);
+    lv.adj_clear = true;
 }
 
 // MultigridMCSampler::sample in reverse: on entry L[lev].adj[0] is the
@@ -1977,6 +1990,7 @@ void Sampler::adjoint_sample(int lev) {
             adj_zero<T>(*this, lv, lv.adj[2]);
             plaunch(false, k_chol_gemv_upper<T, T>, blocks, 256, chol_smem, stream, (const T *)dgv, lv.g, (const T *)dLinvT,
                     chol_ld, (T *)lv.adj[2]);
+            lv.adj_clear = false;
             if (param_adj) pgrad_coarse<T>(tape_pop(EV_COARSE, lev, true));
             adj_axpy<T>(*this, lv, lv.adj[1], lv.adj[2], 1.0);
         } else {
@@ -2003,24 +2017,25 @@ void Sampler::adjoint_sample(int lev) {
                 adjoint_sor<T>(*this, lev, false);
             }
         }
-        // x += alpha P x_c  ->  x_c-bar = alpha R x-bar
-        launch_resid_restrict<T>(*this, lev, lv.adj[0], lv.adj[0], lc.adj[2], nullptr, true);
-        adj_zero<T>(*this, lc, lc.adj[0]);
-        adj_axpy<T>(*this, lc, lc.adj[0], lc.adj[2], P.coarse_scaling);
-        adj_zero<T>(*this, lc, lc.adj[1]);
+        // x += alpha P x_c  ->  x_c-bar = alpha R x-bar; f_c-bar = 0
+        const bool scaled = P.coarse_scaling != 1.0;
+        launch_resid_restrict<T>(*this, lev, lv.adj[0], lv.adj[0], scaled ? lc.adj[2] : lc.adj[0], lc.adj[1], true);
+        if (scaled) {
+            adj_zero<T>(*this, lc, lc.adj[0]);
+            adj_axpy<T>(*this, lc, lc.adj[0], lc.adj[2], P.coarse_scaling);
+            lc.adj_clear = false;
+        }
         adjoint_sample<T>(lev + 1);
         // f_c = R (f - A x)  ->  t = P f_c-bar; f-bar += t; x-bar -= A t
-        void *t = lv.adj[2], *u = lv.adj[3];
-        adj_zero<T>(*this, lv, t);
+        T *t = (T *)lv.adj[2];
+        if (!lv.adj_clear) adj_zero<T>(*this, lv, t);
         prolong(lev, 1.0, lc.adj[1], t);
+        if (m > 0) launch_bt_plain<T>(*this, lv, t);
         if (param_adj) pgrad_minus_udav<T>(lev, t, tape_pop(EV_RESID, lev, true).xin);
-        adj_axpy<T>(*this, lv, lv.adj[1], t, 1.0);
-        adj_apply_a0<T>(*this, lv, t, u);
-        if (m > 0) {
-            launch_bt_plain<T>(*this, lv, t);
-            launch_add_Bq<T>(*this, lv, u, lv.y, 1.0);
-        }
-        adj_axpy<T>(*this, lv, lv.adj[0], u, -1.0);
+        launch_adj_update<T>(*this, lv, t, lv.adj[0], lv.adj[1], lv.adj[3]);
+        if (m > 0) launch_add_Bq<T>(*this, lv, lv.adj[0], lv.y, -1.0);
+        std::swap(lv.adj[2], lv.adj[3]);
+        lv.adj_clear = true;
         for (int k = P.npresmooth - 1; k >= 0; --k) {
             if (ssor) {
                 adjoint_sor<T>(*this, lev, false);
@@ -2074,12 +2089,8 @@ void Sampler::ensure_param_adjoint() {
     tape_last.assign(nl, nullptr);
     tape_f.assign(nl, nullptr);
     const i64 np0 = ((i64)L[0].g.N1 * L[0].g.N2 + SOLVE_ROWS - 1) / SOLVE_ROWS;
-    i64 cap = 8 * np0;
+    i64 cap = std::min<i64>(np0 * SOLVE_ROWS, 8 * (i64)nsm);
     const int mm = std::max(m, 1);
-    pa_Bu = alloc<double>(mm);
-    pa_Bv = alloc<double>(mm);
-    pa_xi = alloc<double>(mm);
-    for (double *p : {pa_Bu, pa_Bv, pa_xi}) CK(cudaMemsetAsync(p, 0, mm * sizeof(double), stream));
     if (chol) {
         Level &lv = L.back();
         const i64 n = lv.geo.n, ld = chol_ld;
@@ -2115,76 +2126,77 @@ void Sampler::ensure_param_adjoint() {
     CK(cudaStreamSynchronize(stream));
 }
 
-static PgradStencils pgrad_stencils(const Level &lv, const std::array<double, 27> &E) {
-    PgradStencils st;
-    for (int k = 0; k < 27; ++k) {
-        st.a[k] = lv.st[k];
-        st.e[k] = E[k];
-        st.af[k] = (float)lv.st[k];
-        st.ef[k] = (float)E[k];
-    }
-    return st;
-}
-
+// partial sums of an event's stencil term; returns their number
 template <typename T>
-static void launch_pgrad_stencil(Sampler &S, const Level &lv, const std::array<double, 27> &E, const void *u,
-                                 const void *v, const void *w, const void *f, int ncol, bool forward, int np) {
-    const PgradStencils st = pgrad_stencils(lv, E);
-    bool has_e = false;
-    for (int k = 0; k < 27; ++k) has_e |= (k != 13 && E[k] != 0.0);
-    const T *U = (const T *)u, *V = (const T *)v, *W = (const T *)w, *F = (const T *)f;
-    const int fw = forward ? 1 : 0;
-    if (lv.npt == 7) {
-        if (has_e)
-            k_pgrad_stencil<T, 7, true><<<np, 256, 0, S.stream>>>(U, V, W, F, lv.g, st, ncol, fw, S.pa_part);
-        else
-            k_pgrad_stencil<T, 7, false><<<np, 256, 0, S.stream>>>(U, V, W, F, lv.g, st, ncol, fw, S.pa_part);
-    } else {
-        if (has_e)
-            k_pgrad_stencil<T, 27, true><<<np, 256, 0, S.stream>>>(U, V, W, F, lv.g, st, ncol, fw, S.pa_part);
-        else
-            k_pgrad_stencil<T, 27, false><<<np, 256, 0, S.stream>>>(U, V, W, F, lv.g, st, ncol, fw, S.pa_part);
-    }
+static int launch_pgrad_stencil(Sampler &S, const Level &lv, const PgradWeights<T> &pw, const void *u, const void *v,
+                                const void *w, const void *f, int ncol, bool forward) {
+    int tx = 8;
+    while (tx < lv.g.N0 && tx < 256) tx *= 2;
+    const dim3 blk(tx, 256 / tx);
+    const int np = (int)std::min<i64>(((i64)lv.g.N1 * lv.g.N2 + blk.y - 1) / blk.y, S.pa_part_cap);
+    auto go = [&](auto kernel) {
+        kernel<<<np, blk, 0, S.stream>>>((const T *)u, (const T *)v, (const T *)w, (const T *)f, lv.g, pw, ncol,
+                                         forward ? 1 : 0, S.pa_part);
+    };
+    if (lv.npt == 7)
+        go(k_pgrad_stencil<T, 7>);
+    else
+        S.dim == 2 ? go(k_pgrad_stencil<T, 9>) : go(k_pgrad_stencil<T, 27>);
+    return np;
 }
 
-// One sweep's contribution: u = M_f^{-T} x-bar'' of the sweep, its input
-// and output states and right hand side from the tape.
+// B^T v for k_pgrad_combine: partial sums into the level's part
+template <typename T>
+static void launch_pgrad_bv(Sampler &S, Level &lv, const void *v) {
+    LowRankArg lr{};
+    lr.m = S.m;
+    lr.Bptr = lv.Bptr;
+    lr.Bidx = lv.Bidx;
+    lr.Bval = lv.Bval;
+    lr.Bvalf = lv.Bvalf;
+    lr.part = lv.part;
+    plaunch(S.pdl, k_bt_partial<T, NOISE_NONE>, dim3(S.m, lv.bt_split), 256, 0, S.stream, (const T *)v, lr, NoiseArgs{});
+}
+
+// One sweep's contribution: u = M_f^{-T} x-bar'' of the sweep (its low-rank
+// coefficients in the level's z), its input and output states and right hand
+// side from the tape.
 template <typename T>
 void Sampler::pgrad_sweep(const TapeEvent &ev, const void *u) {
     Level &lv = L[ev.lev];
     const int ncol = P.ordering == MGMC_ORDER_LEXICOGRAPHIC ? 0 : lv.ncol;
-    const int np = (int)(((i64)lv.g.N1 * lv.g.N2 + SOLVE_ROWS - 1) / SOLVE_ROWS);
-    launch_pgrad_stencil<T>(*this, lv, pa_E[ev.lev], u, ev.xout, ev.xin, ev.f, ncol, ev.forward, np);
-    if (m > 0) {
-        launch_bt_plain<T>(*this, lv, u, pa_Bu);
-        launch_bt_plain<T>(*this, lv, ev.xout, pa_Bv);
-        if (noise_mode == NOISE_PHILOX)
-            k_lowrank_normals<NOISE_PHILOX><<<nblk(m, 256), 256, 0, stream>>>(ev.nzl, m, pa_xi);
-        else
-            k_lowrank_normals<NOISE_INJECTED><<<nblk(m, 256), 256, 0, stream>>>(ev.nzl, m, pa_xi);
-    }
-    const double ac = lv.diag, ec = pa_E[ev.lev][13];
-    const PgradCoef cf{ec / (2.0 * ac), P.omega, ac, ec, 0};
-    k_pgrad_combine<<<1, 256, 0, stream>>>(pa_part, np, pa_Bu, pa_Bv, pa_xi, d_sigma_inv, d_sigma_sqrt, m, cf, pa_gs,
-                                           pa_gsig);
+    const std::array<double, 27> &E = pa_E[ev.lev];
+    const double ac = lv.diag, ec = E[13], kd = ec / (2.0 * ac), io = 1.0 / P.omega;
+    PgradWeights<T> pw;
+    for (int k = 0; k < 27; ++k) pw.c[k] = (T)(kd * lv.st[k] - E[k]);
+    pw.cv = (kd * ac - ec) * io;
+    pw.cw = (kd * ac - ec) * (1.0 - io);
+    pw.cf = -kd;
+    const int np = launch_pgrad_stencil<T>(*this, lv, pw, u, ev.xout, ev.xin, ev.f, ncol, ev.forward);
+    if (m > 0) launch_pgrad_bv<T>(*this, lv, ev.xout);
+    auto combine = [&](auto kernel) {
+        kernel<<<1, 256, 0, stream>>>(pa_part, np, lv.z, 1, lv.part, lv.bt_split, ev.nzl, d_sigma_inv, d_sigma_sqrt, m, kd,
+                                      pa_gs, pa_gsig);
+    };
+    noise_mode == NOISE_PHILOX ? combine(k_pgrad_combine<T, NOISE_PHILOX>) : combine(k_pgrad_combine<T, NOISE_INJECTED>);
     check_launch();
 }
 
 // -u^T dA v on level lev: the residual f - A x (u = P f_c-bar, v = the
 // state entering the residual) and the coarse mean Q^{-1} f (u = Q^{-1}
-// x-bar, v = Q^{-1} f).
+// x-bar, v = Q^{-1} f); the level's y holds B^T u.
 template <typename T>
 void Sampler::pgrad_minus_udav(int lev, const void *u, const void *v) {
     Level &lv = L[lev];
-    const int np = (int)(((i64)lv.g.N1 * lv.g.N2 + SOLVE_ROWS - 1) / SOLVE_ROWS);
-    launch_pgrad_stencil<T>(*this, lv, pa_E[lev], u, v, v, v, 0, true, np);
-    if (m > 0) {
-        launch_bt_plain<T>(*this, lv, u, pa_Bu);
-        launch_bt_plain<T>(*this, lv, v, pa_Bv);
-    }
-    const PgradCoef cf{0.0, P.omega, lv.diag, pa_E[lev][13], 1};
-    k_pgrad_combine<<<1, 256, 0, stream>>>(pa_part, np, pa_Bu, pa_Bv, pa_xi, d_sigma_inv, d_sigma_sqrt, m, cf, pa_gs,
-                                           pa_gsig);
+    const std::array<double, 27> &E = pa_E[lev];
+    PgradWeights<T> pw;
+    for (int k = 0; k < 27; ++k) pw.c[k] = (T)-E[k];
+    pw.cv = pw.cf = 0.0;
+    pw.cw = -E[13];
+    const int np = launch_pgrad_stencil<T>(*this, lv, pw, u, v, v, v, 0, true);
+    if (m > 0) launch_pgrad_bv<T>(*this, lv, v);
+    k_pgrad_combine<T, NOISE_NONE><<<1, 256, 0, stream>>>(pa_part, np, lv.y, 0, lv.part, lv.bt_split, NoiseArgs{}, d_sigma_inv,
+                                                          d_sigma_sqrt, m, 0.0, pa_gs, pa_gsig);
     check_launch();
 }
 
@@ -2210,6 +2222,7 @@ void Sampler::pgrad_coarse(const TapeEvent &ev) {
             (const MT *)dLinv, chol_ld, (MT *)pa_cv, nz);
     plaunch(false, k_chol_gemv_upper<T, MT>, blocks, 256, chol_smem, stream, (const MT *)pa_cv, lv.g, (const MT *)dLinvT,
             chol_ld, (T *)pa_mu);
+    if (m > 0) launch_bt_plain<T>(*this, lv, lv.adj[2]);
     pgrad_minus_udav<T>(ev.lev, lv.adj[2], pa_mu);
 }
 // The replay of one step from level 0's state, recording the tape, and the
@@ -2223,6 +2236,7 @@ void Sampler::param_adjoint_pass() {
     std::fill(tape_last.begin(), tape_last.end(), nullptr);
     std::fill(tape_f.begin(), tape_f.end(), nullptr);
     tape_f[0] = l0.f;
+    for (auto &lv : L) lv.adj_clear = false;
     inv = 0;
     noise_off = noise_pos;
     taping = true;
@@ -3728,6 +3742,7 @@ mgmc_status mgmc_sampler_adjoint_step(mgmc_sampler *s, double *xbar, double *fba
     S.ensure_adjoint();
     Level &l0 = S.L[0];
     put_vec(S, 0, xbar, on_device, l0.adj[0]);
+    for (auto &lv : S.L) lv.adj_clear = false;
     if (S.fp32) {
         adj_zero<float>(S, l0, l0.adj[1]);
         S.adjoint_sample<float>(0);

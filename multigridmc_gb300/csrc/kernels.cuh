@@ -842,6 +842,21 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return v;  // valid in thread 0
 }
 
+// block_sum over the 256 threads of a two-dimensional CTA
+__device__ __forceinline__ double block_sum_2d(double v, double *sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int t = threadIdx.y * blockDim.x + threadIdx.x;
+    if ((t & 31) == 0) sh[t >> 5] = v;
+    __syncthreads();
+    v = t < 8 ? sh[t] : 0.0;
+    if (t < 32) {
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    return v;  // valid in thread 0
+}
+
 // ------------------------------------------------ float-float arithmetic
 // An unevaluated sum hi + lo of two FP32 numbers carries about 48
 // significant bits.  GB300 issues about two FP64 FMAs per clock per SM
@@ -922,6 +937,7 @@ struct LowRankArg {
                         // stores float-float pairs, float2, in the same slots)
     unsigned *counter;  // CTA counter of k_bt_solve (reset by its last CTA)
     void *w;                     // m scratch: Sigma^{1/2} xi' (double, or float2 for the FP32 chain)
+    double *zpub;                // where k_lr_correct leaves z (null: nowhere)
     const float2 *SinvT_ff;      // SinvT as float-float pairs (FP32 chain)
     const float2 *sigma_sqrt_ff; // Sigma^{1/2} as float-float pairs (FP32 chain)
 };
@@ -1403,6 +1419,8 @@ struct CorrJob {
     int multi;       // of the multi-entry rows
     int c0, nc;      // their columns: cols[c0 .. c0 + nc)
 };
+// in the list of columns: the first CTA that has the column
+constexpr int CORR_OWNER = 1 << 30;
 
 template <typename T, int MODE, int NQ>
 __global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
@@ -1439,8 +1457,9 @@ __global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
         for (int i = 0; i < 2; ++i) {
             if (warp + 8 * i >= jb.nc) break;
             kcol[i] = jobcols[jb.c0 + warp + 8 * i];
-            if (lane < m) pv[2 * i] = __ldg(Sinv + lane * m + kcol[i]);
-            if (lane + 32 < m) pv[2 * i + 1] = __ldg(Sinv + (lane + 32) * m + kcol[i]);
+            const int k = kcol[i] & ~CORR_OWNER;
+            if (lane < m) pv[2 * i] = __ldg(Sinv + lane * m + k);
+            if (lane + 32 < m) pv[2 * i + 1] = __ldg(Sinv + (lane + 32) * m + k);
         }
     }
     if (MODE == 1) {
@@ -1498,14 +1517,20 @@ __global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
                 ff32 zk{0.f, 0.f};
                 for (int h = 0; h < groups; ++h)
                     zk = ff_add(zk, ff32{__shfl_sync(0xffffffffu, a.hi, 2 * h), __shfl_sync(0xffffffffu, a.lo, 2 * h)});
-                if (lane == 0) zs[kcol[i]] = ff_to_float(zk);
+                if (lane == 0) {
+                    zs[kcol[i] & ~CORR_OWNER] = ff_to_float(zk);
+                    if (lr.zpub && (kcol[i] & CORR_OWNER)) lr.zpub[kcol[i] & ~CORR_OWNER] = ff_to_double(zk);
+                }
                 __syncwarp();
             } else {
                 double a = lane < m ? pv[2 * i] * u[lane] : 0.0;
                 if (lane + 32 < m) a = fma(pv[2 * i + 1], u[lane + 32], a);
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-                if (lane == 0) zs[kcol[i]] = a;
+                if (lane == 0) {
+                    zs[kcol[i] & ~CORR_OWNER] = a;
+                    if (lr.zpub && (kcol[i] & CORR_OWNER)) lr.zpub[kcol[i] & ~CORR_OWNER] = a;
+                }
             }
         }
         __syncthreads();
@@ -1568,10 +1593,12 @@ __global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
                     ff32 zk{0.f, 0.f};
                     for (int h = 0; h < groups; ++h) zk = ff_add(zk, ff_of(pr[h * cols + tid]));
                     zs[k0 + tid] = ff_to_float(zk);
+                    if (lr.zpub && blockIdx.x == 0) lr.zpub[k0 + tid] = ff_to_double(zk);
                 } else {
                     double zk = 0.0;
                     for (int h = 0; h < groups; ++h) zk += pr[h * cols + tid];
                     zs[k0 + tid] = zk;
+                    if (lr.zpub && blockIdx.x == 0) lr.zpub[k0 + tid] = zk;
                 }
             }
             __syncthreads();
@@ -2331,17 +2358,43 @@ __global__ void __launch_bounds__(256) k_axpy(T *__restrict__ y, const T *__rest
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) y[i] += alpha * x[i];
 }
 
-// out_k = Sigma_k sum_j (S^{-1})_{jk} q_j: the transposed m x m solve of the
-// low-rank correction, scaled by Sigma so that k_add_Bq (which divides by
-// Sigma) applies B S^{-T} q.  One thread per k; SinvT row k is column k of
-// S^{-1}.
-__global__ void __launch_bounds__(256) k_sinvt_q(const double *__restrict__ SinvT, const double *__restrict__ q,
-                                                 const double *__restrict__ sigma_sqrt, double *__restrict__ out, int m) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m) return;
-    double t = 0.0;
-    for (int j = 0; j < m; ++j) t = fma(SinvT[(i64)k * m + j], q[j], t);
-    out[k] = sigma_sqrt[k] * sigma_sqrt[k] * t;
+// a -= A_0 u, b += u (b may be null) and `zero` = 0 (the work vector of the
+// next transposed sweep, may be null) over the interior, in one pass.
+template <typename T, int NPT, int VAR>
+__global__ void __launch_bounds__(256) k_adj_update(const T *u, T *a, T *b, T *zero, Grid3 g, StencilArg<T> s, VarField<T> vf) {
+    if (g.pdl) pdl_begin();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= g.N0 || j >= g.N1) return;
+    const i64 P = g.pad(i, j, blockIdx.z);
+    constexpr int NZ = NPT == 9 ? 1 : 3;
+    T sum[NZ];  // by planes: three sums in flight
+#pragma unroll
+    for (int z = 0; z < NZ; ++z) {
+        const int dz = NZ == 1 ? 0 : z - 1;
+        sum[z] = T(0);
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+            for (int dx = -1; dx <= 1; ++dx) {
+                if (NPT == 7 && (dz != 0) + (dy != 0) + (dx != 0) > 1) continue;
+                sum[z] += vweight<T, VAR>(s, vf, P, (dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * u[P + dz * g.sz + dy * g.sy + dx];
+            }
+    }
+    a[P] -= NZ == 1 ? sum[0] : (sum[0] + sum[NZ - 1]) + sum[NZ / 2];
+    if (b) b[P] += u[P];
+    if (zero) zero[P] = T(0);
+}
+
+// dst[row] += sum_e B_e z_{col_e} over the rows of B
+template <typename T>
+__global__ void __launch_bounds__(256) k_add_Bz(T *dst, i64 nrows, const i64 *__restrict__ rows, const i64 *__restrict__ ptr,
+                                                const int *__restrict__ col, const double *__restrict__ val, const double *z) {
+    pdl_begin();
+    const i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= nrows) return;
+    double acc = 0.0;
+    for (i64 e = ptr[r]; e < ptr[r + 1]; ++e) acc += val[e] * z[col[e]];
+    dst[rows[r]] += (T)acc;
 }
 
 // ------------------------------------------------- deterministic solver
@@ -2475,61 +2528,45 @@ __global__ void __launch_bounds__(256) k_lowrank_perturbation(NoiseArgs nz, cons
 // unit centre weight; the noise part c - f = M x'' + N x + B Sigma^{-1} B^T x''
 // - f is rebuilt from the sweep's input and output states, so the point
 // normals need not be stored.
-struct PgradStencils {
-    double a[27];  // the level's A_0
-    double e[27];  // E_l = dA_0 / ds
-    float af[27], ef[27];  // the same rounded to FP32 (neighbour sums of FP32 chains)
-};
-
-template <typename T>
-__device__ __forceinline__ T pg_a(const PgradStencils &st, int k);
-template <>
-__device__ __forceinline__ float pg_a<float>(const PgradStencils &st, int k) { return st.af[k]; }
-template <>
-__device__ __forceinline__ double pg_a<double>(const PgradStencils &st, int k) { return st.a[k]; }
-template <typename T>
-__device__ __forceinline__ T pg_e(const PgradStencils &st, int k);
-template <>
-__device__ __forceinline__ float pg_e<float>(const PgradStencils &st, int k) { return st.ef[k]; }
-template <>
-__device__ __forceinline__ double pg_e<double>(const PgradStencils &st, int k) { return st.e[k]; }
-
 // Colour of interior point (a, b, c) in the multicolour order (2 colours:
 // parity of a + b + c; 2^dim colours: one parity bit per direction).
 __device__ __forceinline__ int point_colour(int ncol, int a, int b, int c) {
     return ncol == 2 ? ((a + b + c) & 1) : ((a & 1) | ((b & 1) << 1) | ((c & 1) << 2));
 }
 
-// Per CTA of SOLVE_ROWS rows, the eight sums over the level's points p
-// (part[j * gridDim.x + blockIdx.x]):
-//   0: u_p sum_{q before p} A_pq v_q    1: u_p sum_{q after p} A_pq w_q
-//   2: u_p sum_{q before p} E_pq v_q    3: u_p sum_{q before p} E_pq w_q
-//   4: u_p sum_{q after p} E_pq w_q     5: u_p v_p   6: u_p w_p   7: u_p f_p
-// (v = the sweep's output, w = its input; off-diagonal neighbours only, the
-// 6 axis neighbours of a 7-point level or all 26).  "Before" is the order
-// of the sweep of direction `forward`: by linear index for the
-// lexicographic order (ncol = 0), by colour otherwise.  The neighbour sums
-// run in the chain's type T, the u_p-weighted sums in FP64.  Without
-// off-diagonal entries in E (HAS_E false: the fine level's E is the unit
-// centre weight) sums 2 to 4 are zero and skipped.
-template <typename T, int NPT, bool HAS_E>
-__global__ void __launch_bounds__(256) k_pgrad_stencil(const T *__restrict__ u, const T *__restrict__ v,
-                                                       const T *__restrict__ w, const T *__restrict__ f, Grid3 g,
-                                                       PgradStencils st, int ncol, int forward,
-                                                       double *__restrict__ part) {
+// An event's sum over the level's points p, one partial sum per CTA:
+//   sum_p u_p [sum_{q before p} c_pq v_q + sum_{q after p} c_pq w_q
+//              + cv v_p + cw w_p + cf f_p]
+// over the off-diagonal neighbours q (the 6 axis neighbours of a 7-point
+// level, or all), "before" in the order of the sweep of direction `forward`:
+// by linear index for the lexicographic order (ncol = 0), by colour otherwise.
+// A sweep (v = its output, w = its input; kd = dsd/ds / sd = E_c / (2 A_c))
+// has c = kd A - E, cv = kd A_c / omega - E_c / omega,
+// cw = kd A_c (1 - 1/omega) - E_c (1 - 1/omega), cf = -kd; -u^T dA v has
+// v = w, c = -E, cw = -E_c.  The neighbour sums run in the chain's type, the
+// u_p-weighted sum in FP64.  One weight per neighbour instead of one each for
+// the products with A and E (and one sum instead of eight): 30 FP64
+// instructions per point instead of 75, on a unit that takes two per clock.
+template <typename T>
+struct PgradWeights {
+    T c[27];
+    double cv, cw, cf;
+};
+
+template <typename T, int NPT>
+__global__ void __launch_bounds__(256) k_pgrad_stencil(const T *u, const T *v, const T *w, const T *f, Grid3 g,
+                                                       PgradWeights<T> pw, int ncol, int forward, double *part) {
     __shared__ double sh[32];
-    const i64 nrows = (i64)g.N1 * g.N2;
-    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int q = 0; q < SOLVE_ROWS; ++q) {
-        const i64 row = (i64)blockIdx.x * SOLVE_ROWS + q;
-        if (row >= nrows) break;
-        const int bb = (int)(row % g.N1), c = (int)(row / g.N1);
+    const int nrows = g.N1 * g.N2;
+    double acc = 0.0;
+    for (int row = blockIdx.x * blockDim.y + threadIdx.y; row < nrows; row += gridDim.x * blockDim.y) {
+        const int bb = row % g.N1, c = row / g.N1;
         for (int a = threadIdx.x; a < g.N0; a += blockDim.x) {
             const i64 P = g.pad(a, bb, c);
             const T up = u[P];
             if (up == T(0)) continue;
             const int cp = ncol ? point_colour(ncol, a, bb, c) : 0;
-            T lav = 0, uaw = 0, lev = 0, lew = 0, uew = 0;
+            T sum[3] = {T(0), T(0), T(0)};  // by planes
 #pragma unroll
             for (int dz = -1; dz <= 1; ++dz)
 #pragma unroll
@@ -2537,9 +2574,7 @@ __global__ void __launch_bounds__(256) k_pgrad_stencil(const T *__restrict__ u, 
 #pragma unroll
                     for (int dx = -1; dx <= 1; ++dx) {
                         const int nzo = (dx != 0) + (dy != 0) + (dz != 0);
-                        if (nzo == 0 || (NPT == 7 && nzo > 1)) continue;
-                        const int k = (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1);
-                        const T wa = pg_a<T>(st, k), we = pg_e<T>(st, k);
+                        if (nzo == 0 || (NPT == 7 && nzo > 1) || (NPT == 9 && dz != 0)) continue;
                         bool before;
                         if (ncol == 0) {
                             const bool lower = dz < 0 || (dz == 0 && (dy < 0 || (dy == 0 && dx < 0)));
@@ -2548,107 +2583,62 @@ __global__ void __launch_bounds__(256) k_pgrad_stencil(const T *__restrict__ u, 
                             const int cq = point_colour(ncol, a + dx, bb + dy, c + dz);
                             before = forward ? cq < cp : cq > cp;
                         }
-                        const i64 Q = P + dz * g.sz + dy * g.sy + dx;
-                        const T wq = w[Q];
-                        if (before) {
-                            const T vq = v[Q];
-                            lav += wa * vq;
-                            if (HAS_E) {
-                                lev += we * vq;
-                                lew += we * wq;
-                            }
-                        } else {
-                            uaw += wa * wq;
-                            if (HAS_E) uew += we * wq;
-                        }
+                        sum[dz + 1] += pw.c[(dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)] *
+                                       (before ? v : w)[P + dz * g.sz + dy * g.sy + dx];
                     }
-            const double ud = (double)up;
-            acc[0] += ud * (double)lav;
-            acc[1] += ud * (double)uaw;
-            if (HAS_E) {
-                acc[2] += ud * (double)lev;
-                acc[3] += ud * (double)lew;
-                acc[4] += ud * (double)uew;
-            }
-            acc[5] += ud * (double)v[P];
-            acc[6] += ud * (double)w[P];
-            acc[7] += ud * (double)f[P];
+            const double own = fma(pw.cv, (double)v[P], fma(pw.cw, (double)w[P], pw.cf * (double)f[P]));
+            acc = fma((double)up, (double)((sum[0] + sum[2]) + sum[1]) + own, acc);
         }
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const double t = block_sum<256>(acc[j], sh);
-        if (threadIdx.x == 0) part[(i64)j * gridDim.x + blockIdx.x] = t;
-        __syncthreads();
-    }
+    acc = block_sum_2d(acc, sh);
+    if (threadIdx.x == 0 && threadIdx.y == 0) part[blockIdx.x] = acc;
 }
 
-// Adds one event's contribution to the gradients (one CTA).  Sums the eight
-// partial streams of k_pgrad_stencil (np values each) into S0..S7 and, with Bu = B^T u,
-// Bv = B^T v and the low-rank normals xi' of the sweep:
-// sweep (mode 0), kd = dsd/ds / sd = E_c / (2 A_c):
-//   g_s += kd [S0 + A_c/omega S5 + S1 + A_c (1 - 1/omega) S6 - S7
-//              + sum_k Bu_k Bv_k / Sigma_k - sum_k Bu_k xi'_k / Sigma_k^{1/2}]
-//          - [S2 + S4 + E_c S6 + E_c/omega (S5 - S6)]
+// Adds one event's contribution to the gradients (one CTA): S = the sum of the
+// np partial sums of k_pgrad_stencil, Bu = B^T u (a vector, or -Sigma z of the
+// low-rank solve whose result u is: then Bu_k = -Sigma_k z_k), Bv = B^T v from
+// the P partial sums of k_bt_partial, and xi' the sweep's low-rank normals:
+// sweep (kd != 0):
+//   g_s += S + kd [sum_k Bu_k Bv_k / Sigma_k - sum_k Bu_k xi'_k / Sigma_k^{1/2}]
 //   g_k += Bu_k (Bv_k / Sigma_k - xi'_k / (2 Sigma_k^{1/2}))
-// -u^T dA v with v = w (mode 1: the residual f - A x with u = P f_c-bar,
-// and the coarse mean Q^{-1} f with u = Q^{-1} x-bar):
-//   g_s -= S3 + S4 + E_c S6;   g_k += Bu_k Bv_k / Sigma_k
-struct PgradCoef {
-    double kd, omega, ac, ec;
-    int mode;
-};
-__global__ void __launch_bounds__(256) k_pgrad_combine(const double *__restrict__ part, int np,
-                                                       const double *__restrict__ Bu, const double *__restrict__ Bv,
-                                                       const double *__restrict__ xi,
+// -u^T dA v (kd = 0; the residual f - A x with u = P f_c-bar, and the coarse
+// mean Q^{-1} f with u = Q^{-1} x-bar):
+//   g_s += S;   g_k += Bu_k Bv_k / Sigma_k
+template <typename T, int NOISE>
+__global__ void __launch_bounds__(256) k_pgrad_combine(const double *part, int np, const double *Bu, int from_z,
+                                                       const double *bv_part, int P, NoiseArgs nz,
                                                        const double *__restrict__ sigma_inv,
-                                                       const double *__restrict__ sigma_sqrt, int m, PgradCoef cf,
-                                                       double *__restrict__ g_s, double *__restrict__ g_sig) {
+                                                       const double *__restrict__ sigma_sqrt, int m, double kd, double *g_s,
+                                                       double *g_sig) {
     __shared__ double sh[32];
-    double S[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        double a = 0.0;
-        for (int i = threadIdx.x; i < np; i += blockDim.x) a += part[(i64)j * np + i];
-        S[j] = block_sum<256>(a, sh);
-        __syncthreads();
-    }
-    double q1 = 0.0, q2 = 0.0;
+    double acc = 0.0;
+    for (int i = threadIdx.x; i < np; i += blockDim.x) acc += part[i];
     for (int k = threadIdx.x; k < m; k += blockDim.x) {
-        q1 += Bu[k] * Bv[k] * sigma_inv[k];
-        if (cf.mode == 0) q2 += Bu[k] * xi[k] / sigma_sqrt[k];
-        g_sig[k] += cf.mode == 0 ? Bu[k] * (Bv[k] * sigma_inv[k] - 0.5 * xi[k] / sigma_sqrt[k])
-                                 : Bu[k] * Bv[k] * sigma_inv[k];
+        double bv = 0.0;
+        for (int p = 0; p < P; ++p) {
+            if constexpr (sizeof(T) == 4)
+                bv += ff_to_double(ff_of(reinterpret_cast<const float2 *>(bv_part)[(i64)k * P + p]));
+            else
+                bv += bv_part[(i64)k * P + p];
+        }
+        const double sq = sigma_sqrt[k], si = sigma_inv[k], bu = from_z ? -(sq * sq) * Bu[k] : Bu[k], q = bu * bv * si;
+        if (kd != 0.0) {
+            double xi = 0.0;
+            if (NOISE == NOISE_PHILOX)
+                xi = (double)pick(normals4(philox4x32_10(noise_ctr(nz, (unsigned)(k >> 2), PURPOSE_LOWRANK, 0), noise_key(nz))), k & 3);
+            if (NOISE == NOISE_INJECTED) xi = nz.buf[k];
+            const double r = bu * xi / sq;
+            acc += kd * (q - r);
+            g_sig[k] += q - 0.5 * r;
+        } else {
+            g_sig[k] += q;
+        }
     }
-    q1 = block_sum<256>(q1, sh);
-    __syncthreads();
-    q2 = block_sum<256>(q2, sh);
-    if (threadIdx.x == 0) {
-        double c;
-        if (cf.mode == 0)
-            c = cf.kd * (S[0] + cf.ac / cf.omega * S[5] + S[1] + cf.ac * (1.0 - 1.0 / cf.omega) * S[6] - S[7] + q1 - q2) -
-                (S[2] + S[4] + cf.ec * S[6] + cf.ec / cf.omega * (S[5] - S[6]));
-        else
-            c = -(S[3] + S[4] + cf.ec * S[6]);
-        *g_s += c;
-    }
+    acc = block_sum<256>(acc, sh);
+    if (threadIdx.x == 0) *g_s += acc;
 }
 
-// The low-rank normals xi'_k of one sweep (as the low-rank kernels draw
-// them), and the n coarse normals of the Cholesky sample, compact.
-template <int NOISE>
-__global__ void __launch_bounds__(256) k_lowrank_normals(NoiseArgs nz, int m, double *__restrict__ out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m) return;
-    double xi = 0.0;
-    if (NOISE == NOISE_PHILOX) {
-        float4 rn = normals4(philox4x32_10(noise_ctr(nz, (unsigned)(k >> 2), PURPOSE_LOWRANK, 0), noise_key(nz)));
-        xi = (double)pick(rn, k & 3);
-    }
-    if (NOISE == NOISE_INJECTED) xi = nz.buf[k];
-    out[k] = xi;
-}
-
+// The n coarse normals of the Cholesky sample, compact.
 template <int NOISE>
 __global__ void __launch_bounds__(256) k_coarse_normals(NoiseArgs nz, int n, double *__restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
