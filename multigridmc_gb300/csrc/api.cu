@@ -100,13 +100,14 @@ struct Level {
     CorrJob *Cjobs[2] = {nullptr, nullptr};  // the CTAs of k_lr_correct and their columns
     int *Ccols[2] = {nullptr, nullptr};
     int n_Cjobs[2] = {0, 0}, Cmode[2] = {0, 0}, Cquads[2] = {1, 1};
+    std::vector<CorrJob> hCjobs[2];  // the same on the host, for batched groups
     double *SinvT[2] = {nullptr, nullptr};  // S^{-1} transposed, per sweep direction
     float2 *SinvT_ff[2] = {nullptr, nullptr};  // the same as float-float pairs (FP32 chain)
     double *y = nullptr, *z = nullptr, *part = nullptr;
     void *w = nullptr;  // m values: the low-rank noise of the sweep in flight
-    float *zf = nullptr, *Bvalf = nullptr;
+    float *Bvalf = nullptr;
     int bt_split = 1;  // blocks per column of the B^T x reduction
-    unsigned *counter = nullptr;  // CTA counter of k_bt_solve
+    unsigned *counter = nullptr;  // CTA counter of k_bt_full
     int sweep_tx = 0;             // CTA width of the colour passes chosen by the autotuner (0: sweep_block())
     int sweep_threads = 0;        // and its thread count, 128 or 256 (0: RBP_THREADS)
     // constant stencil with equal weights at +-dx, +-dy, +-dz (to rounding):
@@ -610,11 +611,6 @@ static void launch_sweep(Sampler &S, const Level &lv, bool forward, int noise, v
         launch_sweep_noise<double, false>(S, lv, forward, noise, (double *)x, (const double *)f, nz);
 }
 
-// threads of the one-CTA low-rank solve: one per row, up to 256
-static unsigned solve_block(int) { return 256u; }
-// its dynamic shared memory: u (m) and the partial products (256)
-static size_t solve_smem(int m) { return sizeof(double) * ((size_t)m + 256); }
-
 // dynamic shared memory of k_lr_correct: u and z (m values), products and sums
 static size_t lr_correct_smem(int m) {
     return sizeof(double) * (2 * (size_t)m + 64 * 8 + LRC_MAX_M);
@@ -629,13 +625,11 @@ static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, cons
     lr.Bidx = lv.Bidx;
     lr.Bval = lv.Bval;
     lr.Bvalf = lv.Bvalf;
-    lr.zf = lv.zf;
     lr.SinvT = lv.SinvT[dir];
     lr.sigma_sqrt = S.d_sigma_sqrt;
     lr.SinvT_ff = lv.SinvT_ff[dir];
     lr.sigma_sqrt_ff = S.d_sigma_sqrt_ff;
     lr.y = lv.y;
-    lr.z = lv.z;
     lr.part = lv.part;
     lr.counter = lv.counter;
     const CorrRows &C = lv.C[dir];
@@ -785,9 +779,7 @@ static void launch_bt_plain(Sampler &S, Level &lv, const void *x, double *y = nu
     lr.y = y ? y : lv.y;
     lr.part = lv.part;
     lr.counter = lv.counter;
-    NoiseArgs nz{};
-    plaunch(S.pdl, k_bt_solve<T, NOISE_NONE, false>, dim3(S.m, lv.bt_split), 256, solve_smem(S.m), S.stream,
-            (const T *)x, lr, nz);
+    plaunch(S.pdl, k_bt_full<T>, dim3(S.m, lv.bt_split), 256, 0, S.stream, (const T *)x, lr);
     S.launches += 1;
 }
 
@@ -1022,7 +1014,7 @@ __global__ void k_nonzeros(const double *__restrict__ x, Grid3 g, i64 *__restric
 // C = M^{-1} B for both sweep directions, M = D/omega + (strictly lower
 // part of A_0 in the sweep order): column j is one noise-free sweep from
 // x = 0 with right hand side B e_j (sor_smoother.cc:17-37 in solve form).
-// S = Sigma + B^T C (with G = B^T C) gives the m x m system of k_lr_solve.
+// S = Sigma + B^T C (with G = B^T C) gives the m x m system of k_lr_correct.
 void Sampler::build_lowrank(int lev) {
     Level &lv = L[lev];
     const Geometry &geo = lv.geo;
@@ -1064,7 +1056,6 @@ void Sampler::build_lowrank(int lev) {
     lv.y = alloc<double>(m);
     lv.z = alloc<double>(m);
     CK(cudaMemsetAsync(lv.z, 0, m * sizeof(double), stream));
-    lv.zf = alloc<float>(m);
     lv.w = alloc<double>(m);
     {
         i64 maxcol = 1;
@@ -1113,7 +1104,7 @@ void Sampler::build_lowrank(int lev) {
             lr.y = lv.y;
             lr.part = lv.part;
             k_bt_partial<double, NOISE_NONE><<<dim3(m, lv.bt_split), 256, 0, stream>>>(xs, lr, nz);
-            k_lr_solve<double, NOISE_NONE, false><<<1, solve_block(m), 0, stream>>>(lr, lv.bt_split, nz);
+            k_bt_sum<double><<<1, 256, 0, stream>>>(lr, lv.bt_split);
             CK(cudaMemcpyAsync(yh.data(), lv.y, m * sizeof(double), cudaMemcpyDeviceToHost, stream));
             CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), stream));
             k_nonzeros<<<nblk(n, 256), 256, 0, stream>>>(xs, lv.g, nzi, nzv, cnt);
@@ -1232,6 +1223,7 @@ void Sampler::build_lowrank(int lev) {
             lv.Cjobs[dir] = upload(jobs);
             lv.Ccols[dir] = upload(jcols);
             lv.n_Cjobs[dir] = (int)jobs.size();
+            lv.hCjobs[dir] = std::move(jobs);
         }
         CorrRows &C = lv.C[dir];
         C.n1 = (i64)r1.size();
@@ -2839,11 +2831,11 @@ struct BatchGroup {
     std::vector<BatchLevelArg *> la;          // per level: G entries
     BatchChainArg *ca = nullptr;
     std::vector<std::array<BatchLowRank *, 2>> lr;  // per level and sweep direction
-    std::vector<BatchLowRank *> lr_res;       // per level: the residual's y = B^T x
     std::vector<BtJob *> bt_jobs;             // per level
     std::vector<int> n_bt;
-    std::vector<std::array<RowJob *, 2>> sc_jobs;
-    std::vector<std::array<int, 2>> n_sc;
+    // per level and direction: the correction's CTAs by mode (k_lr_correct)
+    std::vector<std::array<std::array<BatchCorrJob *, 3>, 2>> corr_jobs;
+    std::vector<std::array<std::array<int, 3>, 2>> n_corr;
     std::vector<BatchAddBq *> bq;             // per level: rows of the next level's B
     std::vector<RowJob *> bq_jobs;
     std::vector<int> n_bq;
@@ -2865,22 +2857,16 @@ struct BatchGroup {
     void sample(int lev, cudaStream_t st);
 };
 
-// row ranges of `rows` rows per chain in jobs of at most 1024 rows
-static void row_jobs(std::vector<RowJob> &jobs, int chain, i64 rows) {
-    for (i64 r = 0; r < rows; r += 1024) jobs.push_back(RowJob{chain, r, std::min(rows, r + 1024)});
-}
-
 void BatchGroup::build(cudaStream_t st) {
     G = (int)ch.size();
     const Sampler &S0 = *ch[0];
     nlev = (int)S0.L.size();
     la.resize(nlev);
     lr.resize(nlev);
-    lr_res.resize(nlev);
     bt_jobs.resize(nlev);
     n_bt.assign(nlev, 0);
-    sc_jobs.resize(nlev);
-    n_sc.resize(nlev);
+    corr_jobs.resize(nlev);
+    n_corr.resize(nlev);
     bq.resize(nlev);
     bq_jobs.resize(nlev);
     n_bq.assign(nlev, 0);
@@ -2890,9 +2876,10 @@ void BatchGroup::build(cudaStream_t st) {
     }
     for (int lev = 0; lev < nlev; ++lev) {
         std::vector<BatchLevelArg> a(G);
-        std::vector<BatchLowRank> l0(G), l1(G), lres(G);
+        std::vector<BatchLowRank> l0(G), l1(G);
         std::vector<BtJob> jobs;
-        std::vector<RowJob> sj0, sj1, qj;
+        std::vector<BatchCorrJob> cj[2][3];
+        std::vector<RowJob> qj;
         std::vector<BatchAddBq> q(G);
         for (int c = 0; c < G; ++c) {
             Sampler &S = *ch[c];
@@ -2914,45 +2901,43 @@ void BatchGroup::build(cudaStream_t st) {
                 r.Bidx = lv.Bidx;
                 r.Bval = lv.Bval;
                 r.Bvalf = lv.Bvalf;
-                r.zf = lv.zf;
                 r.SinvT = lv.SinvT[dir];
                 r.sigma_sqrt = S.d_sigma_sqrt;
                 r.SinvT_ff = lv.SinvT_ff[dir];
                 r.sigma_sqrt_ff = S.d_sigma_sqrt_ff;
-                r.y = lv.y;
-                r.z = lv.z;
                 r.part = lv.part;
-                r.counter = lv.counter;
-                const CorrRows &C = lv.C[dir];
-                b.C = C;
-                row_jobs(dir == 0 ? sj0 : sj1, c, C.n1 + C.nm);
+                r.w = lv.w;
+                b.C = lv.C[dir];
+                b.jobcols = lv.Ccols[dir];
+                b.P = lv.bt_split;
+                // rows of a CTA beyond four per thread become CTAs of their own
+                for (const CorrJob &full : lv.hCjobs[dir])
+                    for (int r0 = full.r0; r0 < full.r1; r0 += 1024) {
+                        CorrJob jb = full;
+                        jb.r0 = r0;
+                        jb.r1 = std::min(full.r1, r0 + 1024);
+                        cj[dir][lv.Cmode[dir]].push_back(BatchCorrJob{c, jb});
+                    }
             }
-            LowRankArg &r = lres[c].lr;  // launch_bt_plain's arguments
-            r.m = S.m;
-            r.Bptr = lv.Bptr;
-            r.Bidx = lv.Bidx;
-            r.Bval = lv.Bval;
-            r.Bvalf = lv.Bvalf;
-            r.y = lv.y;
-            r.part = lv.part;
-            r.counter = lv.counter;
             for (int j = 0; j < S.m; ++j)
                 for (int p = 0; p < lv.bt_split; ++p) jobs.push_back(BtJob{c, j, p, lv.bt_split});
             if (lev + 1 < nlev) {
                 const Level &lc = S.L[lev + 1];
                 const RowCsr &B = lc.Br;
-                q[c] = BatchAddBq{B.nrows, B.rows, B.ptr, B.col, (const double *)B.val, lv.y, S.d_sigma_inv,
-                                  (float *)lc.f};
-                row_jobs(qj, c, B.nrows);
+                q[c] = BatchAddBq{B.nrows, B.rows, B.ptr, B.col, (const double *)B.val, lv.part, S.d_sigma_inv,
+                                  S.m, lv.bt_split, (float *)lc.f};
+                for (i64 r0 = 0; r0 < B.nrows; r0 += 256) qj.push_back(RowJob{c, r0});
             }
         }
         la[lev] = put(a, st);
         lr[lev] = {put(l0, st), put(l1, st)};
-        lr_res[lev] = put(lres, st);
         bt_jobs[lev] = put(jobs, st);
         n_bt[lev] = (int)jobs.size();
-        sc_jobs[lev] = {put(sj0, st), put(sj1, st)};
-        n_sc[lev] = {(int)sj0.size(), (int)sj1.size()};
+        for (int dir = 0; dir < 2; ++dir)
+            for (int mode = 0; mode < 3; ++mode) {
+                corr_jobs[lev][dir][mode] = put(cj[dir][mode], st);
+                n_corr[lev][dir][mode] = (int)cj[dir][mode].size();
+            }
         bq[lev] = put(q, st);
         bq_jobs[lev] = put(qj, st);
         n_bq[lev] = (int)qj.size();
@@ -2980,18 +2965,12 @@ void BatchGroup::build(cudaStream_t st) {
     CK(cudaStreamSynchronize(st));
 }
 
-template <typename Kern>
-static void batch_launch_check(Kern) {
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) fail(MGMC_ERR_CUDA, std::string("batched kernel launch: ") + cudaGetErrorString(e));
-}
-
 // Sampler::sor for the whole group: one sweep, its low-rank correction
 void BatchGroup::sor(int lev, bool forward, cudaStream_t st) {
     const Sampler &S0 = *ch[0];
     const Level &lv = S0.L[lev];
-    Grid3 g = lv.g;
-    g.pdl = 0;
+    const Grid3 g = lv.g;
+    const bool pdl = S0.pdl;
     if (lv.npt == 7) {
         const int ngrp = (g.N0 + 8) / 8;
         const dim3 blk = level_block(lv, ngrp);
@@ -3001,16 +2980,13 @@ void BatchGroup::sor(int lev, bool forward, cudaStream_t st) {
         for (Sampler *S : ch) fs = fs && S->fsplit;
         for (int pass = 0; pass < 2; ++pass) {
             const int colour = forward ? pass : 1 - pass;
-            if (fs)
-                k_sweep_rb_vec_batch<NOISE_PHILOX, true, true><<<grid, blk, 0, st>>>(la[lev], ca, g, colour, pass, inv,
-                                                                                    (unsigned)lev);
-            else if (v8)
-                k_sweep_rb_vec_batch<NOISE_PHILOX, true, false><<<grid, blk, 0, st>>>(la[lev], ca, g, colour, pass,
-                                                                                     inv, (unsigned)lev);
-            else
-                k_sweep_rb_vec_batch<NOISE_PHILOX, false, false><<<grid, blk, 0, st>>>(la[lev], ca, g, colour, pass,
-                                                                                      inv, (unsigned)lev);
-            batch_launch_check(0);
+            auto go = [&](auto kernel) {
+                plaunch(pdl, kernel, grid, blk, 0, st, (const BatchLevelArg *)la[lev], (const BatchChainArg *)ca, g, colour,
+                        pass, inv, (unsigned)lev);
+            };
+            fs   ? go(k_sweep_rb_vec_batch<NOISE_PHILOX, true, true>)
+            : v8 ? go(k_sweep_rb_vec_batch<NOISE_PHILOX, true, false>)
+                 : go(k_sweep_rb_vec_batch<NOISE_PHILOX, false, false>);
         }
     } else if (g.N0 <= ROW_PAIR_MAX_N0) {
         const int npair = lv.ncol / 2;
@@ -3018,10 +2994,9 @@ void BatchGroup::sor(int lev, bool forward, cudaStream_t st) {
             const int pr = forward ? q : npair - 1 - q, pb = pr & 1, pc = pr >> 1;
             if (g.N1 <= pb || g.N2 <= pc) continue;
             const RowLaunch r = row_launch(g, (g.N0 + 1) / 2, ROW_NT32, pb, pc);
-            const dim3 grid(r.grid.x, r.grid.y, r.grid.z * G);
-            k_sweep_row_pair_batch<NOISE_PHILOX><<<grid, r.block, sizeof(float) * (r.block.x + 1) * r.block.y, st>>>(
-                la[lev], ca, g, pb, pc, forward ? 0 : 1, (int)r.grid.z, inv, (unsigned)lev);
-            batch_launch_check(0);
+            plaunch(pdl, k_sweep_row_pair_batch<NOISE_PHILOX>, dim3(r.grid.x, r.grid.y, r.grid.z * G), r.block,
+                    sizeof(float) * (r.block.x + 1) * r.block.y, st, (const BatchLevelArg *)la[lev],
+                    (const BatchChainArg *)ca, g, pb, pc, forward ? 0 : 1, (int)r.grid.z, inv, (unsigned)lev);
         }
     } else {
         for (int cc = 0; cc < lv.ncol; ++cc) {
@@ -3031,19 +3006,24 @@ void BatchGroup::sor(int lev, bool forward, cudaStream_t st) {
             if (na <= 0 || nb <= 0 || nc <= 0) continue;
             const dim3 blk = level_block(lv, na);
             const dim3 grid((na + blk.x - 1) / blk.x, (nb + blk.y - 1) / blk.y, nc * G);
-            k_sweep_c27_batch<NOISE_PHILOX><<<grid, blk, 0, st>>>(la[lev], ca, g, colour, nc, inv, (unsigned)lev);
-            batch_launch_check(0);
+            plaunch(pdl, k_sweep_c27_batch<NOISE_PHILOX>, grid, blk, 0, st, (const BatchLevelArg *)la[lev],
+                    (const BatchChainArg *)ca, g, colour, nc, inv, (unsigned)lev);
         }
     }
     if (n_bt[lev] > 0) {
         const int dir = forward ? 0 : 1;
-        k_bt_solve_batch<NOISE_PHILOX, true><<<n_bt[lev], 256, solve_smem(max_m), st>>>(la[lev], lr[lev][dir], ca,
-                                                                                       bt_jobs[lev], inv, (unsigned)lev);
-        batch_launch_check(0);
-        if (n_sc[lev][dir] > 0) {
-            k_lr_scatter_batch<<<n_sc[lev][dir], 256, 0, st>>>(la[lev], lr[lev][dir], sc_jobs[lev][dir]);
-            batch_launch_check(0);
-        }
+        const BatchLowRank *low = lr[lev][dir];
+        plaunch(pdl, k_bt_partial_batch<NOISE_PHILOX>, n_bt[lev], 256, 0, st, (const BatchLevelArg *)la[lev], low,
+                (const BatchChainArg *)ca, (const BtJob *)bt_jobs[lev], inv, (unsigned)lev);
+        // chains of different modes correct in launches of their own
+        auto correct = [&](int mode, auto kernel) {
+            if (n_corr[lev][dir][mode] > 0)
+                plaunch(pdl, kernel, n_corr[lev][dir][mode], 256, lr_correct_smem(max_m), st, (const BatchLevelArg *)la[lev],
+                        low, (const BatchCorrJob *)corr_jobs[lev][dir][mode]);
+        };
+        correct(0, k_lr_correct_batch<0>);
+        correct(1, k_lr_correct_batch<1>);
+        correct(2, k_lr_correct_batch<2>);
     }
     inv++;
 }
@@ -3051,22 +3031,23 @@ void BatchGroup::sor(int lev, bool forward, cudaStream_t st) {
 // Sampler::sample for the whole group (multigridmc_sampler.cc:109-136)
 void BatchGroup::sample(int lev, cudaStream_t st) {
     const Sampler &S0 = *ch[0];
+    const bool pdl = S0.pdl;
     if (lev == nlev - 1) {
         const Level &lv = S0.L[lev];
-        Grid3 g = lv.g;
-        g.pdl = 0;
+        const Grid3 g = lv.g;
         const unsigned blocks = (unsigned)((lv.geo.n + 7) / 8);
-        k_chol_lower_batch<NOISE_PHILOX><<<dim3(blocks, G), 256, S0.chol_smem, st>>>(la[lev], ca, g, S0.chol_ld, inv,
-                                                                                     (unsigned)lev);
-        batch_launch_check(0);
-        k_chol_upper_batch<<<dim3(blocks, G), 256, S0.chol_smem, st>>>(la[lev], ca, g, S0.chol_ld);
-        batch_launch_check(0);
+        const BatchLevelArg *la_ = la[lev];
+        const BatchChainArg *ca_ = ca;
+        plaunch(pdl, k_chol_lower_batch<NOISE_PHILOX>, dim3(blocks, G), 256, S0.chol_smem, st, la_, ca_, g, S0.chol_ld, inv,
+                (unsigned)lev);
+        plaunch(pdl, k_chol_upper_batch, dim3(blocks, G), 256, S0.chol_smem, st, la_, ca_, g, S0.chol_ld);
         inv++;
         return;
     }
     const Level &lv = S0.L[lev], &lc = S0.L[lev + 1];
-    Grid3 gf = lv.g, gc = lc.g;
-    gf.pdl = gc.pdl = 0;
+    const Grid3 gf = lv.g, gc = lc.g;
+    const BatchLevelArg *la_ = la[lev];
+    const BatchChainArg *ca_ = ca;
     const int cyc = lev > 0 ? S0.P.cycle : 1;
     for (int j = 0; j < cyc; ++j) {
         for (int k = 0; k < S0.P.npresmooth; ++k) {
@@ -3078,23 +3059,18 @@ void BatchGroup::sample(int lev, cudaStream_t st) {
         const int tz = (gc.N2 + RR_TZ - 1) / RR_TZ;
         const dim3 rgrid((gc.N0 + RR_TX - 1) / RR_TX, (gc.N1 + RR_TY - 1) / RR_TY, tz * G);
         if (lv.npt == 7)
-            k_resid_restrict_batch<7><<<rgrid, RR_THREADS, rr_smem_bytes<float>(), st>>>(la[lev], gf, gc, tz);
+            plaunch(pdl, k_resid_restrict_batch<7>, rgrid, RR_THREADS, rr_smem_bytes<float>(), st, la_, gf, gc, tz);
         else
-            k_resid_restrict_batch<27><<<rgrid, RR_THREADS, rr_smem_bytes<float>(), st>>>(la[lev], gf, gc, tz);
-        batch_launch_check(0);
-        if (n_bt[lev] > 0) {
-            k_bt_solve_batch<NOISE_NONE, false><<<n_bt[lev], 256, solve_smem(max_m), st>>>(la[lev], lr_res[lev], ca,
-                                                                                          bt_jobs[lev], 0u, 0u);
-            batch_launch_check(0);
-            if (n_bq[lev] > 0) {
-                k_add_Bq_batch<<<n_bq[lev], 256, 0, st>>>(bq[lev], bq_jobs[lev]);
-                batch_launch_check(0);
-            }
+            plaunch(pdl, k_resid_restrict_batch<27>, rgrid, RR_THREADS, rr_smem_bytes<float>(), st, la_, gf, gc, tz);
+        if (n_bt[lev] > 0 && n_bq[lev] > 0) {
+            plaunch(pdl, k_bt_partial_batch<NOISE_NONE>, n_bt[lev], 256, 0, st, la_, (const BatchLowRank *)lr[lev][0], ca_,
+                    (const BtJob *)bt_jobs[lev], 0u, 0u);
+            plaunch(pdl, k_resid_Bq_batch, n_bq[lev], 256, sizeof(double) * max_m, st, (const BatchAddBq *)bq[lev],
+                    (const RowJob *)bq_jobs[lev]);
         }
         sample(lev + 1, st);
         const dim3 pgrid((gc.N0 + 1 + 127) / 128, gc.N1 + 1, (gc.N2 + 1) * G);
-        k_prolong_batch<<<pgrid, 128, 0, st>>>(la[lev], gf, gc, (float)S0.P.coarse_scaling, 3, gc.N2 + 1);
-        batch_launch_check(0);
+        plaunch(pdl, k_prolong_batch, pgrid, 128, 0, st, la_, gf, gc, (float)S0.P.coarse_scaling, 3, gc.N2 + 1);
         for (int k = 0; k < S0.P.npostsmooth; ++k) {
             sor(lev, true, st);
             sor(lev, false, st);
@@ -3105,8 +3081,8 @@ void BatchGroup::sample(int lev, cudaStream_t st) {
 void BatchGroup::record(cudaStream_t st) {
     inv = 0;
     sample(0, st);
-    k_step_end_batch<<<dim3(max_probe, G), 256, 0, st>>>(la[0], ca);
-    batch_launch_check(0);
+    plaunch(ch[0]->pdl, k_step_end_batch, dim3(max_probe, G), 256, 0, st, (const BatchLevelArg *)la[0],
+            (const BatchChainArg *)ca);
 }
 
 extern "C" {
@@ -3114,11 +3090,21 @@ extern "C" {
 struct mgmc_batch {
     std::vector<Sampler *> chains;
     std::vector<std::unique_ptr<BatchGroup>> groups;
-    std::vector<cudaGraph_t> group_graphs;
+    std::vector<cudaStream_t> branches;  // one per group while the step is captured
+    std::vector<cudaEvent_t> events;
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     int device = 0;
+    ~mgmc_batch() {
+        if (gexec) cudaGraphExecDestroy(gexec);
+        if (graph) cudaGraphDestroy(graph);
+        for (cudaEvent_t e : events)
+            if (e) cudaEventDestroy(e);
+        for (cudaStream_t st : branches)
+            if (st) cudaStreamDestroy(st);
+        if (stream) cudaStreamDestroy(stream);
+    }
 };
 
 mgmc_status mgmc_batch_create(int nchain, mgmc_sampler *const *samplers, mgmc_batch **out) {
@@ -3138,7 +3124,6 @@ mgmc_status mgmc_batch_create(int nchain, mgmc_sampler *const *samplers, mgmc_ba
     }
     CK(cudaSetDevice(B->device));
     CK(cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking));
-    CK(cudaGraphCreate(&B->graph, 0));
     // groups of chains that step through the batched kernels
     std::vector<Sampler *> solo;
     {
@@ -3165,50 +3150,48 @@ mgmc_status mgmc_batch_create(int nchain, mgmc_sampler *const *samplers, mgmc_ba
                 grp->ch.assign(v.begin() + a, v.begin() + std::min(v.size(), a + (size_t)zmax));
                 for (Sampler *S : grp->ch) CK(cudaStreamSynchronize(S->stream));
                 grp->build(B->stream);
-                cudaGraph_t gg = nullptr;
-                CK(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
-                try {
-                    grp->record(B->stream);
-                } catch (...) {
-                    cudaStreamEndCapture(B->stream, &gg);
-                    if (gg) cudaGraphDestroy(gg);
-                    throw;
-                }
-                CK(cudaStreamEndCapture(B->stream, &gg));
-                B->group_graphs.push_back(gg);
-                cudaGraphNode_t node;
-                CK(cudaGraphAddChildGraphNode(&node, B->graph, nullptr, 0, gg));
                 B->groups.push_back(std::move(grp));
             }
         }
     }
-    for (Sampler *S : solo) {
-        CK(cudaStreamSynchronize(S->stream));
-        // a chain's step graph becomes a child graph: captured with plain
-        // (non-programmatic) dependencies
-        if (S->pdl) {
-            S->pdl = false;
-            if (S->gexec) cudaGraphExecDestroy(S->gexec);
-            if (S->graph) cudaGraphDestroy(S->graph);
-            S->gexec = nullptr;
-            S->graph = nullptr;
-        }
-        ensure_graph(*S);
-        cudaGraphNode_t node;
-        CK(cudaGraphAddChildGraphNode(&node, B->graph, nullptr, 0, S->graph));
+    for (Sampler *S : solo) CK(cudaStreamSynchronize(S->stream));
+    // One capture of the whole step: groups and single chains on streams of
+    // their own, forked from and joined to the batch's stream, so that every
+    // branch keeps its programmatic dependent launches (a child graph would
+    // carry plain dependencies)
+    B->events.resize(B->groups.size() + solo.size() + 1);
+    for (cudaEvent_t &e : B->events) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    B->branches.resize(B->groups.size());
+    for (cudaStream_t &st : B->branches) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    CK(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
+    try {
+        CK(cudaEventRecord(B->events.back(), B->stream));
+        auto branch = [&](size_t k, cudaStream_t st, const std::function<void()> &body) {
+            CK(cudaStreamWaitEvent(st, B->events.back(), 0));
+            body();
+            CK(cudaEventRecord(B->events[k], st));
+            CK(cudaStreamWaitEvent(B->stream, B->events[k], 0));
+        };
+        for (size_t k = 0; k < B->groups.size(); ++k)
+            branch(k, B->branches[k], [&]() { B->groups[k]->record(B->branches[k]); });
+        for (size_t k = 0; k < solo.size(); ++k)
+            branch(B->groups.size() + k, solo[k]->stream, [&]() {
+                solo[k]->launch_step();
+                solo[k]->check_launch();
+            });
+    } catch (...) {
+        cudaGraph_t g = nullptr;
+        cudaStreamEndCapture(B->stream, &g);
+        if (g) cudaGraphDestroy(g);
+        throw;
     }
+    CK(cudaStreamEndCapture(B->stream, &B->graph));
     CK(cudaGraphInstantiate(&B->gexec, B->graph, 0));
     *out = B;
     B = nullptr;
     }
     catch (const Error &e) {
-        if (B) {
-            if (B->gexec) cudaGraphExecDestroy(B->gexec);
-            if (B->graph) cudaGraphDestroy(B->graph);
-            for (cudaGraph_t gg : B->group_graphs) cudaGraphDestroy(gg);
-            if (B->stream) cudaStreamDestroy(B->stream);
-            delete B;
-        }
+        delete B;
         g_err = e.msg;
         return e.st;
     }
@@ -3253,10 +3236,6 @@ mgmc_status mgmc_batch_destroy(mgmc_batch *b) {
     if (!b) return MGMC_OK;
     cudaSetDevice(b->device);
     cudaStreamSynchronize(b->stream);
-    if (b->gexec) cudaGraphExecDestroy(b->gexec);
-    if (b->graph) cudaGraphDestroy(b->graph);
-    for (cudaGraph_t gg : b->group_graphs) cudaGraphDestroy(gg);
-    if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     API_END
 }

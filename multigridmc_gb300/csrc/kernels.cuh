@@ -17,7 +17,7 @@
 //                       (one CTA; parity mode)
 //   k_bt_partial        partial sums of y = B^T x, the low-rank noise
 //   k_lr_correct        the m x m solve and x += C z over the rows of C = M^{-1} B
-//   k_bt_solve          y = B^T x in one launch (k_lr_solve: from partial sums)
+//   k_bt_full           y = B^T x in one launch (k_bt_sum: from partial sums)
 //   k_resid_restrict_tma    f_c = R (f - A_0 x), TMA tiles (fused residual
 //                           + restriction; _tiled / plain variants otherwise)
 //   k_resid_restrict_sym    the same for FP64 chains' symmetric stencils
@@ -930,12 +930,10 @@ struct LowRankArg {
     const double *SinvT; // m x m, S^{-1} = (Sigma + B^T M^{-1} B)^{-1}, transposed (column q contiguous)
     const double *sigma_sqrt; // Sigma^{1/2}
     double *y;          // m scratch: B^T x
-    double *z;          // m scratch: coefficients of C
-    float *zf;          // the same coefficients rounded to FP32 (FP32 chain)
     const float *Bvalf; // B values rounded to FP32 (FP32 chain)
     double *part;       // m x P scratch: partial sums of B^T x (the FP32 chain
                         // stores float-float pairs, float2, in the same slots)
-    unsigned *counter;  // CTA counter of k_bt_solve (reset by its last CTA)
+    unsigned *counter;  // CTA counter of k_bt_full (reset by its last CTA)
     void *w;                     // m scratch: Sigma^{1/2} xi' (double, or float2 for the FP32 chain)
     double *zpub;                // where k_lr_correct leaves z (null: nowhere)
     const float2 *SinvT_ff;      // SinvT as float-float pairs (FP32 chain)
@@ -996,14 +994,13 @@ __device__ __forceinline__ void bt_partial_cta(const T *x, const LowRankArg &lr,
 // Also the low-rank noise Sigma^{1/2} xi' of the column (lr.w, unless null),
 // drawn before the wait by a thread that has little else to do.
 template <typename T, int NOISE>
-__global__ void __launch_bounds__(256) k_bt_partial(const T *x, LowRankArg lr, NoiseArgs nz) {
+__device__ __forceinline__ void bt_partial_body(const T *x, const LowRankArg &lr, const NoiseArgs &nz, int j, int p, int P) {
     __shared__ double sh[32];
-    const int j = blockIdx.x;
-    const bool draws = lr.w && blockIdx.y == 0 && threadIdx.x == 255;
+    const bool draws = lr.w && p == 0 && threadIdx.x == 255;
     float xif = 0.f;
     if (draws && NOISE == NOISE_PHILOX)
         xif = pick(normals4(philox4x32_10(noise_ctr(nz, (unsigned)(j >> 2), PURPOSE_LOWRANK, 0), noise_key(nz))), j & 3);
-    bt_partial_cta<T>(x, lr, sh, j, blockIdx.y, gridDim.y, true);
+    bt_partial_cta<T>(x, lr, sh, j, p, P, true);
     if (draws) {
         if constexpr (sizeof(T) == 4) {
             const ff32 w = ff_mul(ff_of(lr.sigma_sqrt_ff[j]), ff32{NOISE == NOISE_INJECTED ? (float)nz.buf[j] : xif, 0.f});
@@ -1014,286 +1011,67 @@ __global__ void __launch_bounds__(256) k_bt_partial(const T *x, LowRankArg lr, N
     }
 }
 
+template <typename T, int NOISE>
+__global__ void __launch_bounds__(256) k_bt_partial(const T *x, LowRankArg lr, NoiseArgs nz) {
+    bt_partial_body<T, NOISE>(x, lr, nz, blockIdx.x, blockIdx.y, gridDim.y);
+}
+
 // One CTA: y_k = sum_p part[k * P + p] (fixed order, so the result does not
-// depend on block timing).  With SOLVE it then forms the coefficients z of
-// the correction x += C z,
-//   z = w - S^{-1} (y + G w) = S^{-1} (Sigma w - y) = S^{-1} (Sigma^{1/2} xi' - y)
-// with w = Sigma^{-1/2} xi' the low-rank noise of sor_sampler.cc:29-33,
-// G = B^T C and S = Sigma + G (so S - G = Sigma and a single m x m product
-// remains); with_noise == 0 gives z = -S^{-1} y, the smoother's correction
-// x -= Bbar B^T x of sor_smoother.cc:47-51, Bbar = C S^{-1}.
-// One thread per row k: FP64 arithmetic is scarce on this GPU, so every
-// FP64 instruction works on 32 different rows (no shuffle trees); S^{-1} is
-// stored transposed (SinvT[q * m + k]) so that a warp's loads of one column
-// q are contiguous.
-// The low-rank solve of one CTA of 256 threads (see k_lr_solve); with
-// SOLVE the coefficients z end up in zs (shared, m doubles) and, if
-// `publish`, in lr.z / lr.zf.  u and acc are shared scratch of m and 256
-// doubles.
-template <int NOISE, bool SOLVE>
-__device__ __forceinline__ void lr_solve_cta(const LowRankArg &lr, int P, const NoiseArgs &nz, double *u, double *acc,
-                                             double *zs, bool publish) {
-    const int m = lr.m;
-    // rows handled at once and threads per row (blockDim.x = 256)
-    const int rows = m < 256 ? m : 256;
-    const int tpr = 256 / rows;
-    const int g = threadIdx.x / rows, kk = threadIdx.x % rows;
-    // m <= 64: each thread's slice of S^{-1} (at most 16 values) is loaded
-    // here, while the partial sums below are read, instead of after them
-    const int cnt = g < tpr ? (m - g + tpr - 1) / tpr : 0;
-    const bool pre = SOLVE && m <= 64;
-    double pv[16];
-    if (pre) {
+// depend on block timing), in float-float for the FP32 chain
+template <typename T>
+__device__ __forceinline__ void bt_sum_cta(const LowRankArg &lr, int P) {
+    for (int k = threadIdx.x; k < lr.m; k += blockDim.x) {
+        if constexpr (sizeof(T) == 4) {
+            const float2 *part = reinterpret_cast<const float2 *>(lr.part) + (i64)k * P;
+            ff32 t{0.f, 0.f};
+            for (int p0 = 0; p0 < P; p0 += 8) {
+                float2 pp[8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) pv[i] = i < cnt ? __ldg(lr.SinvT + (i64)(g + i * tpr) * m + kk) : 0.0;
-    }
-    for (int k = threadIdx.x; k < m; k += blockDim.x) {
-        double pv[8];
-        double t = 0.0;
-        for (int q0 = 0; q0 < P; q0 += 8) {
+                for (int r = 0; r < 8; ++r) pp[r] = p0 + r < P ? __ldcg(part + p0 + r) : make_float2(0.f, 0.f);
 #pragma unroll
-            for (int r = 0; r < 8; ++r) pv[r] = q0 + r < P ? __ldcg(lr.part + (i64)k * P + q0 + r) : 0.0;
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-                if (q0 + r < P) t += pv[r];
-        }
-        if (publish) lr.y[k] = t;
-        if (SOLVE) {
-            double xi = 0.0;
-            if (NOISE == NOISE_PHILOX) {
-                float4 rn = normals4(philox4x32_10(noise_ctr(nz, (unsigned)(k >> 2), PURPOSE_LOWRANK, 0), noise_key(nz)));
-                xi = (double)pick(rn, k & 3);
+                for (int r = 0; r < 8; ++r)
+                    if (p0 + r < P) t = ff_add(t, ff_of(pp[r]));
             }
-            if (NOISE == NOISE_INJECTED) xi = nz.buf[k];
-            u[k] = lr.sigma_sqrt[k] * xi - t;
-        }
-    }
-    if (!SOLVE) return;
-    __syncthreads();
-    // z = S^{-1} u: thread (g, k) of g < tpr sums the columns q = g, g + tpr, ...
-    // of row k (loads of one column contiguous over k), in batches of 8
-    // loads issued together; the tpr partial sums are then added in order g.
-    if (pre) {  // the same sums from the preloaded slice (one batch of rows: m <= 64)
-        double t0 = 0.0, t1 = 0.0;
-        if (g < tpr) {
+            lr.y[k] = ff_to_double(t);
+        } else {
+            double t = 0.0;
+            for (int p0 = 0; p0 < P; p0 += 8) {
+                double pp[8];
 #pragma unroll
-            for (int i0 = 0; i0 < 16; i0 += 8) {
-                if (i0 + 7 < cnt) {
+                for (int r = 0; r < 8; ++r) pp[r] = p0 + r < P ? __ldcg(lr.part + (i64)k * P + p0 + r) : 0.0;
 #pragma unroll
-                    for (int r = 0; r < 8; r += 2) {
-                        t0 = fma(pv[i0 + r], u[g + (i0 + r) * tpr], t0);
-                        t1 = fma(pv[i0 + r + 1], u[g + (i0 + r + 1) * tpr], t1);
-                    }
-                } else {
-#pragma unroll
-                    for (int r = 0; r < 8; ++r)
-                        if (i0 + r < cnt) t0 = fma(pv[i0 + r], u[g + (i0 + r) * tpr], t0);
-                }
+                for (int r = 0; r < 8; ++r)
+                    if (p0 + r < P) t += pp[r];
             }
-            acc[g * rows + kk] = t0 + t1;
+            lr.y[k] = t;
         }
-        __syncthreads();
-        if (threadIdx.x < rows) {
-            double zk = 0.0;
-            for (int h = 0; h < tpr; ++h) zk += acc[h * rows + threadIdx.x];
-            if (zs) zs[threadIdx.x] = zk;
-            if (publish) {
-                lr.z[threadIdx.x] = zk;
-                if (lr.zf) lr.zf[threadIdx.x] = (float)zk;
-            }
-        }
-        __syncthreads();
-        return;
-    }
-    for (int k0 = 0; k0 < m; k0 += rows) {
-        const int k = k0 + kk;
-        double t0 = 0.0, t1 = 0.0;
-        if (g < tpr && k < m) {
-            int q = g;
-            for (; q + 7 * tpr < m; q += 8 * tpr) {
-                double sv[8];
-#pragma unroll
-                for (int r = 0; r < 8; ++r) sv[r] = __ldg(lr.SinvT + (i64)(q + r * tpr) * m + k);
-#pragma unroll
-                for (int r = 0; r < 8; r += 2) {
-                    t0 = fma(sv[r], u[q + r * tpr], t0);
-                    t1 = fma(sv[r + 1], u[q + (r + 1) * tpr], t1);
-                }
-            }
-            for (; q < m; q += tpr) t0 = fma(__ldg(lr.SinvT + (i64)q * m + k), u[q], t0);
-            acc[g * rows + kk] = t0 + t1;
-        }
-        __syncthreads();
-        if (threadIdx.x < rows && k0 + threadIdx.x < m) {
-            double zk = 0.0;
-            for (int h = 0; h < tpr; ++h) zk += acc[h * rows + threadIdx.x];
-            if (zs) zs[k0 + threadIdx.x] = zk;
-            if (publish) {
-                lr.z[k0 + threadIdx.x] = zk;
-                if (lr.zf) lr.zf[k0 + threadIdx.x] = (float)zk;
-            }
-        }
-        __syncthreads();
     }
 }
 
-// lr_solve_cta for the FP32 chain: the same sums, in the same order and the
-// same thread layout, in float-float arithmetic (partial sums as float2
-// pairs, S^{-1} and Sigma^{1/2} from their float-float copies).  z goes to
-// zsf (shared, m floats, rounded to FP32) and, if `publish`, to lr.z (the
-// float-float value in FP64) and lr.zf.  u and acc are shared scratch of m
-// and 256 float2.
-template <int NOISE, bool SOLVE>
-__device__ __forceinline__ void lr_solve_cta_ff(const LowRankArg &lr, int P, const NoiseArgs &nz, float2 *u,
-                                                float2 *acc, float *zsf, bool publish) {
-    const int m = lr.m;
-    const int rows = m < 256 ? m : 256;
-    const int tpr = 256 / rows;
-    const int g = threadIdx.x / rows, kk = threadIdx.x % rows;
-    const int cnt = g < tpr ? (m - g + tpr - 1) / tpr : 0;
-    const bool pre = SOLVE && m <= 64;
-    const float2 *part = reinterpret_cast<const float2 *>(lr.part);
-    float2 pv[16];
-    if (pre) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            pv[i] = i < cnt ? __ldg(lr.SinvT_ff + (i64)(g + i * tpr) * m + kk) : make_float2(0.f, 0.f);
-    }
-    for (int k = threadIdx.x; k < m; k += blockDim.x) {
-        float2 pp[8];
-        ff32 t{0.f, 0.f};
-        for (int q0 = 0; q0 < P; q0 += 8) {
-#pragma unroll
-            for (int r = 0; r < 8; ++r) pp[r] = q0 + r < P ? __ldcg(part + (i64)k * P + q0 + r) : make_float2(0.f, 0.f);
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-                if (q0 + r < P) t = ff_add(t, ff_of(pp[r]));
-        }
-        if (publish) lr.y[k] = ff_to_double(t);
-        if (SOLVE) {
-            float xi = 0.f;
-            if (NOISE == NOISE_PHILOX) {
-                float4 rn = normals4(philox4x32_10(noise_ctr(nz, (unsigned)(k >> 2), PURPOSE_LOWRANK, 0), noise_key(nz)));
-                xi = pick(rn, k & 3);
-            }
-            if (NOISE == NOISE_INJECTED) xi = (float)nz.buf[k];
-            const ff32 uk = ff_add(ff_mul(ff_of(lr.sigma_sqrt_ff[k]), ff32{xi, 0.f}), ff_neg(t));
-            u[k] = make_float2(uk.hi, uk.lo);
-        }
-    }
-    if (!SOLVE) return;
-    __syncthreads();
-    auto finish = [&](int k, ff32 zk) {
-        if (zsf) zsf[k] = ff_to_float(zk);
-        if (publish) {
-            lr.z[k] = ff_to_double(zk);
-            if (lr.zf) lr.zf[k] = ff_to_float(zk);
-        }
-    };
-    if (pre) {
-        ff32 t0{0.f, 0.f}, t1{0.f, 0.f};
-        if (g < tpr) {
-#pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-                if (i < cnt) t0 = ff_add(t0, ff_mul(ff_of(pv[i]), ff_of(u[g + i * tpr])));
-                if (i + 1 < cnt) t1 = ff_add(t1, ff_mul(ff_of(pv[i + 1]), ff_of(u[g + (i + 1) * tpr])));
-            }
-            const ff32 s = ff_add(t0, t1);
-            acc[g * rows + kk] = make_float2(s.hi, s.lo);
-        }
-        __syncthreads();
-        if (threadIdx.x < rows) {
-            ff32 zk{0.f, 0.f};
-            for (int h = 0; h < tpr; ++h) zk = ff_add(zk, ff_of(acc[h * rows + threadIdx.x]));
-            finish(threadIdx.x, zk);
-        }
-        __syncthreads();
-        return;
-    }
-    for (int k0 = 0; k0 < m; k0 += rows) {
-        const int k = k0 + kk;
-        if (g < tpr && k < m) {
-            ff32 t0{0.f, 0.f}, t1{0.f, 0.f};
-            int q = g;
-            for (; q + 7 * tpr < m; q += 8 * tpr) {
-                float2 sv[8];
-#pragma unroll
-                for (int r = 0; r < 8; ++r) sv[r] = __ldg(lr.SinvT_ff + (i64)(q + r * tpr) * m + k);
-#pragma unroll
-                for (int r = 0; r < 8; r += 2) {
-                    t0 = ff_add(t0, ff_mul(ff_of(sv[r]), ff_of(u[q + r * tpr])));
-                    t1 = ff_add(t1, ff_mul(ff_of(sv[r + 1]), ff_of(u[q + (r + 1) * tpr])));
-                }
-            }
-            for (; q < m; q += tpr) t0 = ff_add(t0, ff_mul(ff_of(__ldg(lr.SinvT_ff + (i64)q * m + k)), ff_of(u[q])));
-            const ff32 s = ff_add(t0, t1);
-            acc[g * rows + kk] = make_float2(s.hi, s.lo);
-        }
-        __syncthreads();
-        if (threadIdx.x < rows && k0 + threadIdx.x < m) {
-            ff32 zk{0.f, 0.f};
-            for (int h = 0; h < tpr; ++h) zk = ff_add(zk, ff_of(acc[h * rows + threadIdx.x]));
-            finish(k0 + threadIdx.x, zk);
-        }
-        __syncthreads();
-    }
-}
-
-// The low-rank solve of a chain in precision T: FP64 for the FP64 chain,
-// float-float for the FP32 chain (its partial sums are float-float pairs).
-// u and acc: shared scratch of m and 256 doubles; z goes to zs (m doubles of
-// shared memory, holding m floats for the FP32 chain) unless it is null.
-template <typename T, int NOISE, bool SOLVE>
-__device__ __forceinline__ void lr_solve_chain(const LowRankArg &lr, int P, const NoiseArgs &nz, double *u,
-                                               double *acc, double *zs, bool publish) {
-    if (sizeof(T) == 4)
-        lr_solve_cta_ff<NOISE, SOLVE>(lr, P, nz, reinterpret_cast<float2 *>(u), reinterpret_cast<float2 *>(acc),
-                                      reinterpret_cast<float *>(zs), publish);
-    else
-        lr_solve_cta<NOISE, SOLVE>(lr, P, nz, u, acc, zs, publish);
-}
-
-template <typename T, int NOISE, bool SOLVE>
-__global__ void __launch_bounds__(256) k_lr_solve(LowRankArg lr, int P, NoiseArgs nz) {
+template <typename T>
+__global__ void __launch_bounds__(256) k_bt_sum(LowRankArg lr, int P) {
     pdl_begin();
-    extern __shared__ double dyn[];
-    lr_solve_chain<T, NOISE, SOLVE>(lr, P, nz, dyn, dyn + lr.m, nullptr, true);
+    bt_sum_cta<T>(lr, P);
 }
 
-// Partial sums and the solve in one launch: the last CTA to finish (block
-// counter, reset by that CTA) forms y -- and with SOLVE z -- from the
-// partial sums in the same fixed order as k_lr_solve, so the result does
-// not depend on block timing.  The thread that wrote the CTA's partial sum
-// counts it with an acquire-release atomic, which orders that write before
-// the count and, in the last CTA, the other CTAs' sums before the barrier
-// after which its threads read them.
-template <typename T, int NOISE, bool SOLVE>
-__device__ __forceinline__ void bt_solve_body(const T *__restrict__ x, const LowRankArg &lr, const NoiseArgs &nz, int j,
-                                              int p, int P, bool wait = false) {
+// y = B^T x in one launch: the last CTA to finish (block counter, reset by
+// that CTA) adds the partial sums in k_bt_sum's order.  The thread that wrote
+// the CTA's partial sum counts it with an acquire-release atomic, which orders
+// that write before the count and, in the last CTA, the other CTAs' sums
+// before the barrier after which its threads read them.
+template <typename T>
+__global__ void __launch_bounds__(256) k_bt_full(const T *x, LowRankArg lr) {
     __shared__ double sh[32];
     __shared__ bool last;
-    bt_partial_cta<T>(x, lr, sh, j, p, P, wait);
+    bt_partial_cta<T>(x, lr, sh, blockIdx.x, blockIdx.y, gridDim.y, true);
     if (threadIdx.x == 0) {
-        // one acquire-release count at GPU scope: it publishes this CTA's
-        // partial sum (written by this thread) and, in the last CTA, makes
-        // every other CTA's visible before the barrier below
         unsigned prev;
         asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(lr.counter) : "memory");
-        last = prev == (unsigned)(lr.m * P) - 1u;
+        last = prev == gridDim.x * gridDim.y - 1u;
         if (last) *lr.counter = 0u;
     }
     __syncthreads();
-    if (!last) return;
-    // every other CTA has exited: the next kernel (the correction) can load
-    // its rows of C while this CTA forms z
-    pdl_trigger();
-    extern __shared__ double dyn[];
-    lr_solve_chain<T, NOISE, SOLVE>(lr, P, nz, dyn, dyn + lr.m, nullptr, true);
-}
-
-template <typename T, int NOISE, bool SOLVE>
-__global__ void __launch_bounds__(256) k_bt_solve(const T *__restrict__ x, LowRankArg lr, NoiseArgs nz) {
-    bt_solve_body<T, NOISE, SOLVE>(x, lr, nz, blockIdx.x, blockIdx.y, gridDim.y, true);
+    if (last) bt_sum_cta<T>(lr, gridDim.y);
 }
 
 // Support rows of C = M^{-1} B as x += C z reads them: the rows with one
@@ -1311,20 +1089,9 @@ struct CorrRows {
     const void *vm = nullptr;
 };
 
-// x[row] += C z over the multi-entry row r: the products added to zero in
-// entry order, then to the state
-template <typename T, typename ZT>
-__device__ __forceinline__ void corr_multi_row(T *__restrict__ x, const CorrRows &C, i64 r, const ZT *z) {
-    const T *vm = static_cast<const T *>(C.vm);
-    T acc = T(0);
-    for (int e = C.pm[r]; e < C.pm[r + 1]; ++e) acc += vm[e] * (T)z[C.cm[e]];
-    const unsigned row = C.rm[r];
-    x[row] = x[row] + acc;
-}
-
 // Four single-entry rows of a thread, r0 + j stride (j < 4) below r1: row index,
-// column, value and state loaded together; the update is the multi-entry
-// arithmetic with one product.  The state of rows loaded before the wait
+// column, value and state loaded together; the update adds the
+// product to zero, then to the state, as a multi-entry row's (FP64: one FMA).  The state of rows loaded before the wait
 // for the previous kernel is read through L2 (see k_lr_correct).
 template <typename T>
 struct CorrQuad {
@@ -1363,8 +1130,8 @@ struct CorrQuad {
 
 // One multi-entry row r (two entries at least) with its row index, entry
 // range, first two entries and state loaded together, before the wait for
-// the previous kernel where the caller says so; the update is
-// corr_multi_row's arithmetic.
+// the previous kernel where the caller says so; its products
+// are added to zero in entry order, then to the state.
 template <typename T>
 struct CorrMulti {
     unsigned row;
@@ -1399,7 +1166,7 @@ struct CorrMulti {
 // only, their products one per thread.  MODE 1, the same where columns overlap
 // throughout (coarse levels): all of z, S^{-1} loaded before the wait.  MODE 2:
 // all of z of more columns.  The FP32 chain forms every z_k in the same order wherever it
-// is formed (lr_solve_cta_ff's: 256 / m groups of terms per column, two
+// is formed (256 / m groups of terms per column, two
 // alternating sums in a group), so all CTAs and the batched kernels agree bit
 // for bit.
 //
@@ -1423,12 +1190,10 @@ struct CorrJob {
 constexpr int CORR_OWNER = 1 << 30;
 
 template <typename T, int MODE, int NQ>
-__global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
-    k_lr_correct(T *x, LowRankArg lr, int P, CorrRows C, const CorrJob *__restrict__ jobs, const int *__restrict__ jobcols) {
+__device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int P, const CorrRows &C, const CorrJob &jb,
+                                                const int *__restrict__ jobcols, bool first, double *dyn) {
     typedef typename std::conditional<sizeof(T) == 4, float2, double>::type V;  // FP32 chain: float-float
-    extern __shared__ double dyn[];
     const int m = lr.m, tid = threadIdx.x;
-    const CorrJob jb = jobs[blockIdx.x];
     V *u = reinterpret_cast<V *>(dyn), *pr = u + m;
     T *zs = reinterpret_cast<T *>(pr + (MODE ? 256 : 64 * 8));
     const V *Sinv;
@@ -1593,12 +1358,12 @@ __global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
                     ff32 zk{0.f, 0.f};
                     for (int h = 0; h < groups; ++h) zk = ff_add(zk, ff_of(pr[h * cols + tid]));
                     zs[k0 + tid] = ff_to_float(zk);
-                    if (lr.zpub && blockIdx.x == 0) lr.zpub[k0 + tid] = ff_to_double(zk);
+                    if (lr.zpub && first) lr.zpub[k0 + tid] = ff_to_double(zk);
                 } else {
                     double zk = 0.0;
                     for (int h = 0; h < groups; ++h) zk += pr[h * cols + tid];
                     zs[k0 + tid] = zk;
-                    if (lr.zpub && blockIdx.x == 0) lr.zpub[k0 + tid] = zk;
+                    if (lr.zpub && first) lr.zpub[k0 + tid] = zk;
                 }
             }
             __syncthreads();
@@ -1613,16 +1378,22 @@ __global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
     }
 }
 
+template <typename T, int MODE, int NQ>
+__global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
+    k_lr_correct(T *x, LowRankArg lr, int P, CorrRows C, const CorrJob *__restrict__ jobs, const int *__restrict__ jobcols) {
+    extern __shared__ double dyn[];
+    lr_correct_body<T, MODE, NQ>(x, lr, P, C, jobs[blockIdx.x], jobcols, blockIdx.x == 0, dyn);
+}
+
 // dst -= B_c Sigma^{-1} y over the rows of the coarse level's B, y from the
 // partial sums of k_bt_partial: the low-rank term of a residual-restriction
 // (k_add_Bq's arithmetic).  The rows are known before the wait; dst was
 // written by the kernel before k_bt_partial.
 template <typename T>
-__global__ void __launch_bounds__(256)
-    k_resid_Bq(T *dst, i64 nrows, const i64 *__restrict__ rows, const i64 *__restrict__ ptr, const int *__restrict__ col,
-               const double *__restrict__ val, const double *lrpart, int m, int P, const double *__restrict__ sigma_inv) {
-    extern __shared__ double qs[];
-    const i64 r = (i64)blockIdx.x * 256 + threadIdx.x;
+__device__ __forceinline__ void resid_Bq_body(T *dst, i64 nrows, const i64 *__restrict__ rows, const i64 *__restrict__ ptr,
+                                              const int *__restrict__ col, const double *__restrict__ val,
+                                              const double *lrpart, int m, int P, const double *__restrict__ sigma_inv,
+                                              i64 r, double *qs) {
     i64 row = 0, e0 = 0, e1 = 0;
     double v0 = 0.0;
     int c0 = 0;
@@ -1654,6 +1425,14 @@ __global__ void __launch_bounds__(256)
     double acc = v0 * qs[c0];
     for (i64 e = e0 + 1; e < e1; ++e) acc += val[e] * qs[col[e]];
     dst[row] = d + (T)(-1.0 * acc);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_resid_Bq(T *dst, i64 nrows, const i64 *__restrict__ rows, const i64 *__restrict__ ptr, const int *__restrict__ col,
+               const double *__restrict__ val, const double *lrpart, int m, int P, const double *__restrict__ sigma_inv) {
+    extern __shared__ double qs[];
+    resid_Bq_body<T>(dst, nrows, rows, ptr, col, val, lrpart, m, P, sigma_inv, (i64)blockIdx.x * 256 + threadIdx.x, qs);
 }
 
 // ------------------------------------------------- residual + restriction
@@ -3111,28 +2890,36 @@ struct BatchChainArg {
 };
 
 // Low-rank data of one chain on one level and sweep direction: the B^T x
-// arguments and C = M^{-1} B by rows.
+// arguments, C = M^{-1} B by rows and its CTAs' columns.
 struct BatchLowRank {
     LowRankArg lr;
     CorrRows C;  // x += C z rows (FP32 values)
+    const int *jobcols;
+    int P;       // partial sums per column
 };
 
 // B^T x work unit: chain, column j, part p of P.
 struct BtJob {
     int chain, j, p, P;
 };
-// Row range [r0, r1) of one chain's sparse rows.
+// A CTA of one chain's correction.
+struct BatchCorrJob {
+    int chain;
+    CorrJob job;
+};
+// Up to 256 rows from r0 on of one chain's B_c Sigma^{-1} y.
 struct RowJob {
     int chain;
-    i64 r0, r1;
+    i64 r0;
 };
 // B_c Sigma^{-1} y rows of one chain's coarse level (the residual's
-// low-rank term), destination its coarse f.
+// low-rank term), y from its partial sums, destination its coarse f.
 struct BatchAddBq {
     i64 nrows;
     const i64 *rows, *ptr;
     const int *col;
-    const double *val, *y, *sigma_inv;
+    const double *val, *part, *sigma_inv;
+    int m, P;
     float *dst;
 };
 
@@ -3164,7 +2951,7 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_vec_batch(const BatchL
     load_stencil_shared(ss, a.s);
     const NoiseArgs nz = batch_noise(ca[chain], invocation, level);
     const float *fsc = FS ? a.fsplit + colour * a.fhalf : nullptr;
-    sweep_rb_vec_body<NOISE, false, V8, FS, false>(a.x, a.f, g, ss, colour, reverse, nz, nullptr, fsc, blockIdx.x, blockIdx.y,
+    sweep_rb_vec_body<NOISE, false, V8, FS, true>(a.x, a.f, g, ss, colour, reverse, nz, nullptr, fsc, blockIdx.x, blockIdx.y,
                                             bz);
 }
 
@@ -3180,7 +2967,7 @@ __global__ void __launch_bounds__(ROW_PAIR_THREADS)
     load_stencil_shared(ss, a.s);
     const NoiseArgs nz = batch_noise(ca[chain], invocation, level);
     sweep_row_pair_body<float, 27, false, NOISE, 0>(a.x, a.f, g, ss, pb, pc, odd_first, nz, VarField<float>{nullptr, 0},
-                                                    blockIdx.y, bz, reinterpret_cast<float *>(row_sm), false, false);
+                                                    blockIdx.y, bz, reinterpret_cast<float *>(row_sm), true, true);
 }
 
 // one colour of an 8-colour level with rows too long for a CTA, grid.z =
@@ -3195,59 +2982,42 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_c27_batch(const BatchLeve
     const BatchLevelArg &a = la[chain];
     load_stencil_shared(ss, a.s);
     const NoiseArgs nz = batch_noise(ca[chain], invocation, level);
+    pdl_begin();
     sweep_c27_body<float, false, NOISE, 0>(a.x, a.f, g, ss, colour, nz, VarField<float>{nullptr, 0}, blockIdx.x,
                                            blockIdx.y, bz);
 }
 
-// B^T x partial sums with the per-chain solve in each chain's last CTA
-// (SOLVE: the low-rank correction's coefficients; otherwise y = B^T x of the
-// residual), one CTA per job
-template <int NOISE, bool SOLVE>
-__global__ void __launch_bounds__(256) k_bt_solve_batch(const BatchLevelArg *__restrict__ la,
-                                                        const BatchLowRank *__restrict__ lrs,
-                                                        const BatchChainArg *__restrict__ ca,
-                                                        const BtJob *__restrict__ jobs, unsigned invocation,
-                                                        unsigned level) {
-    const BtJob jb = jobs[blockIdx.x];
-    const LowRankArg lr = lrs[jb.chain].lr;
-    const NoiseArgs nz = batch_noise(ca[jb.chain], invocation, level);
-    bt_solve_body<float, NOISE, SOLVE>(la[jb.chain].x, lr, nz, jb.j, jb.p, jb.P);
-}
-
-// x += C z over a row range of one chain (the per-row arithmetic of
-// k_lr_scatter)
-__global__ void __launch_bounds__(256) k_lr_scatter_batch(const BatchLevelArg *__restrict__ la,
+// B^T x partial sums and the low-rank noise (NOISE_NONE: the residual's), one
+// CTA per job
+template <int NOISE>
+__global__ void __launch_bounds__(256) k_bt_partial_batch(const BatchLevelArg *__restrict__ la,
                                                           const BatchLowRank *__restrict__ lrs,
-                                                          const RowJob *__restrict__ jobs) {
-    const RowJob jb = jobs[blockIdx.x];
-    const BatchLowRank &c = lrs[jb.chain];
-    const CorrRows &C = c.C;
-    float *x = la[jb.chain].x;
-    const float *z = c.lr.zf;
-    const float *v1 = static_cast<const float *>(C.v1);
-    for (i64 r = jb.r0 + threadIdx.x; r < jb.r1; r += blockDim.x) {
-        if (r < C.n1) {
-            const unsigned row = C.r1[r];
-            float acc = 0.f;
-            acc += v1[r] * z[C.c1[r]];
-            x[row] = x[row] + acc;
-        } else {
-            corr_multi_row(x, C, r - C.n1, z);
-        }
-    }
+                                                          const BatchChainArg *__restrict__ ca,
+                                                          const BtJob *__restrict__ jobs, unsigned invocation,
+                                                          unsigned level) {
+    const BtJob jb = jobs[blockIdx.x];
+    LowRankArg lr = lrs[jb.chain].lr;
+    if (NOISE == NOISE_NONE) lr.w = nullptr;
+    bt_partial_body<float, NOISE>(la[jb.chain].x, lr, batch_noise(ca[jb.chain], invocation, level), jb.j, jb.p, jb.P);
 }
 
-// f_c -= B_c Sigma^{-1} y over a row range of one chain (the per-row
-// arithmetic of k_add_Bq with sign -1)
-__global__ void __launch_bounds__(256) k_add_Bq_batch(const BatchAddBq *__restrict__ bq,
-                                                      const RowJob *__restrict__ jobs) {
+// the solve and x += C z, one CTA per job
+template <int MODE>
+__global__ void __launch_bounds__(256, MODE == 1 ? 2 : 4)
+    k_lr_correct_batch(const BatchLevelArg *__restrict__ la, const BatchLowRank *__restrict__ lrs,
+                       const BatchCorrJob *__restrict__ jobs) {
+    extern __shared__ double dyn[];
+    const BatchCorrJob jb = jobs[blockIdx.x];
+    const BatchLowRank &c = lrs[jb.chain];
+    lr_correct_body<float, MODE, 1>(la[jb.chain].x, c.lr, c.P, c.C, jb.job, c.jobcols, false, dyn);
+}
+
+// f_c -= B_c Sigma^{-1} y, one CTA per job
+__global__ void __launch_bounds__(256) k_resid_Bq_batch(const BatchAddBq *__restrict__ bq, const RowJob *__restrict__ jobs) {
+    extern __shared__ double qs[];
     const RowJob jb = jobs[blockIdx.x];
     const BatchAddBq &a = bq[jb.chain];
-    for (i64 r = jb.r0 + threadIdx.x; r < jb.r1; r += blockDim.x) {
-        double acc = 0.0;
-        for (i64 e = a.ptr[r]; e < a.ptr[r + 1]; ++e) acc += a.val[e] * (a.y[a.col[e]] * a.sigma_inv[a.col[e]]);
-        a.dst[a.rows[r]] += (float)(-1.0 * acc);
-    }
+    resid_Bq_body<float>(a.dst, a.nrows, a.rows, a.ptr, a.col, a.val, a.part, a.m, a.P, a.sigma_inv, jb.r0 + threadIdx.x, qs);
 }
 
 // residual + restriction, grid.z = chains x coarse tiles in z
@@ -3266,6 +3036,7 @@ __global__ void __launch_bounds__(RR_THREADS, MGMC_RR_BATCH_MINB) k_resid_restri
     const int chain = blockIdx.z / tz, bz = blockIdx.z - chain * tz;
     const BatchLevelArg &a = la[chain];
     load_stencil_shared(ss, a.s);
+    pdl_begin();
     resid_restrict_tiled_body<float, NPT>(a.x, a.f, a.fc, a.xc, gf, gc, ss, rr_smem_b, blockIdx.x, blockIdx.y, bz);
 }
 
@@ -3274,6 +3045,7 @@ __global__ void __launch_bounds__(128) k_prolong_batch(const BatchLevelArg *__re
                                                        float alpha, int dim, int nzc) {
     const int chain = blockIdx.z / nzc, bz = blockIdx.z - chain * nzc;
     const BatchLevelArg &a = la[chain];
+    pdl_begin();
     prolong_add_body<float>(a.x, a.xc, gf, gc, alpha, dim, blockIdx.x, blockIdx.y, nzc - 1 - bz);
 }
 
@@ -3285,6 +3057,7 @@ __global__ void __launch_bounds__(256) k_chol_lower_batch(const BatchLevelArg *_
     extern __shared__ __align__(16) unsigned char chol_sm_b[];
     const BatchChainArg &c = ca[blockIdx.y];
     const NoiseArgs nz = batch_noise(c, invocation, level);
+    pdl_begin();
     chol_gemv_lower_body<float, float, NOISE>(la[blockIdx.y].f, g, c.Linv, ld, c.gv, nz, chol_sm_b, blockIdx.x,
                                               gridDim.x);
 }
@@ -3293,6 +3066,7 @@ __global__ void __launch_bounds__(256) k_chol_upper_batch(const BatchLevelArg *_
                                                           const BatchChainArg *__restrict__ ca, Grid3 g, int ld) {
     extern __shared__ __align__(16) unsigned char chol_sm_b[];
     const BatchChainArg &c = ca[blockIdx.y];
+    pdl_begin();
     chol_gemv_upper_body<float, float>(c.gv, g, c.LinvT, ld, la[blockIdx.y].x, chol_sm_b, blockIdx.x, gridDim.x);
 }
 
@@ -3300,6 +3074,7 @@ __global__ void __launch_bounds__(256) k_chol_upper_batch(const BatchLevelArg *_
 __global__ void __launch_bounds__(256) k_step_end_batch(const BatchLevelArg *__restrict__ la,
                                                         const BatchChainArg *__restrict__ ca) {
     const BatchChainArg &c = ca[blockIdx.y];
+    pdl_begin();
     step_end_body<float>(la[blockIdx.y].x, c.nprobe, c.bptr, c.bidx, c.bval, c.obs, c.capacity, c.obs_count, c.d_step,
                          c.err, c.done, blockIdx.x, gridDim.x);
 }
