@@ -158,7 +158,8 @@ struct Sampler {
     unsigned *d_err = nullptr;
     double *d_obs = nullptr;
     i64 obs_cap = 0;
-    int nprobe = 0;
+    int nprobe = 0, obs_split = 1;  // observables, and CTAs per observable
+    double *d_obs_part = nullptr;   // their partial sums
     i64 *d_bptr = nullptr, *d_bidx = nullptr;
     double *d_bval = nullptr;
     unsigned *d_done = nullptr;
@@ -296,6 +297,7 @@ struct Sampler {
     void resid_restrict(int lev);
     void prolong(int lev, double alpha, void *xc, void *x);
     void step_end();
+    StepEnd step_end_args() const;
     void ensure_scratch(int lev);
     void check_launch();
     NoiseArgs noise_args(int lev, i64 count);
@@ -944,13 +946,17 @@ void Sampler::smooth(int lev, bool forward, int nsmooth) {
     for (int k = 0; k < nsmooth; ++k) sor(lev, forward, noisy, lv.x, lv.f, nsmooth);
 }
 
+StepEnd Sampler::step_end_args() const {
+    return StepEnd{nprobe, obs_split, d_bptr, d_bidx, d_bval, d_obs_part, d_obs, obs_cap, d_obs_count, d_step, d_err, d_done};
+}
+
 void Sampler::step_end() {
+    const StepEnd e = step_end_args();
+    const unsigned blocks = (unsigned)std::max(nprobe * obs_split, 1);
     if (fp32)
-        plaunch(pdl, k_step_end<float>, std::max(nprobe, 1), 256, 0, stream, (const float *)L[0].x, nprobe, d_bptr, d_bidx, d_bval, d_obs,
-                                                                  obs_cap, d_obs_count, d_step, d_err, d_done);
+        plaunch(pdl, k_step_end<float>, blocks, 256, 0, stream, (const float *)L[0].x, e);
     else
-        plaunch(pdl, k_step_end<double>, std::max(nprobe, 1), 256, 0, stream, (const double *)L[0].x, nprobe, d_bptr, d_bidx, d_bval,
-                                                                   d_obs, obs_cap, d_obs_count, d_step, d_err, d_done);
+        plaunch(pdl, k_step_end<double>, blocks, 256, 0, stream, (const double *)L[0].x, e);
     launches++;
 }
 
@@ -2529,6 +2535,10 @@ static void set_probes(Sampler &S, int nprobe, const int64_t *ptr, const int64_t
     S.d_bval = S.upload(v);
     S.d_obs = S.alloc<double>((size_t)std::max<int64_t>(capacity, 1) * std::max(nprobe, 1));
     S.nprobe = nprobe;
+    S.obs_split = 1;
+    for (int q = 0; q < nprobe; ++q)  // CTAs of about STEP_END_ENTRIES entries of the longest probe
+        S.obs_split = (int)std::max<i64>(S.obs_split, std::min<i64>(STEP_END_MAX_SPLIT, (pptr[q + 1] - pptr[q] + STEP_END_ENTRIES - 1) / STEP_END_ENTRIES));
+    S.d_obs_part = S.alloc<double>((size_t)std::max(nprobe, 1) * S.obs_split);
     S.obs_cap = capacity;
     CK(cudaMemsetAsync(S.d_obs_count, 0, sizeof(u64), S.stream));
     // the captured step embeds the observable arguments: capture again
@@ -2872,7 +2882,7 @@ void BatchGroup::build(cudaStream_t st) {
     n_bq.assign(nlev, 0);
     for (Sampler *S : ch) {
         max_m = std::max(max_m, S->m);
-        max_probe = std::max(max_probe, S->nprobe);
+        max_probe = std::max(max_probe, S->nprobe * S->obs_split);
     }
     for (int lev = 0; lev < nlev; ++lev) {
         std::vector<BatchLevelArg> a(G);
@@ -2951,15 +2961,7 @@ void BatchGroup::build(cudaStream_t st) {
         A.Linv = (const float *)S.dLinv;
         A.LinvT = (const float *)S.dLinvT;
         A.gv = (float *)S.dgv;
-        A.nprobe = S.nprobe;
-        A.bptr = S.d_bptr;
-        A.bidx = S.d_bidx;
-        A.bval = S.d_bval;
-        A.obs = S.d_obs;
-        A.capacity = S.obs_cap;
-        A.obs_count = S.d_obs_count;
-        A.err = S.d_err;
-        A.done = S.d_done;
+        A.end = S.step_end_args();
     }
     ca = put(c, st);
     CK(cudaStreamSynchronize(st));

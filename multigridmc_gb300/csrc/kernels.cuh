@@ -2517,48 +2517,94 @@ __global__ void __launch_bounds__(256) k_pgrad_coarse_sigma(const double *__rest
 }
 
 // ------------------------------------------------------------ step end
-// Observables z_p = b_p^T x of measure_sampling_time (sampling_time.cc:40),
-// one CTA per probe p (probe p's entries are bptr[p]..bptr[p+1]), stored at
-// obs[k * nprobe + p] for step k while k < capacity; a non-finite value
-// raises the error flag.  The last CTA to finish advances the observation
-// count and the step counter that keys the Philox streams.  Runs after
-// every other kernel of the step.
+// Observables z_p = b_p^T x of measure_sampling_time (sampling_time.cc:40):
+// CTA (p, q), q < split, sums its share of probe p's entries
+// bptr[p]..bptr[p+1] into part[p split + q]; the last CTA to finish adds the
+// shares in order, stores z_p at obs[k * nprobe + p] for step k while
+// k < capacity (a non-finite value raises the error flag) and advances the
+// observation count and the step counter that keys the Philox streams.  Runs
+// after every other kernel of the step.  The entries do not depend on the
+// step: a CTA's first 1024 are loaded before the wait.  (The central ball of
+// 256^3, 8,700 entries: one CTA took 18.6 us under ncu, its loads one after
+// the other and its sums on one SM's FP64 unit; nine CTAs 7.)
+struct StepEnd {
+    int nprobe, split;
+    const i64 *bptr, *bidx;
+    const double *bval;
+    double *part, *obs;
+    i64 capacity;
+    u64 *obs_count, *d_step;
+    unsigned *err, *done;
+};
+constexpr int STEP_END_ENTRIES = 1024, STEP_END_MAX_SPLIT = 16;
+
+__device__ __forceinline__ double to_double(double v) { return v; }
+__device__ __forceinline__ double to_double(float v) {  // widen, for any value
+    const unsigned m = __float_as_uint(v) & 0x7fffffffu;
+    return m - 0x00800000u < 0x7f000000u || m == 0u ? widen(v) : (double)v;
+}
+
 template <typename T>
-__device__ __forceinline__ void step_end_body(const T *__restrict__ x, int nprobe, const i64 *__restrict__ bptr,
-                                              const i64 *__restrict__ bidx, const double *__restrict__ bval,
-                                              double *__restrict__ obs, i64 capacity, u64 *__restrict__ obs_count,
-                                              u64 *__restrict__ d_step, unsigned *__restrict__ err,
-                                              unsigned *__restrict__ done, int p, int nblocks) {
+__device__ __forceinline__ void step_end_body(const T *x, const StepEnd &e, int cta, int nblocks) {
     __shared__ double sh[32];
     __shared__ bool last;
-    if (nprobe > 0 && p < nprobe) {
+    const int p = e.split ? cta / e.split : 0, q = cta - p * e.split;
+    const bool mine = p < e.nprobe;
+    i64 lo = 0, hi = 0, idx[4];
+    double val[4];
+    if (mine) {
+        const i64 b0 = e.bptr[p], b1 = e.bptr[p + 1], len = (b1 - b0 + e.split - 1) / e.split;
+        lo = b0 + q * len + threadIdx.x;
+        hi = min(b1, b0 + (q + 1) * len);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (lo + 256 * t < hi) {
+                idx[t] = e.bidx[lo + 256 * t];
+                val[t] = e.bval[lo + 256 * t];
+            }
+    }
+    pdl_begin();
+    if (mine) {
         double acc = 0.0;
-        for (i64 e = bptr[p] + threadIdx.x; e < bptr[p + 1]; e += blockDim.x) acc += bval[e] * (double)x[bidx[e]];
+        T xv[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (lo + 256 * t < hi) xv[t] = x[idx[t]];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (lo + 256 * t < hi) acc = fma(val[t], to_double(xv[t]), acc);
+#pragma unroll 4
+        for (i64 i = lo + STEP_END_ENTRIES; i < hi; i += 256) acc = fma(e.bval[i], to_double(x[e.bidx[i]]), acc);
         acc = block_sum<256>(acc, sh);
-        if (threadIdx.x == 0) {
-            const u64 k = *obs_count;
-            if ((i64)k < capacity) obs[k * nprobe + p] = acc;
-            if (!isfinite(acc)) atomicOr(err, 1u);
+        if (threadIdx.x == 0) e.part[cta] = acc;
+    }
+    if (threadIdx.x == 0) {
+        unsigned prev;  // publishes the partial sum; in the last CTA, makes the others visible
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(e.done) : "memory");
+        last = prev == (unsigned)nblocks - 1u;
+    }
+    __syncthreads();
+    if (!last) return;
+    if (e.nprobe > 0) {
+        const u64 k = *e.obs_count;
+        for (int r = threadIdx.x; r < e.nprobe; r += blockDim.x) {
+            double z = 0.0;
+            for (int t = 0; t < e.split; ++t) z += __ldcg(e.part + (i64)r * e.split + t);
+            if ((i64)k < e.capacity) e.obs[k * e.nprobe + r] = z;
+            if (!isfinite(z)) atomicOr(e.err, 1u);
         }
     }
-    __threadfence();
-    if (threadIdx.x == 0) last = (atomicAdd(done, 1u) == (unsigned)nblocks - 1u);
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        if (nprobe > 0) *obs_count += 1ull;
-        *d_step += 1ull;
-        *done = 0u;
+    if (threadIdx.x == 0) {
+        if (e.nprobe > 0) *e.obs_count += 1ull;
+        *e.d_step += 1ull;
+        *e.done = 0u;
     }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_step_end(const T *__restrict__ x, int nprobe, const i64 *__restrict__ bptr,
-                                                   const i64 *__restrict__ bidx, const double *__restrict__ bval,
-                                                   double *__restrict__ obs, i64 capacity, u64 *__restrict__ obs_count,
-                                                   u64 *__restrict__ d_step, unsigned *__restrict__ err,
-                                                   unsigned *__restrict__ done) {
-    pdl_begin();
-    step_end_body<T>(x, nprobe, bptr, bidx, bval, obs, capacity, obs_count, d_step, err, done, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(256) k_step_end(const T *x, StepEnd e) {
+    step_end_body<T>(x, e, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------- low-rank Cholesky sampler
@@ -2880,13 +2926,7 @@ struct BatchChainArg {
     u64 *d_step;
     const float *Linv, *LinvT;
     float *gv;
-    int nprobe;
-    const i64 *bptr, *bidx;
-    const double *bval;
-    double *obs;
-    i64 capacity;
-    u64 *obs_count;
-    unsigned *err, *done;
+    StepEnd end;
 };
 
 // Low-rank data of one chain on one level and sweep direction: the B^T x
@@ -3073,10 +3113,7 @@ __global__ void __launch_bounds__(256) k_chol_upper_batch(const BatchLevelArg *_
 // observables and step counters, grid.y = chains
 __global__ void __launch_bounds__(256) k_step_end_batch(const BatchLevelArg *__restrict__ la,
                                                         const BatchChainArg *__restrict__ ca) {
-    const BatchChainArg &c = ca[blockIdx.y];
-    pdl_begin();
-    step_end_body<float>(la[blockIdx.y].x, c.nprobe, c.bptr, c.bidx, c.bval, c.obs, c.capacity, c.obs_count, c.d_step,
-                         c.err, c.done, blockIdx.x, gridDim.x);
+    step_end_body<float>(la[blockIdx.y].x, ca[blockIdx.y].end, blockIdx.x, gridDim.x);
 }
 
 }  // namespace mgmc
