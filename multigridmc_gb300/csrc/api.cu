@@ -155,7 +155,11 @@ struct Sampler {
     // bookkeeping
     cudaStream_t stream = nullptr;
     u64 *d_step = nullptr, *d_obs_count = nullptr;
-    unsigned *d_err = nullptr;
+    // error bits: page-locked host memory that kernels write (rarely) and the
+    // host reads after a synchronisation, without a copy of its own
+    unsigned *h_err = nullptr, *d_err = nullptr;
+    char *h_stage = nullptr;  // behind them, staging of observation counts and values
+    static constexpr size_t STAGE_BYTES = 16 * 1024;
     double *d_obs = nullptr;
     i64 obs_cap = 0;
     int nprobe = 0, obs_split = 1;  // observables, and CTAs per observable
@@ -227,6 +231,7 @@ struct Sampler {
         if (pa_exec) cudaGraphExecDestroy(pa_exec);
         if (pa_graph) cudaGraphDestroy(pa_graph);
         for (void *p : owned) cudaFree(p);
+        if (h_err) cudaFreeHost(h_err);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -1395,12 +1400,14 @@ void Sampler::build(const mgmc_operator_desc &op) {
     raise_smem_limit(k_resid_restrict_tma<double, 27>, rr_tma_smem_bytes<double>());
     d_step = alloc<u64>(1);
     d_obs_count = alloc<u64>(1);
-    d_err = alloc<unsigned>(1);
+    CK(cudaHostAlloc((void **)&h_err, 64 + STAGE_BYTES, cudaHostAllocMapped));
+    *h_err = 0;
+    h_stage = (char *)h_err + 64;
+    CK(cudaHostGetDevicePointer((void **)&d_err, h_err, 0));
     d_done = alloc<unsigned>(1);
     CK(cudaMemsetAsync(d_done, 0, sizeof(unsigned), stream));
     CK(cudaMemsetAsync(d_step, 0, sizeof(u64), stream));
     CK(cudaMemsetAsync(d_obs_count, 0, sizeof(u64), stream));
-    CK(cudaMemsetAsync(d_err, 0, sizeof(unsigned), stream));
     // levels
     Geometry geo(dim, cells[0], cells[1], cells[2]);
     double st[27];
@@ -1705,9 +1712,11 @@ static void get_vec(Sampler &S, int lev, const void *src, double *dst, int on_de
 // step counter).
 // Error bits raised on the device: 1 = non-finite observable, 2 = a tile
 // copy wait ran out.
+static unsigned device_errors(Sampler &S) { return *(volatile unsigned *)S.h_err; }
+
+// after a synchronisation with the sampler's work
 static void check_device_errors(Sampler &S) {
-    unsigned err = 0;
-    CK(cudaMemcpy(&err, S.d_err, sizeof(err), cudaMemcpyDeviceToHost));
+    const unsigned err = device_errors(S);
     if (err & ERR_TILE_TIMEOUT) fail(MGMC_ERR_CUDA, "a shared-memory tile copy did not complete in time");
     if (err) fail(MGMC_ERR_NONFINITE, "non-finite observable in the chain");
 }
@@ -2573,15 +2582,24 @@ mgmc_status mgmc_sampler_read_observations(mgmc_sampler *s, double *out, int64_t
     API_BEGIN
     Sampler &S = impl(s);
     if (!count) fail(MGMC_ERR_INVALID_ARGUMENT, "null count");
-    CK(cudaStreamSynchronize(S.stream));
-    u64 c = 0;
-    CK(cudaMemcpy(&c, S.d_obs_count, sizeof(c), cudaMemcpyDeviceToHost));
-    i64 k = std::min<i64>((i64)c, S.obs_cap);
+    // the count and the values (as many as fit the staging buffer) with one
+    // synchronisation
     const int np = std::max(S.nprobe, 1);
-    k = std::min<i64>(k, capacity / np);
-    if (k > 0 && out) CK(cudaMemcpy(out, S.d_obs, (size_t)k * np * sizeof(double), cudaMemcpyDeviceToHost));
+    const i64 most = std::max<i64>(0, std::min<i64>(S.obs_cap, capacity / np)) * np;  // values the caller takes
+    const i64 staged = std::min<i64>(most, (i64)((Sampler::STAGE_BYTES - sizeof(u64)) / sizeof(double)));
+    double *values = (double *)(S.h_stage + sizeof(u64));
+    CK(cudaMemcpyAsync(S.h_stage, S.d_obs_count, sizeof(u64), cudaMemcpyDeviceToHost, S.stream));
+    if (staged > 0 && out) CK(cudaMemcpyAsync(values, S.d_obs, staged * sizeof(double), cudaMemcpyDeviceToHost, S.stream));
+    CK(cudaMemsetAsync(S.d_obs_count, 0, sizeof(u64), S.stream));
+    CK(cudaStreamSynchronize(S.stream));
+    u64 c;
+    std::memcpy(&c, S.h_stage, sizeof(c));
+    const i64 k = std::min<i64>((i64)std::min<u64>(c, (u64)INT64_MAX / (u64)np) * np, most);
+    if (k > 0 && out) {
+        std::copy(values, values + std::min(k, staged), out);
+        if (k > staged) CK(cudaMemcpy(out + staged, S.d_obs + staged, (k - staged) * sizeof(double), cudaMemcpyDeviceToHost));
+    }
     *count = (int64_t)c;
-    CK(cudaMemset(S.d_obs_count, 0, sizeof(u64)));
     check_device_errors(S);
     API_END
 }
@@ -2629,8 +2647,7 @@ mgmc_status mgmc_sampler_synchronize(mgmc_sampler *s) {
     API_BEGIN
     Sampler &S = impl(s);
     CK(cudaStreamSynchronize(S.stream));
-    unsigned err = 0;
-    CK(cudaMemcpy(&err, S.d_err, sizeof(err), cudaMemcpyDeviceToHost));
+    const unsigned err = device_errors(S);
     if (err & ERR_TILE_TIMEOUT) fail(MGMC_ERR_CUDA, "a shared-memory tile copy did not complete in time");
     API_END
 }

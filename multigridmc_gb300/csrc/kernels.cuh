@@ -1717,7 +1717,7 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict_tma(const __grid_
     }
     const bool ok = mbar_wait_bounded(&bar, 0, TILE_WAIT_NS);
     if (__syncthreads_or(!ok)) {
-        if (threadIdx.x == 0) atomicOr(err, ERR_TILE_TIMEOUT);
+        if (threadIdx.x == 0) atomicOr_system(err, ERR_TILE_TIMEOUT);
         mbar_wait_bounded(&bar, 0, TILE_WAIT_NS);  // let copies in flight land before the CTA exits
         return;
     }
@@ -2591,7 +2591,7 @@ __device__ __forceinline__ void step_end_body(const T *x, const StepEnd &e, int 
             double z = 0.0;
             for (int t = 0; t < e.split; ++t) z += __ldcg(e.part + (i64)r * e.split + t);
             if ((i64)k < e.capacity) e.obs[k * e.nprobe + r] = z;
-            if (!isfinite(z)) atomicOr(e.err, 1u);
+            if (!isfinite(z)) atomicOr_system(e.err, 1u);
         }
     }
     __syncthreads();
