@@ -2901,6 +2901,12 @@ void BatchGroup::build(cudaStream_t st) {
         max_m = std::max(max_m, S->m);
         max_probe = std::max(max_probe, S->nprobe * S->obs_split);
     }
+    // (beyond 2784 columns; the group's largest m sizes the launches of every mode)
+    if (lr_correct_smem(max_m) > 48 * 1024) {
+        raise_smem_limit(k_lr_correct_batch<0>, lr_correct_smem(max_m));
+        raise_smem_limit(k_lr_correct_batch<1>, lr_correct_smem(max_m));
+        raise_smem_limit(k_lr_correct_batch<2>, lr_correct_smem(max_m));
+    }
     for (int lev = 0; lev < nlev; ++lev) {
         std::vector<BatchLevelArg> a(G);
         std::vector<BatchLowRank> l0(G), l1(G);
