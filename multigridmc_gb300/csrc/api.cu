@@ -187,12 +187,17 @@ struct Sampler {
     void refresh_fsplit();
     // deterministic solver: LoopSolver around MultigridPreconditioner
     bool noisy = true;  // false while the preconditioner's noise-free cycle is recorded
-    double *sv_x = nullptr, *sv_b = nullptr, *sv_r = nullptr;  // FP64 iterate, rhs, residual (padded level 0)
-    double *sv_part = nullptr, *sv_norm = nullptr;             // |r|^2 partial sums and total
+    double *sv_x = nullptr, *sv_b = nullptr;     // FP64 iterate, rhs - B Sigma^{-1} B^T iterate (padded level 0)
+    double *sv_bB = nullptr;                     // the rhs on the rows of B
+    double *sv_part = nullptr, *d_norm = nullptr;  // |r|^2: partial sums, and the total in page-locked memory
+    unsigned *sv_counter = nullptr;
     int sv_np = 0;
+    void record_solve_resid(), record_solve_cycle();
+    double solve_norm2() const { return *(volatile double *)((char *)h_err + 32); }
     void *sv_keep_x = nullptr, *sv_keep_f = nullptr;  // the chain's x_0 and f_0 while a solve borrows them
-    cudaGraph_t rgraph = nullptr, pgraph = nullptr;   // residual + norm; preconditioner cycle
-    cudaGraphExec_t rexec = nullptr, pexec = nullptr;
+    // residual + norm; preconditioner cycle; the cycle and the next residual
+    cudaGraph_t rgraph = nullptr, pgraph = nullptr, prgraph = nullptr;
+    cudaGraphExec_t rexec = nullptr, pexec = nullptr, prexec = nullptr;
     std::vector<void *> owned;  // every device allocation
 
     template <typename P_>
@@ -228,6 +233,8 @@ struct Sampler {
         if (rgraph) cudaGraphDestroy(rgraph);
         if (pexec) cudaGraphExecDestroy(pexec);
         if (pgraph) cudaGraphDestroy(pgraph);
+        if (prexec) cudaGraphExecDestroy(prexec);
+        if (prgraph) cudaGraphDestroy(prgraph);
         if (pa_exec) cudaGraphExecDestroy(pa_exec);
         if (pa_graph) cudaGraphDestroy(pa_graph);
         for (void *p : owned) cudaFree(p);
@@ -799,9 +806,10 @@ static void launch_add_Bq(Sampler &S, Level &lv, void *dst, const double *y, dou
     S.launches++;
 }
 
-// dst -= B_c Sigma^{-1} B^T x: x on level lv, dst and B_c on the next one
+// dst -= B_c Sigma^{-1} B^T x: x on level lv, dst and B_c on level lc, the
+// next one or the same (base not null: dst = base - ... on the rows of B_c)
 template <typename T>
-static void launch_resid_lowrank(Sampler &S, Level &lv, Level &lc, const void *x, void *dst) {
+static void launch_resid_lowrank(Sampler &S, Level &lv, Level &lc, const void *x, void *dst, const T *base = nullptr) {
     const RowCsr &B = lc.Br;
     if (B.nrows == 0) return;
     LowRankArg lr{};
@@ -814,7 +822,7 @@ static void launch_resid_lowrank(Sampler &S, Level &lv, Level &lc, const void *x
     plaunch(S.pdl, k_bt_partial<T, NOISE_NONE>, dim3(S.m, lv.bt_split), 256, 0, S.stream, (const T *)x, lr, NoiseArgs{});
     plaunch(S.pdl, k_resid_Bq<T>, nblk(B.nrows, 256), 256, sizeof(double) * S.m, S.stream, (T *)dst, B.nrows,
             (const i64 *)B.rows, (const i64 *)B.ptr, (const int *)B.col, (const double *)B.val, (const double *)lv.part,
-            S.m, lv.bt_split, (const double *)S.d_sigma_inv);
+            S.m, lv.bt_split, (const double *)S.d_sigma_inv, base);
     S.launches += 2;
 }
 
@@ -1758,33 +1766,70 @@ static void run_steps(Sampler &S, i64 nsteps) {
 // preconditioner is the sampler's cycle with the noise switched off: the
 // same sweeps with their low-rank corrections, residual-restriction,
 // prolongation and coarse scaling, from a zero state, with the Cholesky
-// coarse solve.  Two graphs: the FP64 residual r = b - A x with |r|^2 (and
-// the preconditioner's input f_0 = r, x_0 = 0), and the cycle followed by
-// x += P r.
+// coarse solve.  Graphs: the FP64 residual r = b - A x with |r|^2 (and the
+// preconditioner's input f_0 = r, x_0 = 0); the cycle followed by x += P r;
+// and the second followed by the first, which is one iteration between two
+// tests of the norm (one gap between graphs instead of two).
 void Sampler::ensure_solver_buffers() {
     Level &l0 = L[0];
     const i64 na = l0.geo.nalloc;
     if (!sv_x) {
         sv_x = alloc<double>(na);
         sv_b = alloc<double>(na);
-        sv_r = alloc<double>(na);
-        for (double *p : {sv_x, sv_b, sv_r}) CK(cudaMemsetAsync(p, 0, (size_t)na * sizeof(double), stream));
-        const i64 nrows = (i64)l0.g.N1 * l0.g.N2;
-        sv_np = (int)((nrows + SOLVE_ROWS - 1) / SOLVE_ROWS);
+        for (double *p : {sv_x, sv_b}) CK(cudaMemsetAsync(p, 0, (size_t)na * sizeof(double), stream));
+        const i64 ntask = (i64)((l0.g.N0 + SOLVE_SEG - 1) / SOLVE_SEG) * l0.g.N1 * l0.g.N2;
+        sv_np = (int)std::min<i64>((ntask + 7) / 8, 4 * (i64)nsm);
         sv_part = alloc<double>(sv_np);
-        sv_norm = alloc<double>(1);
+        sv_counter = alloc<unsigned>(1);
+        CK(cudaMemsetAsync(sv_counter, 0, sizeof(unsigned), stream));
+        d_norm = (double *)((char *)d_err + 32);
+        if (m > 0 && l0.Br.nrows > 0) sv_bB = alloc<double>(l0.Br.nrows);
         sv_keep_x = talloc(na);
         sv_keep_f = talloc(na);
     }
 }
 
-void Sampler::ensure_solver() {
-    if (rexec && pexec) return;
-    if (!dLinv) build_coarse();
-    ensure_solver_buffers();
+template <typename T>
+static void launch_solve_resid(Sampler &S) {
+    Level &l0 = S.L[0];
+    const StencilArg<double> st = stencil_arg<double>(l0, S.P.omega);
+    const VarField<double> vf{l0.vw64, l0.geo.nalloc};
+    auto go = [&](auto kernel) {
+        kernel<<<S.sv_np, 256, 0, S.stream>>>(S.sv_x, S.sv_b, (T *)l0.f, (T *)l0.x, S.fsplit, S.fhalf, l0.g, st, vf, S.sv_part,
+                                              S.sv_counter, S.d_norm);
+    };
+    if (l0.var == 2)
+        go(k_solve_resid<T, 27, 2>);
+    else if (l0.var == 1)
+        l0.npt == 7 ? go(k_solve_resid<T, 7, 1>) : go(k_solve_resid<T, 27, 1>);
+    else
+        l0.npt == 7 ? go(k_solve_resid<T, 7, 0>) : go(k_solve_resid<T, 27, 0>);
+}
+
+void Sampler::record_solve_resid() {
+    Level &l0 = L[0];
+    if (m > 0) launch_resid_lowrank<double>(*this, l0, l0, sv_x, sv_b, sv_bB);
+    fp32 ? launch_solve_resid<float>(*this) : launch_solve_resid<double>(*this);
+}
+
+void Sampler::record_solve_cycle() {
     Level &l0 = L[0];
     const i64 na = l0.geo.nalloc;
+    noisy = false;
+    sample(0);
+    noisy = true;
+    if (fp32)
+        k_solve_update<float><<<nblk((na + 3) / 4, 256), 256, 0, stream>>>(sv_x, (const float *)l0.x, na);
+    else
+        k_solve_update<double><<<nblk((na + 3) / 4, 256), 256, 0, stream>>>(sv_x, (const double *)l0.x, na);
+}
+
+void Sampler::ensure_solver() {
+    if (rexec && pexec && prexec) return;
+    if (!dLinv) build_coarse();
+    ensure_solver_buffers();
     auto capture = [&](cudaGraph_t &g, cudaGraphExec_t &ge, const std::function<void()> &body) {
+        if (ge) return;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
             body();
@@ -1799,44 +1844,12 @@ void Sampler::ensure_solver() {
         CK(cudaStreamEndCapture(stream, &g));
         CK(cudaGraphInstantiate(&ge, g, 0));
     };
-    if (!rexec)
-        capture(rgraph, rexec, [&]() {
-            const StencilArg<double> st = stencil_arg<double>(l0, P.omega);
-            const VarField<double> vf{l0.vw64, l0.geo.nalloc};
-            if (l0.var == 2) {
-                k_solve_resid<27, 2><<<pack_grid(l0), 256, 0, stream>>>(sv_x, sv_b, sv_r, l0.g, st, vf);
-            } else if (l0.var == 1) {
-                if (l0.npt == 7)
-                    k_solve_resid<7, 1><<<pack_grid(l0), 256, 0, stream>>>(sv_x, sv_b, sv_r, l0.g, st, vf);
-                else
-                    k_solve_resid<27, 1><<<pack_grid(l0), 256, 0, stream>>>(sv_x, sv_b, sv_r, l0.g, st, vf);
-            } else if (l0.npt == 7) {
-                k_solve_resid<7, 0><<<pack_grid(l0), 256, 0, stream>>>(sv_x, sv_b, sv_r, l0.g, st, vf);
-            } else {
-                k_solve_resid<27, 0><<<pack_grid(l0), 256, 0, stream>>>(sv_x, sv_b, sv_r, l0.g, st, vf);
-            }
-            if (m > 0) {
-                launch_bt_plain<double>(*this, l0, sv_x);
-                launch_add_Bq<double>(*this, l0, sv_r, l0.y, -1.0);
-            }
-            if (fp32)
-                k_solve_rhs<float><<<sv_np, 256, 0, stream>>>(sv_r, (float *)l0.f, (float *)l0.x, l0.g, sv_part);
-            else
-                k_solve_rhs<double><<<sv_np, 256, 0, stream>>>(sv_r, (double *)l0.f, (double *)l0.x, l0.g, sv_part);
-            k_solve_norm<<<1, 256, 0, stream>>>(sv_part, sv_np, sv_norm);
-            refresh_fsplit();  // the cycle's fine sweeps read f = r through the colour split
-        });
-    if (!pexec)
-        capture(pgraph, pexec, [&]() {
-            noisy = false;
-            sample(0);
-            noisy = true;
-            const unsigned blocks = (unsigned)std::min<i64>(nblk(na, 256), 8 * nsm);
-            if (fp32)
-                k_solve_update<float><<<blocks, 256, 0, stream>>>(sv_x, (const float *)l0.x, na);
-            else
-                k_solve_update<double><<<blocks, 256, 0, stream>>>(sv_x, (const double *)l0.x, na);
-        });
+    capture(rgraph, rexec, [&]() { record_solve_resid(); });
+    capture(pgraph, pexec, [&]() { record_solve_cycle(); });
+    capture(prgraph, prexec, [&]() {
+        record_solve_cycle();
+        record_solve_resid();
+    });
 }
 
 // Edge weights of the fine stencil for the exact sampler's perturbation
@@ -2095,8 +2108,8 @@ void Sampler::ensure_param_adjoint() {
     tape_next.assign(nl, 0);
     tape_last.assign(nl, nullptr);
     tape_f.assign(nl, nullptr);
-    const i64 np0 = ((i64)L[0].g.N1 * L[0].g.N2 + SOLVE_ROWS - 1) / SOLVE_ROWS;
-    i64 cap = std::min<i64>(np0 * SOLVE_ROWS, 8 * (i64)nsm);
+    const i64 rows0 = ((i64)L[0].g.N1 * L[0].g.N2 + 7) / 8 * 8;
+    i64 cap = std::min<i64>(rows0, 8 * (i64)nsm);
     const int mm = std::max(m, 1);
     if (chol) {
         Level &lv = L.back();
@@ -3624,22 +3637,24 @@ mgmc_status mgmc_sampler_precondition(mgmc_sampler *s, const double *b, double *
 static int loop_solve(Sampler &S, double rtol, double atol, int maxiter, double *rnorm, bool *converged) {
     Level &l0 = S.L[0];
     CK(cudaMemsetAsync(S.sv_x, 0, (size_t)l0.geo.nalloc * sizeof(double), S.stream));
+    if (S.sv_bB) {
+        k_solve_gather<<<nblk(l0.Br.nrows, 256), 256, 0, S.stream>>>(S.sv_bB, S.sv_b, l0.Br.rows, l0.Br.nrows);
+        S.check_launch();
+    }
     int k = 0;
     double r0 = 0.0, rn = -1.0;
     bool conv = false;
+    if (maxiter > 0) CK(cudaGraphLaunch(S.rexec, S.stream));
     for (k = 0; k < maxiter; ++k) {
-        CK(cudaGraphLaunch(S.rexec, S.stream));
-        double r2 = 0.0;
-        CK(cudaMemcpyAsync(&r2, S.sv_norm, sizeof(double), cudaMemcpyDeviceToHost, S.stream));
         CK(cudaStreamSynchronize(S.stream));
-        rn = std::sqrt(r2);
+        rn = std::sqrt(S.solve_norm2());
         if (!std::isfinite(rn)) fail(MGMC_ERR_NONFINITE, "non-finite residual in the solver");
         if (k == 0) r0 = rn;  // |A 0 - b| = |b| (loop_solver.cc:11)
         if (rn / r0 < rtol && rn < atol) {
             conv = true;
             break;
         }
-        CK(cudaGraphLaunch(S.pexec, S.stream));
+        CK(cudaGraphLaunch(k + 1 < maxiter ? S.prexec : S.pexec, S.stream));
     }
     *rnorm = rn;
     *converged = conv;

@@ -27,10 +27,10 @@
 //   k_step_end          observables z = b^T x, step counter
 // Host conversions: k_unpack / k_unpack2 / k_pack; adjoint helpers: k_axpy,
 // k_sinvt_q; deterministic solver (FP64 loop around the noise-free cycle):
-// k_solve_resid, k_solve_rhs, k_solve_norm, k_solve_update; parameter
-// adjoint: k_pgrad_stencil, k_pgrad_combine, k_lowrank_normals,
-// k_coarse_normals, k_pgrad_coarse_phi, k_pgrad_coarse_sigma, k_accum_sum;
-// building blocks: k_apply_stencil.
+// k_solve_resid, k_solve_update, k_solve_gather; parameter adjoint:
+// k_pgrad_stencil, k_pgrad_combine, k_lowrank_normals, k_coarse_normals,
+// k_pgrad_coarse_phi, k_pgrad_coarse_sigma, k_accum_sum; building blocks:
+// k_apply_stencil.
 #pragma once
 
 #include <cstdint>
@@ -171,6 +171,11 @@ __device__ __forceinline__ double widen(float v) {
     const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu;
     const unsigned hi = (u & 0x80000000u) | (m < 0x00800000u ? 0u : (m >> 3) + 0x38000000u);
     return __hiloint2double((int)hi, m < 0x00800000u ? 0 : (int)(u << 29));
+}
+__device__ __forceinline__ double to_double(double v) { return v; }
+__device__ __forceinline__ double to_double(float v) {  // widen, for any value
+    const unsigned m = __float_as_uint(v) & 0x7fffffffu;
+    return m - 0x00800000u < 0x7f000000u || m == 0u ? widen(v) : (double)v;
 }
 
 // ------------------------------------------------------- exact arithmetic
@@ -1388,12 +1393,13 @@ __global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
 // dst -= B_c Sigma^{-1} y over the rows of the coarse level's B, y from the
 // partial sums of k_bt_partial: the low-rank term of a residual-restriction
 // (k_add_Bq's arithmetic).  The rows are known before the wait; dst was
-// written by the kernel before k_bt_partial.
+// written by the kernel before k_bt_partial.  base (not null): dst = base -
+// ... instead, base one value per row.
 template <typename T>
 __device__ __forceinline__ void resid_Bq_body(T *dst, i64 nrows, const i64 *__restrict__ rows, const i64 *__restrict__ ptr,
                                               const int *__restrict__ col, const double *__restrict__ val,
                                               const double *lrpart, int m, int P, const double *__restrict__ sigma_inv,
-                                              i64 r, double *qs) {
+                                              i64 r, double *qs, const T *base = nullptr) {
     i64 row = 0, e0 = 0, e1 = 0;
     double v0 = 0.0;
     int c0 = 0;
@@ -1407,7 +1413,7 @@ __device__ __forceinline__ void resid_Bq_body(T *dst, i64 nrows, const i64 *__re
     const double si = threadIdx.x < m ? sigma_inv[threadIdx.x] : 0.0;
     pdl_begin();
     pdl_trigger();
-    const T d = r < nrows ? dst[row] : T(0);
+    const T d = r < nrows ? (base ? base[r] : dst[row]) : T(0);
     for (int k = threadIdx.x; k < m; k += 256) {
         double y = 0.0;
         if constexpr (sizeof(T) == 4) {
@@ -1430,9 +1436,11 @@ __device__ __forceinline__ void resid_Bq_body(T *dst, i64 nrows, const i64 *__re
 template <typename T>
 __global__ void __launch_bounds__(256)
     k_resid_Bq(T *dst, i64 nrows, const i64 *__restrict__ rows, const i64 *__restrict__ ptr, const int *__restrict__ col,
-               const double *__restrict__ val, const double *lrpart, int m, int P, const double *__restrict__ sigma_inv) {
+               const double *__restrict__ val, const double *lrpart, int m, int P, const double *__restrict__ sigma_inv,
+               const T *base) {
     extern __shared__ double qs[];
-    resid_Bq_body<T>(dst, nrows, rows, ptr, col, val, lrpart, m, P, sigma_inv, (i64)blockIdx.x * 256 + threadIdx.x, qs);
+    resid_Bq_body<T>(dst, nrows, rows, ptr, col, val, lrpart, m, P, sigma_inv, (i64)blockIdx.x * 256 + threadIdx.x, qs,
+                     base);
 }
 
 // ------------------------------------------------- residual + restriction
@@ -2183,59 +2191,101 @@ __global__ void __launch_bounds__(256) k_add_Bz(T *dst, i64 nrows, const i64 *__
 // preconditioner: with an FP32 hierarchy the loop is iterative refinement
 // and still converges to FP64 accuracy.
 //
-// r = b - A_0 x over the interior (the low-rank term is added afterwards by
-// k_add_Bq with sign -1).
-template <int NPT, int VAR = 0>
+// r = b - A_0 x over the interior in FP64, with everything an iteration does
+// with it: |r|^2 (the partial sums of the CTAs, added in their order by the
+// CTA that finishes last, so the norm is reproducible; it goes to page-locked
+// host memory), the preconditioner's right hand side f = (T) r, its split by
+// colour (fs, may be null: k_split_colours' layout) and its zero initial
+// state (multigrid_preconditioner.cc:76).  b has B Sigma^{-1} B^T x
+// subtracted already (k_resid_Bq with k_solve_gather's values).  r itself is
+// not stored.
+//
+// A warp takes segments of SOLVE_SEG points of a row, its lanes consecutive
+// ones (CTAs of 256 threads along a row left half of the threads of 127
+// points idle), at most four CTAs per SM (one segment per warp: 48 us, the
+// reduction at the end of a CTA is FP64 work too).  Bound by the FP64 unit: 9
+// instructions a point of a 7-point stencil, 31 us at 127^3.  Measured there
+// under ncu: 42 us; 71 us for the residual (35), the right hand side with the
+// partial sums of the norm (19), their sum (6) and the split (11) in four
+// launches.
+constexpr int SOLVE_SEG = 128;
+template <typename T, int NPT, int VAR = 0>
 __global__ void __launch_bounds__(256) k_solve_resid(const double *__restrict__ x, const double *__restrict__ b,
-                                                     double *__restrict__ r, Grid3 g, StencilArg<double> s,
-                                                     VarField<double> vf) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x, bb = blockIdx.y, c = blockIdx.z;
-    if (a >= g.N0) return;
-    const i64 P = g.pad(a, bb, c);
-    r[P] = b[P] - stencil_row<double, NPT, false, VAR>(x, g, s, P, vf);
-}
-
-// Per CTA: SOLVE_ROWS rows (b, c) of the interior.  The partial sums of
-// |r|^2 go to part[blockIdx.x] (a fixed grid, so the norm is
-// reproducible); the preconditioner gets f = (T) r and the zero initial
-// state of MultigridPreconditioner::solve (multigrid_preconditioner.cc:76).
-constexpr int SOLVE_ROWS = 8;
-template <typename T>
-__global__ void __launch_bounds__(256) k_solve_rhs(const double *__restrict__ r, T *__restrict__ f,
-                                                   T *__restrict__ x, Grid3 g, double *__restrict__ part) {
+                                                     T *__restrict__ f, T *__restrict__ px, float *__restrict__ fs,
+                                                     i64 fhalf, Grid3 g, StencilArg<double> s, VarField<double> vf,
+                                                     double *part, unsigned *counter, double *norm) {
     __shared__ double sh[32];
-    const i64 nrows = (i64)g.N1 * g.N2;
+    __shared__ bool last;
+    const int nseg = (g.N0 + SOLVE_SEG - 1) / SOLVE_SEG;
+    const i64 ntask = (i64)g.N1 * g.N2 * nseg;
     double acc = 0.0;
-    for (int q = 0; q < SOLVE_ROWS; ++q) {
-        const i64 row = (i64)blockIdx.x * SOLVE_ROWS + q;
-        if (row >= nrows) break;
+    for (i64 task = (i64)blockIdx.x * 8 + (threadIdx.x >> 5); task < ntask; task += (i64)gridDim.x * 8) {
+        const i64 row = task / nseg;
         const int bb = (int)(row % g.N1), c = (int)(row / g.N1);
-        for (int a = threadIdx.x; a < g.N0; a += blockDim.x) {
-            const i64 P = g.pad(a, bb, c);
-            const double v = r[P];
-            acc += v * v;
-            f[P] = (T)v;
-            x[P] = T(0);
+        const int a0 = (int)(task - row * nseg) * SOLVE_SEG + (threadIdx.x & 31);
+        const i64 P0 = g.pad(a0, bb, c);
+#pragma unroll(NPT == 7 ? SOLVE_SEG / 32 : 1)
+        for (int q = 0; q < SOLVE_SEG / 32; ++q) {
+            const i64 P = P0 + 32 * q;
+            if (a0 + 32 * q >= g.N0) break;
+            double v = b[P];
+#pragma unroll
+            for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+                for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+                    for (int dx = -1; dx <= 1; ++dx) {
+                        if (NPT == 7 && (dz != 0) + (dy != 0) + (dx != 0) > 1) continue;
+                        v = fma(-vweight<double, VAR>(s, vf, P, (dz + 1) * 9 + (dy + 1) * 3 + dx + 1),
+                                x[P + dz * g.sz + dy * g.sy + dx], v);
+                    }
+            acc = fma(v, v, acc);
+            const T fv = (T)v;
+            f[P] = fv;
+            px[P] = T(0);
+            if (sizeof(T) == 4 && fs) fs[(i64)((a0 + 32 * q + bb + c) & 1) * fhalf + (P >> 1)] = (float)fv;
         }
     }
     acc = block_sum<256>(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc;
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = acc;
+        unsigned prev;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(counter) : "memory");
+        last = prev == gridDim.x - 1u;
+        if (last) *counter = 0u;
+    }
+    __syncthreads();
+    if (!last) return;
+    acc = 0.0;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += 256) acc += __ldcg(part + i);
+    acc = block_sum<256>(acc, sh);
+    if (threadIdx.x == 0) *norm = acc;
 }
 
-// |r|^2 = the sum of the partial sums, in one CTA.
-__global__ void __launch_bounds__(256) k_solve_norm(const double *__restrict__ part, int np, double *__restrict__ out) {
-    __shared__ double sh[32];
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) acc += part[i];
-    acc = block_sum<256>(acc, sh);
-    if (threadIdx.x == 0) *out = acc;
+// dst[r] = src[rows[r]]
+__global__ void __launch_bounds__(256) k_solve_gather(double *__restrict__ dst, const double *__restrict__ src,
+                                                      const i64 *__restrict__ rows, i64 nrows) {
+    const i64 r = (i64)blockIdx.x * 256 + threadIdx.x;
+    if (r < nrows) dst[r] = src[rows[r]];
 }
 
 // x += P r: the preconditioner's result (type T) added to the FP64 iterate
-// over whole padded arrays (ghosts are zero in both).
+// over whole padded arrays (ghosts are zero in both), four entries per
+// thread.
 template <typename T>
 __global__ void __launch_bounds__(256) k_solve_update(double *__restrict__ x, const T *__restrict__ dx, i64 n) {
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) x[i] += (double)dx[i];
+    typedef typename std::conditional<sizeof(T) == 4, float2, double2>::type T2;
+    const i64 i = 4 * ((i64)blockIdx.x * 256 + threadIdx.x);
+    if (i + 3 < n) {
+        double2 *xv = reinterpret_cast<double2 *>(x + i);
+        const T2 *dv = reinterpret_cast<const T2 *>(dx + i);
+        const double2 a = xv[0], b = xv[1];
+        const T2 d = dv[0], e = dv[1];
+        xv[0] = make_double2(a.x + to_double(d.x), a.y + to_double(d.y));
+        xv[1] = make_double2(b.x + to_double(e.x), b.y + to_double(e.y));
+    } else {
+        for (i64 k = i; k < n; ++k) x[k] += to_double(dx[k]);
+    }
 }
 
 // ------------------------------------------------------ exact sampler
@@ -2538,11 +2588,6 @@ struct StepEnd {
 };
 constexpr int STEP_END_ENTRIES = 1024, STEP_END_MAX_SPLIT = 16;
 
-__device__ __forceinline__ double to_double(double v) { return v; }
-__device__ __forceinline__ double to_double(float v) {  // widen, for any value
-    const unsigned m = __float_as_uint(v) & 0x7fffffffu;
-    return m - 0x00800000u < 0x7f000000u || m == 0u ? widen(v) : (double)v;
-}
 
 template <typename T>
 __device__ __forceinline__ void step_end_body(const T *x, const StepEnd &e, int cta, int nblocks) {
