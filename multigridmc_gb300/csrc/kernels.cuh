@@ -1134,32 +1134,36 @@ struct CorrQuad {
 };
 
 // One multi-entry row r (two entries at least) with its row index, entry
-// range, first two entries and state loaded together, before the wait for
-// the previous kernel where the caller says so; its products
-// are added to zero in entry order, then to the state.
-template <typename T>
+// range, first PF entries and state loaded together, before the wait for
+// the previous kernel where the caller says so; its products are added to
+// zero in entry order, then to the state.
+template <typename T, int PF>
 struct CorrMulti {
     unsigned row;
-    int e0, e1, col0, col1;
-    T val0, val1, xv;
+    int e0, e1, col[PF];
+    T val[PF], xv;
     __device__ __forceinline__ void load(const T *x, const CorrRows &C, i64 r, bool before_wait) {
         const T *vm = static_cast<const T *>(C.vm);
         row = C.rm[r];
         e0 = C.pm[r];
         e1 = C.pm[r + 1];
-        col0 = C.cm[e0];
-        col1 = C.cm[e0 + 1];
-        val0 = vm[e0];
-        val1 = vm[e0 + 1];
+#pragma unroll
+        for (int k = 0; k < PF; ++k)
+            if (k < 2 || e0 + k < e1) {
+                col[k] = C.cm[e0 + k];
+                val[k] = vm[e0 + k];
+            }
         xv = before_wait ? __ldcg(x + row) : x[row];
     }
     template <typename ZT>
     __device__ __forceinline__ void apply(T *x, const CorrRows &C, const ZT *z) const {
         const T *vm = static_cast<const T *>(C.vm);
         T acc = T(0);
-        acc += val0 * (T)z[col0];
-        acc += val1 * (T)z[col1];
-        for (int e = e0 + 2; e < e1; ++e) acc += vm[e] * (T)z[C.cm[e]];
+#pragma unroll
+        for (int k = 0; k < PF; ++k)
+            if (k < 2 || e0 + k < e1) acc += val[k] * (T)z[col[k]];
+#pragma unroll 4
+        for (int e = e0 + PF; e < e1; ++e) acc += vm[e] * (T)z[C.cm[e]];
         x[row] = xv + acc;
     }
 };
@@ -1194,7 +1198,11 @@ struct CorrJob {
 // in the list of columns: the first CTA that has the column
 constexpr int CORR_OWNER = 1 << 30;
 
-template <typename T, int MODE, int NQ>
+// PF entries of a multi-entry row are loaded ahead: 8 in k_lr_correct's mode 1
+// (coarse rows have many: 2D 768 x 480 FP64 step 2.5 % faster than with 2, 3D
+// 128^3 1.3 %), 2 in the batch, whose CTAs need the registers to be resident
+// (20 chains: 2.5 % slower with 8).
+template <typename T, int MODE, int NQ, int PF = 2>
 __device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int P, const CorrRows &C, const CorrJob &jb,
                                                 const int *__restrict__ jobcols, bool first, double *dyn) {
     typedef typename std::conditional<sizeof(T) == 4, float2, double>::type V;  // FP32 chain: float-float
@@ -1208,7 +1216,7 @@ __device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int 
         Sinv = lr.SinvT;
     const int row = jb.r0 + tid;
     CorrQuad<T> q[NQ];
-    CorrMulti<T> mr;
+    CorrMulti<T, PF> mr;
     if (jb.multi) {
         if (row < jb.r1) mr.load(x, C, row, true);
     } else {
@@ -1387,7 +1395,7 @@ template <typename T, int MODE, int NQ>
 __global__ void __launch_bounds__(256, MODE == 1 || NQ > 1 ? 2 : 4)
     k_lr_correct(T *x, LowRankArg lr, int P, CorrRows C, const CorrJob *__restrict__ jobs, const int *__restrict__ jobcols) {
     extern __shared__ double dyn[];
-    lr_correct_body<T, MODE, NQ>(x, lr, P, C, jobs[blockIdx.x], jobcols, blockIdx.x == 0, dyn);
+    lr_correct_body<T, MODE, NQ, MODE == 1 ? 8 : 2>(x, lr, P, C, jobs[blockIdx.x], jobcols, blockIdx.x == 0, dyn);
 }
 
 // dst -= B_c Sigma^{-1} y over the rows of the coarse level's B, y from the
