@@ -848,10 +848,15 @@ void Sampler::prolong(int lev, double alpha, void *xc, void *x) {
     Level &lv = L[lev], &lc = L[lev + 1];
     if (taping) tape_last[lev] = nullptr;
     dim3 grid((lc.g.N0 + 1 + 127) / 128, dim > 1 ? lc.g.N1 + 1 : 1, dim > 2 ? lc.g.N2 + 1 : 1);
+    auto go = [&](auto *xf, auto kernel1, auto kernel2, auto kernel3) {
+        typedef std::remove_pointer_t<decltype(xf)> T;
+        plaunch(pdl && lv.g.pdl, dim == 1 ? kernel1 : dim == 2 ? kernel2 : kernel3, grid, 128, 0, stream, xf, (const T *)xc, lv.g,
+                lc.g, (T)alpha);
+    };
     if (fp32)
-        plaunch(pdl && lv.g.pdl, k_prolong_add<float>, grid, 128, 0, stream, (float *)x, (const float *)xc, lv.g, lc.g, (float)alpha, dim);
+        go((float *)x, k_prolong_add<float, 1>, k_prolong_add<float, 2>, k_prolong_add<float, 3>);
     else
-        plaunch(pdl && lv.g.pdl, k_prolong_add<double>, grid, 128, 0, stream, (double *)x, (const double *)xc, lv.g, lc.g, alpha, dim);
+        go((double *)x, k_prolong_add<double, 1>, k_prolong_add<double, 2>, k_prolong_add<double, 3>);
     launches++;
 }
 
@@ -3108,7 +3113,7 @@ void BatchGroup::sample(int lev, cudaStream_t st) {
         }
         sample(lev + 1, st);
         const dim3 pgrid((gc.N0 + 1 + 127) / 128, gc.N1 + 1, (gc.N2 + 1) * G);
-        plaunch(pdl, k_prolong_batch, pgrid, 128, 0, st, la_, gf, gc, (float)S0.P.coarse_scaling, 3, gc.N2 + 1);
+        plaunch(pdl, k_prolong_batch, pgrid, 128, 0, st, la_, gf, gc, (float)S0.P.coarse_scaling, gc.N2 + 1);
         for (int k = 0; k < S0.P.npostsmooth; ++k) {
             sor(lev, true, st);
             sor(lev, false, st);

@@ -56,6 +56,15 @@ __device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;
 // pdl_begin until this grid has completed).  Used where one CTA is left
 // working alone, so that the next kernel's independent loads overlap it.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Both, for a kernel between two sweeps: a grid of at most two CTAs per SM
+// lets the next kernel start at once (it draws its noise and loads what does
+// not depend on this one meanwhile; see k_chol_gemv_lower for what it gave);
+// a larger one needs the SM slots.
+constexpr unsigned PDL_SMALL_GRID = 304;
+__device__ __forceinline__ void pdl_begin_trigger() {
+    pdl_begin();
+    if (gridDim.x * gridDim.y * gridDim.z <= PDL_SMALL_GRID) pdl_trigger();
+}
 
 // ------------------------------------------------------------- geometry
 struct Grid3 {
@@ -1470,7 +1479,7 @@ constexpr int RRS_TX = 16, RRS_FW = 2 * RRS_TX + 1, RRS_THREADS = 320;  // >= 33
 template <typename T, int NPT, int VAR, bool ZERO>
 __global__ void __launch_bounds__(RRS_THREADS) k_resid_restrict(const T *x, const T *f, T *fc, T *xc, Grid3 gf, Grid3 gc,
                                                                 StencilArg<T> s, int dim, VarField<T> vf) {
-    if (gf.pdl) pdl_begin();
+    if (gf.pdl) pdl_begin_trigger();
     __shared__ T res[9 * RRS_FW];
     const int ca0 = blockIdx.x * RRS_TX, cb = blockIdx.y, cc = blockIdx.z;
     const int nr = dim > 2 ? 9 : dim > 1 ? 3 : 1;  // rows of the footprint
@@ -1621,7 +1630,7 @@ template <typename T, int NPT>
 __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict_tiled(const T *__restrict__ x, const T *__restrict__ f,
                                                                       T *__restrict__ fc, T *__restrict__ xc, Grid3 gf, Grid3 gc,
                                                                       StencilArg<T> s) {
-    if (gf.pdl) pdl_begin();
+    if (gf.pdl) pdl_begin_trigger();
     extern __shared__ __align__(16) unsigned char rr_smem[];
     resid_restrict_tiled_body<T, NPT>(x, f, fc, xc, gf, gc, s, rr_smem, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -1715,7 +1724,7 @@ __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict_tma(const __grid_
                                                                    const __grid_constant__ CUtensorMap fmap,
                                                                    T *__restrict__ fc, T *__restrict__ xc, Grid3 gf, Grid3 gc,
                                                                    StencilArg<T> s, unsigned *__restrict__ err) {
-    if (gf.pdl) pdl_begin();
+    if (gf.pdl) pdl_begin_trigger();
     extern __shared__ __align__(1024) unsigned char rr_tma_smem[];
     __shared__ unsigned long long bar;
     T *xs = reinterpret_cast<T *>(rr_tma_smem);                      // [RR_XD][RR_XH][RR_BW]
@@ -1769,7 +1778,7 @@ template <int NPT>
 __global__ void __launch_bounds__(256)
     k_resid_restrict_sym(const double *x, const double *f, double *fc, double *xc, Grid3 gf, Grid3 gc, SymWeights w,
                          int whole) {
-    if (gf.pdl) pdl_begin();
+    if (gf.pdl) pdl_begin_trigger();
     constexpr bool D3 = NPT == 27 || NPT == 7, FULL = NPT == 27 || NPT == 9;
     constexpr int NPX = D3 ? 5 : 1, NPF = D3 ? 3 : 1;  // planes of x and f
     extern __shared__ __align__(16) unsigned char rr_sym_sm[];
@@ -1854,75 +1863,92 @@ __global__ void __launch_bounds__(256) k_add_Bq(T *__restrict__ dst, i64 nrows, 
 // x += alpha P x_c (intergrid_operator.hh:106-120): every fine vertex
 // gathers its <= 2^d coarse parents, weight 1 (even coordinate) or 1/2 for
 // each of the two parents (odd coordinate).
-template <typename T>
+//
+// A thread owns the 2^d fine vertices of a coarse cell.  FP64: the sums of the
+// parents direction by direction, 12 additions in 3D, and one FMA per vertex
+// with alpha times the weight (the sums parent by parent, with the weights as
+// run-time values, took over 80 FP64 instructions; k_sweep_row_sym says why
+// their number counts).  FP32 adds the parents in their order.
+// On 127^3, FP64, under ncu: 24.4 -> 16.5 us, of which the FP64 unit 10.
+template <typename T, int DIM>
 __device__ __forceinline__ void prolong_add_body(T *__restrict__ x, const T *__restrict__ xc, const Grid3 &gf,
-                                                 const Grid3 &gc, T alpha, int dim, int bx, int by, int bz_from_top) {
+                                                 const Grid3 &gc, T alpha, int bx, int by, int bz_from_top) {
     // coarse cell (i, j, k), 0 <= i <= Nc0 etc., owns the fine vertices with
     // 1-based coordinates 2 i + {0, 1} (those inside the interior); its
     // corners are the coarse vertices i, i+1 (1-based, ghosts are zero)
     // planes from the top: the residual-restriction before ends there, and
     // the sweep after starts at the bottom, which this kernel writes last
     // (both find their first planes in L2)
+    constexpr int NY = DIM > 1 ? 2 : 1, NZ = DIM > 2 ? 2 : 1;
     const int i = bx * blockDim.x + threadIdx.x;
-    const int j = dim > 1 ? by : 0, k = dim > 2 ? bz_from_top : 0;
+    const int j = DIM > 1 ? by : 0, k = DIM > 2 ? bz_from_top : 0;
     if (i > gc.N0) return;
-    const int ny = dim > 1 ? 2 : 1, nz = dim > 2 ? 2 : 1;
-    T cv[2][2][2];
+    const i64 Pc = (i64)(DIM > 2 ? k : 1) * gc.sz + (i64)(DIM > 1 ? j : 1) * gc.sy + i;
+    const i64 Pf = (i64)(DIM > 2 ? 2 * k : 1) * gf.sz + (i64)(DIM > 1 ? 2 * j : 1) * gf.sy + 2 * i;
+    T v[NZ][NY][2], xv[NZ][NY][2];
+    bool in[NZ][NY][2];
 #pragma unroll
-    for (int dz = 0; dz < 2; ++dz)
+    for (int z = 0; z < NZ; ++z)
 #pragma unroll
-        for (int dy = 0; dy < 2; ++dy)
+        for (int y = 0; y < NY; ++y)
 #pragma unroll
-            for (int dx = 0; dx < 2; ++dx) {
-                const int ci = i + dx, cj = dim > 1 ? j + dy : 1, ck = dim > 2 ? k + dz : 1;
-                const bool use = (dy < ny) && (dz < nz);
-                cv[dz][dy][dx] = use ? xc[(i64)ck * gc.sz + (i64)cj * gc.sy + ci] : T(0);
+            for (int q = 0; q < 2; ++q) {
+                v[z][y][q] = xc[Pc + z * gc.sz + y * gc.sy + q];
+                const int fk = DIM > 2 ? 2 * k + z : 1, fj = DIM > 1 ? 2 * j + y : 1, fi = 2 * i + q;
+                in[z][y][q] = fk >= 1 && fk <= gf.N2 && fj >= 1 && fj <= gf.N1 && fi >= 1 && fi <= gf.N0;
+                xv[z][y][q] = in[z][y][q] ? x[Pf + z * gf.sz + y * gf.sy + q] : T(0);
             }
+    if constexpr (sizeof(T) == 8) {
+        const T a[4] = {alpha, T(0.5) * alpha, T(0.25) * alpha, T(0.125) * alpha};
 #pragma unroll
-    for (int oz = 0; oz < 2; ++oz) {
-        if (oz >= nz) break;
-        const int fk = dim > 2 ? 2 * k + oz : 1;
-        if (fk < 1 || fk > gf.N2) continue;
+        for (int z = 0; z < NZ; ++z)
 #pragma unroll
-        for (int oy = 0; oy < 2; ++oy) {
-            if (oy >= ny) break;
-            const int fj = dim > 1 ? 2 * j + oy : 1;
-            if (fj < 1 || fj > gf.N1) continue;
+            for (int y = 0; y < NY; ++y) v[z][y][1] += v[z][y][0];
+        if (DIM > 1) {
 #pragma unroll
-            for (int ox = 0; ox < 2; ++ox) {
-                const int fi = 2 * i + ox;
-                if (fi < 1 || fi > gf.N0) continue;
-                // even coordinate: the vertex itself (weight 1); odd: half
-                // of each neighbour
-                T acc = T(0);
+            for (int z = 0; z < NZ; ++z)
 #pragma unroll
-                for (int dz = 0; dz < 2; ++dz) {
-                    const T wz = dim > 2 ? (oz == 0 ? (dz == 0 ? T(1) : T(0)) : T(0.5)) : (dz == 0 ? T(1) : T(0));
-                    if (wz == T(0)) continue;
-#pragma unroll
-                    for (int dy = 0; dy < 2; ++dy) {
-                        const T wy = dim > 1 ? (oy == 0 ? (dy == 0 ? T(1) : T(0)) : T(0.5)) : (dy == 0 ? T(1) : T(0));
-                        if (wy == T(0)) continue;
-#pragma unroll
-                        for (int dx = 0; dx < 2; ++dx) {
-                            const T wx = ox == 0 ? (dx == 0 ? T(1) : T(0)) : T(0.5);
-                            if (wx == T(0)) continue;
-                            acc += wx * wy * wz * cv[dz][dy][dx];
-                        }
-                    }
-                }
-                const i64 P = (i64)fk * gf.sz + (i64)fj * gf.sy + fi;
-                x[P] += alpha * acc;
-            }
+                for (int q = 0; q < 2; ++q) v[z][NY - 1][q] += v[z][0][q];
         }
+        if (DIM > 2) {
+#pragma unroll
+            for (int y = 0; y < NY; ++y)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) v[NZ - 1][y][q] += v[0][y][q];
+        }
+#pragma unroll
+        for (int z = 0; z < NZ; ++z)
+#pragma unroll
+            for (int y = 0; y < NY; ++y)
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    if (in[z][y][q]) x[Pf + z * gf.sz + y * gf.sy + q] = fma(a[z + y + q], v[z][y][q], xv[z][y][q]);
+    } else {
+#pragma unroll
+        for (int oz = 0; oz < NZ; ++oz)
+#pragma unroll
+            for (int oy = 0; oy < NY; ++oy)
+#pragma unroll
+                for (int ox = 0; ox < 2; ++ox) {
+                    // even coordinate: the vertex itself; odd: half of each neighbour
+                    const T w = (oz ? T(0.5) : T(1)) * (oy ? T(0.5) : T(1)) * (ox ? T(0.5) : T(1));
+                    T acc = T(0);
+#pragma unroll
+                    for (int dz = 0; dz <= oz; ++dz)
+#pragma unroll
+                        for (int dy = 0; dy <= oy; ++dy)
+#pragma unroll
+                            for (int dx = 0; dx <= ox; ++dx) acc += w * v[dz][dy][dx];
+                    if (in[oz][oy][ox]) x[Pf + oz * gf.sz + oy * gf.sy + ox] = xv[oz][oy][ox] + alpha * acc;
+                }
     }
 }
 
-template <typename T>
+template <typename T, int DIM>
 __global__ void __launch_bounds__(128) k_prolong_add(T *__restrict__ x, const T *__restrict__ xc, Grid3 gf, Grid3 gc,
-                                                      T alpha, int dim) {
-    if (gf.pdl) pdl_begin();
-    prolong_add_body<T>(x, xc, gf, gc, alpha, dim, blockIdx.x, blockIdx.y, (int)(gridDim.z - 1 - blockIdx.z));
+                                                      T alpha) {
+    if (gf.pdl) pdl_begin_trigger();
+    prolong_add_body<T, DIM>(x, xc, gf, gc, alpha, blockIdx.x, blockIdx.y, (int)(gridDim.z - 1 - blockIdx.z));
 }
 
 // ----------------------------------------------------- stencil apply
@@ -2052,98 +2078,130 @@ struct Vec16<double> {
     static __device__ __forceinline__ double dot(double2 a, const double *v) { return a.x * v[0] + a.y * v[1]; }
 };
 
-// sum over vectors q0..q1-1 of row . vs, lanes strided, four vectors in flight
+// A warp's row, vectors q0 .. q1 - 1: sum of row . vs, lanes strided, four
+// vectors in flight.  The first four of a lane are loaded by load(), which a
+// kernel calls before it waits for vs.
 template <typename MT>
-__device__ __forceinline__ MT warp_row_dot(const MT *__restrict__ row, const MT *vs, int q0, int q1, int lane) {
+struct WarpRow {
     typedef typename Vec16<MT>::type V;
-    constexpr int NV = Vec16<MT>::N;
-    const V *r = reinterpret_cast<const V *>(row);
-    MT a0 = MT(0), a1 = MT(0), a2 = MT(0), a3 = MT(0);
-    int q = q0 + lane;
-    for (; q + 96 < q1; q += 128) {
-        V v0 = __ldg(r + q), v1 = __ldg(r + q + 32), v2 = __ldg(r + q + 64), v3 = __ldg(r + q + 96);
-        a0 += Vec16<MT>::dot(v0, vs + NV * q);
-        a1 += Vec16<MT>::dot(v1, vs + NV * (q + 32));
-        a2 += Vec16<MT>::dot(v2, vs + NV * (q + 64));
-        a3 += Vec16<MT>::dot(v3, vs + NV * (q + 96));
-    }
-    for (; q < q1; q += 32) a0 += Vec16<MT>::dot(__ldg(r + q), vs + NV * q);
-    MT acc = (a0 + a1) + (a2 + a3);
+    static constexpr int NV = Vec16<MT>::N;
+    const V *r;
+    int q, q1;
+    V first[4];
+    __device__ __forceinline__ void load(const MT *__restrict__ row, int q0, int end, int lane) {
+        r = reinterpret_cast<const V *>(row);
+        q = q0 + lane;
+        q1 = end;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    return acc;
-}
+        for (int k = 0; k < 4; ++k)
+            if (q + 32 * k < q1) first[k] = __ldg(r + q + 32 * k);
+    }
+    __device__ __forceinline__ MT dot(const MT *vs) const {
+        MT a0 = MT(0), a1 = MT(0), a2 = MT(0), a3 = MT(0);
+        int p = q;
+        if (p + 96 < q1) {
+            a0 += Vec16<MT>::dot(first[0], vs + NV * p);
+            a1 += Vec16<MT>::dot(first[1], vs + NV * (p + 32));
+            a2 += Vec16<MT>::dot(first[2], vs + NV * (p + 64));
+            a3 += Vec16<MT>::dot(first[3], vs + NV * (p + 96));
+            p += 128;
+            for (; p + 96 < q1; p += 128) {
+                V v0 = __ldg(r + p), v1 = __ldg(r + p + 32), v2 = __ldg(r + p + 64), v3 = __ldg(r + p + 96);
+                a0 += Vec16<MT>::dot(v0, vs + NV * p);
+                a1 += Vec16<MT>::dot(v1, vs + NV * (p + 32));
+                a2 += Vec16<MT>::dot(v2, vs + NV * (p + 64));
+                a3 += Vec16<MT>::dot(v3, vs + NV * (p + 96));
+            }
+            for (; p < q1; p += 32) a0 += Vec16<MT>::dot(__ldg(r + p), vs + NV * p);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (p + 32 * k < q1) a0 += Vec16<MT>::dot(first[k], vs + NV * (p + 32 * k));
+        }
+        MT acc = (a0 + a1) + (a2 + a3);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        return acc;
+    }
+};
 
-// v = xi + Linv f (row i: vectors 0 .. i / NV)
+// v = xi + Linv f (row i: vectors 0 .. i / NV), one warp per row: row, noise
+// and addresses before the wait for f.
 template <typename T, typename MT, int NOISE>
 __device__ __forceinline__ void chol_gemv_lower_body(const T *__restrict__ f, const Grid3 &g, const MT *__restrict__ Linv,
-                                                     int ld, MT *__restrict__ v, const NoiseArgs &nz,
-                                                     unsigned char *chol_sm, int bx, int nbx) {
+                                                     int ld, MT *__restrict__ v, const NoiseArgs &nz, bool wait,
+                                                     unsigned char *chol_sm, int bx) {
     MT *fs = reinterpret_cast<MT *>(chol_sm);
     const int n = g.N0 * g.N1 * g.N2;
-    for (int i = threadIdx.x; i < ld; i += blockDim.x) {
-        MT val = MT(0);
-        if (i < n) {
-            const int a = i % g.N0, t = i / g.N0;
-            val = (MT)f[g.pad(a, t % g.N1, t / g.N1)];
-        }
-        fs[i] = val;
-    }
-    __syncthreads();
     constexpr int NV = Vec16<MT>::N;
-    const int lane = threadIdx.x & 31;
-    const int warps = nbx * (blockDim.x >> 5);
-    for (int ii = bx * (blockDim.x >> 5) + (threadIdx.x >> 5); ii < n; ii += warps) {
-        const int i = (ii & 1) ? n - 1 - (ii >> 1) : (ii >> 1);
-        const MT acc = warp_row_dot<MT>(Linv + (i64)i * ld, fs, 0, i / NV + 1, lane);
-        if (lane == 0) {
-            double xi = 0.0;
-            if (NOISE == NOISE_INJECTED) xi = nz.buf[i];
-            if (NOISE == NOISE_PHILOX) {
-                float4 r = normals4(philox4x32_10(noise_ctr(nz, (unsigned)(i >> 2), PURPOSE_COARSE, 0), noise_key(nz)));
-                xi = (double)pick(r, i & 3);
-            }
-            v[i] = (MT)xi + acc;
+    const int lane = threadIdx.x & 31, ii = bx * 8 + (threadIdx.x >> 5);
+    const int i = (ii & 1) ? n - 1 - (ii >> 1) : (ii >> 1);
+    WarpRow<MT> row;
+    MT xi = MT(0);
+    if (ii < n) {
+        row.load(Linv + (i64)i * ld, 0, i / NV + 1, lane);
+        if (NOISE == NOISE_PHILOX) {
+            const float4 r = normals4(philox4x32_10(noise_ctr(nz, (unsigned)(i >> 2), PURPOSE_COARSE, 0), noise_key(nz)));
+            if constexpr (sizeof(MT) == 4)
+                xi = pick(r, i & 3);
+            else
+                xi = widen(pick(r, i & 3));
         }
     }
+    auto padded = [&](int k) {
+        const int a = k % g.N0, t = k / g.N0;
+        return g.pad(a, t % g.N1, t / g.N1);
+    };
+    const i64 P0 = (int)threadIdx.x < n ? padded(threadIdx.x) : 0;
+    if (wait) pdl_begin_trigger();
+    for (int k = threadIdx.x; k < ld; k += 256) fs[k] = k < n ? (MT)f[k < 256 ? P0 : padded(k)] : MT(0);
+    __syncthreads();
+    if (ii >= n) return;
+    const MT acc = row.dot(fs);
+    if (lane == 0) v[i] = (NOISE == NOISE_INJECTED ? (MT)nz.buf[i] : xi) + acc;
 }
 
+// (With the row and the noise loaded and drawn after the wait, and no early
+// start here, in the residual-restriction and in the prolongation, whole
+// steps were slower: 2D 64 x 64 FP64 59.0 us, now 56.4; 3D 32^3 FP64 128 ->
+// 122 us; 96x48x80 27-point FP32 258 -> 240 us.)
 template <typename T, typename MT, int NOISE>
 __global__ void __launch_bounds__(256) k_chol_gemv_lower(const T *__restrict__ f, Grid3 g, const MT *__restrict__ Linv,
                                                           int ld, MT *__restrict__ v, NoiseArgs nz) {
-    if (g.pdl) pdl_begin();
     extern __shared__ __align__(16) unsigned char chol_sm[];
-    chol_gemv_lower_body<T, MT, NOISE>(f, g, Linv, ld, v, nz, chol_sm, blockIdx.x, gridDim.x);
+    chol_gemv_lower_body<T, MT, NOISE>(f, g, Linv, ld, v, nz, g.pdl != 0, chol_sm, blockIdx.x);
 }
 
 // ... x = Linv^T v (row j of Linv^T: vectors j / NV .. ld / NV - 1).
 template <typename T, typename MT>
 __device__ __forceinline__ void chol_gemv_upper_body(const MT *__restrict__ v, const Grid3 &g,
-                                                     const MT *__restrict__ LinvT, int ld, T *__restrict__ x,
-                                                     unsigned char *chol_sm, int bx, int nbx) {
+                                                     const MT *__restrict__ LinvT, int ld, T *__restrict__ x, bool wait,
+                                                     unsigned char *chol_sm, int bx) {
     MT *vs = reinterpret_cast<MT *>(chol_sm);
     const int n = g.N0 * g.N1 * g.N2;
-    for (int i = threadIdx.x; i < ld; i += blockDim.x) vs[i] = i < n ? v[i] : MT(0);
-    __syncthreads();
     constexpr int NV = Vec16<MT>::N;
-    const int lane = threadIdx.x & 31;
-    const int warps = nbx * (blockDim.x >> 5);
-    for (int jj = bx * (blockDim.x >> 5) + (threadIdx.x >> 5); jj < n; jj += warps) {
-        const int j = (jj & 1) ? n - 1 - (jj >> 1) : (jj >> 1);
-        const MT acc = warp_row_dot<MT>(LinvT + (i64)j * ld, vs, j / NV, ld / NV, lane);
-        if (lane == 0) {
-            const int a = j % g.N0, t = j / g.N0;
-            x[g.pad(a, t % g.N1, t / g.N1)] = (T)acc;
-        }
+    const int lane = threadIdx.x & 31, jj = bx * 8 + (threadIdx.x >> 5);
+    const int j = (jj & 1) ? n - 1 - (jj >> 1) : (jj >> 1);
+    WarpRow<MT> row;
+    i64 P = 0;
+    if (jj < n) {
+        row.load(LinvT + (i64)j * ld, j / NV, ld / NV, lane);
+        const int a = j % g.N0, t = j / g.N0;
+        P = g.pad(a, t % g.N1, t / g.N1);
     }
+    if (wait) pdl_begin_trigger();
+    for (int i = threadIdx.x; i < ld; i += 256) vs[i] = i < n ? v[i] : MT(0);
+    __syncthreads();
+    if (jj >= n) return;
+    const MT acc = row.dot(vs);
+    if (lane == 0) x[P] = (T)acc;
 }
 
 template <typename T, typename MT>
 __global__ void __launch_bounds__(256) k_chol_gemv_upper(const MT *__restrict__ v, Grid3 g,
                                                           const MT *__restrict__ LinvT, int ld, T *__restrict__ x) {
-    if (g.pdl) pdl_begin();
     extern __shared__ __align__(16) unsigned char chol_sm[];
-    chol_gemv_upper_body<T, MT>(v, g, LinvT, ld, x, chol_sm, blockIdx.x, gridDim.x);
+    chol_gemv_upper_body<T, MT>(v, g, LinvT, ld, x, g.pdl != 0, chol_sm, blockIdx.x);
 }
 
 // ------------------------------------------------------------- adjoint
@@ -2511,7 +2569,9 @@ __global__ void __launch_bounds__(256) k_pgrad_coarse_phi(const MT *__restrict__
     const int warps = gridDim.x * (blockDim.x >> 5);
     double acc = 0.0;
     for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-        const MT r = warp_row_dot<MT>(Phi + (i64)i * ld, ws, 0, i / NV + 1, lane);
+        WarpRow<MT> row;
+        row.load(Phi + (i64)i * ld, 0, i / NV + 1, lane);
+        const MT r = row.dot(ws);
         if (lane == 0) acc += xi[i] * (double)r;
     }
     acc = block_sum<256>(acc, sh);
@@ -3135,11 +3195,11 @@ __global__ void __launch_bounds__(RR_THREADS, MGMC_RR_BATCH_MINB) k_resid_restri
 
 // x += alpha P x_c, grid.z = chains x (coarse planes + 1)
 __global__ void __launch_bounds__(128) k_prolong_batch(const BatchLevelArg *__restrict__ la, Grid3 gf, Grid3 gc,
-                                                       float alpha, int dim, int nzc) {
+                                                       float alpha, int nzc) {
     const int chain = blockIdx.z / nzc, bz = blockIdx.z - chain * nzc;
     const BatchLevelArg &a = la[chain];
     pdl_begin();
-    prolong_add_body<float>(a.x, a.xc, gf, gc, alpha, dim, blockIdx.x, blockIdx.y, nzc - 1 - bz);
+    prolong_add_body<float, 3>(a.x, a.xc, gf, gc, alpha, blockIdx.x, blockIdx.y, nzc - 1 - bz);  // batched chains are 3D
 }
 
 // coarse Cholesky sample, grid.y = chains
@@ -3150,17 +3210,14 @@ __global__ void __launch_bounds__(256) k_chol_lower_batch(const BatchLevelArg *_
     extern __shared__ __align__(16) unsigned char chol_sm_b[];
     const BatchChainArg &c = ca[blockIdx.y];
     const NoiseArgs nz = batch_noise(c, invocation, level);
-    pdl_begin();
-    chol_gemv_lower_body<float, float, NOISE>(la[blockIdx.y].f, g, c.Linv, ld, c.gv, nz, chol_sm_b, blockIdx.x,
-                                              gridDim.x);
+    chol_gemv_lower_body<float, float, NOISE>(la[blockIdx.y].f, g, c.Linv, ld, c.gv, nz, true, chol_sm_b, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(256) k_chol_upper_batch(const BatchLevelArg *__restrict__ la,
                                                           const BatchChainArg *__restrict__ ca, Grid3 g, int ld) {
     extern __shared__ __align__(16) unsigned char chol_sm_b[];
     const BatchChainArg &c = ca[blockIdx.y];
-    pdl_begin();
-    chol_gemv_upper_body<float, float>(c.gv, g, c.LinvT, ld, la[blockIdx.y].x, chol_sm_b, blockIdx.x, gridDim.x);
+    chol_gemv_upper_body<float, float>(c.gv, g, c.LinvT, ld, la[blockIdx.y].x, true, chol_sm_b, blockIdx.x);
 }
 
 // observables and step counters, grid.y = chains
