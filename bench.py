@@ -43,7 +43,7 @@ RB_VEC_DRAM_BYTES = 110.47e6
 RB_VEC_TRAFFIC_SOURCE = ("constant: ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch, capture of "
                          "`python bench.py --profile-steps 1` (profiles/k_sweep_rb_vec_256cubed.md, launch 1): "
                          "100.68 MB read + 9.79 MB written")
-RB_VEC_KERNEL = ("k_sweep_rb_vec<1, 0, 1, 1> (one colour pass of the fine-level red-black SOR sweep: FP32, Philox "
+RB_VEC_KERNEL = ("k_sweep_rb_vec<1, 0, 1, 1, 0> (one colour pass of the fine-level red-black SOR sweep: FP32, Philox "
                  "noise, 256-bit spans, colour-split f)")
 METRIC = "indep. samples/s (rate/IACT), 3D 256³ posterior: mixed vs FP64 plain, 1 GB300"
 UNIT = "indep_samples/s"

@@ -47,14 +47,13 @@ typedef unsigned long long u64;
 // stream has completed and its writes are visible (a kernel launched with
 // the programmatic-serialization attribute may start while its predecessor
 // drains; the predecessor triggers it implicitly as its CTAs exit).  Without
-// the attribute this is a no-op.  (An explicit griddepcontrol.launch_dependents
-// right after the wait, which schedules the next kernel's CTAs while this
-// grid runs, made the 256^3 step 1.8 % slower: the waiting CTAs hold SM
-// slots the running grid needs.)
+// the attribute this is a no-op.
 __device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Let the next kernel on the stream start its CTAs now (they still wait in
-// pdl_begin until this grid has completed).  Used where one CTA is left
-// working alone, so that the next kernel's independent loads overlap it.
+// pdl_begin until this grid has completed), so that its noise and independent
+// loads overlap this one.  For grids that leave room: the waiting CTAs hold SM
+// slots, and after the wait of every kernel, whatever its grid, it made the
+// 256^3 step 1.8 % slower.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Both, for a kernel between two sweeps: a grid of at most two CTAs per SM
 // lets the next kernel start at once (it draws its noise and loads what does
