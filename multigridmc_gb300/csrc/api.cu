@@ -346,11 +346,12 @@ NoiseArgs Sampler::noise_args(int lev, i64 count) {
     return nz;
 }
 
-// Launch with programmatic stream serialization (pdl): the kernel's CTAs
-// may be scheduled while its predecessor on the stream drains; every step
-// kernel starts with griddepcontrol.wait (pdl_begin), so no kernel touches
-// memory before its predecessor has completed and flushed.  This hides the launch latency between the short
-// dependent kernels of a multigrid step.
+// Launch with programmatic stream serialization (pdl): the kernel's CTAs may
+// start while its predecessor on the stream is still running.  That is safe by
+// the rules at pdl_begin (kernels.cuh): a kernel lets its successor start only
+// after its own wait, and before the wait it reads nothing that an unfinished
+// launch writes.  It hides the launch latency between the short dependent
+// kernels of a multigrid step.
 constexpr i64 PDL_MAX_POINTS = i64(1) << 22;
 template <typename... KArgs, typename... Args>
 static void plaunch(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -45,9 +45,20 @@ typedef unsigned long long u64;
 
 // Programmatic dependent launch: wait until the previous kernel on the
 // stream has completed and its writes are visible (a kernel launched with
-// the programmatic-serialization attribute may start while its predecessor
-// drains; the predecessor triggers it implicitly as its CTAs exit).  Without
-// the attribute this is a no-op.
+// the programmatic-serialization attribute may start once every CTA of its
+// predecessor has let it, with pdl_trigger or by its exit).  Without the
+// attribute this is a no-op.
+//
+// The rules of every kernel that waits:
+// - It waits before it lets the next one start.  Then "the kernel before has
+//   completed" holds for all kernels before that one too.
+// - Before the wait it writes nothing outside its CTA and reads only what no
+//   launch of the step writes: operators, factors, index lists, and the step
+//   counter, which the step's last launch advances.  One exception: the
+//   correction reads the state before its wait (k_lr_correct says why it may).
+// - Memory that a launch of the step writes carries no __restrict__ and is not
+//   read by ld.global.nc or __ldg: a compiler may move loads of memory promised
+//   to be constant, or private to a pointer, above the wait.
 __device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Let the next kernel on the stream start its CTAs now (they still wait in
 // pdl_begin until this grid has completed), so that its noise and independent
@@ -272,7 +283,7 @@ __device__ __forceinline__ T sor_value(const XA &xa, T xo, T fv, const StencilAr
 }
 
 template <typename T, int NPT, bool EXACT, int VAR = 0>
-__device__ __forceinline__ void sor_point(T *__restrict__ x, const T *__restrict__ f, const Grid3 &g,
+__device__ __forceinline__ void sor_point(T *x, const T *f, const Grid3 &g,
                                           const StencilArg<T> &s, i64 P, bool noisy, T xi,
                                           const VarField<T> &vf = VarField<T>{nullptr, 0}) {
     x[P] = sor_value<T, NPT, EXACT, VAR>([&](int dz, int dy, int dx) { return x[P + dz * g.sz + dy * g.sy + dx]; },
@@ -371,7 +382,9 @@ __device__ __forceinline__ void ld8(const float *p, float *v) {
 // Read-once streams (f and the centre field of the fine sweep): no L1
 // allocation, and first in line for L2 eviction, so that the L2 keeps x --
 // which the next colour pass reads again -- rather than f, which it does
-// not.  (Measured at 256^3: 53.3 -> 49.7 us per two-pass sweep.)
+// not.  (Measured at 256^3: 53.3 -> 49.7 us per two-pass sweep.)  An earlier
+// launch may have written f: ordinary loads, kept behind the wait by the
+// clobber, not loads of memory that is constant while the kernel runs.
 __device__ __forceinline__ unsigned long long l2_evict_first_policy() {
     unsigned long long p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -379,15 +392,17 @@ __device__ __forceinline__ unsigned long long l2_evict_first_policy() {
 }
 __device__ __forceinline__ float4 ld4_stream(const float *p, unsigned long long pol) {
     float4 r;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
-        : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
-        : "l"(p), "l"(pol));
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
+                 : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+                 : "l"(p), "l"(pol)
+                 : "memory");
     return r;
 }
 __device__ __forceinline__ void ld8_stream(const float *p, float *v, unsigned long long pol) {
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-        : "l"(p), "l"(pol));
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p), "l"(pol)
+                 : "memory");
 }
 __device__ __forceinline__ void st8(float *p, const float *v) {
     asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
@@ -412,10 +427,10 @@ __device__ __forceinline__ void st8(float *p, const float *v) {
 // EARLY (levels in programmatic dependent launch): the normals are drawn before
 // the wait for the launch before, and the next launch starts early.
 template <int NOISE, bool VD, bool V8, bool FS, bool EARLY>
-__device__ __forceinline__ void sweep_rb_vec_body(float *__restrict__ x, const float *__restrict__ f, const Grid3 &g,
+__device__ __forceinline__ void sweep_rb_vec_body(float *x, const float *f, const Grid3 &g,
                                                   const StencilArg<float> &s, int colour, int reverse,
                                                   const NoiseArgs &nz, const float *__restrict__ vd,
-                                                  const float *__restrict__ fsc, int bx, int by, int bz) {
+                                                  const float *fsc, int bx, int by, int bz) {
     const int b = by * blockDim.y + threadIdx.y;
     const int c = reverse ? g.N2 - 1 - bz : bz;
     const int q = bx * blockDim.x + threadIdx.x;
@@ -536,10 +551,10 @@ __device__ __forceinline__ void sweep_rb_vec_body(float *__restrict__ x, const f
 }
 
 template <int NOISE, bool VD, bool V8, bool FS, bool EARLY>
-__global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_vec(float *__restrict__ x, const float *__restrict__ f,
+__global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_vec(float *x, const float *f,
                                                               Grid3 g, StencilArg<float> s, int colour, int reverse,
                                                               NoiseArgs nz, const float *__restrict__ vd,
-                                                              const float *__restrict__ fsc) {
+                                                              const float *fsc) {
     sweep_rb_vec_body<NOISE, VD, V8, FS, EARLY>(x, f, g, s, colour, reverse, nz, vd, fsc, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -559,7 +574,7 @@ __global__ void __launch_bounds__(256) k_split_colours(const float *__restrict__
 // One colour of an 8-colour (27-point) sweep, one thread per point (colour
 // index (a & 1) | (b & 1) << 1 | (c & 1) << 2).
 template <typename T, bool EXACT, int NOISE, int VAR>
-__device__ __forceinline__ void sweep_c27_body(T *__restrict__ x, const T *__restrict__ f, const Grid3 &g,
+__device__ __forceinline__ void sweep_c27_body(T *x, const T *f, const Grid3 &g,
                                                const StencilArg<T> &s, int colour, const NoiseArgs &nz,
                                                const VarField<T> &vf, int bx, int by, int bz) {
     const int pa = colour & 1, pb = (colour >> 1) & 1, pc = (colour >> 2) & 1;
@@ -607,7 +622,7 @@ __device__ __forceinline__ void sweep_c27_body(T *__restrict__ x, const T *__res
 }
 
 template <typename T, bool EXACT, int NOISE, int VAR = 0>
-__global__ void __launch_bounds__(RBP_THREADS) k_sweep_c27_pass(T *__restrict__ x, const T *__restrict__ f, Grid3 g,
+__global__ void __launch_bounds__(RBP_THREADS) k_sweep_c27_pass(T *x, const T *f, Grid3 g,
                                                                 StencilArg<T> s, int colour, NoiseArgs nz,
                                                                 VarField<T> vf) {
     if (g.pdl) pdl_begin();
@@ -631,10 +646,6 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_c27_pass(T *__restrict__ 
 // (GB300, a whole sweep with Philox noise in a graph of dependent launches,
 // one-colour passes -> row pairs: FP32 127^3 31.5 -> 17.7 us, 63^3 15.4 ->
 // 6.8, 31^3 14.1 -> 5.9; FP64 31^3 22.3 -> 13.0, 15^3 20.8 -> 12.7.)
-//
-// x and f carry no __restrict__ here and in the kernels below that wait for
-// the launch before: loads of memory promised to be read-only may move above
-// the wait.
 //
 // Thread t of a row owns the points 2t and 2t + 1: the four positions 2t ..
 // 2t + 3 of the nine (three) rows around, two aligned pair loads each where
@@ -818,7 +829,7 @@ __global__ void __launch_bounds__(ROW_SYM_THREADS)
 // ((1,1,1) for axis stencils, (1,2,4) for 27-point stencils), points on one
 // hyperplane are independent.  One CTA, one __syncthreads per hyperplane.
 template <typename T, int NPT, bool EXACT, int NOISE>
-__global__ void __launch_bounds__(1024) k_sweep_wavefront(T *__restrict__ x, const T *__restrict__ f, Grid3 g,
+__global__ void __launch_bounds__(1024) k_sweep_wavefront(T *x, const T *f, Grid3 g,
                                                            StencilArg<T> s, int forward, int hb, int hc, NoiseArgs nz) {
     if (g.pdl) pdl_begin();
     const int tmax = (g.N0 - 1) + hb * (g.N1 - 1) + hc * (g.N2 - 1);
@@ -1530,8 +1541,8 @@ constexpr int RR_RZ = RR_TZ * RR_FH * RR_FW;  // z-restricted residuals of a til
 // product of those weights is the trilinear restriction of
 // intergrid_operator.hh:74-88.
 template <typename T, int NPT, int XP, typename FV>
-__device__ __forceinline__ void rr_tile_compute(const T *xs, const FV &fv, T *rz, T *__restrict__ fc,
-                                                T *__restrict__ xc, const Grid3 &gf, const Grid3 &gc,
+__device__ __forceinline__ void rr_tile_compute(const T *xs, const FV &fv, T *rz, T *fc,
+                                                T *xc, const Grid3 &gf, const Grid3 &gc,
                                                 const StencilArg<T> &s, int ca0, int cb0, int cc0) {
     constexpr int SY = XP, SZ = XP * RR_XH;
     const int fa0 = 2 * ca0, fb0 = 2 * cb0, fz0 = 2 * cc0;
@@ -1596,8 +1607,8 @@ constexpr size_t rr_smem_bytes() {
 }
 
 template <typename T, int NPT>
-__device__ __forceinline__ void resid_restrict_tiled_body(const T *__restrict__ x, const T *__restrict__ f,
-                                                          T *__restrict__ fc, T *__restrict__ xc, const Grid3 &gf,
+__device__ __forceinline__ void resid_restrict_tiled_body(const T *x, const T *f,
+                                                          T *fc, T *xc, const Grid3 &gf,
                                                           const Grid3 &gc, const StencilArg<T> &s, unsigned char *smem,
                                                           int bx, int by, int bz) {
     T *xs = reinterpret_cast<T *>(smem);  // [RR_XD][RR_XH][RR_XW]
@@ -1626,8 +1637,8 @@ __device__ __forceinline__ void resid_restrict_tiled_body(const T *__restrict__ 
 }
 
 template <typename T, int NPT>
-__global__ void __launch_bounds__(RR_THREADS) k_resid_restrict_tiled(const T *__restrict__ x, const T *__restrict__ f,
-                                                                      T *__restrict__ fc, T *__restrict__ xc, Grid3 gf, Grid3 gc,
+__global__ void __launch_bounds__(RR_THREADS) k_resid_restrict_tiled(const T *x, const T *f,
+                                                                      T *fc, T *xc, Grid3 gf, Grid3 gc,
                                                                       StencilArg<T> s) {
     if (gf.pdl) pdl_begin_trigger();
     extern __shared__ __align__(16) unsigned char rr_smem[];
@@ -1710,8 +1721,8 @@ __host__ __device__ constexpr size_t rr_tma_smem_bytes() {
 // (rr_tile_compute; the f box's footprint point (la, lb, lc) at
 // (lc RR_FH + lb) RR_BW + la + 1).
 template <typename T, int NPT>
-__device__ __forceinline__ void resid_restrict_tile(const T *xs, const T *fs, T *rz, T *__restrict__ fc,
-                                                    T *__restrict__ xc, const Grid3 &gf, const Grid3 &gc,
+__device__ __forceinline__ void resid_restrict_tile(const T *xs, const T *fs, T *rz, T *fc,
+                                                    T *xc, const Grid3 &gf, const Grid3 &gc,
                                                     const StencilArg<T> &s, int ca0, int cb0, int cc0) {
     rr_tile_compute<T, NPT, RR_BW>(
         xs, [&](int la, int lb, int lc) { return fs[(lc * RR_FH + lb) * RR_BW + la + 1]; }, rz, fc, xc, gf, gc, s,
@@ -1721,8 +1732,8 @@ __device__ __forceinline__ void resid_restrict_tile(const T *xs, const T *fs, T 
 template <typename T, int NPT>
 __global__ void __launch_bounds__(RR_THREADS) k_resid_restrict_tma(const __grid_constant__ CUtensorMap xmap,
                                                                    const __grid_constant__ CUtensorMap fmap,
-                                                                   T *__restrict__ fc, T *__restrict__ xc, Grid3 gf, Grid3 gc,
-                                                                   StencilArg<T> s, unsigned *__restrict__ err) {
+                                                                   T *fc, T *xc, Grid3 gf, Grid3 gc,
+                                                                   StencilArg<T> s, unsigned *err) {
     if (gf.pdl) pdl_begin_trigger();
     extern __shared__ __align__(1024) unsigned char rr_tma_smem[];
     __shared__ unsigned long long bar;
@@ -1846,9 +1857,9 @@ __global__ void __launch_bounds__(256)
 // dst[row] += sign * sum_e B_e y_{col_e} / Sigma_{col_e} over the rows of B
 // (row-compressed): the B Sigma^{-1} B^T x part of A x.
 template <typename T>
-__global__ void __launch_bounds__(256) k_add_Bq(T *__restrict__ dst, i64 nrows, const i64 *__restrict__ rows,
+__global__ void __launch_bounds__(256) k_add_Bq(T *dst, i64 nrows, const i64 *__restrict__ rows,
                                                  const i64 *__restrict__ ptr, const int *__restrict__ col,
-                                                 const double *__restrict__ val, const double *__restrict__ y,
+                                                 const double *__restrict__ val, const double *y,
                                                  const double *__restrict__ sigma_inv, double sign) {
     pdl_begin();
     for (i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (i64)gridDim.x * blockDim.x) {
@@ -1870,7 +1881,7 @@ __global__ void __launch_bounds__(256) k_add_Bq(T *__restrict__ dst, i64 nrows, 
 // their number counts).  FP32 adds the parents in their order.
 // On 127^3, FP64, under ncu: 24.4 -> 16.5 us, of which the FP64 unit 10.
 template <typename T, int DIM>
-__device__ __forceinline__ void prolong_add_body(T *__restrict__ x, const T *__restrict__ xc, const Grid3 &gf,
+__device__ __forceinline__ void prolong_add_body(T *x, const T *xc, const Grid3 &gf,
                                                  const Grid3 &gc, T alpha, int bx, int by, int bz_from_top) {
     // coarse cell (i, j, k), 0 <= i <= Nc0 etc., owns the fine vertices with
     // 1-based coordinates 2 i + {0, 1} (those inside the interior); its
@@ -1944,7 +1955,7 @@ __device__ __forceinline__ void prolong_add_body(T *__restrict__ x, const T *__r
 }
 
 template <typename T, int DIM>
-__global__ void __launch_bounds__(128) k_prolong_add(T *__restrict__ x, const T *__restrict__ xc, Grid3 gf, Grid3 gc,
+__global__ void __launch_bounds__(128) k_prolong_add(T *x, const T *xc, Grid3 gf, Grid3 gc,
                                                       T alpha) {
     if (gf.pdl) pdl_begin_trigger();
     prolong_add_body<T, DIM>(x, xc, gf, gc, alpha, blockIdx.x, blockIdx.y, (int)(gridDim.z - 1 - blockIdx.z));
@@ -1955,7 +1966,6 @@ __global__ void __launch_bounds__(128) k_prolong_add(T *__restrict__ x, const T 
 template <typename T, int VAR = 0>
 __global__ void __launch_bounds__(256) k_apply_stencil(const T *__restrict__ x, T *__restrict__ y, Grid3 g,
                                                         StencilArg<T> s, VarField<T> vf) {
-    if (g.pdl) pdl_begin();
     i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     i64 n = (i64)g.N0 * g.N1 * g.N2;
     if (t >= n) return;
@@ -1972,7 +1982,6 @@ __global__ void __launch_bounds__(256) k_apply_stencil(const T *__restrict__ x, 
 // ---------------------------------------------------- layout conversion
 template <typename T>
 __global__ void __launch_bounds__(256) k_unpack(const double *__restrict__ src, T *__restrict__ dst, Grid3 g) {
-    if (g.pdl) pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, c = blockIdx.z;
     if (a >= g.N0) return;
     dst[g.pad(a, b, c)] = (T)src[((i64)c * g.N1 + b) * g.N0 + a];
@@ -1983,7 +1992,6 @@ __global__ void __launch_bounds__(256) k_unpack(const double *__restrict__ src, 
 template <typename T>
 __global__ void __launch_bounds__(256) k_unpack2(const double *__restrict__ f_src, const double *__restrict__ x_src,
                                                  T *__restrict__ f_dst, T *__restrict__ x_dst, Grid3 g) {
-    if (g.pdl) pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, c = blockIdx.z;
     if (a >= g.N0) return;
     const i64 i = ((i64)c * g.N1 + b) * g.N0 + a, P = g.pad(a, b, c);
@@ -1994,7 +2002,6 @@ __global__ void __launch_bounds__(256) k_unpack2(const double *__restrict__ f_sr
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_pack(const T *__restrict__ src, double *__restrict__ dst, Grid3 g) {
-    if (g.pdl) pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, c = blockIdx.z;
     if (a >= g.N0) return;
     dst[((i64)c * g.N1 + b) * g.N0 + a] = (double)src[g.pad(a, b, c)];
@@ -2006,8 +2013,8 @@ __global__ void __launch_bounds__(256) k_pack(const T *__restrict__ src, double 
 // Parity form: column-oriented substitution in one CTA (same operation
 // order as the oracle, one rounding per operation).
 template <typename T, int NOISE>
-__global__ void __launch_bounds__(1024) k_chol_subst(const T *__restrict__ f, T *__restrict__ x, Grid3 g,
-                                                      const double *__restrict__ L, double *__restrict__ gv,
+__global__ void __launch_bounds__(1024) k_chol_subst(const T *f, T *x, Grid3 g,
+                                                      const double *__restrict__ L, double *gv,
                                                       NoiseArgs nz) {
     if (g.pdl) pdl_begin();
     const i64 n = (i64)g.N0 * g.N1 * g.N2;
@@ -2127,8 +2134,8 @@ struct WarpRow {
 // v = xi + Linv f (row i: vectors 0 .. i / NV), one warp per row: row, noise
 // and addresses before the wait for f.
 template <typename T, typename MT, int NOISE>
-__device__ __forceinline__ void chol_gemv_lower_body(const T *__restrict__ f, const Grid3 &g, const MT *__restrict__ Linv,
-                                                     int ld, MT *__restrict__ v, const NoiseArgs &nz, bool wait,
+__device__ __forceinline__ void chol_gemv_lower_body(const T *f, const Grid3 &g, const MT *__restrict__ Linv,
+                                                     int ld, MT *v, const NoiseArgs &nz, bool wait,
                                                      unsigned char *chol_sm, int bx) {
     MT *fs = reinterpret_cast<MT *>(chol_sm);
     const int n = g.N0 * g.N1 * g.N2;
@@ -2170,16 +2177,16 @@ __device__ __forceinline__ void chol_gemv_lower_body(const T *__restrict__ f, co
 // steps were slower: 2D 64 x 64 FP64 59.0 us, now 56.4; 3D 32^3 FP64 128 ->
 // 122 us; 96x48x80 27-point FP32 258 -> 240 us.)
 template <typename T, typename MT, int NOISE>
-__global__ void __launch_bounds__(256) k_chol_gemv_lower(const T *__restrict__ f, Grid3 g, const MT *__restrict__ Linv,
-                                                          int ld, MT *__restrict__ v, NoiseArgs nz) {
+__global__ void __launch_bounds__(256) k_chol_gemv_lower(const T *f, Grid3 g, const MT *__restrict__ Linv,
+                                                          int ld, MT *v, NoiseArgs nz) {
     extern __shared__ __align__(16) unsigned char chol_sm[];
     chol_gemv_lower_body<T, MT, NOISE>(f, g, Linv, ld, v, nz, g.pdl != 0, chol_sm, blockIdx.x);
 }
 
 // ... x = Linv^T v (row j of Linv^T: vectors j / NV .. ld / NV - 1).
 template <typename T, typename MT>
-__device__ __forceinline__ void chol_gemv_upper_body(const MT *__restrict__ v, const Grid3 &g,
-                                                     const MT *__restrict__ LinvT, int ld, T *__restrict__ x, bool wait,
+__device__ __forceinline__ void chol_gemv_upper_body(const MT *v, const Grid3 &g,
+                                                     const MT *__restrict__ LinvT, int ld, T *x, bool wait,
                                                      unsigned char *chol_sm, int bx) {
     MT *vs = reinterpret_cast<MT *>(chol_sm);
     const int n = g.N0 * g.N1 * g.N2;
@@ -2202,8 +2209,8 @@ __device__ __forceinline__ void chol_gemv_upper_body(const MT *__restrict__ v, c
 }
 
 template <typename T, typename MT>
-__global__ void __launch_bounds__(256) k_chol_gemv_upper(const MT *__restrict__ v, Grid3 g,
-                                                          const MT *__restrict__ LinvT, int ld, T *__restrict__ x) {
+__global__ void __launch_bounds__(256) k_chol_gemv_upper(const MT *v, Grid3 g,
+                                                          const MT *__restrict__ LinvT, int ld, T *x) {
     extern __shared__ __align__(16) unsigned char chol_sm[];
     chol_gemv_upper_body<T, MT>(v, g, LinvT, ld, x, g.pdl != 0, chol_sm, blockIdx.x);
 }
