@@ -297,6 +297,15 @@ struct SymWeights {
     double sd, od, om1;  // noise scale, omega / d, 1 - omega (kernels' UNIT: omega = 1, om1 = 0)
 };
 
+// With omega = 1 a point's new value does not need its old one.  A non-finite
+// old value still has to stay (x + (omega / d)(c - A x) keeps it, and an
+// observable reports it), so v becomes NaN there: by its bits, without an FP64
+// instruction.
+__device__ __forceinline__ double keep_nonfinite(double v, double old) {
+    const bool bad = (__double2hiint(old) & 0x7ff00000) == 0x7ff00000;
+    return __hiloint2double(bad ? 0x7ff80000 : __double2hiint(v), __double2loint(v));
+}
+
 // ------------------------------------------------- red-black SOR sweep
 // Noise of a 7-point level: the normals of the 4 points of one x-parity in
 // the 8-aligned group of padded positions P = a + 1 in [8q, 8q + 8) of row
@@ -362,12 +371,13 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_sym(double *x, const d
     if (NOISE == NOISE_INJECTED) xi = nz.buf[g.compact(a, b, c)];
     double *q = x + g.pad(a, b, c);
     double cv = f[g.pad(a, b, c)];
+    const double old = *q;
     const double sx = q[-1] + q[1], sy = q[-g.sy] + q[g.sy], sz = D3 ? q[-g.sz] + q[g.sz] : 0.0;
     if (NOISE != NOISE_NONE) cv = fma(w.sd, xi, cv);
     if (D3) cv = fma(-w.wc[4], sz, cv);
     cv = fma(-w.wc[2], sy, cv);
     cv = fma(-w.wc[1], sx, cv);
-    *q = UNIT ? w.od * cv : fma(w.od, cv, w.om1 * *q);
+    *q = UNIT ? keep_nonfinite(w.od * cv, old) : fma(w.od, cv, w.om1 * old);
 }
 
 // 256-bit vector access (sm_100 and later): 8 floats at a 32-byte aligned
@@ -814,7 +824,8 @@ __global__ void __launch_bounds__(ROW_SYM_THREADS)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         if ((a & 1) == (h ^ odd_first)) {
-            const double c1 = fma(-w.wc[1], row[-1] + row[1], cv), v = UNIT ? w.od * c1 : fma(w.od, c1, keep);
+            const double c1 = fma(-w.wc[1], row[-1] + row[1], cv);
+            const double v = UNIT ? keep_nonfinite(w.od * c1, s[0]) : fma(w.od, c1, keep);
             if (h == 0) row[0] = v;
             if (in) x[P] = v;
             if (h == 0 && !in) row[0] = 0.0;
