@@ -937,6 +937,25 @@ __device__ __forceinline__ ff32 ff_of(float2 v) { return {v.x, v.y}; }
 __device__ __forceinline__ double ff_to_double(ff32 a) { return (double)a.hi + (double)a.lo; }
 __device__ __forceinline__ float ff_to_float(ff32 a) { return __fadd_rn(a.hi, a.lo); }
 
+// A sum of products of a thread.  FP32 values: the products and the sum with
+// their rounding errors (exact products, TwoSum), so that a sum whose terms
+// cancel keeps the bits of its result.  FP64: one FMA per term.
+template <typename T>
+struct ProductSum {
+    T hi = T(0), lo = T(0);
+    __device__ __forceinline__ void add(T w, T v) {
+        if constexpr (sizeof(T) == 4) {
+            const float p = __fmul_rn(w, v);
+            const ff32 s = two_sum(hi, p);
+            lo = __fadd_rn(lo, __fadd_rn(s.lo, __fmaf_rn(w, v, -p)));
+            hi = s.hi;
+        } else {
+            hi = fma(w, v, hi);
+        }
+    }
+    __device__ __forceinline__ double value() const { return sizeof(T) == 4 ? (double)hi + (double)lo : (double)hi; }
+};
+
 // block_sum's shuffle tree in float-float; the result is valid in thread 0
 template <int NT>
 __device__ __forceinline__ ff32 block_sum_ff(ff32 v, float2 *sh) {
@@ -2234,7 +2253,9 @@ __global__ void __launch_bounds__(256) k_axpy(T *__restrict__ y, const T *__rest
 }
 
 // a -= A_0 u, b += u (b may be null) and `zero` = 0 (the work vector of the
-// next transposed sweep, may be null) over the interior, in one pass.
+// next transposed sweep, may be null) over the interior, in one pass.  A_0 u
+// cancels most of a (u is about A_0^{-1} a): FP32 forms the difference without
+// intermediate roundings.
 template <typename T, int NPT, int VAR>
 __global__ void __launch_bounds__(256) k_adj_update(const T *u, T *a, T *b, T *zero, Grid3 g, StencilArg<T> s, VarField<T> vf) {
     if (g.pdl) pdl_begin();
@@ -2242,20 +2263,26 @@ __global__ void __launch_bounds__(256) k_adj_update(const T *u, T *a, T *b, T *z
     if (i >= g.N0 || j >= g.N1) return;
     const i64 P = g.pad(i, j, blockIdx.z);
     constexpr int NZ = NPT == 9 ? 1 : 3;
-    T sum[NZ];  // by planes: three sums in flight
+    ProductSum<T> sum[NZ];  // by planes: three sums in flight
 #pragma unroll
     for (int z = 0; z < NZ; ++z) {
         const int dz = NZ == 1 ? 0 : z - 1;
-        sum[z] = T(0);
 #pragma unroll
         for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
             for (int dx = -1; dx <= 1; ++dx) {
                 if (NPT == 7 && (dz != 0) + (dy != 0) + (dx != 0) > 1) continue;
-                sum[z] += vweight<T, VAR>(s, vf, P, (dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * u[P + dz * g.sz + dy * g.sy + dx];
+                sum[z].add(vweight<T, VAR>(s, vf, P, (dz + 1) * 9 + (dy + 1) * 3 + dx + 1), u[P + dz * g.sz + dy * g.sy + dx]);
             }
     }
-    a[P] -= NZ == 1 ? sum[0] : (sum[0] + sum[NZ - 1]) + sum[NZ / 2];
+    if constexpr (sizeof(T) == 4) {
+        ff32 t{sum[0].hi, sum[0].lo};
+#pragma unroll
+        for (int z = 1; z < NZ; ++z) t = ff_add(t, ff32{sum[z].hi, sum[z].lo});
+        a[P] = ff_to_float(ff_add(ff32{a[P], 0.f}, ff_neg(t)));
+    } else {
+        a[P] -= NZ == 1 ? sum[0].hi : (sum[0].hi + sum[NZ - 1].hi) + sum[NZ / 2].hi;
+    }
     if (b) b[P] += u[P];
     if (zero) zero[P] = T(0);
 }
@@ -2460,10 +2487,11 @@ __device__ __forceinline__ int point_colour(int ncol, int a, int b, int c) {
 // A sweep (v = its output, w = its input; kd = dsd/ds / sd = E_c / (2 A_c))
 // has c = kd A - E, cv = kd A_c / omega - E_c / omega,
 // cw = kd A_c (1 - 1/omega) - E_c (1 - 1/omega), cf = -kd; -u^T dA v has
-// v = w, c = -E, cw = -E_c.  The neighbour sums run in the chain's type, the
-// u_p-weighted sum in FP64.  One weight per neighbour instead of one each for
-// the products with A and E (and one sum instead of eight): 30 FP64
-// instructions per point instead of 75, on a unit that takes two per clock.
+// v = w, c = -E, cw = -E_c.  The neighbour sums are FP64 ones, or those of
+// ProductSum over FP32 values; the u_p-weighted sum is FP64.  One weight per
+// neighbour instead of one each for the products with A and E (and one sum
+// instead of eight): 30 FP64 instructions per point instead of 75, on a unit
+// that takes two per clock.
 template <typename T>
 struct PgradWeights {
     T c[27];
@@ -2483,7 +2511,7 @@ __global__ void __launch_bounds__(256) k_pgrad_stencil(const T *u, const T *v, c
             const T up = u[P];
             if (up == T(0)) continue;
             const int cp = ncol ? point_colour(ncol, a, bb, c) : 0;
-            T sum[3] = {T(0), T(0), T(0)};  // by planes
+            ProductSum<T> sum[3];  // by planes
 #pragma unroll
             for (int dz = -1; dz <= 1; ++dz)
 #pragma unroll
@@ -2500,11 +2528,11 @@ __global__ void __launch_bounds__(256) k_pgrad_stencil(const T *u, const T *v, c
                             const int cq = point_colour(ncol, a + dx, bb + dy, c + dz);
                             before = forward ? cq < cp : cq > cp;
                         }
-                        sum[dz + 1] += pw.c[(dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)] *
-                                       (before ? v : w)[P + dz * g.sz + dy * g.sy + dx];
+                        sum[dz + 1].add(pw.c[(dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)],
+                                        (before ? v : w)[P + dz * g.sz + dy * g.sy + dx]);
                     }
             const double own = fma(pw.cv, (double)v[P], fma(pw.cw, (double)w[P], pw.cf * (double)f[P]));
-            acc = fma((double)up, (double)((sum[0] + sum[2]) + sum[1]) + own, acc);
+            acc = fma((double)up, ((sum[0].value() + sum[2].value()) + sum[1].value()) + own, acc);
         }
     }
     acc = block_sum_2d(acc, sh);
