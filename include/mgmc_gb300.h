@@ -344,7 +344,9 @@ mgmc_status mgmc_batch_destroy(mgmc_batch *b);
  * MGMC_NOISE_INJECTED in the reference's draw order), g = L^{-1} f
  * corrected by the low-rank factors, x = L^{-T}(xi + g) corrected likewise.
  * The host set-up costs about 2 nb p^3 flops (nb blocks of p vertices) and
- * the device holds 2 nb p^2 + 3 n m doubles.  apply: x <- a sample (x's
+ * the device holds 3 nb p^2 + n m doubles, or 2 nb p^2 + n m in a compact,
+ * slower form: where two of the nb p^2 are more than half of the free memory
+ * at creation, or with MGMC_LRCHOL_COMPACT=1 in the environment.  apply: x <- a sample (x's
  * input value is not used); f == NULL samples with the fixed f. */
 typedef struct mgmc_lrchol mgmc_lrchol;
 mgmc_status mgmc_lrchol_create(const mgmc_operator_desc *op, int noise, uint64_t seed, int device, mgmc_lrchol **out);

@@ -3310,13 +3310,19 @@ mgmc_status mgmc_batch_destroy(mgmc_batch *b) {
 // the low-rank part, and x = L^{-T} xi, each solve a product of all
 // triangular blocks and a chain of dense ones (k_chol_tri, k_chol_step),
 // captured into one CUDA graph.
+//
+// Memory: D and D^T share one array of nb p^2 values, E and G take two more.
+// Where these two are more than half of what is free, or with
+// MGMC_LRCHOL_COMPACT=1, the chain keeps O instead (two arrays in all; about
+// 95^3 cells are the limit of the larger form on an empty GPU, 112^3 of this
+// one) and runs with two products per block.
 struct LrChol {
     int device = 0, nb = 0, m = 0, noise = NOISE_PHILOX, nsm = 152;
     i64 n = 0;
     int p = 0, ld = 0;
     u64 seed = 0;
     cudaStream_t stream = nullptr;
-    double *D = nullptr, *DT = nullptr, *E = nullptr, *G = nullptr, *Q = nullptr, *W = nullptr;
+    double *D = nullptr, *E = nullptr, *G = nullptr, *O = nullptr, *Q = nullptr, *W = nullptr;
     double *f = nullptr, *x = nullptr, *xi = nullptr, *g = nullptr, *v = nullptr, *part = nullptr;  // blocks of ld
     double *cvec = nullptr;  // n values: a caller's vector
     double *noise_buf = nullptr;
@@ -3362,13 +3368,22 @@ struct LrChol {
         } else {
             k_cholesky_normals<NOISE_PHILOX><<<nblk(np, 256), 256, 0, stream>>>(nz, nb, p, ld, xi);
         }
-        auto triangular = [&](auto kernel, const double *A, const double *from, double *to) {
-            for (i64 k0 = 0; k0 < nb; k0 += 65535)  // grid.y carries the blocks
-                plaunch(true, kernel, dim3(((p + 1) / 2 + 7) / 8, (unsigned)std::min<i64>(nb - k0, 65535)), 256, 0, stream,
-                        A + k0 * mat, p, ld, from + k0 * ld, to + k0 * ld);
+        // y_k = (triangle of D_k) v_k, blocks a <= k < b
+        auto triangular = [&](auto kernel, i64 a, i64 b, const double *from, double *to) {
+            for (i64 k0 = a; k0 < b; k0 += 65535)  // grid.y carries the blocks
+                plaunch(true, kernel, dim3(((p + 1) / 2 + 7) / 8, (unsigned)std::min<i64>(b - k0, 65535)), 256, 0, stream,
+                        (const double *)D + k0 * mat, p, ld, from + k0 * ld, to + k0 * ld);
         };
-        triangular(k_chol_tri<false>, D, f, g);
-        for (int k = 1; k < nb; ++k) link(E + k * mat, g + (i64)(k - 1) * ld, g + (i64)k * ld);
+        if (O) {
+            CK(cudaMemcpyAsync(x, f, (size_t)np * sizeof(double), cudaMemcpyDeviceToDevice, stream));
+            for (int k = 0; k < nb; ++k) {
+                if (k > 0) link(O + k * mat, g + (i64)(k - 1) * ld, x + (i64)k * ld);
+                triangular(k_chol_tri<false>, k, k + 1, x, g);
+            }
+        } else {
+            triangular(k_chol_tri<false>, 0, nb, f, g);
+            for (int k = 1; k < nb; ++k) link(E + k * mat, g + (i64)(k - 1) * ld, g + (i64)k * ld);
+        }
         const unsigned rows = nblk(np, 128);
         const size_t sm = m * sizeof(double);
         if (m > 0) {
@@ -3384,8 +3399,17 @@ struct LrChol {
             plaunch(true, k_chol_add<true>, rows, 128, 0, stream, xi, (const double *)g, (const double *)nullptr, np, 0,
                     (const double *)nullptr);
         }
-        triangular(k_chol_tri<true>, DT, xi, x);
-        for (int k = nb - 2; k >= 0; --k) link(G + k * mat, x + (i64)(k + 1) * ld, x + (i64)k * ld);
+        if (O) {
+            for (int k = nb - 1; k >= 0; --k) {
+                if (k + 1 < nb)
+                    plaunch(true, k_chol_step_t, (p + 31) / 32, 256, 0, stream, (const double *)O + (k + 1) * mat, p, ld,
+                            (const double *)x + (i64)(k + 1) * ld, xi + (i64)k * ld);
+                triangular(k_chol_tri<true>, k, k + 1, xi, x);
+            }
+        } else {
+            triangular(k_chol_tri<true>, 0, nb, xi, x);
+            for (int k = nb - 2; k >= 0; --k) link(G + k * mat, x + (i64)(k + 1) * ld, x + (i64)k * ld);
+        }
         plaunch(true, k_counter_advance, 1, 1, 0, stream, d_step);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) fail(MGMC_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
@@ -3416,39 +3440,12 @@ struct LrChol {
     }
 };
 
-// The factors on the device: D and D^T with rows of ld, E_k = D_k O_k and
-// G_k = D_k^T O_{k+1}^T, Q by the blocks' rows (zero rows behind each block).
+// The factors on the device: the triangles of D_k and D_k^T in one block with
+// rows of ld, E_k = D_k O_k and G_k = D_k^T O_{k+1}^T or O_k, Q by the blocks'
+// rows (zero rows behind each block).  Called with every other buffer in place.
 void LrChol::set_factors(const LowRankCholeskyFactors &F) {
-    ld = (p + 3) / 4 * 4;
     const i64 mat = (i64)p * ld, pp = (i64)p * p;
-    D = zeros((size_t)nb * mat);
-    DT = zeros((size_t)nb * mat);
-    E = zeros((size_t)nb * mat);
-    G = zeros((size_t)nb * mat);
-    struct Temp {
-        std::vector<double *> ptrs;
-        ~Temp() {
-            for (double *q : ptrs) cudaFree(q);
-        }
-    } temp;
-    auto up = [&](const std::vector<double> &h) {
-        temp.ptrs.push_back(dupload(h, stream));
-        return temp.ptrs.back();
-    };
-    const double *Dc = up(F.D), *Oc = up(F.O);
-    // grid.z carries the blocks: at most 65535 at a time
-    for (int k0 = 0; k0 < nb; k0 += 65535) {
-        const int nk = std::min(nb - k0, 65535), ne = std::min(nb - 1 - k0, 65535);
-        const dim3 t32((p + 31) / 32, (p + 31) / 32, nk);
-        k_chol_copy<false><<<t32, 256, 0, stream>>>(Dc + k0 * pp, D + k0 * mat, p, ld);
-        k_chol_copy<true><<<t32, 256, 0, stream>>>(Dc + k0 * pp, DT + k0 * mat, p, ld);
-        if (ne <= 0) continue;
-        const dim3 t64((p + 63) / 64, (p + 63) / 64, ne);
-        k_chol_gemm<<<t64, 256, 0, stream>>>(Dc + (k0 + 1) * pp, pp, p, 1, Oc + (k0 + 1) * pp, pp, p, 1,
-                                             E + (k0 + 1) * mat, mat, ld, p);
-        k_chol_gemm<<<t64, 256, 0, stream>>>(Dc + k0 * pp, pp, 1, p, Oc + (k0 + 1) * pp, pp, 1, p, G + k0 * mat, mat, ld, p);
-    }
-    CK(cudaGetLastError());
+    const size_t all = (size_t)nb * mat;
     std::vector<double> Qp;
     if (m > 0) {
         Qp.assign((size_t)padded() * m, 0.0);
@@ -3458,6 +3455,48 @@ void LrChol::set_factors(const LowRankCholeskyFactors &F) {
         W = alloc<double>(F.W.size());
         CK(cudaMemcpyAsync(Q, Qp.data(), Qp.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
         CK(cudaMemcpyAsync(W, F.W.data(), F.W.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
+    }
+    D = zeros(all);
+    auto rows = [&](double *dst, const std::vector<double> &src) {
+        CK(cudaMemcpy2DAsync(dst, ld * sizeof(double), src.data(), p * sizeof(double), p * sizeof(double), (size_t)nb * p,
+                             cudaMemcpyHostToDevice, stream));
+    };
+    rows(D, F.D);
+    // grid.z carries the blocks: at most 65535 at a time
+    for (int k0 = 0; k0 < nb; k0 += 65535) {
+        k_chol_mirror<<<dim3((p + 31) / 32, (p + 31) / 32, std::min(nb - k0, 65535)), 256, 0, stream>>>(D + k0 * mat, p, ld);
+        CK(cudaGetLastError());
+    }
+    // O in pieces of about 256 MB, each with the first block of the next
+    const int piece = (int)std::max<i64>(1, std::min<i64>(nb, std::min<i64>(65535, (i64(1) << 25) / pp)));
+    size_t free_bytes = 0, total_bytes = 0;
+    CK(cudaMemGetInfo(&free_bytes, &total_bytes));
+    const char *e = std::getenv("MGMC_LRCHOL_COMPACT");
+    if ((e && e[0] == '1') || (2 * all + (piece + 1) * pp) * sizeof(double) > free_bytes / 2) {
+        O = zeros(all);
+        rows(O, F.O);
+    } else {
+        E = zeros(all);
+        G = zeros(all);
+        struct Temp {
+            double *p = nullptr;
+            ~Temp() { cudaFree(p); }
+        } temp;
+        temp.p = dalloc<double>((size_t)(piece + 1) * pp);
+        for (int k0 = 0; k0 < nb; k0 += piece) {
+            const int k1 = std::min(nb, k0 + piece), k2 = std::min(nb, k1 + 1);
+            CK(cudaMemcpyAsync(temp.p, F.O.data() + k0 * pp, (size_t)(k2 - k0) * pp * sizeof(double), cudaMemcpyHostToDevice, stream));
+            const dim3 tiles((p + 63) / 64, (p + 63) / 64);
+            const int first = std::max(k0, 1);
+            if (k1 > first)
+                k_chol_gemm<false><<<dim3(tiles.x, tiles.y, k1 - first), 256, 0, stream>>>(
+                    D + first * mat, mat, ld, temp.p + (first - k0) * pp, pp, p, 1, E + first * mat, p);
+            if (k2 - 1 > k0)
+                k_chol_gemm<true><<<dim3(tiles.x, tiles.y, k2 - 1 - k0), 256, 0, stream>>>(
+                    D + k0 * mat, mat, ld, temp.p + pp, pp, 1, p, G + k0 * mat, p);
+            CK(cudaGetLastError());
+        }
+        CK(cudaStreamSynchronize(stream));  // before the pieces' buffer goes
     }
     CK(cudaStreamSynchronize(stream));
 }
@@ -3527,7 +3566,7 @@ mgmc_status mgmc_lrchol_create(const mgmc_operator_desc *op, int noise, uint64_t
     CK(cudaDeviceGetAttribute(&S.nsm, cudaDevAttrMultiProcessorCount, device));
     S.noise = noise == MGMC_NOISE_INJECTED ? NOISE_INJECTED : NOISE_PHILOX;
     S.seed = seed;
-    S.set_factors(F);
+    S.ld = (S.p + 3) / 4 * 4;
     if (S.m > 0) {
         S.v = S.alloc<double>(S.m);
         S.part = S.alloc<double>((size_t)((S.padded() + CHOL_QT_ROWS - 1) / CHOL_QT_ROWS) * S.m);
@@ -3542,6 +3581,7 @@ mgmc_status mgmc_lrchol_create(const mgmc_operator_desc *op, int noise, uint64_t
     for (double **q : {&S.f, &S.x, &S.xi, &S.g}) *q = S.zeros((size_t)S.padded());
     S.d_step = S.alloc<u64>(1);
     CK(cudaMemsetAsync(S.d_step, 0, sizeof(u64), S.stream));
+    S.set_factors(F);
     CK(cudaStreamSynchronize(S.stream));
     *out = h;
     h = nullptr;

@@ -2779,12 +2779,15 @@ __global__ void __launch_bounds__(256) k_step_end(const T *x, StepEnd e) {
 // one dense product per block (k_chol_step): half the dependent launches of
 // the form with two products per block, and every product reads rows.
 // Vectors are stored by blocks of ld doubles (p, padded with zeros to a
-// multiple of 4), matrices with rows of ld.
+// multiple of 4), matrices with rows of ld.  D_k and D_k^T share one symmetric
+// array: row i holds row i of D_k up to the diagonal and row i of D_k^T from
+// there on.  Where E and G do not fit, the chain keeps O and runs the first
+// form, one block at a time (k_chol_step with O_k, k_chol_step_t, k_chol_tri).
 
-// y_k = A_k v_k for all blocks k = blockIdx.y, A_k triangular (UPPER: columns
-// j >= i).  A warp takes the rows i and p - 1 - i, together one full row, and
-// reduces both sums in five steps instead of ten: FP64 instructions, two per
-// clock per SM, bound it.
+// y_k = A_k v_k for all blocks k = blockIdx.y, A_k the lower or (UPPER: columns
+// j >= i) the upper triangle of the stored block.  A warp takes the rows i and
+// p - 1 - i, together one full row, and reduces both sums in five steps instead
+// of ten: FP64 instructions, two per clock per SM, bound it.
 template <bool UPPER>
 __global__ void __launch_bounds__(256) k_chol_tri(const double *__restrict__ A, int p, int ld, const double *v, double *y) {
     const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5), k = blockIdx.y;
@@ -2795,12 +2798,16 @@ __global__ void __launch_bounds__(256) k_chol_tri(const double *__restrict__ A, 
     auto row_sum = [&](int r) {
         const double2 *a = reinterpret_cast<const double2 *>(A + ((i64)k * p + r) * ld);
         const int q0 = UPPER ? r / 2 : 0, q1 = UPPER ? ld / 2 : r / 2 + 1;
+        // the pair at the diagonal, a lane's first (UPPER) or last one, may hold a value of the other triangle
+        const int qd = UPPER == (r & 1) ? r / 2 : -1;
         double s0 = 0.0, s1 = 0.0;
         int q = q0 + lane;
         for (; q + 96 < q1; q += 128) {
             double2 av[4], vv[4];
 #pragma unroll
             for (int t = 0; t < 4; ++t) av[t] = __ldcs(a + q + 32 * t);
+            if (UPPER && q == qd) av[0].x = 0.0;
+            if (!UPPER && q + 96 == qd) av[3].y = 0.0;
 #pragma unroll
             for (int t = 0; t < 4; ++t) vv[t] = vk[q + 32 * t];
 #pragma unroll
@@ -2810,7 +2817,9 @@ __global__ void __launch_bounds__(256) k_chol_tri(const double *__restrict__ A, 
             }
         }
         for (; q < q1; q += 32) {
-            const double2 av = __ldcs(a + q), vv = vk[q];
+            double2 av = __ldcs(a + q);
+            const double2 vv = vk[q];
+            if (q == qd) (UPPER ? av.x : av.y) = 0.0;
             s0 = fma(av.x, vv.x, s0);
             s1 = fma(av.y, vv.y, s1);
         }
@@ -2871,6 +2880,26 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(const double *__restrict__
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0 && row < p) y[row] -= s;
+}
+
+// y -= A^T v, A p x p dense: a CTA takes 32 columns, its warps every eighth row.
+__global__ void __launch_bounds__(256) k_chol_step_t(const double *__restrict__ A, int p, int ld, const double *v, double *y) {
+    __shared__ double sh[8][32];
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5, j = blockIdx.x * 32 + l;
+    pdl_begin();
+    double t = 0.0;
+    if (j < p) {
+#pragma unroll 4
+        for (int i = w; i < p; i += 8) t = fma(A[(i64)i * ld + j], v[i], t);
+    }
+    sh[w][l] = t;
+    __syncthreads();
+    if (w == 0 && j < p) {
+        t = 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t += sh[i][l];
+        y[j] -= t;
+    }
 }
 
 // Low-rank part, xi += g + Q (W^T - Id) Q^T g, then xi += Q (W - Id) Q^T xi:
@@ -3003,23 +3032,24 @@ __global__ void __launch_bounds__(256) k_chol_unpad(const double *__restrict__ s
     if (k < nb && j < p) dst[(i64)k * p + j] = src[t];
 }
 
-// Set-up: C_k(i, j) = sum_l A_k(i, l) B_k(l, j), p x p each, through strides
-// (A_k(i, l) at k as + i ai + l al, and so on); tiles of 64 x 64, 4 x 4 per
-// thread.
-__global__ void __launch_bounds__(256) k_chol_gemm(const double *__restrict__ A, i64 as, i64 ai, i64 al,
-                                                   const double *__restrict__ B, i64 bs, i64 bl, i64 bj,
-                                                   double *__restrict__ C, i64 cs, i64 ci, int p) {
+// Set-up: C_k(i, j) = sum_l A_k(i, l) B_k(l, j), p x p each, A_k the lower or
+// (UPPER) the upper triangle of a block of S, B_k through strides (B_k(l, j) at
+// k bs + l bl + j bj); tiles of 64 x 64, 4 x 4 per thread.
+template <bool UPPER>
+__global__ void __launch_bounds__(256) k_chol_gemm(const double *__restrict__ S, i64 mat, int ld, const double *__restrict__ B,
+                                                   i64 bs, i64 bl, i64 bj, double *__restrict__ C, int p) {
     __shared__ double At[16][64 + 1], Bt[16][64 + 1];
-    A += blockIdx.z * as;
+    S += blockIdx.z * mat;
     B += blockIdx.z * bs;
-    C += blockIdx.z * cs;
+    C += blockIdx.z * mat;
     const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     double acc[4][4] = {};
-    for (int l0 = 0; l0 < p; l0 += 16) {
+    const int l1 = UPPER ? p : min(p, i0 + 64);
+    for (int l0 = UPPER ? i0 : 0; l0 < l1; l0 += 16) {
         for (int t = threadIdx.x; t < 16 * 64; t += 256) {
+            const int la = t & 15, i = i0 + (t >> 4), l = l0 + la;
+            At[la][t >> 4] = i < p && l < p && (UPPER ? l >= i : l <= i) ? S[(i64)i * ld + l] : 0.0;
             // the index with the unit stride runs over the threads
-            const int la = al == 1 ? t & 15 : t >> 6, ia = al == 1 ? t >> 4 : t & 63;
-            At[la][ia] = i0 + ia < p && l0 + la < p ? A[(i0 + ia) * ai + (l0 + la) * al] : 0.0;
             const int lb = bl == 1 ? t & 15 : t >> 6, jb = bl == 1 ? t >> 4 : t & 63;
             Bt[lb][jb] = j0 + jb < p && l0 + lb < p ? B[(l0 + lb) * bl + (j0 + jb) * bj] : 0.0;
         }
@@ -3036,26 +3066,20 @@ __global__ void __launch_bounds__(256) k_chol_gemm(const double *__restrict__ A,
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b)
-            if (i0 + ty + 16 * a < p && j0 + tx + 16 * b < p) C[(i0 + ty + 16 * a) * ci + j0 + tx + 16 * b] = acc[a][b];
+            if (i0 + ty + 16 * a < p && j0 + tx + 16 * b < p) C[(i64)(i0 + ty + 16 * a) * ld + j0 + tx + 16 * b] = acc[a][b];
 }
 
-// blocks of p x p values to blocks of p rows of ld, transposed or not
-template <bool TRANSPOSE>
-__global__ void __launch_bounds__(256) k_chol_copy(const double *__restrict__ src, double *__restrict__ dst, int p, int ld) {
+// the upper triangles of blocks of p rows of ld from the lower ones
+__global__ void __launch_bounds__(256) k_chol_mirror(double *S, int p, int ld) {
     __shared__ double tile[32][33];
-    src += (i64)blockIdx.z * p * p;
-    dst += (i64)blockIdx.z * p * ld;
+    S += (i64)blockIdx.z * p * ld;
     const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    if (i0 < j0) return;
     for (int r = ty; r < 32; r += 8)
-        if (i0 + r < p && j0 + tx < p) tile[r][tx] = src[(i64)(i0 + r) * p + j0 + tx];
+        if (i0 + r < p && j0 + tx < p) tile[r][tx] = S[(i64)(i0 + r) * ld + j0 + tx];
     __syncthreads();
-    for (int r = ty; r < 32; r += 8) {
-        if (TRANSPOSE) {
-            if (j0 + r < p && i0 + tx < p) dst[(i64)(j0 + r) * ld + i0 + tx] = tile[tx][r];
-        } else {
-            if (i0 + r < p && j0 + tx < p) dst[(i64)(i0 + r) * ld + j0 + tx] = tile[r][tx];
-        }
-    }
+    for (int r = ty; r < 32; r += 8)
+        if (i0 + tx < p && i0 + tx > j0 + r) S[(i64)(j0 + r) * ld + i0 + tx] = tile[tx][r];
 }
 
 __global__ void k_counter_advance(u64 *step) {
