@@ -3385,18 +3385,22 @@ struct LrChol {
             for (int k = 1; k < nb; ++k) link(E + k * mat, g + (i64)(k - 1) * ld, g + (i64)k * ld);
         }
         const unsigned rows = nblk(np, 128);
-        const size_t sm = m * sizeof(double);
         if (m > 0) {
             const int parts = (int)((np + CHOL_QT_ROWS - 1) / CHOL_QT_ROWS);
+            const bool wide = m > CHOL_STAGE_M;
+            const size_t sm = wide ? 0 : m * sizeof(double);
             const double *cQ = Q, *cW = W, *cg = g, *cxi = xi, *cv = v, *cp = part;
-            plaunch(true, k_chol_qt, parts, 256, 0, stream, cQ, np, m, cg, part);
-            plaunch(true, k_chol_v<true>, 1, 1024, sm, stream, cp, parts, m, cW, v);
-            plaunch(true, k_chol_add<true>, rows, 128, sm, stream, xi, cg, cQ, np, m, cv);
-            plaunch(true, k_chol_qt, parts, 256, 0, stream, cQ, np, m, cxi, part);
-            plaunch(true, k_chol_v<false>, 1, 1024, sm, stream, cp, parts, m, cW, v);
-            plaunch(true, k_chol_add<false>, rows, 128, sm, stream, xi, cg, cQ, np, m, cv);
+            auto lowrank = [&](auto kernel_v, auto kernel_add, const double *from) {
+                plaunch(true, k_chol_qt, parts, 256, 0, stream, cQ, np, m, from, part);
+                plaunch(true, kernel_v, 1, 1024, sm, stream, cp, parts, m, cW, v, v + m);
+                plaunch(true, kernel_add, rows, 128, sm, stream, xi, cg, cQ, np, m, cv);
+            };
+            wide ? lowrank(k_chol_v<true, true>, k_chol_add<true, true>, cg)
+                 : lowrank(k_chol_v<true, false>, k_chol_add<true, false>, cg);
+            wide ? lowrank(k_chol_v<false, true>, k_chol_add<false, true>, cxi)
+                 : lowrank(k_chol_v<false, false>, k_chol_add<false, false>, cxi);
         } else {
-            plaunch(true, k_chol_add<true>, rows, 128, 0, stream, xi, (const double *)g, (const double *)nullptr, np, 0,
+            plaunch(true, k_chol_add<true, false>, rows, 128, 0, stream, xi, (const double *)g, (const double *)nullptr, np, 0,
                     (const double *)nullptr);
         }
         if (O) {
@@ -3568,13 +3572,14 @@ mgmc_status mgmc_lrchol_create(const mgmc_operator_desc *op, int noise, uint64_t
     S.seed = seed;
     S.ld = (S.p + 3) / 4 * 4;
     if (S.m > 0) {
-        S.v = S.alloc<double>(S.m);
+        S.v = S.alloc<double>(2 * (size_t)S.m);  // and k_chol_v's t
         S.part = S.alloc<double>((size_t)((S.padded() + CHOL_QT_ROWS - 1) / CHOL_QT_ROWS) * S.m);
-        if (S.m * sizeof(double) > 48 * 1024) {
-            raise_smem_limit(k_chol_v<true>, S.m * sizeof(double));
-            raise_smem_limit(k_chol_v<false>, S.m * sizeof(double));
-            raise_smem_limit(k_chol_add<true>, S.m * sizeof(double));
-            raise_smem_limit(k_chol_add<false>, S.m * sizeof(double));
+        const size_t sm = S.m * sizeof(double);
+        if (sm > 48 * 1024 && S.m <= CHOL_STAGE_M) {
+            raise_smem_limit(k_chol_v<true, false>, sm);
+            raise_smem_limit(k_chol_v<false, false>, sm);
+            raise_smem_limit(k_chol_add<true, false>, sm);
+            raise_smem_limit(k_chol_add<false, false>, sm);
         }
     }
     S.cvec = S.alloc<double>(S.n);

@@ -2938,11 +2938,14 @@ __global__ void __launch_bounds__(256) k_chol_qt(const double *__restrict__ Q, i
 }
 
 // t = the sum of the parts and v = (W - Id) t (TRANSPOSE: (W^T - Id) t) in one
-// CTA of 1024 threads, eight lanes per sum
-template <bool TRANSPOSE>
+// CTA of 1024 threads, eight lanes per sum.  WIDE, more columns than shared
+// memory takes (CHOL_STAGE_M): t in tbuf, in global memory.
+constexpr int CHOL_STAGE_M = 28672;
+template <bool TRANSPOSE, bool WIDE>
 __global__ void __launch_bounds__(1024) k_chol_v(const double *part, int nparts, int m, const double *__restrict__ W,
-                                                 double *v) {
-    extern __shared__ double ts[];
+                                                 double *v, double *tbuf) {
+    extern __shared__ double t_sm[];
+    double *ts = WIDE ? tbuf : t_sm;
     pdl_begin();
     pdl_trigger();
     const int l = threadIdx.x & 7, q = threadIdx.x >> 3;
@@ -2973,15 +2976,18 @@ __global__ void __launch_bounds__(1024) k_chol_v(const double *part, int nparts,
     }
 }
 
-// xi += Q v (ADD_G: + g), one thread per row
-template <bool ADD_G>
+// xi += Q v (ADD_G: + g), one thread per row, v in shared memory unless WIDE
+template <bool ADD_G, bool WIDE>
 __global__ void __launch_bounds__(128) k_chol_add(double *xi, const double *g, const double *__restrict__ Q, i64 rows, int m,
                                                   const double *v) {
-    extern __shared__ double vs[];
+    extern __shared__ double v_sm[];
+    const double *vs = WIDE ? v : v_sm;
     pdl_begin();
     pdl_trigger();
-    for (int j = threadIdx.x; j < m; j += blockDim.x) vs[j] = v[j];
-    __syncthreads();
+    if (!WIDE) {
+        for (int j = threadIdx.x; j < m; j += blockDim.x) v_sm[j] = v[j];
+        __syncthreads();
+    }
     const i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
     double a0 = 0.0, a1 = 0.0;

@@ -1,11 +1,14 @@
 """The low-rank Cholesky sampler's two forms: with the products E and G of the
 factor's blocks (three arrays of the blocks' size) and compact (two), which
-lattices whose three arrays do not fit fall back to."""
+lattices whose three arrays do not fit fall back to; any number of columns."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import multigridmc_gb300 as M
 import oracle as O
+from gpu_helpers.build import build as gpu_build
 from problems import posterior
 
 pytestmark = pytest.mark.gpu
@@ -68,3 +71,27 @@ def test_both_forms_draw_the_same(monkeypatch):
         s.close()
     # the same normals; 64 eps per unit of the prior's condition number, below 1e4 here
     assert np.linalg.norm(out[0] - out[1]) < 64 * np.finfo(float).eps * 1e4 * np.linalg.norm(out[0])
+
+
+@pytest.mark.parametrize("m", [1, 300, 6200, 28672, 28673, 30000])
+def test_columns_beyond_shared_memory(m):
+    """m x m and Q products up to and beyond the columns that shared memory
+    takes (W = 0 where it would be gigabytes of host data)."""
+    lib = C.CDLL(gpu_build("chol_wide_check"))
+    rng = np.random.default_rng(m)
+    part, Q = rng.standard_normal((3, m)), rng.standard_normal((130, m))
+    W = rng.standard_normal((m, m)) if m <= 300 else None
+    g, xi0 = rng.standard_normal(130), rng.standard_normal(130)
+    P = lambda a: a.ctypes.data_as(C.POINTER(C.c_double)) if a is not None else None
+    out = []
+    for wide in (-1, 1):
+        xi, v = xi0.copy(), np.zeros(m)
+        assert lib.chol_wide_check(P(part), 3, m, P(W), P(Q), 130, P(g), P(xi), P(v), wide) == 0
+        out.append((xi, v))
+    t = part.sum(0)
+    want = (W.T @ t if W is not None else 0.0) - t
+    # sums of m products of size below 6 x 18 in FP64
+    for xi, v in out:
+        assert np.max(np.abs(v - want)) < 1e-15 * 110 * (m if W is not None else 3)
+        assert np.max(np.abs(xi - (xi0 + g + Q @ want))) < 1e-15 * m * 6 * max(1.0, np.abs(want).max())
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
