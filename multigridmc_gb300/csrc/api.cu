@@ -611,7 +611,7 @@ static void launch_sweep_noise(Sampler &S, const Level &lv, bool forward, int no
         launch_sweep_npt<T, EXACT, NOISE_NONE>(S, lv, forward, x, f, nz);
     else if (noise == NOISE_PHILOX)
         launch_sweep_npt<T, EXACT, NOISE_PHILOX>(S, lv, forward, x, f, nz);
-    else
+    else if constexpr (sizeof(T) == 4 || EXACT)  // an FP64 chain with injected noise is exact
         launch_sweep_npt<T, EXACT, NOISE_INJECTED>(S, lv, forward, x, f, nz);
 }
 

@@ -368,7 +368,6 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_rb_sym(double *x, const d
     if (g.pdl) pdl_begin();
     if (trigger) pdl_trigger();
     if (a >= g.N0 || b >= g.N1) return;
-    if (NOISE == NOISE_INJECTED) xi = nz.buf[g.compact(a, b, c)];
     double *q = x + g.pad(a, b, c);
     double cv = f[g.pad(a, b, c)];
     const double old = *q;
@@ -789,7 +788,6 @@ __global__ void __launch_bounds__(ROW_SYM_THREADS)
     if (g.pdl) pdl_begin();
     if (trigger) pdl_trigger();
     const i64 P = g.pad(a, b, c);
-    if (NOISE == NOISE_INJECTED && in) xi = nz.buf[g.compact(a, b, c)];
     // position a + 1 of the class rows; positions 0 and N0 + 1 are ghosts
     const int pitch = blockDim.x + 2;
     double *row = reinterpret_cast<double *>(row_sm) + threadIdx.y * (NC + 1) * pitch + 1 + a;
@@ -1003,8 +1001,7 @@ struct LowRankArg {
 // thread's first index/value loads are issued before the wait for the
 // kernel that wrote x (`wait`: the caller has not waited yet).
 template <typename T>
-__device__ __forceinline__ void bt_partial_cta(const T *x, const LowRankArg &lr, double *sh, int j, int p, int P,
-                                               bool wait = false) {
+__device__ __forceinline__ void bt_partial_cta(const T *x, const LowRankArg &lr, double *sh, int j, int p, int P) {
     const i64 e0 = lr.Bptr[j], e1 = lr.Bptr[j + 1];
     const i64 len = P == 1 ? e1 - e0 : (e1 - e0 + P - 1) / P;
     const i64 lo = e0 + p * len, hi = min(e1, lo + len);
@@ -1021,10 +1018,8 @@ __device__ __forceinline__ void bt_partial_cta(const T *x, const LowRankArg &lr,
     };
     i64 e = lo + threadIdx.x;
     load(e);
-    if (wait) {
-        pdl_begin();
-        pdl_trigger();  // the correction's rows, S^{-1} and normals load meanwhile
-    }
+    pdl_begin();
+    pdl_trigger();  // the correction's rows, S^{-1} and normals load meanwhile
     // eight index/value loads, then the eight gathers, in flight at once;
     // the products are added in entry order
     for (; e < hi; e += 8 * 256) {
@@ -1054,7 +1049,7 @@ __device__ __forceinline__ void bt_partial_body(const T *x, const LowRankArg &lr
     float xif = 0.f;
     if (draws && NOISE == NOISE_PHILOX)
         xif = pick(normals4(philox4x32_10(noise_ctr(nz, (unsigned)(j >> 2), PURPOSE_LOWRANK, 0), noise_key(nz))), j & 3);
-    bt_partial_cta<T>(x, lr, sh, j, p, P, true);
+    bt_partial_cta<T>(x, lr, sh, j, p, P);
     if (draws) {
         if constexpr (sizeof(T) == 4) {
             const ff32 w = ff_mul(ff_of(lr.sigma_sqrt_ff[j]), ff32{NOISE == NOISE_INJECTED ? (float)nz.buf[j] : xif, 0.f});
@@ -1117,7 +1112,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_bt_full(const T *x, LowRankArg lr) {
     __shared__ double sh[32];
     __shared__ bool last;
-    bt_partial_cta<T>(x, lr, sh, blockIdx.x, blockIdx.y, gridDim.y, true);
+    bt_partial_cta<T>(x, lr, sh, blockIdx.x, blockIdx.y, gridDim.y);
     if (threadIdx.x == 0) {
         unsigned prev;
         asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(lr.counter) : "memory");
@@ -1144,15 +1139,15 @@ struct CorrRows {
 };
 
 // Four single-entry rows of a thread, r0 + j stride (j < 4) below r1: row index,
-// column, value and state loaded together; the update adds the
-// product to zero, then to the state, as a multi-entry row's (FP64: one FMA).  The state of rows loaded before the wait
-// for the previous kernel is read through L2 (see k_lr_correct).
+// column, value and state loaded together, before the wait (the state through
+// L2: see k_lr_correct); the update adds the product to zero, then to the state,
+// as a multi-entry row's (FP64: one FMA).
 template <typename T>
 struct CorrQuad {
     unsigned row[4];
     int col[4];
     T val[4], xv[4];
-    __device__ __forceinline__ void load(const T *x, const CorrRows &C, int r0, int stride, int r1, bool before_wait) {
+    __device__ __forceinline__ void load(const T *x, const CorrRows &C, int r0, int stride, int r1) {
         const T *v1 = static_cast<const T *>(C.v1);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -1164,7 +1159,7 @@ struct CorrQuad {
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            xv[j] = r0 + j * stride < r1 ? (before_wait ? __ldcg(x + row[j]) : x[row[j]]) : T(0);
+            xv[j] = r0 + j * stride < r1 ? __ldcg(x + row[j]) : T(0);
     }
     template <typename ZT>
     __device__ __forceinline__ void apply(T *x, int r0, int stride, int r1, const ZT *z) const {
@@ -1183,15 +1178,14 @@ struct CorrQuad {
 };
 
 // One multi-entry row r (two entries at least) with its row index, entry
-// range, first PF entries and state loaded together, before the wait for
-// the previous kernel where the caller says so; its products are added to
-// zero in entry order, then to the state.
+// range, first PF entries and state loaded together, before the wait; its
+// products are added to zero in entry order, then to the state.
 template <typename T, int PF>
 struct CorrMulti {
     unsigned row;
     int e0, e1, col[PF];
     T val[PF], xv;
-    __device__ __forceinline__ void load(const T *x, const CorrRows &C, i64 r, bool before_wait) {
+    __device__ __forceinline__ void load(const T *x, const CorrRows &C, i64 r) {
         const T *vm = static_cast<const T *>(C.vm);
         row = C.rm[r];
         e0 = C.pm[r];
@@ -1202,7 +1196,7 @@ struct CorrMulti {
                 col[k] = C.cm[e0 + k];
                 val[k] = vm[e0 + k];
             }
-        xv = before_wait ? __ldcg(x + row) : x[row];
+        xv = __ldcg(x + row);
     }
     template <typename ZT>
     __device__ __forceinline__ void apply(T *x, const CorrRows &C, const ZT *z) const {
@@ -1267,11 +1261,11 @@ __device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int 
     CorrQuad<T> q[NQ];
     CorrMulti<T, PF> mr;
     if (jb.multi) {
-        if (row < jb.r1) mr.load(x, C, row, true);
+        if (row < jb.r1) mr.load(x, C, row);
     } else {
 #pragma unroll
         for (int i = 0; i < NQ; ++i)
-            if (row + 1024 * i < jb.r1) q[i].load(x, C, row + 1024 * i, 256, jb.r1, true);
+            if (row + 1024 * i < jb.r1) q[i].load(x, C, row + 1024 * i, 256, jb.r1);
     }
     // terms of a column in groups g = 0 .. tpr - 1: columns g, g + tpr, ... of S^{-1}
     const int cols = m < 256 ? m : 256, tpr = 256 / cols, groups = min(tpr, m);
