@@ -1211,8 +1211,8 @@ void Sampler::build_lowrank(int lev) {
             pm.swap(ps);
             cm.swap(cs);
             vm.swap(vs);
-            if (r1.size() > (size_t)INT32_MAX || cm.size() > (size_t)INT32_MAX)
-                fail(MGMC_ERR_UNSUPPORTED, "more than 2^31 support rows of C on a level");
+            if (cm.size() > (size_t)INT32_MAX)
+                fail(MGMC_ERR_UNSUPPORTED, "more than 2^31 entries in the rows of C with several entries on a level");
             std::vector<CorrJob> jobs;
             std::vector<int> jcols;
             int widest = 1;
@@ -1224,9 +1224,9 @@ void Sampler::build_lowrank(int lev) {
             while (rows1 < 3072 && (i64)rows1 * 2 * nsm < (i64)r1.size()) rows1 = rows1 < 1024 ? 1024 : rows1 + 1024;
             lv.Cquads[dir] = (rows1 + 1023) / 1024;
             std::vector<int> mark(m, -1);
-            auto add_jobs = [&](int multi, int n, int most, auto first, auto last) {  // entries first(r) .. last(r) of row r
-                for (int r = 0; r < n;) {
-                    CorrJob jb{r, r, multi, (int)jcols.size(), 0};
+            auto add_jobs = [&](int multi, i64 n, int most, auto first, auto last) {  // entries first(r) .. last(r) of row r
+                for (i64 r = 0; r < n;) {
+                    CorrJob jb{r, 0, multi, (int)jcols.size(), 0};
                     while (r < n && r - jb.r0 < most) {
                         int fresh = 0;
                         for (const int *c = first(r); c != last(r); ++c) fresh += mark[*c] != (int)jobs.size();
@@ -1239,12 +1239,12 @@ void Sampler::build_lowrank(int lev) {
                             }
                         ++r;
                     }
-                    jb.r1 = r;
+                    jb.n = (int)(r - jb.r0);
                     jobs.push_back(jb);
                 }
             };
-            add_jobs(0, (int)r1.size(), rows1, [&](int r) { return c1.data() + r; }, [&](int r) { return c1.data() + r + 1; });
-            add_jobs(1, (int)nm, 256, [&](int r) { return cm.data() + pm[r]; }, [&](int r) { return cm.data() + pm[r + 1]; });
+            add_jobs(0, (i64)r1.size(), rows1, [&](i64 r) { return c1.data() + r; }, [&](i64 r) { return c1.data() + r + 1; });
+            add_jobs(1, (i64)nm, 256, [&](i64 r) { return cm.data() + pm[r]; }, [&](i64 r) { return cm.data() + pm[r + 1]; });
             lv.Cjobs[dir] = upload(jobs);
             lv.Ccols[dir] = upload(jcols);
             lv.n_Cjobs[dir] = (int)jobs.size();
@@ -2979,10 +2979,10 @@ void BatchGroup::build(cudaStream_t st) {
                 b.P = lv.bt_split;
                 // rows of a CTA beyond four per thread become CTAs of their own
                 for (const CorrJob &full : lv.hCjobs[dir])
-                    for (int r0 = full.r0; r0 < full.r1; r0 += 1024) {
+                    for (int r = 0; r < full.n; r += 1024) {
                         CorrJob jb = full;
-                        jb.r0 = r0;
-                        jb.r1 = std::min(full.r1, r0 + 1024);
+                        jb.r0 = full.r0 + r;
+                        jb.n = std::min(full.n - r, 1024);
                         cj[dir][lv.Cmode[dir]].push_back(BatchCorrJob{c, jb});
                     }
             }

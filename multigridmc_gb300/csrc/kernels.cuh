@@ -1138,34 +1138,36 @@ struct CorrRows {
     const void *vm = nullptr;
 };
 
-// Four single-entry rows of a thread, r0 + j stride (j < 4) below r1: row index,
-// column, value and state loaded together, before the wait (the state through
-// L2: see k_lr_correct); the update adds the product to zero, then to the state,
-// as a multi-entry row's (FP64: one FMA).
+// Four single-entry rows of a thread, r0 + j stride (j < 4) of the n rows from
+// `base` on: row index, column, value and state loaded together, before the wait
+// (the state through L2: see k_lr_correct); the update adds the product to zero,
+// then to the state, as a multi-entry row's (FP64: one FMA).
 template <typename T>
 struct CorrQuad {
     unsigned row[4];
     int col[4];
     T val[4], xv[4];
-    __device__ __forceinline__ void load(const T *x, const CorrRows &C, int r0, int stride, int r1) {
-        const T *v1 = static_cast<const T *>(C.v1);
+    __device__ __forceinline__ void load(const T *x, const CorrRows &C, i64 base, int r0, int stride, int n) {
+        const unsigned *r1 = C.r1 + base;
+        const int *c1 = C.c1 + base;
+        const T *v1 = static_cast<const T *>(C.v1) + base;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int r = r0 + j * stride;
-            const bool ok = r < r1;
-            row[j] = ok ? C.r1[r] : 0u;
-            col[j] = ok ? C.c1[r] : 0;
+            const bool ok = r < n;
+            row[j] = ok ? r1[r] : 0u;
+            col[j] = ok ? c1[r] : 0;
             val[j] = ok ? v1[r] : T(0);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            xv[j] = r0 + j * stride < r1 ? __ldcg(x + row[j]) : T(0);
+            xv[j] = r0 + j * stride < n ? __ldcg(x + row[j]) : T(0);
     }
     template <typename ZT>
-    __device__ __forceinline__ void apply(T *x, int r0, int stride, int r1, const ZT *z) const {
+    __device__ __forceinline__ void apply(T *x, int r0, int stride, int n, const ZT *z) const {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (r0 + j * stride >= r1) continue;
+            if (r0 + j * stride >= n) continue;
             if (sizeof(T) == 4) {
                 T acc = T(0);
                 acc += val[j] * (T)z[col[j]];
@@ -1234,7 +1236,8 @@ struct CorrMulti {
 constexpr int LRC_MAX_M = 64, LRC_MAX_COLS = 16;  // columns of S^{-1}, and of a CTA's rows, in mode 0
 
 struct CorrJob {
-    int r0, r1;      // rows
+    i64 r0;          // first row (a level may have more than 2^31 single-entry rows)
+    int n;           // rows
     int multi;       // of the multi-entry rows
     int c0, nc;      // their columns: cols[c0 .. c0 + nc)
 };
@@ -1257,15 +1260,14 @@ __device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int 
         Sinv = lr.SinvT_ff;
     else
         Sinv = lr.SinvT;
-    const int row = jb.r0 + tid;
     CorrQuad<T> q[NQ];
     CorrMulti<T, PF> mr;
     if (jb.multi) {
-        if (row < jb.r1) mr.load(x, C, row);
+        if (tid < jb.n) mr.load(x, C, jb.r0 + tid);
     } else {
 #pragma unroll
         for (int i = 0; i < NQ; ++i)
-            if (row + 1024 * i < jb.r1) q[i].load(x, C, row + 1024 * i, 256, jb.r1);
+            if (tid + 1024 * i < jb.n) q[i].load(x, C, jb.r0, tid + 1024 * i, 256, jb.n);
     }
     // terms of a column in groups g = 0 .. tpr - 1: columns g, g + tpr, ... of S^{-1}
     const int cols = m < 256 ? m : 256, tpr = 256 / cols, groups = min(tpr, m);
@@ -1426,11 +1428,11 @@ __device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int 
         }
     }
     if (jb.multi) {
-        if (row < jb.r1) mr.apply(x, C, zs);
+        if (tid < jb.n) mr.apply(x, C, zs);
     } else {
 #pragma unroll
         for (int i = 0; i < NQ; ++i)
-            if (row + 1024 * i < jb.r1) q[i].apply(x, row + 1024 * i, 256, jb.r1, zs);
+            if (tid + 1024 * i < jb.n) q[i].apply(x, tid + 1024 * i, 256, jb.n, zs);
     }
 }
 
