@@ -109,7 +109,8 @@ struct Level {
     int bt_split = 1;  // blocks per column of the B^T x reduction
     unsigned *counter = nullptr;  // CTA counter of k_bt_full
     int sweep_tx = 0;             // CTA width of the colour passes chosen by the autotuner (0: sweep_block())
-    int sweep_threads = 0;        // and its thread count, 128 or 256 (0: RBP_THREADS)
+    int sweep_threads = 0;        // and its thread count, 64 to 256 (0: RBP_THREADS)
+    bool one_colour = false;      // rows fit a CTA, but one colour per launch is faster (autotune_sweeps)
     // constant stencil with equal weights at +-dx, +-dy, +-dz (to rounding):
     // wc[|dz| * 4 + |dy| * 2 + |dx|] (k_sweep_row_sym)
     bool sym = false;
@@ -526,7 +527,7 @@ static void launch_colour_passes(Sampler &S, const Level &lv, bool forward, T *x
                                  const NoiseArgs &nz) {
     const bool pdl = S.pdl && lv.g.pdl;
     const VarField<T> vf = var_field<T>(lv);
-    if (lv.g.N0 <= ROW_PAIR_MAX_N0) {
+    if (lv.g.N0 <= ROW_PAIR_MAX_N0 && !lv.one_colour) {
         const int npair = lv.ncol / 2;
         for (int q = 0; q < npair; ++q) {
             const int pr = forward ? q : npair - 1 - q, pb = pr & 1, pc = pr >> 1;
@@ -1584,11 +1585,22 @@ void Sampler::upload_field(Level &lv) {
     }
 }
 
-// Autotuner of the colour passes' CTA shape: for every level that sweeps,
-// time a few sweeps on scratch vectors for each CTA of 128 or 256 threads
-// whose width fits the level's rows (the block shape does not change any
-// result: every thread owns whole points or spans) and keep the fastest.
-// MGMC_AUTOTUNE=0 keeps the heuristic shapes.
+// Autotuner of the colour passes: for every level that sweeps one colour per
+// launch (small ones and whole rows excepted), time a few sweeps on scratch
+// vectors for each CTA of 128 or 256 threads whose width fits the level's rows
+// and keep the fastest.  No choice changes a result: every thread owns whole
+// points or spans, and their sums are the same in every kernel.
+//
+// FP64 levels in 3D that add weight by weight (per-vertex or unsymmetric
+// stencils; k_sweep_row_pair) are timed both ways where they have more than
+// 2^18 points.  Below, two colours of a row per launch always won (64^3
+// per-vertex: 40 us a sweep, one colour 50; 32^3 23, 39).  Above, the launches
+// saved no longer decide: an FP64 instruction takes a warp's time whether its
+// lanes have points or not, and rows leave lanes idle by their length
+// (per-vertex 80^3: 105, one colour 79; 72^3 100, 75; 96^3 155, 114; 128^3 247,
+// 272; unsymmetric constants 80^3: 61, 52; 128 x 64 x 64 40, 47).
+// MGMC_AUTOTUNE=0 keeps the heuristic shapes and whole rows.
+constexpr i64 ROW_PAIR64_SURE = i64(1) << 18;
 void Sampler::autotune_sweeps() {
     if (const char *e = std::getenv("MGMC_AUTOTUNE"))
         if (e[0] == '0') return;
@@ -1600,7 +1612,10 @@ void Sampler::autotune_sweeps() {
     for (int lev = 0; lev < nlev; ++lev) {
         if (lev == nlev - 1 && chol) break;
         Level &lv = L[lev];
-        if (lv.npt != 7 && lv.g.N0 <= ROW_PAIR_MAX_N0) continue;  // whole rows: no width to choose
+        // whole rows have no width to choose
+        const bool whole = lv.npt != 7 && lv.g.N0 <= ROW_PAIR_MAX_N0;
+        const bool by_class = !exact && lv.sym && lv.var == 0;  // k_sweep_row_sym
+        if (whole && (fp32 || dim < 3 || by_class || lv.geo.n <= ROW_PAIR64_SURE)) continue;
         const bool vec = fp32 && !exact && lv.npt == 7 && (lv.g.sy % 4) == 0 && (lv.g.sz % 4) == 0 && lv.var != 2;
         const int count = vec ? (lv.g.N0 + 8) / 8 : (lv.g.N0 + 1) / 2;
         // a level of at most eight warps per SM: small CTAs spread it best, and
@@ -1621,26 +1636,34 @@ void Sampler::autotune_sweeps() {
         int best_tx = 0, best_nt = RBP_THREADS;
         // the level's own f (still zero, only read): level 0 then runs the
         // kernel variant the chain runs (the colour-split f); best of three
+        auto time_sweeps = [&]() {
+            float least = 1e30f;
+            for (int r = 0; r < 2; ++r) launch_sweep(*this, lv, true, noise, lv.s1, lv.f, nz, fp32, exact);
+            for (int trial = 0; trial < 3; ++trial) {
+                CK(cudaEventRecord(e0, stream));
+                for (int r = 0; r < 4; ++r) launch_sweep(*this, lv, r % 2 == 0, noise, lv.s1, lv.f, nz, fp32, exact);
+                CK(cudaEventRecord(e1, stream));
+                CK(cudaEventSynchronize(e1));
+                float ms = 0.f;
+                CK(cudaEventElapsedTime(&ms, e0, e1));
+                least = std::min(least, ms);
+            }
+            return least;
+        };
+        const float pairs = whole ? time_sweeps() : 1e30f;
+        lv.one_colour = whole;
         for (int nt : {RBP_THREADS, RBP_THREADS / 2})
             for (int tx = 8; tx <= std::min(nt, 2 * cap); tx *= 2) {
                 lv.sweep_tx = tx;
                 lv.sweep_threads = nt;
-                for (int r = 0; r < 2; ++r) launch_sweep(*this, lv, true, noise, lv.s1, lv.f, nz, fp32, exact);
-                for (int trial = 0; trial < 3; ++trial) {
-                    CK(cudaEventRecord(e0, stream));
-                    for (int r = 0; r < 4; ++r)
-                        launch_sweep(*this, lv, r % 2 == 0, noise, lv.s1, lv.f, nz, fp32, exact);
-                    CK(cudaEventRecord(e1, stream));
-                    CK(cudaEventSynchronize(e1));
-                    float ms = 0.f;
-                    CK(cudaEventElapsedTime(&ms, e0, e1));
-                    if (ms < best) {
-                        best = ms;
-                        best_tx = tx;
-                        best_nt = nt;
-                    }
+                const float ms = time_sweeps();
+                if (ms < best) {
+                    best = ms;
+                    best_tx = tx;
+                    best_nt = nt;
                 }
             }
+        if (pairs <= best) lv.one_colour = false;
         lv.sweep_tx = best_tx;
         lv.sweep_threads = best_nt;
         CK(cudaMemsetAsync(lv.s1, 0, (size_t)lv.geo.nalloc * tsize(), stream));
