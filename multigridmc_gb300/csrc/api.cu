@@ -705,13 +705,22 @@ void Sampler::sor(int lev, bool forward, bool noisy, void *x, void *f, int nspar
     if (noisy) inv++;
 }
 
-// k_resid_restrict_sym, CTAs of 64 threads at least
+// k_resid_restrict_sym, CTAs of 64 threads at least.  Whole warps beyond a
+// row's end would run its FP64 instructions all the same, so rows of more than
+// 32 points take the next multiple of 32, and rows longer than a CTA equal
+// windows.  (7-point, plain launches, CTAs of the next power of two and now:
+// 80^3 cells 22.6 and 18.5 us, 144^3 111 and 74, 160^3 135 and 90, 272 x 64 x 64
+// 45 and 31; tiles of point residuals, k_resid_restrict_tma, take 21.7, 96, 119
+// and 39.)
 static void launch_resid_restrict_sym(Sampler &S, const Level &lv, const Level &lc, const double *x, const double *f,
                                       double *fc, double *xc, const StencilArg<double> &s) {
     const SymWeights w = sym_weights(lv, s);
     const int whole = lv.g.N0 <= 256;
-    int tx = 16;
-    while (tx < lv.g.N0 && tx < 256) tx *= 2;
+    int tx = lv.g.N0 <= 16 ? 16 : (lv.g.N0 + 31) / 32 * 32;
+    if (!whole) {  // windows of 2 txc + 3 columns
+        const int windows = (lc.g.N0 + 125) / 126;
+        tx = (2 * ((lc.g.N0 + windows - 1) / windows) + 3 + 31) / 32 * 32;
+    }
     const dim3 blk(tx, std::max(1, 64 / tx), 1);
     const int txc = whole ? lc.g.N0 : (tx - 3) / 2;
     const dim3 grid((lc.g.N0 + txc - 1) / txc, (lc.g.N1 + blk.y - 1) / blk.y, S.dim == 3 ? lc.g.N2 : 1);
