@@ -104,7 +104,8 @@ struct Level {
     double *SinvT[2] = {nullptr, nullptr};  // S^{-1} transposed, per sweep direction
     float2 *SinvT_ff[2] = {nullptr, nullptr};  // the same as float-float pairs (FP32 chain)
     double *y = nullptr, *z = nullptr, *part = nullptr;
-    void *w = nullptr;  // m values: the low-rank noise of the sweep in flight
+    void *w = nullptr;   // m values: the low-rank noise of the sweep in flight
+    void *zv = nullptr;  // m values: its coefficients z, where k_lr_z forms them
     float *Bvalf = nullptr;
     int bt_split = 1;  // blocks per column of the B^T x reduction
     unsigned *counter = nullptr;  // CTA counter of k_bt_full
@@ -627,10 +628,13 @@ static void launch_sweep(Sampler &S, const Level &lv, bool forward, int noise, v
         launch_sweep_noise<double, false>(S, lv, forward, noise, (double *)x, (const double *)f, nz);
 }
 
-// dynamic shared memory of k_lr_correct: u and z (m values), products and sums
-static size_t lr_correct_smem(int m) {
-    return sizeof(double) * (2 * (size_t)m + 64 * 8 + LRC_MAX_M);
+// dynamic shared memory of k_lr_correct: z (mode 2), or u, z, products and
+// sums; and of k_lr_z: u and the warps' sums (24 KB and 26 KB at most)
+static size_t lr_correct_smem(int m, int mode) {
+    return sizeof(double) * (mode == 2 ? (size_t)m : 2 * (size_t)m + 64 * 8);
 }
+static size_t lr_z_smem(int m) { return sizeof(double) * ((size_t)m + 8 * 32); }
+static unsigned lr_z_ctas(int m) { return (unsigned)((m + LRZ_COLS - 1) / LRZ_COLS); }
 
 template <typename T>
 static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, const NoiseArgs &nz, double *zpub = nullptr) {
@@ -652,6 +656,7 @@ static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, cons
     const i64 nrows = C.n1 + C.nm;
     if (nrows == 0) return;  // empty columns: nothing to correct
     lr.w = lv.w;
+    lr.zv = lv.zv;
     auto gather = [&](auto kernel) {
         plaunch(S.pdl, kernel, dim3(S.m, lv.bt_split), 256, 0, S.stream, (const T *)x, lr, nz);
     };
@@ -662,7 +667,7 @@ static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, cons
     else
         gather(k_bt_partial<T, NOISE_INJECTED>);
     auto correct = [&](auto kernel) {
-        plaunch(S.pdl, kernel, lv.n_Cjobs[dir], 256, lr_correct_smem(S.m), S.stream, x, lr, lv.bt_split, C,
+        plaunch(S.pdl, kernel, lv.n_Cjobs[dir], 256, lr_correct_smem(S.m, lv.Cmode[dir]), S.stream, x, lr, lv.bt_split, C,
                 (const CorrJob *)lv.Cjobs[dir], (const int *)lv.Ccols[dir]);
     };
     const int nq = lv.Cquads[dir];
@@ -670,8 +675,11 @@ static void launch_lowrank(Sampler &S, Level &lv, int dir, int noise, T *x, cons
         nq == 1 ? correct(k_lr_correct<T, 0, 1>) : nq == 2 ? correct(k_lr_correct<T, 0, 2>) : correct(k_lr_correct<T, 0, 3>);
     else if (lv.Cmode[dir] == 1)
         nq == 1 ? correct(k_lr_correct<T, 1, 1>) : nq == 2 ? correct(k_lr_correct<T, 1, 2>) : correct(k_lr_correct<T, 1, 3>);
-    else
+    else {
+        plaunch(S.pdl, k_lr_z<T>, lr_z_ctas(S.m), 256, lr_z_smem(S.m), S.stream, lr, lv.bt_split);
+        S.launches++;
         nq == 1 ? correct(k_lr_correct<T, 2, 1>) : nq == 2 ? correct(k_lr_correct<T, 2, 2>) : correct(k_lr_correct<T, 2, 3>);
+    }
     S.launches += 2;
 }
 
@@ -1092,6 +1100,7 @@ void Sampler::build_lowrank(int lev) {
     lv.z = alloc<double>(m);
     CK(cudaMemsetAsync(lv.z, 0, m * sizeof(double), stream));
     lv.w = alloc<double>(m);
+    lv.zv = alloc<double>(m);
     {
         i64 maxcol = 1;
         for (int j = 0; j < m; ++j) maxcol = std::max<i64>(maxcol, lv.Bh.ptr[j + 1] - lv.Bh.ptr[j]);
@@ -1188,7 +1197,17 @@ void Sampler::build_lowrank(int lev) {
         // 4.6, 4.4, 4.5, 4.6).  Where most rows have one entry (and none has
         // too many), a run has at most LRC_MAX_COLS columns and its CTA forms
         // those z only (mode 0: 256,000 rows 4.8 us, all of z in every CTA
-        // 6.0)
+        // 6.0).  Otherwise every CTA repeats the m x m product (mode 1).  With
+        // more CTAs than the SMs hold at once a launch of its own forms z
+        // (mode 2), and always above LRC_MAX_M columns.  Gather to correction:
+        // mode 1 against 2, FP64, 48^3 cells with 32 balls, 243 CTAs, 10.9 and
+        // 11.0 us; with 64 balls, 322 CTAs, 13.5 and 12.4; 64^3 with 16, 654
+        // CTAs, 29 and 13; 128^3 with 32, 6335 CTAs, 229 and 64; mode 0 against
+        // 2, 128^3 with 3, 310 CTAs, 9.8 and 12.9; 2D 1024^2 with 10, 420 CTAs,
+        // 12.6 and 10.9; 160^3 with 3, FP32, 879 CTAs, 19.8 and 14.3.  (300
+        // balls on 64^3 in mode 1's way: 259 us, now 25.)  Beyond 16 CTAs per
+        // SM a CTA of mode 2 takes 1024 multi-entry rows (128^3 with 32: 70 us
+        // with 256 each, 64; 64^3 with 300 and 978 CTAs: 118 and 147).
         {
             std::vector<size_t> ord(r1.size());
             for (size_t k = 0; k < ord.size(); ++k) ord[k] = k;
@@ -1227,20 +1246,22 @@ void Sampler::build_lowrank(int lev) {
             std::vector<int> jcols;
             int widest = 1;
             for (size_t k = 0; k < nm; ++k) widest = std::max(widest, pm[k + 1] - pm[k]);
-            const int mode = m > LRC_MAX_M ? 2 : r1.size() >= 2 * nm && widest <= LRC_MAX_COLS ? 0 : 1;
-            const int max_cols = mode == 0 ? LRC_MAX_COLS : m;
-            lv.Cmode[dir] = mode;
             int rows1 = 512;
             while (rows1 < 3072 && (i64)rows1 * 2 * nsm < (i64)r1.size()) rows1 = rows1 < 1024 ? 1024 : rows1 + 1024;
             lv.Cquads[dir] = (rows1 + 1023) / 1024;
-            std::vector<int> mark(m, -1);
+            int mode = r1.size() >= 2 * nm && widest <= LRC_MAX_COLS ? 0 : 1;
+            const i64 ctas = ((i64)r1.size() + rows1 - 1) / rows1 + ((i64)nm + 255) / 256;
+            if (m > LRC_MAX_M || (mode == 1 ? ctas > 2 * (i64)nsm : 2 * ctas > 5 * (i64)nsm)) mode = 2;
+            lv.Cmode[dir] = mode;
+            std::vector<int> mark(m, -1);  // mode 0: the last CTA that has the column
             auto add_jobs = [&](int multi, i64 n, int most, auto first, auto last) {  // entries first(r) .. last(r) of row r
                 for (i64 r = 0; r < n;) {
                     CorrJob jb{r, 0, multi, (int)jcols.size(), 0};
-                    while (r < n && r - jb.r0 < most) {
+                    if (mode != 0) r = std::min<i64>(n, r + most);
+                    while (mode == 0 && r < n && r - jb.r0 < most) {
                         int fresh = 0;
                         for (const int *c = first(r); c != last(r); ++c) fresh += mark[*c] != (int)jobs.size();
-                        if (jb.nc + fresh > max_cols) break;
+                        if (jb.nc + fresh > LRC_MAX_COLS) break;
                         for (const int *c = first(r); c != last(r); ++c)
                             if (mark[*c] != (int)jobs.size()) {
                                 jcols.push_back(*c | (mark[*c] < 0 ? CORR_OWNER : 0));
@@ -1254,7 +1275,7 @@ void Sampler::build_lowrank(int lev) {
                 }
             };
             add_jobs(0, (i64)r1.size(), rows1, [&](i64 r) { return c1.data() + r; }, [&](i64 r) { return c1.data() + r + 1; });
-            add_jobs(1, (i64)nm, 256, [&](i64 r) { return cm.data() + pm[r]; }, [&](i64 r) { return cm.data() + pm[r + 1]; });
+            add_jobs(1, (i64)nm, mode == 2 && ctas > 16 * (i64)nsm ? 1024 : 256, [&](i64 r) { return cm.data() + pm[r]; }, [&](i64 r) { return cm.data() + pm[r + 1]; });
             lv.Cjobs[dir] = upload(jobs);
             lv.Ccols[dir] = upload(jcols);
             lv.n_Cjobs[dir] = (int)jobs.size();
@@ -1536,14 +1557,6 @@ void Sampler::build(const mgmc_operator_desc &op) {
         d_sigma_inv = upload(si);
         d_sigma_sqrt = upload(ss);
         d_sigma_sqrt_ff = upload(float_float(ss));
-        if (lr_correct_smem(m) > 48 * 1024) {
-            raise_smem_limit(k_lr_correct<float, 2, 1>, lr_correct_smem(m));
-            raise_smem_limit(k_lr_correct<float, 2, 2>, lr_correct_smem(m));
-            raise_smem_limit(k_lr_correct<float, 2, 3>, lr_correct_smem(m));
-            raise_smem_limit(k_lr_correct<double, 2, 1>, lr_correct_smem(m));
-            raise_smem_limit(k_lr_correct<double, 2, 2>, lr_correct_smem(m));
-            raise_smem_limit(k_lr_correct<double, 2, 3>, lr_correct_smem(m));
-        }
         for (size_t lev = 0; lev < L.size(); ++lev) build_lowrank((int)lev);
     }
     if (chol) build_coarse();
@@ -2929,6 +2942,8 @@ struct BatchGroup {
     // per level and direction: the correction's CTAs by mode (k_lr_correct)
     std::vector<std::array<std::array<BatchCorrJob *, 3>, 2>> corr_jobs;
     std::vector<std::array<std::array<int, 3>, 2>> n_corr;
+    std::vector<std::array<BatchZJob *, 2>> z_jobs;  // the solves of mode 2
+    std::vector<std::array<int, 2>> n_z;
     std::vector<BatchAddBq *> bq;             // per level: rows of the next level's B
     std::vector<RowJob *> bq_jobs;
     std::vector<int> n_bq;
@@ -2960,6 +2975,8 @@ void BatchGroup::build(cudaStream_t st) {
     n_bt.assign(nlev, 0);
     corr_jobs.resize(nlev);
     n_corr.resize(nlev);
+    z_jobs.resize(nlev);
+    n_z.resize(nlev);
     bq.resize(nlev);
     bq_jobs.resize(nlev);
     n_bq.assign(nlev, 0);
@@ -2967,17 +2984,12 @@ void BatchGroup::build(cudaStream_t st) {
         max_m = std::max(max_m, S->m);
         max_probe = std::max(max_probe, S->nprobe * S->obs_split);
     }
-    // (beyond 2784 columns; the group's largest m sizes the launches of every mode)
-    if (lr_correct_smem(max_m) > 48 * 1024) {
-        raise_smem_limit(k_lr_correct_batch<0>, lr_correct_smem(max_m));
-        raise_smem_limit(k_lr_correct_batch<1>, lr_correct_smem(max_m));
-        raise_smem_limit(k_lr_correct_batch<2>, lr_correct_smem(max_m));
-    }
     for (int lev = 0; lev < nlev; ++lev) {
         std::vector<BatchLevelArg> a(G);
         std::vector<BatchLowRank> l0(G), l1(G);
         std::vector<BtJob> jobs;
         std::vector<BatchCorrJob> cj[2][3];
+        std::vector<BatchZJob> zj[2];
         std::vector<RowJob> qj;
         std::vector<BatchAddBq> q(G);
         for (int c = 0; c < G; ++c) {
@@ -3006,9 +3018,12 @@ void BatchGroup::build(cudaStream_t st) {
                 r.sigma_sqrt_ff = S.d_sigma_sqrt_ff;
                 r.part = lv.part;
                 r.w = lv.w;
+                r.zv = lv.zv;
                 b.C = lv.C[dir];
                 b.jobcols = lv.Ccols[dir];
                 b.P = lv.bt_split;
+                if (lv.Cmode[dir] == 2 && !lv.hCjobs[dir].empty())
+                    for (int t = 0; t < (int)lr_z_ctas(S.m); ++t) zj[dir].push_back(BatchZJob{c, t});
                 // rows of a CTA beyond four per thread become CTAs of their own
                 for (const CorrJob &full : lv.hCjobs[dir])
                     for (int r = 0; r < full.n; r += 1024) {
@@ -3032,11 +3047,14 @@ void BatchGroup::build(cudaStream_t st) {
         lr[lev] = {put(l0, st), put(l1, st)};
         bt_jobs[lev] = put(jobs, st);
         n_bt[lev] = (int)jobs.size();
-        for (int dir = 0; dir < 2; ++dir)
+        for (int dir = 0; dir < 2; ++dir) {
+            z_jobs[lev][dir] = put(zj[dir], st);
+            n_z[lev][dir] = (int)zj[dir].size();
             for (int mode = 0; mode < 3; ++mode) {
                 corr_jobs[lev][dir][mode] = put(cj[dir][mode], st);
                 n_corr[lev][dir][mode] = (int)cj[dir][mode].size();
             }
+        }
         bq[lev] = put(q, st);
         bq_jobs[lev] = put(qj, st);
         n_bq[lev] = (int)qj.size();
@@ -3106,11 +3124,13 @@ void BatchGroup::sor(int lev, bool forward, cudaStream_t st) {
         const BatchLowRank *low = lr[lev][dir];
         plaunch(pdl, k_bt_partial_batch<NOISE_PHILOX>, n_bt[lev], 256, 0, st, (const BatchLevelArg *)la[lev], low,
                 (const BatchChainArg *)ca, (const BtJob *)bt_jobs[lev], inv, (unsigned)lev);
+        if (n_z[lev][dir] > 0)
+            plaunch(pdl, k_lr_z_batch, n_z[lev][dir], 256, lr_z_smem(max_m), st, low, (const BatchZJob *)z_jobs[lev][dir]);
         // chains of different modes correct in launches of their own
         auto correct = [&](int mode, auto kernel) {
             if (n_corr[lev][dir][mode] > 0)
-                plaunch(pdl, kernel, n_corr[lev][dir][mode], 256, lr_correct_smem(max_m), st, (const BatchLevelArg *)la[lev],
-                        low, (const BatchCorrJob *)corr_jobs[lev][dir][mode]);
+                plaunch(pdl, kernel, n_corr[lev][dir][mode], 256, lr_correct_smem(mode < 2 ? std::min(max_m, LRC_MAX_M) : max_m, mode), st,
+                        (const BatchLevelArg *)la[lev], low, (const BatchCorrJob *)corr_jobs[lev][dir][mode]);
         };
         correct(0, k_lr_correct_batch<0>);
         correct(1, k_lr_correct_batch<1>);

@@ -17,6 +17,7 @@
 //                       (one CTA; parity mode)
 //   k_bt_partial        partial sums of y = B^T x, the low-rank noise
 //   k_lr_correct        the m x m solve and x += C z over the rows of C = M^{-1} B
+//   k_lr_z              the solve alone, for k_lr_correct on large m or supports
 //   k_bt_full           y = B^T x in one launch (k_bt_sum: from partial sums)
 //   k_resid_restrict_tma    f_c = R (f - A_0 x), TMA tiles (fused residual
 //                           + restriction; _tiled / plain variants otherwise)
@@ -987,7 +988,8 @@ struct LowRankArg {
                         // stores float-float pairs, float2, in the same slots)
     unsigned *counter;  // CTA counter of k_bt_full (reset by its last CTA)
     void *w;                     // m scratch: Sigma^{1/2} xi' (double, or float2 for the FP32 chain)
-    double *zpub;                // where k_lr_correct leaves z (null: nowhere)
+    double *zpub;                // where the solve leaves z (null: nowhere)
+    void *zv;                    // m scratch: z of k_lr_z in the chain's type
     const float2 *SinvT_ff;      // SinvT as float-float pairs (FP32 chain)
     const float2 *sigma_sqrt_ff; // Sigma^{1/2} as float-float pairs (FP32 chain)
 };
@@ -1218,11 +1220,12 @@ struct CorrMulti {
 // multi-entry ones, both sorted by column).  MODE 0, up to LRC_MAX_M columns
 // and mostly single-entry rows: it forms the z of the columns of its own rows
 // only, their products one per thread.  MODE 1, the same where columns overlap
-// throughout (coarse levels): all of z, S^{-1} loaded before the wait.  MODE 2:
-// all of z of more columns.  The FP32 chain forms every z_k in the same order wherever it
-// is formed (256 / m groups of terms per column, two
-// alternating sums in a group), so all CTAs and the batched kernels agree bit
-// for bit.
+// throughout (coarse levels): all of z, S^{-1} loaded before the wait.  MODE 2,
+// more columns, or overlapping ones on more CTAs than should repeat the solve:
+// z comes from a launch of its own (k_lr_z).  The FP32 chain forms every z_k of
+// modes 0 and 1 in the same order wherever it is formed (256 / m groups of
+// terms per column, two alternating sums in a group), so all CTAs and the
+// batched kernels agree bit for bit.
 //
 // What bounds it is the chain of dependent loads and sums behind the launch
 // that gathered x, so everything that does not depend on it -- the rows of C
@@ -1232,8 +1235,8 @@ struct CorrMulti {
 // the sweep's writes are visible), and few registers keep all CTAs of a large
 // support resident.  (Gather and correction behind a short launch, the
 // kernels before -> these: FP64 m = 32, 8,000 rows 7.5 -> 4.5 us, 54,000 rows
-// 9.4 -> 6.0; FP32 m = 64, 19,000 rows 7.1 -> 4.4, 256,000 rows 9.6 -> 6.5.)
-constexpr int LRC_MAX_M = 64, LRC_MAX_COLS = 16;  // columns of S^{-1}, and of a CTA's rows, in mode 0
+// 9.4 -> 6.0; FP32 m = 64, 19,000 rows 7.1 -> 4.4, 256,000 rows 9.6 -> 4.8.)
+constexpr int LRC_MAX_M = 64, LRC_MAX_COLS = 16;  // columns of S^{-1} in modes 0 and 1, and of a CTA's rows in mode 0
 
 struct CorrJob {
     i64 r0;          // first row (a level may have more than 2^31 single-entry rows)
@@ -1244,56 +1247,10 @@ struct CorrJob {
 // in the list of columns: the first CTA that has the column
 constexpr int CORR_OWNER = 1 << 30;
 
-// PF entries of a multi-entry row are loaded ahead: 8 in k_lr_correct's mode 1
-// (coarse rows have many: 2D 768 x 480 FP64 step 2.5 % faster than with 2, 3D
-// 128^3 1.3 %), 2 in the batch, whose CTAs need the registers to be resident
-// (20 chains: 2.5 % slower with 8).
-template <typename T, int MODE, int NQ, int PF = 2>
-__device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int P, const CorrRows &C, const CorrJob &jb,
-                                                const int *__restrict__ jobcols, bool first, double *dyn) {
-    typedef typename std::conditional<sizeof(T) == 4, float2, double>::type V;  // FP32 chain: float-float
-    const int m = lr.m, tid = threadIdx.x;
-    V *u = reinterpret_cast<V *>(dyn), *pr = u + m;
-    T *zs = reinterpret_cast<T *>(pr + (MODE ? 256 : 64 * 8));
-    const V *Sinv;
-    if constexpr (sizeof(T) == 4)
-        Sinv = lr.SinvT_ff;
-    else
-        Sinv = lr.SinvT;
-    CorrQuad<T> q[NQ];
-    CorrMulti<T, PF> mr;
-    if (jb.multi) {
-        if (tid < jb.n) mr.load(x, C, jb.r0 + tid);
-    } else {
-#pragma unroll
-        for (int i = 0; i < NQ; ++i)
-            if (tid + 1024 * i < jb.n) q[i].load(x, C, jb.r0, tid + 1024 * i, 256, jb.n);
-    }
-    // terms of a column in groups g = 0 .. tpr - 1: columns g, g + tpr, ... of S^{-1}
-    const int cols = m < 256 ? m : 256, tpr = 256 / cols, groups = min(tpr, m);
-    const int g = MODE ? tid / cols : 0, kk = tid - g * cols, cnt = g < groups ? (m - g + tpr - 1) / tpr : 0;
-    const int warp = tid >> 5, lane = tid & 31;
-    V pv[MODE == 1 ? 16 : 4];
-    int kcol[2] = {0, 0};
-    if (MODE == 0) {  // warp w takes the columns w and w + 8, lanes l and l + 32 their terms
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            if (warp + 8 * i >= jb.nc) break;
-            kcol[i] = jobcols[jb.c0 + warp + 8 * i];
-            const int k = kcol[i] & ~CORR_OWNER;
-            if (lane < m) pv[2 * i] = __ldg(Sinv + lane * m + k);
-            if (lane + 32 < m) pv[2 * i + 1] = __ldg(Sinv + (lane + 32) * m + k);
-        }
-    }
-    if (MODE == 1) {
-#pragma unroll
-        for (int i = 0; i < (MODE == 1 ? 16 : 0); ++i)
-            if (i < cnt) pv[i] = __ldg(Sinv + (g + i * tpr) * m + kk);
-    }
-    pdl_begin();
-    pdl_trigger();
-    // u = Sigma^{1/2} xi' - y, the partial sums of y in order
-    for (int k = tid; k < m; k += 256) {
+// u = Sigma^{1/2} xi' - y, the partial sums of y in order (a CTA of 256 threads)
+template <typename T, typename V>
+__device__ __forceinline__ void lr_rhs(const LowRankArg &lr, int P, V *u) {
+    for (int k = threadIdx.x; k < lr.m; k += 256) {
         const V *part = reinterpret_cast<const V *>(lr.part) + (i64)k * P;
         const V w = __ldcg(static_cast<const V *>(lr.w) + k);
         if constexpr (sizeof(T) == 4) {
@@ -1318,6 +1275,141 @@ __device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int 
             }
             u[k] = w - t;
         }
+    }
+}
+
+// z = S^{-1} u, LRZ_COLS values per CTA: a lane per column, warp w the terms w,
+// w + 8, ..., the warps' sums added in order.  The first LRZ_PF of a thread's
+// entries of S^{-1} are loaded before the wait.
+constexpr int LRZ_COLS = 32, LRZ_PF = 16;
+template <typename T>
+__device__ __forceinline__ void lr_z_body(const LowRankArg &lr, int P, int tile, double *dyn) {
+    typedef typename std::conditional<sizeof(T) == 4, float2, double>::type V;  // FP32 chain: float-float
+    const int m = lr.m, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = tile * LRZ_COLS + lane;
+    V *u = reinterpret_cast<V *>(dyn), *pr = u + m;
+    const V *Sinv;
+    if constexpr (sizeof(T) == 4)
+        Sinv = lr.SinvT_ff;
+    else
+        Sinv = lr.SinvT;
+    Sinv += k;
+    auto entry = [&](int c) {  // zero beyond the m terms and columns
+        if constexpr (sizeof(T) == 4)
+            return c < m && k < m ? __ldg(Sinv + (i64)c * m) : make_float2(0.f, 0.f);
+        else
+            return c < m && k < m ? __ldg(Sinv + (i64)c * m) : 0.0;
+    };
+    V first[LRZ_PF];
+#pragma unroll
+    for (int i = 0; i < LRZ_PF; ++i) first[i] = entry(warp + 8 * i);
+    pdl_begin();
+    pdl_trigger();
+    lr_rhs<T>(lr, P, u);
+    __syncthreads();
+    if constexpr (sizeof(T) == 4) {
+        ff32 t[2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+        for (int i = 0; i < LRZ_PF; ++i)
+            if (warp + 8 * i < m) t[i & 1] = ff_add(t[i & 1], ff_mul(ff_of(first[i]), ff_of(u[warp + 8 * i])));
+        for (int c0 = warp + 8 * LRZ_PF; c0 < m; c0 += 64) {
+            float2 s[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[i] = entry(c0 + 8 * i);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (c0 + 8 * i < m) t[i & 1] = ff_add(t[i & 1], ff_mul(ff_of(s[i]), ff_of(u[c0 + 8 * i])));
+        }
+        const ff32 a = ff_add(t[0], t[1]);
+        pr[warp * 32 + lane] = make_float2(a.hi, a.lo);
+        __syncthreads();
+        if (warp > 0 || k >= m) return;
+        ff32 z{0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z = ff_add(z, ff_of(pr[i * 32 + lane]));
+        static_cast<float *>(lr.zv)[k] = ff_to_float(z);
+        if (lr.zpub) lr.zpub[k] = ff_to_double(z);
+    } else {
+        double t[2] = {0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < LRZ_PF; ++i)
+            if (warp + 8 * i < m) t[i & 1] = fma(first[i], u[warp + 8 * i], t[i & 1]);
+        for (int c0 = warp + 8 * LRZ_PF; c0 < m; c0 += 64) {
+            double s[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[i] = entry(c0 + 8 * i);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (c0 + 8 * i < m) t[i & 1] = fma(s[i], u[c0 + 8 * i], t[i & 1]);
+        }
+        pr[warp * 32 + lane] = t[0] + t[1];
+        __syncthreads();
+        if (warp > 0 || k >= m) return;
+        double z = 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z += pr[i * 32 + lane];
+        static_cast<double *>(lr.zv)[k] = z;
+        if (lr.zpub) lr.zpub[k] = z;
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_lr_z(LowRankArg lr, int P) {
+    extern __shared__ double dyn[];
+    lr_z_body<T>(lr, P, blockIdx.x, dyn);
+}
+
+// PF entries of a multi-entry row are loaded ahead: 8 in k_lr_correct's mode 1
+// (coarse rows have many: 2D 768 x 480 FP64 step 2.5 % faster than with 2, 3D
+// 128^3 1.3 %), 2 in the batch, whose CTAs need the registers to be resident
+// (20 chains: 2.5 % slower with 8).
+template <typename T, int MODE, int NQ, int PF = 2>
+__device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int P, const CorrRows &C, const CorrJob &jb,
+                                                const int *__restrict__ jobcols, bool first, double *dyn) {
+    typedef typename std::conditional<sizeof(T) == 4, float2, double>::type V;  // FP32 chain: float-float
+    const int m = lr.m, tid = threadIdx.x;
+    V *u = reinterpret_cast<V *>(dyn), *pr = u + m;
+    T *zs = MODE == 2 ? reinterpret_cast<T *>(dyn) : reinterpret_cast<T *>(pr + (MODE ? 256 : 64 * 8));
+    const V *Sinv;
+    if constexpr (sizeof(T) == 4)
+        Sinv = lr.SinvT_ff;
+    else
+        Sinv = lr.SinvT;
+    CorrQuad<T> q[NQ];
+    CorrMulti<T, PF> mr;
+    if (jb.multi) {
+        if (tid < jb.n) mr.load(x, C, jb.r0 + tid);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NQ; ++i)
+            if (tid + 1024 * i < jb.n) q[i].load(x, C, jb.r0, tid + 1024 * i, 256, jb.n);
+    }
+    // terms of a column in groups g = 0 .. tpr - 1: columns g, g + tpr, ... of S^{-1}
+    const int tpr = MODE == 2 ? 1 : 256 / m, groups = min(tpr, m);
+    const int g = MODE == 1 ? tid / m : 0, kk = tid - g * m, cnt = g < groups ? (m - g + tpr - 1) / tpr : 0;
+    const int warp = tid >> 5, lane = tid & 31;
+    V pv[MODE == 1 ? 16 : 4];
+    int kcol[2] = {0, 0};
+    if (MODE == 0) {  // warp w takes the columns w and w + 8, lanes l and l + 32 their terms
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (warp + 8 * i >= jb.nc) break;
+            kcol[i] = jobcols[jb.c0 + warp + 8 * i];
+            const int k = kcol[i] & ~CORR_OWNER;
+            if (lane < m) pv[2 * i] = __ldg(Sinv + lane * m + k);
+            if (lane + 32 < m) pv[2 * i + 1] = __ldg(Sinv + (lane + 32) * m + k);
+        }
+    }
+    if (MODE == 1) {
+#pragma unroll
+        for (int i = 0; i < (MODE == 1 ? 16 : 0); ++i)
+            if (i < cnt) pv[i] = __ldg(Sinv + (g + i * tpr) * m + kk);
+    }
+    pdl_begin();
+    pdl_trigger();
+    if constexpr (MODE == 2) {
+        for (int k = tid; k < m; k += 256) zs[k] = __ldcg(static_cast<const T *>(lr.zv) + k);
+    } else {
+        lr_rhs<T>(lr, P, u);
     }
     __syncthreads();
     if constexpr (MODE == 0) {
@@ -1357,78 +1449,50 @@ __device__ __forceinline__ void lr_correct_body(T *x, const LowRankArg &lr, int 
             }
         }
         __syncthreads();
-    } else {  // every CTA forms all of z
-        for (int k0 = 0; k0 < m; k0 += cols) {
-            const int k = k0 + kk;
-            if (g < groups && k < m) {
-                const V *col = Sinv + k;
-                int c = g;
-                if constexpr (sizeof(T) == 4) {
-                    ff32 t0{0.f, 0.f}, t1{0.f, 0.f};
-                    if constexpr (MODE == 1) {
+    } else if constexpr (MODE == 1) {  // every CTA forms all of z
+        if (g < groups) {
+            if constexpr (sizeof(T) == 4) {
+                ff32 t0{0.f, 0.f}, t1{0.f, 0.f};
 #pragma unroll
-                        for (int i = 0; i < 16; i += 2) {
-                            if (i < cnt) t0 = ff_add(t0, ff_mul(ff_of(pv[i]), ff_of(u[g + i * tpr])));
-                            if (i + 1 < cnt) t1 = ff_add(t1, ff_mul(ff_of(pv[i + 1]), ff_of(u[g + (i + 1) * tpr])));
-                        }
-                    } else {  // blocks of eight terms, the rest to the first sum
-                        for (; c + 7 * tpr < m; c += 8 * tpr) {
-                            float2 sv[8];
-#pragma unroll
-                            for (int r = 0; r < 8; ++r) sv[r] = __ldg(col + (i64)(c + r * tpr) * m);
-#pragma unroll
-                            for (int r = 0; r < 8; r += 2) {
-                                t0 = ff_add(t0, ff_mul(ff_of(sv[r]), ff_of(u[c + r * tpr])));
-                                t1 = ff_add(t1, ff_mul(ff_of(sv[r + 1]), ff_of(u[c + (r + 1) * tpr])));
-                            }
-                        }
-                        for (; c < m; c += tpr) t0 = ff_add(t0, ff_mul(ff_of(__ldg(col + (i64)c * m)), ff_of(u[c])));
-                    }
-                    const ff32 v = ff_add(t0, t1);
-                    pr[g * cols + kk] = make_float2(v.hi, v.lo);
-                } else {
-                    double t0 = 0.0, t1 = 0.0;
-                    if constexpr (MODE == 1) {
-#pragma unroll
-                        for (int i = 0; i < 16; i += 2) {
-                            if (i < cnt) t0 = fma(pv[i], u[g + i * tpr], t0);
-                            if (i + 1 < cnt) t1 = fma(pv[i + 1], u[g + (i + 1) * tpr], t1);
-                        }
-                    } else {
-                        for (; c + 7 * tpr < m; c += 8 * tpr) {
-                            double sv[8];
-#pragma unroll
-                            for (int r = 0; r < 8; ++r) sv[r] = __ldg(col + (i64)(c + r * tpr) * m);
-#pragma unroll
-                            for (int r = 0; r < 8; r += 2) {
-                                t0 = fma(sv[r], u[c + r * tpr], t0);
-                                t1 = fma(sv[r + 1], u[c + (r + 1) * tpr], t1);
-                            }
-                        }
-                        for (; c < m; c += tpr) t0 = fma(__ldg(col + (i64)c * m), u[c], t0);
-                    }
-                    pr[g * cols + kk] = t0 + t1;
+                for (int i = 0; i < 16; i += 2) {
+                    if (i < cnt) t0 = ff_add(t0, ff_mul(ff_of(pv[i]), ff_of(u[g + i * tpr])));
+                    if (i + 1 < cnt) t1 = ff_add(t1, ff_mul(ff_of(pv[i + 1]), ff_of(u[g + (i + 1) * tpr])));
                 }
-            }
-            __syncthreads();
-            if (tid < cols && k0 + tid < m) {
-                if constexpr (sizeof(T) == 4) {
-                    ff32 zk{0.f, 0.f};
-                    for (int h = 0; h < groups; ++h) zk = ff_add(zk, ff_of(pr[h * cols + tid]));
-                    zs[k0 + tid] = ff_to_float(zk);
-                    if (lr.zpub && first) lr.zpub[k0 + tid] = ff_to_double(zk);
-                } else {
-                    double zk = 0.0;
-                    for (int h = 0; h < groups; ++h) zk += pr[h * cols + tid];
-                    zs[k0 + tid] = zk;
-                    if (lr.zpub && first) lr.zpub[k0 + tid] = zk;
+                const ff32 v = ff_add(t0, t1);
+                pr[g * m + kk] = make_float2(v.hi, v.lo);
+            } else {
+                double t0 = 0.0, t1 = 0.0;
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    if (i < cnt) t0 = fma(pv[i], u[g + i * tpr], t0);
+                    if (i + 1 < cnt) t1 = fma(pv[i + 1], u[g + (i + 1) * tpr], t1);
                 }
+                pr[g * m + kk] = t0 + t1;
             }
-            __syncthreads();
         }
+        __syncthreads();
+        if (tid < m) {
+            if constexpr (sizeof(T) == 4) {
+                ff32 zk{0.f, 0.f};
+                for (int h = 0; h < groups; ++h) zk = ff_add(zk, ff_of(pr[h * m + tid]));
+                zs[tid] = ff_to_float(zk);
+                if (lr.zpub && first) lr.zpub[tid] = ff_to_double(zk);
+            } else {
+                double zk = 0.0;
+                for (int h = 0; h < groups; ++h) zk += pr[h * m + tid];
+                zs[tid] = zk;
+                if (lr.zpub && first) lr.zpub[tid] = zk;
+            }
+        }
+        __syncthreads();
     }
     if (jb.multi) {
         if (tid < jb.n) mr.apply(x, C, zs);
+        if (MODE == 2)  // large supports: up to 1024 rows per CTA
+            for (int r = tid + 256; r < jb.n; r += 256) {
+                mr.load(x, C, jb.r0 + r);
+                mr.apply(x, C, zs);
+            }
     } else {
 #pragma unroll
         for (int i = 0; i < NQ; ++i)
@@ -3136,6 +3200,10 @@ struct BatchCorrJob {
     int chain;
     CorrJob job;
 };
+// A CTA of one chain's solve (k_lr_z).
+struct BatchZJob {
+    int chain, tile;
+};
 // Up to 256 rows from r0 on of one chain's B_c Sigma^{-1} y.
 struct RowJob {
     int chain;
@@ -3230,7 +3298,15 @@ __global__ void __launch_bounds__(256) k_bt_partial_batch(const BatchLevelArg *_
     bt_partial_body<float, NOISE>(la[jb.chain].x, lr, batch_noise(ca[jb.chain], invocation, level), jb.j, jb.p, jb.P);
 }
 
-// the solve and x += C z, one CTA per job
+// the solve of chains whose corrections do not form z themselves (mode 2)
+__global__ void __launch_bounds__(256) k_lr_z_batch(const BatchLowRank *__restrict__ lrs, const BatchZJob *__restrict__ jobs) {
+    extern __shared__ double dyn[];
+    const BatchZJob jb = jobs[blockIdx.x];
+    const BatchLowRank &c = lrs[jb.chain];
+    lr_z_body<float>(c.lr, c.P, jb.tile, dyn);
+}
+
+// the solve (modes 0 and 1) and x += C z, one CTA per job
 template <int MODE>
 __global__ void __launch_bounds__(256, MODE == 1 ? 2 : 4)
     k_lr_correct_batch(const BatchLevelArg *__restrict__ la, const BatchLowRank *__restrict__ lrs,
