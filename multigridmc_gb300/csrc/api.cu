@@ -3442,15 +3442,20 @@ struct LrChol {
             const bool wide = m > CHOL_STAGE_M;
             const size_t sm = wide ? 0 : m * sizeof(double);
             const double *cQ = Q, *cW = W, *cg = g, *cxi = xi, *cv = v, *cp = part;
-            auto lowrank = [&](auto kernel_v, auto kernel_add, const double *from) {
+            auto product = [&](auto kernel_v, auto kernel_w, bool transpose, const double *from) {
                 plaunch(true, k_chol_qt, parts, 256, 0, stream, cQ, np, m, from, part);
-                plaunch(true, kernel_v, 1, 1024, sm, stream, cp, parts, m, cW, v, v + m);
-                plaunch(true, kernel_add, rows, 128, sm, stream, xi, cg, cQ, np, m, cv);
+                if (m <= CHOL_V_COLS) {
+                    plaunch(true, kernel_v, 1, 8 * CHOL_V_COLS, 0, stream, cp, parts, m, cW, v);
+                } else {
+                    plaunch(true, k_chol_t, (m + 31) / 32, 256, 0, stream, cp, parts, m, v + m);
+                    plaunch(true, kernel_w, transpose ? (m + 31) / 32 : (m + 7) / 8, 256, 0, stream, cW, m, cv + m, v);
+                }
             };
-            wide ? lowrank(k_chol_v<true, true>, k_chol_add<true, true>, cg)
-                 : lowrank(k_chol_v<true, false>, k_chol_add<true, false>, cg);
-            wide ? lowrank(k_chol_v<false, true>, k_chol_add<false, true>, cxi)
-                 : lowrank(k_chol_v<false, false>, k_chol_add<false, false>, cxi);
+            auto add = [&](auto kernel) { plaunch(true, kernel, rows, 128, sm, stream, xi, cg, cQ, np, m, cv); };
+            product(k_chol_v<true>, k_chol_w<true>, true, cg);
+            wide ? add(k_chol_add<true, true>) : add(k_chol_add<true, false>);
+            product(k_chol_v<false>, k_chol_w<false>, false, cxi);
+            wide ? add(k_chol_add<false, true>) : add(k_chol_add<false, false>);
         } else {
             plaunch(true, k_chol_add<true, false>, rows, 128, 0, stream, xi, (const double *)g, (const double *)nullptr, np, 0,
                     (const double *)nullptr);
@@ -3624,12 +3629,10 @@ mgmc_status mgmc_lrchol_create(const mgmc_operator_desc *op, int noise, uint64_t
     S.seed = seed;
     S.ld = (S.p + 3) / 4 * 4;
     if (S.m > 0) {
-        S.v = S.alloc<double>(2 * (size_t)S.m);  // and k_chol_v's t
+        S.v = S.alloc<double>(2 * (size_t)S.m);  // and k_chol_t's t
         S.part = S.alloc<double>((size_t)((S.padded() + CHOL_QT_ROWS - 1) / CHOL_QT_ROWS) * S.m);
         const size_t sm = S.m * sizeof(double);
         if (sm > 48 * 1024 && S.m <= CHOL_STAGE_M) {
-            raise_smem_limit(k_chol_v<true, false>, sm);
-            raise_smem_limit(k_chol_v<false, false>, sm);
             raise_smem_limit(k_chol_add<true, false>, sm);
             raise_smem_limit(k_chol_add<false, false>, sm);
         }

@@ -2963,7 +2963,8 @@ __global__ void __launch_bounds__(256) k_chol_step_t(const double *__restrict__ 
 }
 
 // Low-rank part, xi += g + Q (W^T - Id) Q^T g, then xi += Q (W - Id) Q^T xi:
-// each a product with Q^T (k_chol_qt), an m x m one (k_chol_v) and one with Q
+// each a product with Q^T (k_chol_qt), an m x m one (k_chol_v, or k_chol_t and
+// k_chol_w) and one with Q
 // (k_chol_add).  Q^T xi is formed from the updated xi although W^T Q^T g +
 // Q^T xi would save a pass over Q: W is small where the measurements are
 // accurate, and only the product with the rounded xi damps its rounding too
@@ -2998,45 +2999,98 @@ __global__ void __launch_bounds__(256) k_chol_qt(const double *__restrict__ Q, i
 }
 
 // t = the sum of the parts and v = (W - Id) t (TRANSPOSE: (W^T - Id) t) in one
-// CTA of 1024 threads, eight lanes per sum.  WIDE, more columns than shared
-// memory takes (CHOL_STAGE_M): t in tbuf, in global memory.
-constexpr int CHOL_STAGE_M = 28672;
-template <bool TRANSPOSE, bool WIDE>
-__global__ void __launch_bounds__(1024) k_chol_v(const double *part, int nparts, int m, const double *__restrict__ W,
-                                                 double *v, double *tbuf) {
-    extern __shared__ double t_sm[];
-    double *ts = WIDE ? tbuf : t_sm;
+// CTA, eight lanes per sum, for up to CHOL_V_COLS columns; more take k_chol_t
+// and k_chol_w, whose CTAs share the m^2 terms.  (A sample of 16^3 cells, both
+// products in one CTA and in two launches each: 8 columns 103 and 105 us, 32 109
+// and 109, 64 124 and 120, 128 163 and 145; of 24^3 with 1000: 2085 and 1027.)
+constexpr int CHOL_V_COLS = 32;
+template <bool TRANSPOSE>
+__global__ void __launch_bounds__(8 * CHOL_V_COLS) k_chol_v(const double *part, int nparts, int m, const double *__restrict__ W,
+                                                 double *v) {
+    __shared__ double ts[CHOL_V_COLS];
     pdl_begin();
     pdl_trigger();
-    const int l = threadIdx.x & 7, q = threadIdx.x >> 3;
+    const int l = threadIdx.x & 7, c = threadIdx.x >> 3;
     auto over8 = [](double a) {
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         return a;
     };
-    for (int c0 = 0; c0 < m; c0 += 128) {
-        const int c = c0 + q;
-        double a = 0.0;
+    double a = 0.0;
+    if (c < m) {
+#pragma unroll 4
+        for (int i = l; i < nparts; i += 8) a += part[(i64)i * m + c];
+    }
+    a = over8(a);
+    if (l == 0 && c < m) ts[c] = a;
+    __syncthreads();
+    a = 0.0;
+    if (c < m)
+        for (int k = l; k < m; k += 8)
+            a = fma((TRANSPOSE ? W[(i64)k * m + c] : W[(i64)c * m + k]) - (k == c ? 1.0 : 0.0), ts[k], a);
+    a = over8(a);
+    if (l == 0 && c < m) v[c] = a;
+}
+
+// the sum over the warps of a CTA of 256 threads, lane by lane, in warp 0
+__device__ __forceinline__ double sum_over_warps(double a) {
+    __shared__ double sh[8][32];
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    sh[w][l] = a;
+    __syncthreads();
+    a = 0.0;
+    if (w == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a += sh[i][l];
+    }
+    return a;
+}
+
+// t = the sum of the parts, 32 columns per CTA
+__global__ void __launch_bounds__(256) k_chol_t(const double *part, int nparts, int m, double *t) {
+    pdl_begin();
+    pdl_trigger();
+    const int c = blockIdx.x * 32 + (threadIdx.x & 31);
+    double a = 0.0;
+    if (c < m) {
+#pragma unroll 4
+        for (int i = threadIdx.x >> 5; i < nparts; i += 8) a += part[(i64)i * m + c];
+    }
+    a = sum_over_warps(a);
+    if (threadIdx.x < 32 && c < m) t[c] = a;
+}
+
+// v = (W - Id) t, a warp per row and 8 rows per CTA, or (TRANSPOSE) (W^T - Id) t,
+// 32 columns per CTA, its warps every eighth row
+template <bool TRANSPOSE>
+__global__ void __launch_bounds__(256) k_chol_w(const double *__restrict__ W, int m, const double *t, double *v) {
+    pdl_begin();
+    pdl_trigger();
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double a = 0.0;
+    if (TRANSPOSE) {
+        const int c = blockIdx.x * 32 + l;
         if (c < m) {
 #pragma unroll 4
-            for (int i = l; i < nparts; i += 8) a += part[(i64)i * m + c];
+            for (int k = w; k < m; k += 8) a = fma(W[(i64)k * m + c] - (k == c ? 1.0 : 0.0), t[k], a);
         }
-        a = over8(a);
-        if (l == 0 && c < m) ts[c] = a;
-    }
-    __syncthreads();
-    for (int c0 = 0; c0 < m; c0 += 128) {
-        const int c = c0 + q;
-        double a = 0.0;
-        if (c < m)
-            for (int k = l; k < m; k += 8)
-                a = fma((TRANSPOSE ? W[(i64)k * m + c] : W[(i64)c * m + k]) - (k == c ? 1.0 : 0.0), ts[k], a);
-        a = over8(a);
+        a = sum_over_warps(a);
+        if (w == 0 && c < m) v[c] = a;
+    } else {
+        const int c = blockIdx.x * 8 + w;
+        if (c < m) {
+#pragma unroll 4
+            for (int k = l; k < m; k += 32) a = fma(W[(i64)c * m + k] - (k == c ? 1.0 : 0.0), t[k], a);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         if (l == 0 && c < m) v[c] = a;
     }
 }
 
 // xi += Q v (ADD_G: + g), one thread per row, v in shared memory unless WIDE
+// (more columns than it takes)
+constexpr int CHOL_STAGE_M = 28672;
 template <bool ADD_G, bool WIDE>
 __global__ void __launch_bounds__(128) k_chol_add(double *xi, const double *g, const double *__restrict__ Q, i64 rows, int m,
                                                   const double *v) {

@@ -19,13 +19,16 @@ extern "C" int chol_wide_check(const double *part, int nparts, int m, const doub
     cudaMemcpy(dx, xi, rows * sz, cudaMemcpyHostToDevice);
     const size_t sm = m * sz;
     const unsigned blocks = (rows + 127) / 128;
+    if (m <= CHOL_V_COLS) {
+        k_chol_v<true><<<1, 8 * CHOL_V_COLS>>>(dp, nparts, m, dW, dv);
+    } else {
+        k_chol_t<<<(m + 31) / 32, 256>>>(dp, nparts, m, dv + m);
+        k_chol_w<true><<<(m + 31) / 32, 256>>>(dW, m, dv + m, dv);
+    }
     if (wide < 0 ? m > CHOL_STAGE_M : wide) {
-        k_chol_v<true, true><<<1, 1024>>>(dp, nparts, m, dW, dv, dv + m);
         k_chol_add<true, true><<<blocks, 128>>>(dx, dg, dQ, rows, m, dv);
     } else {
-        cudaFuncSetAttribute(k_chol_v<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         cudaFuncSetAttribute(k_chol_add<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_chol_v<true, false><<<1, 1024, sm>>>(dp, nparts, m, dW, dv, dv + m);
         k_chol_add<true, false><<<blocks, 128, sm>>>(dx, dg, dQ, rows, m, dv);
     }
     cudaMemcpy(xi, dx, rows * sz, cudaMemcpyDeviceToHost);

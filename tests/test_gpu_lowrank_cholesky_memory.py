@@ -73,10 +73,10 @@ def test_both_forms_draw_the_same(monkeypatch):
     assert np.linalg.norm(out[0] - out[1]) < 64 * np.finfo(float).eps * 1e4 * np.linalg.norm(out[0])
 
 
-@pytest.mark.parametrize("m", [1, 300, 6200, 28672, 28673, 30000])
+@pytest.mark.parametrize("m", [1, 32, 33, 300, 6200, 28672, 28673, 30000])
 def test_columns_beyond_shared_memory(m):
-    """m x m and Q products up to and beyond the columns that shared memory
-    takes (W = 0 where it would be gigabytes of host data)."""
+    """m x m and Q products up to and beyond the columns that one CTA and that
+    shared memory take (W = 0 where it would be gigabytes of host data)."""
     lib = C.CDLL(gpu_build("chol_wide_check"))
     rng = np.random.default_rng(m)
     part, Q = rng.standard_normal((3, m)), rng.standard_normal((130, m))
@@ -95,3 +95,25 @@ def test_columns_beyond_shared_memory(m):
         assert np.max(np.abs(v - want)) < 1e-15 * 110 * (m if W is not None else 3)
         assert np.max(np.abs(xi - (xi0 + g + Q @ want))) < 1e-15 * m * 6 * max(1.0, np.abs(want).max())
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("m", [31, 32, 33, 100, 400])
+def test_many_columns_equal_oracle(m):
+    op_o, op = posterior((9, 9, 9))
+    B = np.zeros((op.n, m))
+    B[np.random.default_rng(2).permutation(op.n)[:m], np.arange(m)] = 1.0
+    sig = 0.5 * np.ones(m)
+    op_o.set_lowrank(B, sig)
+    op = op.with_lowrank(B, sig)
+    noise = O.CLCG().draw_normal(2 * op.n)
+    orc = O.lowrank_cholesky_sampler(op_o, O.Source(noise))
+    gpu = M.LowRankCholeskySampler(op, noise=M.INJECTED)
+    gpu.inject_noise(noise)
+    f = np.random.default_rng(3).standard_normal(op.n)
+    tol = 64 * np.finfo(float).eps * np.linalg.cond(op.to_scipy().toarray())
+    xo, xg = np.zeros(op.n), np.zeros(op.n)
+    for _ in range(2):
+        orc.apply(f, xo)
+        gpu.apply(f, xg)
+        assert np.linalg.norm(xg - xo) < tol * np.linalg.norm(xo)
+    gpu.close()
