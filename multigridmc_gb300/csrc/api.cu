@@ -743,6 +743,22 @@ static void launch_resid_restrict_sym(Sampler &S, const Level &lv, const Level &
     S.launches++;
 }
 
+// One coarse point per thread (k_resid_restrict_point) instead of a row segment
+// per CTA.  Both in microseconds, segments and points, by fine cells: 3D FP32,
+// per-vertex centre, 64^3 3.8 and 5.6, 88^3 8.6 and 9.6, 96^3 9.8 and 9.3, 160^3
+// 41 and 29 (27-point fields and FP64: segments throughout); 1D 8192 1.7 and 1.9
+// (FP64 1.8, 3.7), 32768 2.5 and 2.0 (3.9, 3.8), 4 million 166 and 24; 2D FP32
+// 5-point 192^2 1.9 and 2.8, 256^2 3.2 and 2.9, 2048^2 87 and 22; 9-point 256^2
+// 3.0 and 3.0 (centre 3.2, 3.4), 384^2 4.4 and 3.2, 2048^2 76 and 31; 9-point
+// fields 384^2 4.9 and 6.0, 512^2 7.2 and 6.2, 2048^2 139 and 65; 2D FP64 768 x
+// 480 19 and 21, 1024^2 49 and 47, 2048^2 215 and 178.
+static bool restrict_by_point(const Sampler &S, const Level &lv, const Level &lc, bool fp32) {
+    const i64 n = lc.geo.n;
+    if (S.dim == 3) return fp32 && lv.npt == 7 && n > 90000;
+    if (S.dim == 2 && !fp32) return n > 250000;
+    return n > (lv.npt == 7 ? 12000 : lv.var == 2 ? 50000 : 30000);
+}
+
 template <typename T>
 static void launch_resid_restrict(Sampler &S, int lev, const void *x, const void *f, void *fc, void *xc, bool zero_stencil) {
     Level &lv = S.L[lev], &lc = S.L[lev + 1];
@@ -757,13 +773,26 @@ static void launch_resid_restrict(Sampler &S, int lev, const void *x, const void
         plain(k_resid_restrict<T, 7, 0, true>);
         return;
     }
+    auto point = [&](auto kernel) {  // k_resid_restrict_point
+        plaunch(S.pdl && lv.g.pdl, kernel, nblk(lc.geo.n, 256), 256, 0, S.stream, (const T *)x, (const T *)f, (T *)fc, (T *)xc,
+                lv.g, lc.g, s, S.dim, var_field<T>(lv));
+        S.launches++;
+    };
+    const bool by_point = restrict_by_point(S, lv, lc, sizeof(T) == 4);
     if (lv.var) {  // variable coefficients
         if (lv.npt == 7 && lv.var == 1)
-            plain(k_resid_restrict<T, 7, 1, false>);
-        else if (lv.var == 1)
-            S.dim == 2 ? plain(k_resid_restrict<T, 9, 1, false>) : plain(k_resid_restrict<T, 27, 1, false>);
-        else
-            S.dim == 2 ? plain(k_resid_restrict<T, 9, 2, false>) : plain(k_resid_restrict<T, 27, 2, false>);
+            by_point ? point(k_resid_restrict_point<T, 7, 1>) : plain(k_resid_restrict<T, 7, 1, false>);
+        else if (lv.var == 1) {
+            if (S.dim == 2)
+                by_point ? point(k_resid_restrict_point<T, 9, 1>) : plain(k_resid_restrict<T, 9, 1, false>);
+            else
+                plain(k_resid_restrict<T, 27, 1, false>);
+        } else {
+            if (S.dim == 2)
+                by_point ? point(k_resid_restrict_point<T, 9, 2>) : plain(k_resid_restrict<T, 9, 2, false>);
+            else
+                plain(k_resid_restrict<T, 27, 2, false>);
+        }
         return;
     }
     if constexpr (std::is_same<T, double>::value) {
@@ -795,9 +824,11 @@ static void launch_resid_restrict(Sampler &S, int lev, const void *x, const void
         return;
     }
     if (lv.npt == 7)
-        plain(k_resid_restrict<T, 7, 0, false>);
+        by_point ? point(k_resid_restrict_point<T, 7, 0>) : plain(k_resid_restrict<T, 7, 0, false>);
+    else if (S.dim == 2)
+        by_point ? point(k_resid_restrict_point<T, 9, 0>) : plain(k_resid_restrict<T, 9, 0, false>);
     else
-        S.dim == 2 ? plain(k_resid_restrict<T, 9, 0, false>) : plain(k_resid_restrict<T, 27, 0, false>);
+        plain(k_resid_restrict<T, 27, 0, false>);
 }
 
 // y = B^T x on the level (into the level's y unless `y` is given)

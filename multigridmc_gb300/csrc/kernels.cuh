@@ -1608,6 +1608,33 @@ __global__ void __launch_bounds__(RRS_THREADS) k_resid_restrict(const T *x, cons
     if (xc) xc[Pc] = T(0);  // the coarse sample starts from zero
 }
 
+// The same with one thread per coarse point, for levels with enough of them
+// (restrict_by_point has the line and both sides' times): every residual is
+// formed 27/8 (2D 9/4) times instead of 9/4 (3/2), but no CTA is a mere row
+// segment, of whose threads one to three tenths work in 2D and 1D.
+template <typename T, int NPT, int VAR>
+__global__ void __launch_bounds__(256) k_resid_restrict_point(const T *x, const T *f, T *fc, T *xc, Grid3 gf, Grid3 gc,
+                                                              StencilArg<T> s, int dim, VarField<T> vf) {
+    if (gf.pdl) pdl_begin_trigger();
+    const i64 t = (i64)blockIdx.x * 256 + threadIdx.x;
+    if (t >= (i64)gc.N0 * gc.N1 * gc.N2) return;
+    const int a = (int)(t % gc.N0), b = (int)(t / gc.N0 % gc.N1), c = (int)(t / ((i64)gc.N0 * gc.N1));
+    const int hy = dim > 1, hz = dim > 2;  // half widths of the footprint
+    T acc = T(0);
+    for (int z = -hz; z <= hz; ++z)
+        for (int y = -hy; y <= hy; ++y) {
+            const i64 row = gf.pad(2 * a + 1, hy ? 2 * b + 1 + y : 0, hz ? 2 * c + 1 + z : 0);
+#pragma unroll
+            for (int q = -1; q <= 1; ++q) {
+                const T wr = T((q ? 0.5 : 1.0) * (y ? 0.5 : 1.0) * (z ? 0.5 : 1.0));
+                acc += wr * (f[row + q] - stencil_row<T, NPT, false, VAR>(x, gf, s, row + q, vf));
+            }
+        }
+    const i64 Pc = gc.pad(a, hy ? b : 0, hz ? c : 0);
+    fc[Pc] = acc;
+    if (xc) xc[Pc] = T(0);  // the coarse sample starts from zero
+}
+
 // 3D-tiled variant: a CTA owns RR_TX x RR_TY x RR_TZ coarse points.  It
 // stages the x values of the tile's fine footprint plus a one-point halo in
 // shared memory (all loads issued at once), computes each fine residual of
