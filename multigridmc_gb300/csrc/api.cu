@@ -535,9 +535,12 @@ static void launch_colour_passes(Sampler &S, const Level &lv, bool forward, T *x
             if (lv.g.N1 <= pb || lv.g.N2 <= pc) continue;
             if constexpr (std::is_same<T, double>::value && !EXACT) {
                 // FP64 chains (FP32 chains' set-up sweeps keep the ordered
-                // sums): symmetric stencils by classes of rows, in 3D and,
-                // for rows of up to 128 points, in 2D (383 x 239: 6.9 us per
-                // sweep against 6.2 for the pairs, 63 x 63: 3.1 against 3.9)
+                // sums): symmetric stencils by classes of rows, in 3D (31 x 31
+                // to 255 x 255 rows of 31 to 511 points: 1.4 to 1.7 times as
+                // fast as the pairs) and, for rows of up to 128 points, in 2D
+                // (sweeps of 63^2, 127^2, 159^2, 191^2, 255^2 and 511^2 points:
+                // 5.1, 5.1, 6.2, 7.2, 7.2, 12.3 us, pairs 6.2, 6.2, 6.2, 6.2, 7.2,
+                // 13.3)
                 if (!S.fp32 && lv.sym && lv.var == 0 && lv.g.N0 <= (S.dim == 2 ? 128 : ROW_SYM_THREADS)) {
                     RowLaunch r = row_launch(lv.g, lv.g.N0, ROW_NT64, pb, pc);
                     r.trigger = row_warps(r) <= 4 * S.nsm;

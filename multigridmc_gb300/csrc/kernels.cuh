@@ -22,16 +22,18 @@
 //   k_resid_restrict_tma    f_c = R (f - A_0 x), TMA tiles (fused residual
 //                           + restriction; _tiled / plain variants otherwise)
 //   k_resid_restrict_sym    the same for FP64 chains' symmetric stencils
+//   k_resid_restrict_point  the same, one coarse point per thread
 //   k_resid_Bq          f_c -= B_c Sigma^{-1} y (k_add_Bq: elsewhere)
 //   k_prolong_add       x += alpha P x_c
 //   k_chol_gemv_*       coarse-level Cholesky sample (k_chol_subst: parity)
 //   k_step_end          observables z = b^T x, step counter
 // Host conversions: k_unpack / k_unpack2 / k_pack; adjoint helpers: k_axpy,
-// k_sinvt_q; deterministic solver (FP64 loop around the noise-free cycle):
-// k_solve_resid, k_solve_update, k_solve_gather; parameter adjoint:
-// k_pgrad_stencil, k_pgrad_combine, k_lowrank_normals, k_coarse_normals,
-// k_pgrad_coarse_phi, k_pgrad_coarse_sigma, k_accum_sum; building blocks:
-// k_apply_stencil.
+// k_adj_update, k_add_Bz; deterministic solver (FP64 loop around the noise-free
+// cycle): k_solve_resid, k_solve_update, k_solve_gather; parameter adjoint:
+// k_pgrad_stencil, k_pgrad_combine, k_coarse_normals, k_pgrad_coarse_phi,
+// k_pgrad_coarse_sigma, k_accum_sum; building blocks: k_apply_stencil; the
+// low-rank Cholesky sampler: k_chol_tri, k_chol_step, k_chol_step_t, k_chol_qt,
+// k_chol_v / k_chol_t / k_chol_w, k_chol_add.
 #pragma once
 
 #include <cstdint>
@@ -654,8 +656,11 @@ __global__ void __launch_bounds__(RBP_THREADS) k_sweep_c27_pass(T *x, const T *f
 // are drawn before the wait for it (`wait`), and with `trigger` the next
 // launch's CTAs start, and draw theirs, while this one's loads are in flight.
 // (GB300, a whole sweep with Philox noise in a graph of dependent launches,
-// one-colour passes -> row pairs: FP32 127^3 31.5 -> 17.7 us, 63^3 15.4 ->
-// 6.8, 31^3 14.1 -> 5.9; FP64 31^3 22.3 -> 13.0, 15^3 20.8 -> 12.7.)
+// one-colour passes -> row pairs: FP32 127^3 31.5 -> 14.9 us, 63^3 15.4 ->
+// 6.2, 31^3 14.1 -> 5.9; FP64 31^3 22.3 -> 13.0, 15^3 20.8 -> 12.7; FP32 rows
+// of 255, 383 and 511 points, 64 x 64 of them: 22.6 -> 11.3, 27.7 -> 16.4, 31.8
+// -> 17.3.  FP64 levels above 2^18 points that add weight by weight choose at
+// set-up: see autotune_sweeps.)
 //
 // Thread t of a row owns the points 2t and 2t + 1: the four positions 2t ..
 // 2t + 3 of the nine (three) rows around, two aligned pair loads each where
@@ -2925,7 +2930,8 @@ __global__ void __launch_bounds__(256) k_chol_tri(const double *__restrict__ A, 
 // does not depend on the launch before, so its first 1024 values are in
 // registers before the wait, and the next link starts at once to load its own:
 // what is left between two links is the read of v, 30 FP64 multiplications and
-// five additions.  (32^3 cells, p = 961: about 3.1 us per link.)
+// five additions.  (32^3 cells, p = 961: a sample of 425 us is a chain of 60
+// links beside the triangular and low-rank products, 5 to 6 us each.)
 __global__ void __launch_bounds__(256, 2) k_chol_step(const double *__restrict__ A, int p, int ld, const double *v, double *y) {
     const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), n2 = ld / 2;
     const double2 *a = reinterpret_cast<const double2 *>(A + (i64)min(row, p - 1) * ld);
