@@ -759,7 +759,7 @@ static bool restrict_by_point(const Sampler &S, const Level &lv, const Level &lc
     const i64 n = lc.geo.n;
     if (S.dim == 3) return fp32 && lv.npt == 7 && n > 90000;
     if (S.dim == 2 && !fp32) return n > 250000;
-    return n > (lv.npt == 7 ? 12000 : lv.var == 2 ? 50000 : 30000);
+    return n > (lv.var == 2 ? 50000 : lv.npt == 7 ? 12000 : 30000);
 }
 
 template <typename T>
